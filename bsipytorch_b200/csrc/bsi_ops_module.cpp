@@ -135,14 +135,15 @@ struct PrebuiltBSIKeysCUDA {
     ~PrebuiltBSIKeysCUDA() {
         if (abs_sum.defined() && b.q8.defined()) bsi_b200_unregister_key_bounds(b.q8.data_ptr<int8_t>());
     }
-    // Row sums of |k| for the exact-integer route of the tensor-core dots (bsi_b200_register_key_bounds).
+    // Row bounds for the exact-integer route of the tensor-core dots (bsi_b200_register_key_bounds) of an image that was
+    // not made by pack() (which leaves them in the same pass).
     void compute_bounds() {
         if (!b.q8.defined() || b.q8.numel() == 0 || b.variable) return;
         c10::cuda::CUDAGuard guard(b.q8.device());
-        at::Tensor k32 = b.q8.to(at::kInt);
-        at::Tensor squares = (k32 * k32).sum(1);                                             // at most 2^24 for 16384 x 32^2
-        at::Tensor per_chunk = k32.abs_().view({b.q8.size(0), -1, 256}).sum(2);              // [R, chunks]
-        abs_sum = at::stack({per_chunk.sum(1), per_chunk.amax(1), squares}, 0).to(at::kFloat).contiguous();
+        abs_sum = at::empty({3, b.q8.size(0)}, b.q8.options().dtype(at::kFloat));
+        check_status(bsi_b200_key_bounds(b.q8.data_ptr<int8_t>(), b.q8.size(1), b.q8.size(0), b.q8.size(1) / 256,
+                                         abs_sum.data_ptr<float>(), current_stream()),
+                     "bsi_b200_key_bounds");
     }
     // Called before every dot on these keys: the bound depends on the width of the queries of that dot.
     void register_bounds(int query_bits) const {
@@ -202,9 +203,9 @@ uint64_t g_last_quantize_ns = 0, g_last_pack_ns = 0, g_last_total_ns = 0;
 
 // Quantise + pack `x` ([rows, d], f32/f16/bf16, CPU or CUDA) in one kernel.
 // lean = true skips the bit slices and slice weights (only the int8 image and the scales are
-// produced): what the fused linear path needs.
+// produced): what the fused linear path needs. key_bounds (row mode): receives the [3, rows] bounds of the image.
 PackedBatch pack(const at::Tensor& input, int decimal_places, int bits, bool chunk_mode, bool profile,
-                 bool lean = false) {
+                 bool lean = false, at::Tensor* key_bounds = nullptr) {
     TORCH_CHECK(input.dim() == 2, "expects 2D tensor [rows, d]");
     const float clip_k = clip_k_from_env();
     const auto dev = work_device(input);
@@ -224,20 +225,22 @@ PackedBatch pack(const at::Tensor& input, int decimal_places, int bits, bool chu
     b.chunk_mode = chunk_mode;
     const int64_t ld8 = std::max<int64_t>(b.chunks, 1) * 256;
     auto opt = [&](at::ScalarType t) { return at::TensorOptions().dtype(t).device(dev); };
-    // Partial last words / empty inputs rely on zero-initialised words, as the reference's do.
-    const bool ragged = (b.d % 64) != 0 || b.rows == 0 || b.d == 0;
-    if (!lean)
-        b.words = ragged ? at::zeros({b.rows, bits, b.W}, opt(at::kLong)) : at::empty({b.rows, bits, b.W}, opt(at::kLong));
-    if (chunk_mode) b.scales = at::ones({b.rows, std::max<int64_t>(b.chunks, 0)}, opt(at::kFloat));
-    else b.scales = at::ones({b.rows}, opt(at::kFloat));
-    b.q8 = at::empty({b.rows, ld8}, opt(at::kChar));
-    if (chunk_mode && b.rows > 0 && b.d > 0) b.sq_norms = at::empty({b.rows, b.chunks}, opt(at::kFloat));
     if (b.rows == 0 || b.d == 0) {
-        b.q8.zero_();
-        if (lean) b.words = at::zeros({b.rows, bits, b.W}, opt(at::kLong));
+        b.words = at::zeros({b.rows, bits, b.W}, opt(at::kLong));
+        b.scales = chunk_mode ? at::ones({b.rows, b.chunks}, opt(at::kFloat)) : at::ones({b.rows}, opt(at::kFloat));
+        b.q8 = at::zeros({b.rows, ld8}, opt(at::kChar));
         b.slice_weights = slice_weight_base(bits, dev).unsqueeze(0).expand({b.rows, bits}).contiguous();
         return b;
     }
+    // the kernels write every element: partial last words and padding columns of the image as zeros
+    if (!lean) {
+        b.words = at::empty({b.rows, bits, b.W}, opt(at::kLong));
+        b.slice_weights = at::empty({b.rows, bits}, opt(at::kFloat));
+    }
+    b.scales = chunk_mode ? at::empty({b.rows, b.chunks}, opt(at::kFloat)) : at::empty({b.rows}, opt(at::kFloat));
+    b.q8 = at::empty({b.rows, ld8}, opt(at::kChar));
+    if (chunk_mode) b.sq_norms = at::empty({b.rows, b.chunks}, opt(at::kFloat));
+    if (key_bounds != nullptr) *key_bounds = at::empty({3, b.rows}, opt(at::kFloat));
 
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     auto stream = at::cuda::getCurrentCUDAStream();
@@ -246,13 +249,15 @@ PackedBatch pack(const at::Tensor& input, int decimal_places, int bits, bool chu
         cudaEventCreate(&e1);
         cudaEventRecord(e0, stream.stream());
     }
-    check_status(bsi_b200_quantize_pack_norms(x.data_ptr(), dtype_code(x), b.rows, b.d, b.d, decimal_places, bits,
-                                              chunk_mode ? 1 : 0, clip_k,
-                                              lean ? nullptr : reinterpret_cast<uint64_t*>(b.words.data_ptr<int64_t>()),
-                                              b.scales.data_ptr<float>(), nullptr, b.q8.data_ptr<int8_t>(), ld8,
-                                              b.sq_norms.defined() ? b.sq_norms.data_ptr<float>() : nullptr,
-                                              current_stream()),
-                 "bsi_b200_quantize_pack_norms");
+    auto floats = [](const at::Tensor& t) { return t.defined() ? t.data_ptr<float>() : nullptr; };
+    check_status(bsi_b200_quantize_pack_all(x.data_ptr(), dtype_code(x), b.rows, b.d, b.d, decimal_places, bits,
+                                            chunk_mode ? 1 : 0, clip_k,
+                                            lean ? nullptr : reinterpret_cast<uint64_t*>(b.words.data_ptr<int64_t>()),
+                                            b.scales.data_ptr<float>(), nullptr, b.q8.data_ptr<int8_t>(), ld8,
+                                            floats(b.sq_norms), floats(b.slice_weights),
+                                            key_bounds != nullptr ? key_bounds->data_ptr<float>() : nullptr,
+                                            current_stream()),
+                 "bsi_b200_quantize_pack_all");
     if (profile) {
         cudaEventRecord(e1, stream.stream());
         cudaEventSynchronize(e1);
@@ -260,10 +265,6 @@ PackedBatch pack(const at::Tensor& input, int decimal_places, int bits, bool chu
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
     }
-    if (lean) return b;
-    auto base = slice_weight_base(bits, dev).unsqueeze(0);
-    if (chunk_mode) b.slice_weights = base.expand({b.rows, bits}).contiguous();
-    else b.slice_weights = (base * b.scales.unsqueeze(1)).contiguous();  // bsi_vector_cuda.cpp:1042,1157
     return b;
 }
 
@@ -381,10 +382,10 @@ py::tuple build_bsi_keys_cuda(torch::Tensor K, int decimalPlaces, float compress
     auto* holder = new PrebuiltBSIKeysCUDA();
     const int kbits = bits_keys();
     holder->b = kbits == 0 ? pack_variable(K, decimalPlaces, /*for_keys=*/true)
-                           : pack(K, decimalPlaces, kbits, /*chunk_mode=*/false, /*profile=*/false);
+                           : pack(K, decimalPlaces, kbits, /*chunk_mode=*/false, /*profile=*/false, /*lean=*/false,
+                                  &holder->abs_sum);
     holder->num_keys = K.size(0);
     holder->threshold = compress_threshold;
-    holder->compute_bounds();
     uint64_t total_mem_bytes = static_cast<uint64_t>(holder->b.words.numel() * holder->b.words.element_size());
     if (holder->b.variable) {   // what the reference's per-row vectors would hold: each row its own slice count
         total_mem_bytes = 0;

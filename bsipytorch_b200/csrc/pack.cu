@@ -14,6 +14,8 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "quant_bytes.cuh"
 
@@ -180,10 +182,8 @@ __device__ __forceinline__ void store_packed(u64 packed, int bits, int lane, int
     }
 }
 
-// Quantises the lane's 8 integers with `shift`, clamps, writes slices and the int8 image.
-__device__ __forceinline__ void emit_chunk(const long long (&v)[8], int shift, int bits, int lane,
-                                           int64_t chunk, int64_t W, u64* __restrict__ words_row,
-                                           int8_t* __restrict__ q8_row) {
+// Quantises the lane's 8 integers with `shift` and clamps: one byte each.
+__device__ __forceinline__ u64 quantise8(const long long (&v)[8], int shift, int bits) {
     const long long qmax = (1ll << (bits - 1)) - 1ll;
     const long long qmin = -(1ll << (bits - 1));
     const u64 round_add = shift > 0 ? (1ull << (shift - 1)) : 0ull;
@@ -196,7 +196,13 @@ __device__ __forceinline__ void emit_chunk(const long long (&v)[8], int shift, i
         q = q > qmax ? qmax : q;
         packed |= (static_cast<u64>(q) & 0xffull) << (8 * e);
     }
-    store_packed(packed, bits, lane, chunk, W, words_row, q8_row);
+    return packed;
+}
+
+__device__ __forceinline__ void emit_chunk(const long long (&v)[8], int shift, int bits, int lane,
+                                           int64_t chunk, int64_t W, u64* __restrict__ words_row,
+                                           int8_t* __restrict__ q8_row) {
+    store_packed(quantise8(v, shift, bits), bits, lane, chunk, W, words_row, q8_row);
 }
 
 // 32-bit variant of the quantiser for the common case (10^dp <= 127 and every |x| of the warp's chunk
@@ -275,6 +281,30 @@ __global__ void __launch_bounds__(256) quantize_pack_chunk_generic_kernel(
                         vec_ok != 0, lane, clip_k, sq_norms);
 }
 
+// After the 8x8 bit transposition a lane holds one byte of each slice. Four neighbouring lanes (half a 64-bit word)
+// trade bytes in two shuffle steps so that each ends up with the four bytes of two slices, first_slice(lane) and the
+// one after it: two 4-byte stores per lane instead of seven 1-byte stores.
+__device__ __forceinline__ int first_slice(int lane) { return ((lane & 2) << 1) + ((lane & 1) << 1); }
+__device__ __forceinline__ void slice_pieces(u64 packed, int lane, uint32_t& w0, uint32_t& w1) {
+    uint32_t tl = static_cast<uint32_t>(packed), th = static_cast<uint32_t>(packed >> 32);
+    transpose8x8_halves(tl, th);
+    const bool upper = (lane & 2) != 0;     // lanes 2, 3 of the group collect slices 4..7, lanes 0, 1 slices 0..3
+    const bool odd = (lane & 1) != 0;       // odd lanes keep the second slice pair of their group
+    const uint32_t got = __shfl_xor_sync(0xffffffffu, upper ? tl : th, 2);
+    const uint32_t x = upper ? got : tl;    // the slice group's bytes of group lane (lane & 1)
+    const uint32_t y = upper ? th : got;    // ... and of group lane (lane & 1) + 2
+    const uint32_t keep = __byte_perm(x, y, odd ? 0x7632 : 0x5410);
+    const uint32_t other = __shfl_xor_sync(0xffffffffu, __byte_perm(x, y, odd ? 0x5410 : 0x7632), 1);
+    w0 = __byte_perm(keep, other, odd ? 0x2604 : 0x6240);   // bytes of group lanes 0, 1, 2, 3
+    w1 = __byte_perm(keep, other, odd ? 0x3715 : 0x7351);
+}
+
+// +-2^i with the top slice negative (bsi_cuda.cpp:217-236), times the row scale where there is one
+__device__ __forceinline__ float slice_weight(int slice, int bits, float scale) {
+    const float w = __uint_as_float(static_cast<uint32_t>(127 + slice) << 23) * scale;
+    return slice == bits - 1 ? -w : w;
+}
+
 // Fast path of one chunk: true when the chunk was quantised and stored, false when it needs the generic
 // path (some |x * 10^dp| >= 2^23, NaN or inf). Same integers as the generic path, far fewer instructions.
 //
@@ -285,34 +315,52 @@ __global__ void __launch_bounds__(256) quantize_pack_chunk_generic_kernel(
 //    again: u = fma(r1, 2^-s, 0.5 - 2^(23-s)) is exact and its 2^23-truncation carries the result in the
 //    low mantissa byte. All of this runs on the FMA pipe.
 //  * float32 inputs, 10^dp <= 127: 32-bit integer arithmetic on the float's bit pattern.
+// The shift of a group whose largest |x| has the bit pattern amax_bits; -1: the group needs the generic path.
 template <typename T>
-__device__ __forceinline__ bool fast_quantise(const float (&f)[8], uint32_t dec_mult, int bits, int& shift, u64& packed) {
-    uint32_t amax_bits = 0;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) amax_bits = max(amax_bits, __float_as_uint(f[e]) & 0x7fffffffu);
-    amax_bits = __reduce_max_sync(0xffffffffu, amax_bits);   // NaN and inf order above every finite value
+__device__ __forceinline__ int fast_group_shift(uint32_t amax_bits, uint32_t dec_mult, int bits) {
+    if constexpr (sizeof(T) == 2) {
+        const float ymax = __uint_as_float(amax_bits) * static_cast<float>(dec_mult);
+        if (!(amax_bits < 0x7f800000u && ymax < 8388608.0f)) return -1;
+        return fast_shift(ymax, bits);   // rounding is monotonic: half_away(ymax) is the largest |v|
+    } else {
+        if (!(amax_bits < (150u << 23))) return -1;
+        const int shift = (32 - __clz(static_cast<int>(decimal_round_mag32(amax_bits, dec_mult)))) - (bits - 1);
+        return shift < 0 ? 0 : shift;
+    }
+}
 
+// The lane's 8 values quantised with the group's shift.
+template <typename T>
+__device__ __forceinline__ u64 fast_pack8(const float (&f)[8], uint32_t dec_mult, int shift, int bits) {
     uint32_t u[8];
     if constexpr (sizeof(T) == 2) {
         const float fmult = static_cast<float>(dec_mult);
-        const float ymax = __uint_as_float(amax_bits) * fmult;
-        if (!(amax_bits < 0x7f800000u && ymax < 8388608.0f)) return false;
-        shift = fast_shift(ymax, bits);   // rounding is monotonic: half_away(ymax) is the largest |v|
         float inv, c;
         fast_round_consts(shift, inv, c);
 #pragma unroll
         for (int e = 0; e < 8; ++e) u[e] = fast_magnitude(f[e], fmult, inv, c);
     } else {
-        if (!(amax_bits < (150u << 23))) return false;
-        const uint32_t mx = decimal_round_mag32(amax_bits, dec_mult);
-        shift = (32 - __clz(static_cast<int>(mx))) - (bits - 1);
-        shift = shift < 0 ? 0 : shift;
         const uint32_t round_add = shift > 0 ? (1u << (shift - 1)) : 0u;
 #pragma unroll
         for (int e = 0; e < 8; ++e)
             u[e] = (decimal_round_mag32(__float_as_uint(f[e]), dec_mult) + round_add) >> shift;
     }
-    packed = sign_clamp_bytes(u, f, bits);
+    return sign_clamp_bytes(u, f, bits);
+}
+
+__device__ __forceinline__ uint32_t abs_max_bits(const float (&f)[8]) {
+    uint32_t m = 0;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) m = max(m, __float_as_uint(f[e]) & 0x7fffffffu);
+    return m;
+}
+
+template <typename T>
+__device__ __forceinline__ bool fast_quantise(const float (&f)[8], uint32_t dec_mult, int bits, int& shift, u64& packed) {
+    const uint32_t amax_bits = __reduce_max_sync(0xffffffffu, abs_max_bits(f));   // NaN and inf order above every finite value
+    shift = fast_group_shift<T>(amax_bits, dec_mult, bits);
+    if (shift < 0) return false;
+    packed = fast_pack8<T>(f, dec_mult, shift, bits);
     return true;
 }
 
@@ -340,22 +388,10 @@ __device__ __forceinline__ bool fast_chunk(const float (&f)[8], uint32_t unit, u
     }
     if constexpr (kQ8) *reinterpret_cast<u64*>(q8 + q8_off) = packed;
     if constexpr (kWords) {
-        // After the 8x8 bit transposition a lane holds one byte of each slice. Four neighbouring lanes (half a
-        // 64-bit word) trade bytes in two shuffle steps so that each ends up with the four bytes of two slices:
-        // two 4-byte stores per lane instead of seven 1-byte stores.
-        uint32_t tl = static_cast<uint32_t>(packed), th = static_cast<uint32_t>(packed >> 32);
-        transpose8x8_halves(tl, th);
-        const bool upper = (lane & 2) != 0;     // lanes 2, 3 of the group collect slices 4..7, lanes 0, 1 slices 0..3
-        const bool odd = (lane & 1) != 0;       // odd lanes keep the second slice pair of their group
-        const uint32_t got = __shfl_xor_sync(0xffffffffu, upper ? tl : th, 2);
-        const uint32_t x = upper ? got : tl;    // the slice group's bytes of group lane (lane & 1)
-        const uint32_t y = upper ? th : got;    // ... and of group lane (lane & 1) + 2
-        const uint32_t keep = __byte_perm(x, y, odd ? 0x7632 : 0x5410);
-        const uint32_t other = __shfl_xor_sync(0xffffffffu, __byte_perm(x, y, odd ? 0x5410 : 0x7632), 1);
-        const uint32_t w0 = __byte_perm(keep, other, odd ? 0x2604 : 0x6240);   // bytes of group lanes 0, 1, 2, 3
-        const uint32_t w1 = __byte_perm(keep, other, odd ? 0x3715 : 0x7351);
+        uint32_t w0, w1;
+        slice_pieces(packed, lane, w0, w1);
         if (word_ok) {
-            const int s0 = ((lane & 2) << 1) + ((lane & 1) << 1);              // first of the lane's two slices
+            const int s0 = first_slice(lane);
             uint8_t* out = reinterpret_cast<uint8_t*>(words);
             // word_off addresses the lane's own byte (word lane / 8, byte lane % 8); the 4-byte store goes to
             // the start of its half word
@@ -376,6 +412,21 @@ struct RawLane {
     __device__ __forceinline__ void load(const T* __restrict__ p) {
 #pragma unroll
         for (int i = 0; i < kVecs; ++i) v[i] = __ldg(reinterpret_cast<const uint4*>(p) + i);
+    }
+    // the first n (at most 8) elements at p one by one, zeros behind them
+    __device__ __forceinline__ void load_tail(const T* __restrict__ p, int64_t n) {
+        using Bits = typename std::conditional<sizeof(T) == 2, unsigned short, unsigned int>::type;
+        const Bits* src = reinterpret_cast<const Bits*>(p);
+        Bits b[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) b[e] = e < n ? __ldg(src + e) : static_cast<Bits>(0);
+        if constexpr (sizeof(T) == 2) {
+            v[0] = make_uint4(b[0] | (static_cast<uint32_t>(b[1]) << 16), b[2] | (static_cast<uint32_t>(b[3]) << 16),
+                              b[4] | (static_cast<uint32_t>(b[5]) << 16), b[6] | (static_cast<uint32_t>(b[7]) << 16));
+        } else {
+            v[0] = make_uint4(b[0], b[1], b[2], b[3]);
+            v[kVecs - 1] = make_uint4(b[4], b[5], b[6], b[7]);
+        }
     }
     __device__ __forceinline__ void to_floats(float (&f)[8]) const {
         if constexpr (sizeof(T) == 2) {
@@ -414,7 +465,7 @@ template <typename T, bool kDense, bool kWords, bool kQ8>
 __global__ void __launch_bounds__(256, BSI_PACK_MIN_BLOCKS) quantize_pack_chunk_fast_kernel(
     const T* __restrict__ x, FastGeom g, double dec_scale, uint32_t dec_mult, int bits,
     u64* __restrict__ words, float* __restrict__ scales, int32_t* __restrict__ shifts, int8_t* __restrict__ q8,
-    int vec_ok, float* __restrict__ sq_norms) {
+    int vec_ok, float* __restrict__ sq_norms, float* __restrict__ slice_weights) {
     __shared__ uint32_t slow_queue[8][kSlowQueue];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -451,6 +502,11 @@ __global__ void __launch_bounds__(256, BSI_PACK_MIN_BLOCKS) quantize_pack_chunk_
         const uint32_t q8_off = kDense ? p.unit * 256u + lane_col : p.row * g.ld8 + p.chunk * 256u + lane_col;
         const uint32_t word_off = kWords ? p.row * g.row_bytes + p.chunk * 32u + lane_word : 0u;
         const bool word_ok = kDense || p.chunk * 4u + (lane >> 3) < g.W;
+        if constexpr (kWords) {
+            // the slice weights of a row do not depend on its values in chunk mode
+            if (p.chunk == 0u && slice_weights != nullptr && lane < bits)
+                slice_weights[p.row * static_cast<uint32_t>(bits) + lane] = slice_weight(lane, bits, 1.0f);
+        }
         if (!fast_chunk<T, kWords, kQ8>(f, p.unit, q8_off, word_off, word_ok, lane, dec_mult, bits, g.slice_bytes,
                                         words, scales, shifts, q8, sq_norms)) {
             if (nslow < kSlowQueue && lane == 0) slow_queue[warp][nslow] = p.unit;
@@ -514,20 +570,8 @@ __device__ __noinline__ void generic_quantise(float f0, float f1, float f2, floa
     }
     mx = warp_max_u64(mx);
     const int shift = shift_for(mx, bits);
-    const long long qmax = (1ll << (bits - 1)) - 1ll;
-    const long long qmin = -(1ll << (bits - 1));
-    const u64 round_add = shift > 0 ? (1ull << (shift - 1)) : 0ull;
-    u64 packed = 0;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-        const u64 uq = (uabs(v[e]) + round_add) >> shift;
-        long long q = v[e] < 0 ? -static_cast<long long>(uq) : static_cast<long long>(uq);
-        q = q < qmin ? qmin : q;
-        q = q > qmax ? qmax : q;
-        packed |= (static_cast<u64>(q) & 0xffull) << (8 * e);
-    }
     *shift_out = shift;
-    *packed_out = packed;
+    *packed_out = quantise8(v, shift, bits);
 }
 
 // Chunk-mode pack whose int8 image and chunk scales are stored to several destinations at once (own
@@ -849,6 +893,189 @@ __global__ void __launch_bounds__(256) quantize_pack_row_kernel(
     }
 }
 
+// What a dot's exactness test needs of one 256-element chunk of keys: sum of |k| and sum of k^2 over the warp's bytes.
+__device__ __forceinline__ void chunk_sums(u64 packed, int& abs_sum, int& sq_sum) {
+    const uint32_t lo = static_cast<uint32_t>(packed), hi = static_cast<uint32_t>(packed >> 32);
+    // +-1 per byte by its sign: k * sign(k) = |k|
+    const int slo = static_cast<int>(prmt(lo, lo, 0xba98u) | 0x01010101u), shi = static_cast<int>(prmt(hi, hi, 0xba98u) | 0x01010101u);
+    const int a = __dp4a(static_cast<int>(hi), shi, __dp4a(static_cast<int>(lo), slo, 0));
+    const int q = __dp4a(static_cast<int>(hi), static_cast<int>(hi), __dp4a(static_cast<int>(lo), static_cast<int>(lo), 0));
+    abs_sum = __reduce_add_sync(0xffffffffu, a);
+    sq_sum = __reduce_add_sync(0xffffffffu, q);
+}
+
+// One chunk of a row on the 64-bit path with the row's shift; returns the lane's bytes.
+template <typename T>
+__device__ __noinline__ u64 generic_row_chunk(const T* xr, int64_t chunk, int64_t D, double dec_scale, uint32_t dec_mult,
+                                              int bits, int vec_ok, int lane, int shift) {
+    float f[8];
+    load8<T>(xr, chunk * 256 + lane * 8, D, vec_ok != 0, f);
+    long long v[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = decimal_round(f[e], dec_scale, dec_mult);
+    return quantise8(v, shift, bits);
+}
+
+// The shift of a row on the 64-bit path, found by one warp.
+template <typename T>
+__device__ __noinline__ int generic_row_shift(const T* xr, int64_t chunks, int64_t D, double dec_scale, uint32_t dec_mult,
+                                              int bits, int vec_ok, int lane) {
+    u64 mx = 0;
+    for (int64_t chunk = 0; chunk < chunks; ++chunk) {
+        float f[8];
+        load8<T>(xr, chunk * 256 + lane * 8, D, vec_ok != 0, f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const u64 a = uabs(decimal_round(f[e], dec_scale, dec_mult));
+            mx = a > mx ? a : mx;
+        }
+    }
+    return shift_for(warp_max_u64(mx), bits);
+}
+
+// Row mode (keys) with the row kept in registers: x is read once. 2^wpr_log2 warps share a row, CPW chunks each, and
+// a block of 8 warps takes 8 >> wpr_log2 rows; the row's largest |x| goes through shared memory once, and because
+// rounding is monotonic its bit pattern alone gives the shift. The bytes go to the int8 image and, traded among four
+// lanes, to the slices; the same pass leaves the slice weights and the row's bounds (sum of |k|, largest such sum
+// over a chunk, sum of k^2), which took ten library kernels over 32-bit copies of the image before.
+// Bound by HBM: 4 bytes in and 1 + bits / 8 out per element (float32). A row with NaN, inf or |x * 10^dp| beyond the
+// fast range is redone from memory on the 64-bit path, every warp finding the shift for itself.
+template <typename T, int CPW>
+__global__ void __launch_bounds__(256, CPW * RawLane<T>::kVecs <= 2 ? 4 : (CPW * RawLane<T>::kVecs <= 4 ? 3 : 2)) quantize_pack_row_fast_kernel(
+    const T* __restrict__ x, int64_t rows, int64_t D, int64_t ldx, double dec_scale, uint32_t dec_mult, int bits,
+    int chunks, int64_t W, int wpr_log2, u64* __restrict__ words, float* __restrict__ scales,
+    int32_t* __restrict__ shifts, int8_t* __restrict__ q8, int64_t ld8, int vec_ok, float* __restrict__ slice_weights,
+    float* __restrict__ bounds) {
+    __shared__ uint32_t wmax[8];
+    __shared__ int wsum[3][8];
+    const int lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
+    const int wpr = 1 << wpr_log2;
+    const int sub = warp & (wpr - 1);
+    const int64_t row = static_cast<int64_t>(blockIdx.x) * (8 >> wpr_log2) + (warp >> wpr_log2);
+    const bool row_ok = row < rows;
+    const T* xr = x + (row_ok ? row : 0) * ldx;
+
+    RawLane<T> raw[CPW];
+#pragma unroll
+    for (int i = 0; i < CPW; ++i) {
+        const int64_t col = static_cast<int64_t>(sub + i * wpr) * 256 + lane * 8;
+        const int64_t left = row_ok ? D - col : 0;
+        if (vec_ok && left >= 8) raw[i].load(xr + col);
+        else raw[i].load_tail(xr + (left > 0 ? col : 0), left);
+    }
+    uint32_t amax_bits = 0;
+#pragma unroll
+    for (int i = 0; i < CPW; ++i) {
+        float f[8];
+        raw[i].to_floats(f);
+        amax_bits = max(amax_bits, abs_max_bits(f));
+    }
+    amax_bits = __reduce_max_sync(0xffffffffu, amax_bits);
+    if (lane == 0) wmax[warp] = amax_bits;
+    __syncthreads();
+    const int group = warp & ~(wpr - 1);
+    for (int i = 0; i < wpr; ++i) amax_bits = max(amax_bits, wmax[group + i]);
+    int shift = fast_group_shift<T>(amax_bits, dec_mult, bits);
+    const bool fast = shift >= 0;
+    if (!fast) shift = generic_row_shift<T>(xr, chunks, D, dec_scale, dec_mult, bits, vec_ok, lane);
+
+    int asum = 0, amax_chunk = 0, qsum = 0;
+#pragma unroll
+    for (int i = 0; i < CPW; ++i) {
+        const int chunk = sub + i * wpr;
+        if (row_ok && chunk < chunks) {
+            u64 packed;
+            if (fast) {
+                float f[8];
+                raw[i].to_floats(f);
+                packed = fast_pack8<T>(f, dec_mult, shift, bits);
+            } else {
+                packed = generic_row_chunk<T>(xr, chunk, D, dec_scale, dec_mult, bits, vec_ok, lane, shift);
+            }
+            if (q8 != nullptr) *reinterpret_cast<u64*>(q8 + row * ld8 + chunk * 256 + lane * 8) = packed;
+            if (words != nullptr) {
+                uint32_t w0, w1;
+                slice_pieces(packed, lane, w0, w1);
+                const int64_t word = static_cast<int64_t>(chunk) * 4 + (lane >> 3);
+                if (word < W) {
+                    const int s0 = first_slice(lane);
+                    // half word (lane / 4) % 2 of the lane's word in slice s0
+                    uint32_t* dst = reinterpret_cast<uint32_t*>(words + (row * bits + s0) * W + word) + ((lane >> 2) & 1);
+                    if (s0 < bits) *dst = w0;
+                    if (s0 + 1 < bits) dst[2 * W] = w1;
+                }
+            }
+            if (bounds != nullptr) {
+                int a, q;
+                chunk_sums(packed, a, q);
+                asum += a;
+                qsum += q;
+                amax_chunk = max(amax_chunk, a);
+            }
+        }
+    }
+    const float scale = static_cast<float>(1ull << shift);
+    if (row_ok && sub == 0) {
+        if (lane == 0) {
+            if (scales != nullptr) scales[row] = scale;
+            if (shifts != nullptr) shifts[row] = shift;
+        }
+        if (slice_weights != nullptr && lane < bits) slice_weights[row * bits + lane] = slice_weight(lane, bits, scale);
+    }
+    if (bounds != nullptr) {
+        if (lane == 0) {
+            wsum[0][warp] = asum;
+            wsum[1][warp] = amax_chunk;
+            wsum[2][warp] = qsum;
+        }
+        __syncthreads();
+        if (row_ok && sub == 0 && lane == 0) {
+            for (int i = 1; i < wpr; ++i) {
+                asum += wsum[0][warp + i];
+                amax_chunk = max(amax_chunk, wsum[1][warp + i]);
+                qsum += wsum[2][warp + i];
+            }
+            bounds[row] = static_cast<float>(asum);
+            bounds[rows + row] = static_cast<float>(amax_chunk);
+            bounds[2 * rows + row] = static_cast<float>(qsum);
+        }
+    }
+}
+
+// Bounds of an int8 image that exists already (loaded key sets, rows too long for the kernel above): one warp per row.
+__global__ void __launch_bounds__(256) key_bounds_kernel(const int8_t* __restrict__ q8, int64_t rows, int64_t chunks,
+                                                         int64_t ld8, float* __restrict__ bounds) {
+    const int lane = threadIdx.x & 31;
+    const int64_t row = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+    if (row >= rows) return;
+    const u64* src = reinterpret_cast<const u64*>(q8 + row * ld8) + lane;
+    long long asum = 0, qsum = 0;
+    int amax_chunk = 0;
+#pragma unroll 4
+    for (int64_t c = 0; c < chunks; ++c) {
+        int a, q;
+        chunk_sums(__ldg(src + c * 32), a, q);
+        asum += a;
+        qsum += q;
+        amax_chunk = max(amax_chunk, a);
+    }
+    if (lane == 0) {
+        bounds[row] = static_cast<float>(asum);
+        bounds[rows + row] = static_cast<float>(amax_chunk);
+        bounds[2 * rows + row] = static_cast<float>(qsum);
+    }
+}
+
+// Slice weights behind the generic kernels; scales: one per row, or null for chunk mode.
+__global__ void __launch_bounds__(256) slice_weights_kernel(const float* __restrict__ scales, int64_t n, int bits,
+                                                            float* __restrict__ slice_weights) {
+    const int64_t i = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x;
+    if (i >= n) return;
+    const int64_t row = i / bits;
+    slice_weights[i] = slice_weight(static_cast<int>(i - row * bits), bits, scales != nullptr ? scales[row] : 1.0f);
+}
+
 __global__ void __launch_bounds__(256) recombine_i8_kernel(
     const u64* __restrict__ words, int64_t rows, int bits, int64_t W, int64_t chunks,
     int8_t* __restrict__ q8, int64_t ld8) {
@@ -934,7 +1161,7 @@ int64_t resident_blocks(K kernel) {
     }
     return cached;
 }
-struct ChunkArgs {
+struct PackArgs {
     int64_t rows, D, ldx, ld8, chunks, W;
     double dec_scale;
     uint32_t dec_mult;
@@ -947,10 +1174,12 @@ struct ChunkArgs {
     cudaStream_t stream;
     float clip_k;
     float* sq_norms;
+    float* slice_weights;
+    float* key_bounds;    // row mode only
 };
 
 template <typename T, bool kDense, bool kWords, bool kQ8>
-int launch_chunk_fast(const T* x, const ChunkArgs& a) {
+int launch_chunk_fast(const T* x, const PackArgs& a) {
     const int64_t resident = resident_blocks(quantize_pack_chunk_fast_kernel<T, kDense, kWords, kQ8>);
     if (resident <= 0) return BSI_ERR_CUDA;
     int64_t blocks = (a.rows * a.chunks + 7) / 8;
@@ -965,14 +1194,58 @@ int launch_chunk_fast(const T* x, const ChunkArgs& a) {
     g.row_bytes = static_cast<uint32_t>(a.bits * a.W * 8);
     g.slice_bytes = static_cast<uint32_t>(a.W * 8);
     quantize_pack_chunk_fast_kernel<T, kDense, kWords, kQ8><<<static_cast<unsigned>(blocks), 256, 0, a.stream>>>(
-        x, g, a.dec_scale, a.dec_mult, a.bits, a.words, a.scales, a.shifts, a.q8, a.vec_ok, a.sq_norms);
+        x, g, a.dec_scale, a.dec_mult, a.bits, a.words, a.scales, a.shifts, a.q8, a.vec_ok, a.sq_norms, a.slice_weights);
+    return BSI_OK;
+}
+
+int launch_slice_weights(const float* scales, const PackArgs& a) {
+    if (a.slice_weights == nullptr) return BSI_OK;
+    const int64_t n = a.rows * a.bits;
+    slice_weights_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, a.stream>>>(scales, n, a.bits, a.slice_weights);
+    return BSI_OK;
+}
+
+// Row mode: the register-resident kernel for rows of up to 64 chunks (8 warps x 8 chunks), 10^dp small enough for
+// the input type and no clipping; the two-pass 64-bit kernel otherwise. Rows of fewer than 8 chunks share a block:
+// as many warps per row as it has chunks (rounded up to a power of two), then chunks per warp.
+template <typename T>
+int launch_row(const T* x, const PackArgs& a) {
+    const uint32_t mult_limit = sizeof(T) == 2 ? 1000u : 127u;
+    if (a.dec_mult == 0u || a.dec_mult > mult_limit || a.clip_k > 0.0f || a.chunks > 64) {
+        quantize_pack_row_kernel<T><<<static_cast<unsigned>(a.rows), 256, 0, a.stream>>>(
+            x, a.rows, a.D, a.ldx, a.dec_scale, a.dec_mult, a.bits, a.chunks, a.W, a.words, a.scales, a.shifts, a.q8, a.ld8,
+            a.vec_ok, a.clip_k);
+        if (a.slice_weights != nullptr && a.scales == nullptr)
+            return fail(BSI_ERR_INVALID, "quantize_pack: row-mode slice weights need the scales as well");
+        if (int rc = launch_slice_weights(a.scales, a)) return rc;
+        if (a.key_bounds != nullptr) {
+            if (a.q8 == nullptr) return fail(BSI_ERR_INVALID, "quantize_pack: key bounds need the int8 image as well");
+            key_bounds_kernel<<<static_cast<unsigned>((a.rows + 7) / 8), 256, 0, a.stream>>>(a.q8, a.rows, a.chunks, a.ld8,
+                                                                                          a.key_bounds);
+        }
+        return BSI_OK;
+    }
+    int wpr_log2 = 0;
+    while (wpr_log2 < 3 && (1 << wpr_log2) < a.chunks) ++wpr_log2;
+    const int64_t per_block = 8 >> wpr_log2;
+    const unsigned grid = static_cast<unsigned>((a.rows + per_block - 1) / per_block);
+    const int cpw = static_cast<int>((a.chunks + (1 << wpr_log2) - 1) >> wpr_log2);
+#define BSI_ROW_FAST(CPW)                                                                                              \
+    quantize_pack_row_fast_kernel<T, CPW><<<grid, 256, 0, a.stream>>>(                                                 \
+        x, a.rows, a.D, a.ldx, a.dec_scale, a.dec_mult, a.bits, static_cast<int>(a.chunks), a.W, wpr_log2, a.words,    \
+        a.scales, a.shifts, a.q8, a.ld8, a.vec_ok, a.slice_weights, a.key_bounds)
+    if (cpw <= 1) BSI_ROW_FAST(1);
+    else if (cpw <= 2) BSI_ROW_FAST(2);
+    else if (cpw <= 4) BSI_ROW_FAST(4);
+    else BSI_ROW_FAST(8);
+#undef BSI_ROW_FAST
     return BSI_OK;
 }
 
 // Chunk mode: the fast kernel when its preconditions hold (10^dp small enough for the input type, scales
 // wanted, every offset below 2^31, no outlier clipping), else the generic kernel.
 template <typename T>
-int launch_chunk(const T* x, const ChunkArgs& a) {
+int launch_chunk(const T* x, const PackArgs& a) {
     int64_t widest = a.chunks * 256;
     if (a.ldx > widest) widest = a.ldx;
     if (a.q8 != nullptr && a.ld8 > widest) widest = a.ld8;
@@ -986,7 +1259,7 @@ int launch_chunk(const T* x, const ChunkArgs& a) {
         quantize_pack_chunk_generic_kernel<T><<<static_cast<unsigned>(blocks), 256, 0, a.stream>>>(
             x, a.rows, a.D, a.ldx, a.dec_scale, a.dec_mult, a.bits, a.chunks, a.W, a.words, a.scales, a.shifts, a.q8,
             a.ld8, a.vec_ok, a.clip_k, a.sq_norms);
-        return BSI_OK;
+        return launch_slice_weights(nullptr, a);
     }
     const bool dense = a.vec_ok && a.ldx == a.D && (a.D & 255) == 0 && (a.q8 == nullptr || a.ld8 == a.D);
     const bool w = a.words != nullptr, q = a.q8 != nullptr;
@@ -1022,7 +1295,18 @@ extern "C" int bsi_b200_quantize_pack_norms(const void* x, int dtype, int64_t ro
                                             int decimal_places, int bits, int chunk_mode, float clip_k,
                                             uint64_t* words, float* scales, int32_t* shifts,
                                             int8_t* q8, int64_t ld8, float* sq_norms, bsi_stream_t stream_) {
+    return bsi_b200_quantize_pack_all(x, dtype, rows, D, ldx, decimal_places, bits, chunk_mode, clip_k, words, scales,
+                                      shifts, q8, ld8, sq_norms, nullptr, nullptr, stream_);
+}
+
+extern "C" int bsi_b200_quantize_pack_all(const void* x, int dtype, int64_t rows, int64_t D, int64_t ldx,
+                                          int decimal_places, int bits, int chunk_mode, float clip_k,
+                                          uint64_t* words, float* scales, int32_t* shifts,
+                                          int8_t* q8, int64_t ld8, float* sq_norms, float* slice_weights,
+                                          float* key_bounds, bsi_stream_t stream_) {
     using namespace bsi;
+    if (key_bounds != nullptr && chunk_mode)
+        return fail(BSI_ERR_UNSUPPORTED, "quantize_pack: key bounds are per row: row mode only");
     if (sq_norms != nullptr && !chunk_mode)
         return fail(BSI_ERR_UNSUPPORTED, "quantize_pack: sums of squares are per (row, chunk): chunk mode only");
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
@@ -1049,24 +1333,18 @@ extern "C" int bsi_b200_quantize_pack_norms(const void* x, int dtype, int64_t ro
     }
     u64* w = reinterpret_cast<u64*>(words);
 
-    if (chunk_mode) {
-        ChunkArgs a{rows, D, ldx, ld8, chunks, W, dec_scale, dec_mult, bits, w, scales, shifts, q8, vec_ok, stream, clip_k,
-                    sq_norms};
-        int rc;
-        if (dtype == BSI_DTYPE_F32) rc = launch_chunk<float>(static_cast<const float*>(x), a);
-        else if (dtype == BSI_DTYPE_F16) rc = launch_chunk<__half>(static_cast<const __half*>(x), a);
-        else rc = launch_chunk<__nv_bfloat16>(static_cast<const __nv_bfloat16*>(x), a);
-        if (rc != BSI_OK) return rc;
-    } else {
-        if (rows > 0x7fffffffll) return fail(BSI_ERR_UNSUPPORTED, "quantize_pack: too many rows for one launch");
-#define BSI_LAUNCH_ROW(T)                                                                              \
-    quantize_pack_row_kernel<T><<<static_cast<unsigned>(rows), 256, 0, stream>>>(                      \
-        static_cast<const T*>(x), rows, D, ldx, dec_scale, dec_mult, bits, chunks, W, w, scales, shifts, q8, ld8, vec_ok, clip_k)
-        if (dtype == BSI_DTYPE_F32) BSI_LAUNCH_ROW(float);
-        else if (dtype == BSI_DTYPE_F16) BSI_LAUNCH_ROW(__half);
-        else BSI_LAUNCH_ROW(__nv_bfloat16);
-#undef BSI_LAUNCH_ROW
-    }
+    if (!chunk_mode && rows > 0x7fffffffll) return fail(BSI_ERR_UNSUPPORTED, "quantize_pack: too many rows for one launch");
+    const PackArgs a{rows, D, ldx, ld8, chunks, W, dec_scale, dec_mult, bits, w, scales, shifts, q8, vec_ok, stream, clip_k,
+                     sq_norms, slice_weights, key_bounds};
+    int rc;
+    if (dtype == BSI_DTYPE_F32)
+        rc = chunk_mode ? launch_chunk<float>(static_cast<const float*>(x), a) : launch_row<float>(static_cast<const float*>(x), a);
+    else if (dtype == BSI_DTYPE_F16)
+        rc = chunk_mode ? launch_chunk<__half>(static_cast<const __half*>(x), a) : launch_row<__half>(static_cast<const __half*>(x), a);
+    else
+        rc = chunk_mode ? launch_chunk<__nv_bfloat16>(static_cast<const __nv_bfloat16*>(x), a)
+                        : launch_row<__nv_bfloat16>(static_cast<const __nv_bfloat16*>(x), a);
+    if (rc != BSI_OK) return rc;
     return check_launch("quantize_pack launch");
 }
 
@@ -1270,6 +1548,21 @@ extern "C" int bsi_b200_recombine_i8(const uint64_t* words, int64_t rows, int bi
     recombine_i8_kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(
         reinterpret_cast<const u64*>(words), rows, bits, W, chunks, q8, ld8);
     return check_launch("recombine_i8 launch");
+}
+
+extern "C" int bsi_b200_key_bounds(const int8_t* q8, int64_t ld8, int64_t rows, int64_t chunks, float* bounds,
+                                   bsi_stream_t stream_) {
+    using namespace bsi;
+    if (rows < 0 || chunks <= 0) return fail(BSI_ERR_INVALID, "key_bounds: bad rows / chunks");
+    if (rows == 0) return BSI_OK;
+    if (q8 == nullptr || bounds == nullptr) return fail(BSI_ERR_INVALID, "key_bounds: null pointer");
+    if (ld8 < chunks * 256 || (ld8 & 7) != 0 || (reinterpret_cast<uintptr_t>(q8) & 7) != 0)
+        return fail(BSI_ERR_INVALID, "key_bounds: q8 needs 8-byte aligned rows of at least 256 * chunks bytes");
+    if (rows > 0x7fffffffll) return fail(BSI_ERR_UNSUPPORTED, "key_bounds: too many rows for one launch");
+    if (int rc = require_sm100()) return rc;
+    key_bounds_kernel<<<static_cast<unsigned>((rows + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream_)>>>(q8, rows, chunks,
+                                                                                                       ld8, bounds);
+    return check_launch("key_bounds launch");
 }
 
 extern "C" int bsi_b200_cast_bias(const float* out, int64_t ldo, const float* bias, int64_t Q, int64_t R,

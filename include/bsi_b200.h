@@ -101,6 +101,18 @@ int bsi_b200_quantize_pack_norms(const void* x, int dtype, int64_t rows, int64_t
                                  uint64_t* words, float* scales, int32_t* shifts,
                                  int8_t* q8, int64_t ld8, float* sq_norms, bsi_stream_t stream);
 
+/* Everything one pass over x can leave behind; the entry points above are this one with NULLs.
+ * slice_weights [rows, bits] float32: +-2^i with the top slice negative (bsi_cuda.cpp:217-236), times the row's 2^shift
+ * in row mode. key_bounds (row mode) float32 [3, rows]: what bsi_b200_register_key_bounds takes for this q8. */
+int bsi_b200_quantize_pack_all(const void* x, int dtype, int64_t rows, int64_t D, int64_t ldx,
+                               int decimal_places, int bits, int chunk_mode, float clip_k,
+                               uint64_t* words, float* scales, int32_t* shifts,
+                               int8_t* q8, int64_t ld8, float* sq_norms, float* slice_weights,
+                               float* key_bounds, bsi_stream_t stream);
+
+/* key_bounds of an int8 image that exists already. */
+int bsi_b200_key_bounds(const int8_t* q8, int64_t ld8, int64_t rows, int64_t chunks, float* bounds, bsi_stream_t stream);
+
 /* ---- variable-slice mode (the reference's default when no BSI_FIXED_BITS* variable is set) ------
  * The decimal integers v = half_away(double(float(x)) * 10^decimal_places) are sliced as they are,
  * without a shift; the number of slices follows from the largest |v| (bit_width(max|v|) + 2, at least
