@@ -639,15 +639,15 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                         amax_bits = max(amax_bits, __float_as_uint(static_cast<float>(other_t)) & 0x7fffffffu);
                         ++tiles_done;
                     }
-                    float ymax = __uint_as_float(amax_bits) * requant.mult;
-                    if (!(amax_bits < 0x7f800000u && ymax < 8388608.0f)) {
+                    float amax = __uint_as_float(amax_bits);
+                    if (!(amax_bits < 0x7f800000u && amax * requant.mult < 8388608.0f)) {
                         // NaN / inf / out of the exact range: not representable on this path; report, store zeros
                         atomicCAS(&g_device_status, 0, 48);
-                        ymax = 0.0f;
+                        amax = 0.0f;
 #pragma unroll
                         for (int j = 0; j < kCols; ++j) acc[j] = 0.0f;
                     }
-                    const int shift = fast_shift(ymax, requant.bits);
+                    const int shift = fast_shift(amax, requant.mult, requant.bits);
                     float inv, cst;
                     fast_round_consts(shift, inv, cst);
                     // stage 32 rows x 128 bytes through this warp's 4 KB (16-byte chunks XOR-swizzled by row)

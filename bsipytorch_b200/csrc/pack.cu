@@ -205,26 +205,6 @@ __device__ __forceinline__ void emit_chunk(const long long (&v)[8], int shift, i
     store_packed(quantise8(v, shift, bits), bits, lane, chunk, W, words_row, q8_row);
 }
 
-// 32-bit variant of the quantiser for the common case (10^dp <= 127 and every |x| of the warp's chunk
-// below 2^23, so that every product and magnitude fits 32 bits). Same integers as the 64-bit path.
-__device__ __forceinline__ uint32_t decimal_round_mag32(uint32_t fbits, uint32_t mult) {
-    const uint32_t exp = (fbits >> 23) & 0xffu;
-    const uint32_t man = (fbits & 0x7fffffu) | (exp ? 0x800000u : 0u);
-    const uint32_t sh = 150u - exp;  // >= 1 on this path; denormals get sh = 150
-    const uint32_t P = man * mult;   // < 2^31
-    return sh >= 32u ? 0u : ((P + (1u << (sh - 1u))) >> sh);
-}
-
-// Byte-wise tail of the fast paths: u[e] carries the unsigned quantised magnitude of element e in its
-// low byte (0 .. 2^(bits-1)), f[e] the sign; returns the 8 two's-complement bytes.
-__device__ __forceinline__ u64 sign_clamp_bytes(const uint32_t (&u)[8], const float (&f)[8], int bits) {
-    const uint32_t lo = sign_clamp4(u[0], u[1], u[2], u[3], __float_as_uint(f[0]), __float_as_uint(f[1]),
-                                    __float_as_uint(f[2]), __float_as_uint(f[3]), bits);
-    const uint32_t hi = sign_clamp4(u[4], u[5], u[6], u[7], __float_as_uint(f[4]), __float_as_uint(f[5]),
-                                    __float_as_uint(f[6]), __float_as_uint(f[7]), bits);
-    return static_cast<u64>(lo) | (static_cast<u64>(hi) << 32);
-}
-
 // One (row, chunk) unit on the generic path (any decimal_places, any magnitude, NaN/inf, any layout):
 // 64-bit integers and 64-bit offsets throughout.
 template <typename T>
@@ -305,75 +285,124 @@ __device__ __forceinline__ float slice_weight(int slice, int bits, float scale) 
     return slice == bits - 1 ? -w : w;
 }
 
-// Fast path of one chunk: true when the chunk was quantised and stored, false when it needs the generic
-// path (some |x * 10^dp| >= 2^23, NaN or inf). Same integers as the generic path, far fewer instructions.
-//
-//  * 16-bit inputs, 10^dp <= 1000: an 11-bit (8-bit for bfloat16) significand times a 10-bit constant
-//    has at most 21 bits, so y = |x| * 10^dp and y + 0.5 are exact in float32. Adding 2^23 with
-//    round-toward-zero leaves 2^23 + floor(y + 0.5) = 2^23 + |v| (floats in [2^23, 2^24) are the
-//    integers). The second rounding (|v| + 2^(s-1)) >> s = floor(|v| * 2^-s + 0.5) is the same step
-//    again: u = fma(r1, 2^-s, 0.5 - 2^(23-s)) is exact and its 2^23-truncation carries the result in the
-//    low mantissa byte. All of this runs on the FMA pipe.
-//  * float32 inputs, 10^dp <= 127: 32-bit integer arithmetic on the float's bit pattern.
-// The shift of a group whose largest |x| has the bit pattern amax_bits; -1: the group needs the generic path.
+// ---- fast path: |x * 10^dp| < 2^23 throughout the group ----------------------------------------------------------
+// A lane's 8 elements as loaded: one 16-byte vector for 16-bit types, two for float32. Kept in this form until it is
+// quantised, so that loads of later units stay in flight.
 template <typename T>
-__device__ __forceinline__ int fast_group_shift(uint32_t amax_bits, uint32_t dec_mult, int bits) {
-    if constexpr (sizeof(T) == 2) {
-        const float ymax = __uint_as_float(amax_bits) * static_cast<float>(dec_mult);
-        if (!(amax_bits < 0x7f800000u && ymax < 8388608.0f)) return -1;
-        return fast_shift(ymax, bits);   // rounding is monotonic: half_away(ymax) is the largest |v|
-    } else {
-        if (!(amax_bits < (150u << 23))) return -1;
-        const int shift = (32 - __clz(static_cast<int>(decimal_round_mag32(amax_bits, dec_mult)))) - (bits - 1);
-        return shift < 0 ? 0 : shift;
+struct RawLane {
+    static constexpr int kVecs = sizeof(T) == 2 ? 1 : 2;
+    uint4 v[kVecs];
+    __device__ __forceinline__ void load(const T* __restrict__ p) {
+#pragma unroll
+        for (int i = 0; i < kVecs; ++i) v[i] = __ldg(reinterpret_cast<const uint4*>(p) + i);
     }
-}
-
-// The lane's 8 values quantised with the group's shift.
-template <typename T>
-__device__ __forceinline__ u64 fast_pack8(const float (&f)[8], uint32_t dec_mult, int shift, int bits) {
-    uint32_t u[8];
-    if constexpr (sizeof(T) == 2) {
-        const float fmult = static_cast<float>(dec_mult);
+    // the first n (at most 8) elements at p one by one, zeros behind them
+    __device__ __forceinline__ void load_tail(const T* __restrict__ p, int64_t n) {
+        using Bits = typename std::conditional<sizeof(T) == 2, unsigned short, unsigned int>::type;
+        const Bits* src = reinterpret_cast<const Bits*>(p);
+        Bits b[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) b[e] = e < n ? __ldg(src + e) : static_cast<Bits>(0);
+        if constexpr (sizeof(T) == 2) {
+            v[0] = make_uint4(b[0] | (static_cast<uint32_t>(b[1]) << 16), b[2] | (static_cast<uint32_t>(b[3]) << 16),
+                              b[4] | (static_cast<uint32_t>(b[5]) << 16), b[6] | (static_cast<uint32_t>(b[7]) << 16));
+        } else {
+            v[0] = make_uint4(b[0], b[1], b[2], b[3]);
+            v[kVecs - 1] = make_uint4(b[4], b[5], b[6], b[7]);
+        }
+    }
+    __device__ __forceinline__ void from_floats(const float (&f)[8]) {   // values of type T held as floats
+        if constexpr (sizeof(T) == 2) {
+            T h[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) h[e] = static_cast<T>(f[e]);
+            v[0] = *reinterpret_cast<const uint4*>(h);
+        } else {
+            v[0] = make_uint4(__float_as_uint(f[0]), __float_as_uint(f[1]), __float_as_uint(f[2]), __float_as_uint(f[3]));
+            v[kVecs - 1] = make_uint4(__float_as_uint(f[4]), __float_as_uint(f[5]), __float_as_uint(f[6]), __float_as_uint(f[7]));
+        }
+    }
+    // Largest |x| of the lane as a bit pattern of T that orders like the value: NaN and inf above every finite value.
+    __device__ __forceinline__ uint32_t abs_max() const {
+        if constexpr (sizeof(T) == 2) {
+            const uint32_t m = __vmaxu2(__vmaxu2(v[0].x & 0x7fff7fffu, v[0].y & 0x7fff7fffu),
+                                        __vmaxu2(v[0].z & 0x7fff7fffu, v[0].w & 0x7fff7fffu));
+            return max(m & 0xffffu, m >> 16);
+        } else {
+            const uint4& a = v[0];
+            const uint4& b = v[kVecs - 1];
+            const uint32_t m = max(max(max(a.x & 0x7fffffffu, a.y & 0x7fffffffu), max(a.z & 0x7fffffffu, a.w & 0x7fffffffu)),
+                                   max(max(b.x & 0x7fffffffu, b.y & 0x7fffffffu), max(b.z & 0x7fffffffu, b.w & 0x7fffffffu)));
+            return m;
+        }
+    }
+    // The pattern abs_max() returns as a float.
+    static __device__ __forceinline__ float abs_value(uint32_t bits) {
+        if constexpr (std::is_same<T, float>::value) return __uint_as_float(bits);
+        else if constexpr (std::is_same<T, __half>::value) return __half2float(__ushort_as_half(static_cast<unsigned short>(bits)));
+        else return __uint_as_float(bits << 16);
+    }
+    // The 8 values quantised with the group's shift, one byte each.
+    __device__ __forceinline__ u64 quantise(float mult, int shift, int bits) const {
         float inv, c;
         fast_round_consts(shift, inv, c);
+        if constexpr (sizeof(T) == 2) {
+            uint32_t w[2];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) u[e] = fast_magnitude(f[e], fmult, inv, c);
-    } else {
-        const uint32_t round_add = shift > 0 ? (1u << (shift - 1)) : 0u;
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t p = h == 0 ? v[0].x : v[0].z, q = h == 0 ? v[0].y : v[0].w;
+                w[h] = mask_clamp4(mag(p, 0, mult, inv, c), mag(p, 1, mult, inv, c), mag(q, 0, mult, inv, c),
+                                   mag(q, 1, mult, inv, c), prmt(p, q, 0xfdb9u), bits);
+            }
+            return static_cast<u64>(w[0]) | (static_cast<u64>(w[1]) << 32);
+        } else {
+            uint32_t w[2];
 #pragma unroll
-        for (int e = 0; e < 8; ++e)
-            u[e] = (decimal_round_mag32(__float_as_uint(f[e]), dec_mult) + round_add) >> shift;
+            for (int h = 0; h < 2; ++h) {
+                const uint4& a = v[h == 0 ? 0 : kVecs - 1];
+                w[h] = sign_clamp4(fast_magnitude(__uint_as_float(a.x), mult, inv, c), fast_magnitude(__uint_as_float(a.y), mult, inv, c),
+                                   fast_magnitude(__uint_as_float(a.z), mult, inv, c), fast_magnitude(__uint_as_float(a.w), mult, inv, c),
+                                   a.x, a.y, a.z, a.w, bits);
+            }
+            return static_cast<u64>(w[0]) | (static_cast<u64>(w[1]) << 32);
+        }
     }
-    return sign_clamp_bytes(u, f, bits);
+private:
+    static __device__ __forceinline__ uint32_t mag(uint32_t pair, int half, float mult, float inv, float c) {
+        if constexpr (std::is_same<T, __half>::value) {
+            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&pair));
+            return fast_magnitude(half == 0 ? f.x : f.y, mult, inv, c);
+        } else {
+            return fast_magnitude(__uint_as_float(half == 0 ? pair << 16 : pair & 0xffff0000u), mult, inv, c);
+        }
+    }
+};
+
+// The shift of a group whose largest |x| is amax; -1: NaN, inf or |x * 10^dp| >= 2^23 somewhere, the group needs the
+// generic path.
+__device__ __forceinline__ int fast_group_shift(float amax, float mult, int bits) {
+    return amax * mult < 8388608.0f ? fast_shift(amax, mult, bits) : -1;
 }
 
-__device__ __forceinline__ uint32_t abs_max_bits(const float (&f)[8]) {
-    uint32_t m = 0;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) m = max(m, __float_as_uint(f[e]) & 0x7fffffffu);
-    return m;
-}
-
+// One chunk per warp: false when it needs the generic path. Same integers as that path, far fewer instructions.
 template <typename T>
-__device__ __forceinline__ bool fast_quantise(const float (&f)[8], uint32_t dec_mult, int bits, int& shift, u64& packed) {
-    const uint32_t amax_bits = __reduce_max_sync(0xffffffffu, abs_max_bits(f));   // NaN and inf order above every finite value
-    shift = fast_group_shift<T>(amax_bits, dec_mult, bits);
+__device__ __forceinline__ bool fast_quantise(const RawLane<T>& r, float mult, int bits, int& shift, u64& packed) {
+    shift = fast_group_shift(RawLane<T>::abs_value(__reduce_max_sync(0xffffffffu, r.abs_max())), mult, bits);
     if (shift < 0) return false;
-    packed = fast_pack8<T>(f, dec_mult, shift, bits);
+    packed = r.quantise(mult, shift, bits);
     return true;
 }
 
 // Fast path of one chunk including its stores: true when the chunk was quantised and stored.
 template <typename T, bool kWords, bool kQ8>
-__device__ __forceinline__ bool fast_chunk(const float (&f)[8], uint32_t unit, uint32_t q8_off, uint32_t word_off,
-                                           bool word_ok, int lane, uint32_t dec_mult, int bits, uint32_t slice_bytes,
+__device__ __forceinline__ bool fast_chunk(const RawLane<T>& r, uint32_t unit, uint32_t q8_off, uint32_t word_off,
+                                           bool word_ok, int lane, float mult, int bits, uint32_t slice_bytes,
                                            u64* __restrict__ words, float* __restrict__ scales,
                                            int32_t* __restrict__ shifts, int8_t* __restrict__ q8,
                                            float* __restrict__ sq_norms) {
     int shift;
     u64 packed;
-    if (!fast_quantise<T>(f, dec_mult, bits, shift, packed)) return false;
+    if (!fast_quantise<T>(r, mult, bits, shift, packed)) return false;
     if (sq_norms != nullptr) {
         // sum of squares of the chunk's de-shifted integers, (2^shift)^2 * sum a^2: an exact float (the integer
         // sum is at most 256 * 128^2 = 2^22), which a dot's exactness test turns into a Cauchy-Schwarz bound
@@ -403,44 +432,6 @@ __device__ __forceinline__ bool fast_chunk(const float (&f)[8], uint32_t unit, u
     return true;
 }
 
-// Raw 16-byte vectors holding a lane's 8 elements (one for 16-bit types, two for float32). Keeping
-// the next unit's data in this form lets its load stay in flight while the current unit is processed.
-template <typename T>
-struct RawLane {
-    static constexpr int kVecs = sizeof(T) == 2 ? 1 : 2;
-    uint4 v[kVecs];
-    __device__ __forceinline__ void load(const T* __restrict__ p) {
-#pragma unroll
-        for (int i = 0; i < kVecs; ++i) v[i] = __ldg(reinterpret_cast<const uint4*>(p) + i);
-    }
-    // the first n (at most 8) elements at p one by one, zeros behind them
-    __device__ __forceinline__ void load_tail(const T* __restrict__ p, int64_t n) {
-        using Bits = typename std::conditional<sizeof(T) == 2, unsigned short, unsigned int>::type;
-        const Bits* src = reinterpret_cast<const Bits*>(p);
-        Bits b[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) b[e] = e < n ? __ldg(src + e) : static_cast<Bits>(0);
-        if constexpr (sizeof(T) == 2) {
-            v[0] = make_uint4(b[0] | (static_cast<uint32_t>(b[1]) << 16), b[2] | (static_cast<uint32_t>(b[3]) << 16),
-                              b[4] | (static_cast<uint32_t>(b[5]) << 16), b[6] | (static_cast<uint32_t>(b[7]) << 16));
-        } else {
-            v[0] = make_uint4(b[0], b[1], b[2], b[3]);
-            v[kVecs - 1] = make_uint4(b[4], b[5], b[6], b[7]);
-        }
-    }
-    __device__ __forceinline__ void to_floats(float (&f)[8]) const {
-        if constexpr (sizeof(T) == 2) {
-            const T* h = reinterpret_cast<const T*>(&v[0]);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) f[e] = to_float(h[e]);
-        } else {
-            const float* g = reinterpret_cast<const float*>(&v[0]);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) f[e] = g[e];
-        }
-    }
-};
-
 #ifndef BSI_PACK_MIN_BLOCKS
 #define BSI_PACK_MIN_BLOCKS 4
 #endif
@@ -454,11 +445,11 @@ struct FastGeom {
 
 constexpr int kSlowQueue = 8;   // units per warp that may wait for the generic path
 
-// Persistent fast chunk kernel. The grid is sized to what is resident at once and every warp walks the
-// (row, chunk) units with stride gridDim.x * 8, loading its next unit before it processes the current one
-// (the loop is written out twice so that the two register buffers swap roles without copies). Units the
-// fast path cannot take are queued and redone on the generic path after the loop, which keeps the 64-bit
-// code out of the loop's register budget; a warp whose queue overflows redoes all of its units.
+// Persistent fast chunk kernel. The grid is sized to what is resident at once and every warp walks the (row, chunk)
+// units with stride gridDim.x * 8, kDepth units' loads in flight: at 32 warps per SM one unit of a 16-bit type is 16 KB
+// per SM, and HBM at full rate needs 40 KB and more in flight per SM. Units the fast path cannot take are queued and
+// redone on the generic path after the loop, which keeps the 64-bit code out of the loop's register budget; a warp
+// whose queue overflows redoes all of its units.
 // kDense: x and q8 are contiguous (ldx == ld8 == D), D is a multiple of 256 and x is 16-byte aligned, so
 // a unit's element offset is unit * 256 and no lane ever needs the scalar tail loads.
 template <typename T, bool kDense, bool kWords, bool kQ8>
@@ -467,72 +458,74 @@ __global__ void __launch_bounds__(256, BSI_PACK_MIN_BLOCKS) quantize_pack_chunk_
     u64* __restrict__ words, float* __restrict__ scales, int32_t* __restrict__ shifts, int8_t* __restrict__ q8,
     int vec_ok, float* __restrict__ sq_norms, float* __restrict__ slice_weights) {
     __shared__ uint32_t slow_queue[8][kSlowQueue];
+    constexpr int kDepth = sizeof(T) == 2 ? 4 : 2;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const uint32_t stride = gridDim.x * 8u;
     const uint32_t first = blockIdx.x * 8u + warp;
+    if (kWords && slice_weights != nullptr) {   // in chunk mode a row's slice weights do not depend on its values
+        const uint32_t n = (g.total / g.chunks) * static_cast<uint32_t>(bits);
+        for (uint32_t i = blockIdx.x * 256u + threadIdx.x; i < n; i += gridDim.x * 256u)
+            slice_weights[i] = slice_weight(static_cast<int>(i % static_cast<uint32_t>(bits)), bits, 1.0f);
+    }
     if (first >= g.total) return;
     constexpr bool kRows = !kDense || kWords;   // row / chunk are needed, not just the unit number
     const uint32_t stride_rows = kRows ? stride / g.chunks : 0u;
     const uint32_t stride_chunks = kRows ? stride - stride_rows * g.chunks : 0u;
+    const float mult = static_cast<float>(dec_mult);
     const bool vec = kDense || vec_ok != 0;
     const uint32_t lane_col = lane * 8u;
     const uint32_t lane_word = (lane >> 3) * 8u + (lane & 7u);   // byte within the chunk's 4 words
     int nslow = 0;
 
     struct Pos { uint32_t unit, row, chunk; };
-    auto advance = [&](Pos p) {
+    auto advance = [&](Pos& p) {
         p.unit += stride;
         if constexpr (kRows) {
             p.row += stride_rows; p.chunk += stride_chunks;
             if (p.chunk >= g.chunks) { p.chunk -= g.chunks; ++p.row; }
         }
-        return p;
     };
-    auto lane_vec = [&](const Pos& p) { return kDense || (vec && p.chunk * 256u + lane_col + 8u <= g.D); };
     auto fetch = [&](RawLane<T>& r, const Pos& p) {
-        if constexpr (kDense) r.load(x + (p.unit * 256u + lane_col));
-        else if (lane_vec(p)) r.load(x + (p.row * g.ldx + p.chunk * 256u + lane_col));
-    };
-    auto process = [&](const RawLane<T>& r, const Pos& p) {
-        float f[8];
-        if (lane_vec(p)) r.to_floats(f);
-        else load8<T>(x + static_cast<int64_t>(p.row) * g.ldx, static_cast<int64_t>(p.chunk) * 256 + lane_col,
-                      static_cast<int64_t>(g.D), false, f);
-        const uint32_t q8_off = kDense ? p.unit * 256u + lane_col : p.row * g.ld8 + p.chunk * 256u + lane_col;
-        const uint32_t word_off = kWords ? p.row * g.row_bytes + p.chunk * 32u + lane_word : 0u;
-        const bool word_ok = kDense || p.chunk * 4u + (lane >> 3) < g.W;
-        if constexpr (kWords) {
-            // the slice weights of a row do not depend on its values in chunk mode
-            if (p.chunk == 0u && slice_weights != nullptr && lane < bits)
-                slice_weights[p.row * static_cast<uint32_t>(bits) + lane] = slice_weight(lane, bits, 1.0f);
-        }
-        if (!fast_chunk<T, kWords, kQ8>(f, p.unit, q8_off, word_off, word_ok, lane, dec_mult, bits, g.slice_bytes,
-                                        words, scales, shifts, q8, sq_norms)) {
-            if (nslow < kSlowQueue && lane == 0) slow_queue[warp][nslow] = p.unit;
-            ++nslow;
+        if constexpr (kDense) {
+            r.load(x + (p.unit * 256u + lane_col));
+        } else {
+            const uint32_t col = p.chunk * 256u + lane_col;
+            const T* src = x + static_cast<int64_t>(p.row) * g.ldx;
+            if (vec && col + 8u <= g.D) r.load(src + col);
+            else r.load_tail(src + (col < g.D ? col : 0u), static_cast<int64_t>(g.D) - static_cast<int64_t>(col));
         }
     };
 
-    Pos cur;
+    Pos cur, nxt;
     cur.unit = first;
     cur.row = kRows ? first / g.chunks : 0u;
     cur.chunk = kRows ? first - cur.row * g.chunks : 0u;
-    RawLane<T> a, b;
-    fetch(a, cur);
-    for (;;) {
-        Pos nxt = advance(cur);
-        bool more = nxt.unit < g.total;
-        if (more) fetch(b, nxt);
-        process(a, cur);
-        if (!more) break;
-        cur = nxt;
-        nxt = advance(cur);
-        more = nxt.unit < g.total;
-        if (more) fetch(a, nxt);
-        process(b, cur);
-        if (!more) break;
-        cur = nxt;
+    nxt = cur;
+    RawLane<T> buf[kDepth];
+#pragma unroll
+    for (int j = 0; j < kDepth; ++j) {
+        if (nxt.unit < g.total) fetch(buf[j], nxt);
+        advance(nxt);
+    }
+    while (cur.unit < g.total) {
+#pragma unroll
+        for (int j = 0; j < kDepth; ++j) {
+            if (cur.unit < g.total) {
+                const RawLane<T> r = buf[j];
+                if (nxt.unit < g.total) fetch(buf[j], nxt);
+                const uint32_t q8_off = kDense ? cur.unit * 256u + lane_col : cur.row * g.ld8 + cur.chunk * 256u + lane_col;
+                const uint32_t word_off = kWords ? cur.row * g.row_bytes + cur.chunk * 32u + lane_word : 0u;
+                const bool word_ok = kDense || cur.chunk * 4u + (lane >> 3) < g.W;
+                if (!fast_chunk<T, kWords, kQ8>(r, cur.unit, q8_off, word_off, word_ok, lane, mult, bits, g.slice_bytes,
+                                                words, scales, shifts, q8, sq_norms)) {
+                    if (nslow < kSlowQueue && lane == 0) slow_queue[warp][nslow] = cur.unit;
+                    ++nslow;
+                }
+                advance(cur);
+                advance(nxt);
+            }
+        }
     }
     if (nslow == 0) return;
     __syncwarp();
@@ -556,10 +549,13 @@ struct MultiDst {
 };
 
 // Generic quantiser of one chunk without the stores (the multi-destination kernel's fallback).
-__device__ __noinline__ void generic_quantise(float f0, float f1, float f2, float f3, float f4, float f5, float f6,
-                                              float f7, double dec_scale, uint32_t dec_mult, int bits, int* shift_out,
+template <typename T>
+__device__ __noinline__ void generic_quantise(uint4 v0, uint4 v1, double dec_scale, uint32_t dec_mult, int bits, int* shift_out,
                                               u64* packed_out) {
-    const float f[8] = {f0, f1, f2, f3, f4, f5, f6, f7};
+    const uint4 raw[2] = {v0, v1};
+    float f[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) f[e] = to_float(reinterpret_cast<const T*>(raw)[e]);
     long long v[8];
     u64 mx = 0;
 #pragma unroll
@@ -581,7 +577,7 @@ __device__ __noinline__ void generic_quantise(float f0, float f1, float f2, floa
 template <typename T>
 __global__ void __launch_bounds__(256, BSI_PACK_MIN_BLOCKS) quantize_pack_multi_kernel(
     const T* __restrict__ x, uint32_t total, uint32_t chunks, uint32_t ldx, uint32_t ld8, uint32_t scale_ld,
-    double dec_scale, uint32_t dec_mult, uint32_t fast_limit, int bits, const MultiDst dst) {
+    double dec_scale, uint32_t dec_mult, int bits, const MultiDst dst) {
     const int lane = threadIdx.x & 31;
     const uint32_t stride = gridDim.x * 8u;
     const uint32_t first = blockIdx.x * 8u + (threadIdx.x >> 5);
@@ -589,7 +585,7 @@ __global__ void __launch_bounds__(256, BSI_PACK_MIN_BLOCKS) quantize_pack_multi_
     const uint32_t stride_rows = stride / chunks;
     const uint32_t stride_chunks = stride - stride_rows * chunks;
     const uint32_t lane_col = lane * 8u;
-    const bool try_fast = dec_mult != 0u && dec_mult <= fast_limit;
+    const bool try_fast = dec_mult != 0u;
 
     struct Pos { uint32_t unit, row, chunk; };
     auto advance = [&](Pos p) {
@@ -599,12 +595,10 @@ __global__ void __launch_bounds__(256, BSI_PACK_MIN_BLOCKS) quantize_pack_multi_
     };
     auto fetch = [&](RawLane<T>& r, const Pos& p) { r.load(x + (p.row * ldx + p.chunk * 256u + lane_col)); };
     auto process = [&](const RawLane<T>& r, const Pos& p) {
-        float f[8];
-        r.to_floats(f);
         int shift;
         u64 packed;
-        if (!(try_fast && fast_quantise<T>(f, dec_mult, bits, shift, packed)))
-            generic_quantise(f[0], f[1], f[2], f[3], f[4], f[5], f[6], f[7], dec_scale, dec_mult, bits, &shift, &packed);
+        if (!(try_fast && fast_quantise<T>(r, static_cast<float>(dec_mult), bits, shift, packed)))
+            generic_quantise<T>(r.v[0], r.v[RawLane<T>::kVecs - 1], dec_scale, dec_mult, bits, &shift, &packed);
         const uint32_t q8_off = p.row * ld8 + p.chunk * 256u + lane_col;
         const uint32_t sc_off = p.row * scale_ld + p.chunk;
         const float scale = __uint_as_float(static_cast<uint32_t>(127 + shift) << 23);   // 2^shift, shift <= 62
@@ -648,11 +642,11 @@ template <typename T, int CPW>
 __global__ void __launch_bounds__(256) add_layernorm_pack_kernel(
     const T* __restrict__ x, const T* __restrict__ delta, const T* __restrict__ gamma, const T* __restrict__ beta,
     float eps, int rows, int H, int chunks, T* __restrict__ x_out, double dec_scale, uint32_t dec_mult,
-    uint32_t fast_limit, int bits, int64_t ld8, int64_t scale_ld, const MultiDst dst) {
+    int bits, int64_t ld8, int64_t scale_ld, const MultiDst dst) {
     __shared__ float red[2][8];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    const bool try_fast = dec_mult != 0u && dec_mult <= fast_limit;
+    const bool try_fast = dec_mult != 0u;
     const float inv_h = 1.0f / static_cast<float>(H);
     for (int row = blockIdx.x; row < rows; row += gridDim.x) {
         const int64_t base = static_cast<int64_t>(row) * H;
@@ -727,11 +721,12 @@ __global__ void __launch_bounds__(256) add_layernorm_pack_kernel(
 #pragma unroll
                 for (int e = 0; e < 8; ++e)
                     f[e] = to_float(static_cast<T>(fmaf((v[i][e] - mean) * rstd, to_float(gv[e]), to_float(bv[e]))));
+                RawLane<T> r;
+                r.from_floats(f);
                 int shift;
                 u64 packed;
-                if (!(try_fast && fast_quantise<T>(f, dec_mult, bits, shift, packed)))
-                    generic_quantise(f[0], f[1], f[2], f[3], f[4], f[5], f[6], f[7], dec_scale, dec_mult, bits, &shift,
-                                     &packed);
+                if (!(try_fast && fast_quantise<T>(r, static_cast<float>(dec_mult), bits, shift, packed)))
+                    generic_quantise<T>(r.v[0], r.v[RawLane<T>::kVecs - 1], dec_scale, dec_mult, bits, &shift, &packed);
                 const int64_t q8_off = static_cast<int64_t>(row) * ld8 + col;
                 const int64_t sc_off = static_cast<int64_t>(row) * scale_ld + c;
                 const float scale = __uint_as_float(static_cast<uint32_t>(127 + shift) << 23);
@@ -966,17 +961,14 @@ __global__ void __launch_bounds__(256, CPW * RawLane<T>::kVecs <= 2 ? 4 : (CPW *
     }
     uint32_t amax_bits = 0;
 #pragma unroll
-    for (int i = 0; i < CPW; ++i) {
-        float f[8];
-        raw[i].to_floats(f);
-        amax_bits = max(amax_bits, abs_max_bits(f));
-    }
+    for (int i = 0; i < CPW; ++i) amax_bits = max(amax_bits, raw[i].abs_max());
     amax_bits = __reduce_max_sync(0xffffffffu, amax_bits);
     if (lane == 0) wmax[warp] = amax_bits;
     __syncthreads();
     const int group = warp & ~(wpr - 1);
     for (int i = 0; i < wpr; ++i) amax_bits = max(amax_bits, wmax[group + i]);
-    int shift = fast_group_shift<T>(amax_bits, dec_mult, bits);
+    const float mult = static_cast<float>(dec_mult);
+    int shift = fast_group_shift(RawLane<T>::abs_value(amax_bits), mult, bits);
     const bool fast = shift >= 0;
     if (!fast) shift = generic_row_shift<T>(xr, chunks, D, dec_scale, dec_mult, bits, vec_ok, lane);
 
@@ -987,9 +979,7 @@ __global__ void __launch_bounds__(256, CPW * RawLane<T>::kVecs <= 2 ? 4 : (CPW *
         if (row_ok && chunk < chunks) {
             u64 packed;
             if (fast) {
-                float f[8];
-                raw[i].to_floats(f);
-                packed = fast_pack8<T>(f, dec_mult, shift, bits);
+                packed = raw[i].quantise(mult, shift, bits);
             } else {
                 packed = generic_row_chunk<T>(xr, chunk, D, dec_scale, dec_mult, bits, vec_ok, lane, shift);
             }
@@ -1205,13 +1195,12 @@ int launch_slice_weights(const float* scales, const PackArgs& a) {
     return BSI_OK;
 }
 
-// Row mode: the register-resident kernel for rows of up to 64 chunks (8 warps x 8 chunks), 10^dp small enough for
-// the input type and no clipping; the two-pass 64-bit kernel otherwise. Rows of fewer than 8 chunks share a block:
+// Row mode: the register-resident kernel for rows of up to 64 chunks (8 warps x 8 chunks), decimal_places in [0, 8]
+// and no clipping; the two-pass 64-bit kernel otherwise. Rows of fewer than 8 chunks share a block:
 // as many warps per row as it has chunks (rounded up to a power of two), then chunks per warp.
 template <typename T>
 int launch_row(const T* x, const PackArgs& a) {
-    const uint32_t mult_limit = sizeof(T) == 2 ? 1000u : 127u;
-    if (a.dec_mult == 0u || a.dec_mult > mult_limit || a.clip_k > 0.0f || a.chunks > 64) {
+    if (a.dec_mult == 0u || a.clip_k > 0.0f || a.chunks > 64) {
         quantize_pack_row_kernel<T><<<static_cast<unsigned>(a.rows), 256, 0, a.stream>>>(
             x, a.rows, a.D, a.ldx, a.dec_scale, a.dec_mult, a.bits, a.chunks, a.W, a.words, a.scales, a.shifts, a.q8, a.ld8,
             a.vec_ok, a.clip_k);
@@ -1242,15 +1231,14 @@ int launch_row(const T* x, const PackArgs& a) {
     return BSI_OK;
 }
 
-// Chunk mode: the fast kernel when its preconditions hold (10^dp small enough for the input type, scales
+// Chunk mode: the fast kernel when its preconditions hold (decimal_places in [0, 8], scales
 // wanted, every offset below 2^31, no outlier clipping), else the generic kernel.
 template <typename T>
 int launch_chunk(const T* x, const PackArgs& a) {
     int64_t widest = a.chunks * 256;
     if (a.ldx > widest) widest = a.ldx;
     if (a.q8 != nullptr && a.ld8 > widest) widest = a.ld8;
-    const uint32_t mult_limit = sizeof(T) == 2 ? 1000u : 127u;
-    const bool fast = a.dec_mult != 0u && a.dec_mult <= mult_limit && a.scales != nullptr && !(a.clip_k > 0.0f) &&
+    const bool fast = a.dec_mult != 0u && a.scales != nullptr && !(a.clip_k > 0.0f) &&
                       a.rows * widest < (1ll << 31) && (a.words != nullptr || a.q8 != nullptr);
     if (!fast) {
         int64_t blocks = (a.rows * a.chunks + 7) / 8;
@@ -1391,7 +1379,7 @@ extern "C" int bsi_b200_quantize_pack_multi(const void* x, int dtype, int64_t ro
         dec_mult = 1;
         for (int i = 0; i < decimal_places; ++i) dec_mult *= 10u;
     }
-#define BSI_LAUNCH_MULTI(T, LIMIT)                                                                          \
+#define BSI_LAUNCH_MULTI(T)                                                                                 \
     do {                                                                                                    \
         const int64_t resident = resident_blocks(quantize_pack_multi_kernel<T>);                            \
         if (resident <= 0) return BSI_ERR_CUDA;                                                             \
@@ -1400,11 +1388,11 @@ extern "C" int bsi_b200_quantize_pack_multi(const void* x, int dtype, int64_t ro
         quantize_pack_multi_kernel<T><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(                   \
             static_cast<const T*>(x), static_cast<uint32_t>(rows * chunks), static_cast<uint32_t>(chunks),  \
             static_cast<uint32_t>(ldx), static_cast<uint32_t>(ld8), static_cast<uint32_t>(scale_ld), dec_scale, \
-            dec_mult, LIMIT, bits, dst);                                                                    \
+            dec_mult, bits, dst);                                                                    \
     } while (0)
-    if (dtype == BSI_DTYPE_F32) BSI_LAUNCH_MULTI(float, 127u);
-    else if (dtype == BSI_DTYPE_F16) BSI_LAUNCH_MULTI(__half, 1000u);
-    else BSI_LAUNCH_MULTI(__nv_bfloat16, 1000u);
+    if (dtype == BSI_DTYPE_F32) BSI_LAUNCH_MULTI(float);
+    else if (dtype == BSI_DTYPE_F16) BSI_LAUNCH_MULTI(__half);
+    else BSI_LAUNCH_MULTI(__nv_bfloat16);
 #undef BSI_LAUNCH_MULTI
     return check_launch("quantize_pack_multi launch");
 }
@@ -1457,7 +1445,7 @@ extern "C" int bsi_b200_add_layernorm_pack(const void* x, const void* delta, con
     add_layernorm_pack_kernel<T, CPW_><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(                       \
         static_cast<const T*>(x), static_cast<const T*>(delta), static_cast<const T*>(gamma),                    \
         static_cast<const T*>(beta), eps, static_cast<int>(rows), static_cast<int>(H), static_cast<int>(chunks), \
-        static_cast<T*>(x_out), dec_scale, dec_mult, 1000u, bits, ld8, scale_ld, dst)
+        static_cast<T*>(x_out), dec_scale, dec_mult, bits, ld8, scale_ld, dst)
 #define BSI_LAUNCH_ALP_T(T)                       \
     do {                                          \
         if (cpw <= 1) BSI_LAUNCH_ALP(T, 1);       \

@@ -1,5 +1,5 @@
-// Device helpers shared by the pack kernels and the re-quantising linear epilogue: the exact
-// float32 form of the reference's two roundings and the byte-wise sign / clamp.
+// Device helpers shared by the pack kernels and the re-quantising linear epilogue: the exact float32 form of the
+// reference's two roundings and the byte-wise sign / clamp.
 #pragma once
 
 #include <stdint.h>
@@ -14,14 +14,12 @@ __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
     return d;
 }
 
-// u0..u3 carry the unsigned quantised magnitudes of four elements in their low bytes (0 .. 2^(bits-1)),
-// s0..s3 the sign bits (bit 31, e.g. the float bit patterns). Clamps positives to 2^(bits-1)-1, negates
-// the negatives and returns the four two's-complement bytes.
-__device__ __forceinline__ uint32_t sign_clamp4(uint32_t u0, uint32_t u1, uint32_t u2, uint32_t u3, uint32_t s0,
-                                                uint32_t s1, uint32_t s2, uint32_t s3, int bits) {
+// u0..u3 carry the unsigned quantised magnitudes of four elements in their low bytes (0 .. 2^(bits-1)), m is 0xff in
+// the bytes of the negative ones. Clamps positives to 2^(bits-1)-1, negates the negatives and returns the four
+// two's-complement bytes.
+__device__ __forceinline__ uint32_t mask_clamp4(uint32_t u0, uint32_t u1, uint32_t u2, uint32_t u3, uint32_t m, int bits) {
     const uint32_t top = 0x01010101u << (bits - 1);
     uint32_t w = __byte_perm(__byte_perm(u0, u1, 0x0040), __byte_perm(u2, u3, 0x0040), 0x5410);   // the low bytes
-    const uint32_t m = prmt(prmt(s0, s1, 0x00fbu), prmt(s2, s3, 0x00fbu), 0x5410u);               // 0xff per negative
     // positive 2^(bits-1) -> 2^(bits-1) - 1 (the byte is exactly `top` there, so the borrow stays inside it)
     const uint32_t over = w & ~m & top;
     w -= over >> (bits - 1);
@@ -31,26 +29,37 @@ __device__ __forceinline__ uint32_t sign_clamp4(uint32_t u0, uint32_t u1, uint32
     return t ^ (x & 0x80808080u);
 }
 
-// Shift of a chunk whose largest |x * 10^dp| is ymax (exact in float32, below 2^23): the reference's
-// bits(max|v|) - (b - 1), clamped at 0, with max|v| = half_away(ymax).
-__device__ __forceinline__ int fast_shift(float ymax, int bits) {
-    const uint32_t mx = __float2uint_rz(ymax + 0.5f);
+// The same with the signs in bit 31 of s0..s3 (e.g. the float bit patterns).
+__device__ __forceinline__ uint32_t sign_clamp4(uint32_t u0, uint32_t u1, uint32_t u2, uint32_t u3, uint32_t s0,
+                                                uint32_t s1, uint32_t s2, uint32_t s3, int bits) {
+    return mask_clamp4(u0, u1, u2, u3, prmt(prmt(s0, s1, 0x00fbu), prmt(s2, s3, 0x00fbu), 0x5410u), bits);
+}
+
+// The reference's two roundings, |v| = floor(|x| * 10^dp + 0.5) and (|v| + [shift > 0] * 2^(shift-1)) >> shift, as two
+// FMAs with round toward zero. An FMA rounds the exact product and sum once, so no operand width matters:
+//   r1 = fma_rz(|x|, mult, 2^22 + 0.5)   floats in [2^22, 2^23) are the multiples of 1/2 and those in [2^23, 2^24) the
+//                                        integers, so the truncation leaves 2^22 + |v| + h/2 with h in {0, 1}
+//   u  = fma_rz(r1, 2^-shift, c)         c = 2^23 + [shift > 0] / 2 - 2^(22-shift), exact in float32 for shift <= 23:
+//                                        2^23 + the wanted integer (h/2 never reaches the next one), truncated
+// Valid while |x| * mult < 2^23; mult = 10^dp is exact in float32 up to 10^10.
+__device__ __forceinline__ float fast_round1(float abs_x, float mult) { return __fmaf_rz(abs_x, mult, 4194304.5f); }
+
+// Shift of a group whose largest |x| is amax (amax * mult < 2^23): bits(max|v|) - (b - 1), clamped at 0.
+__device__ __forceinline__ int fast_shift(float amax, float mult, int bits) {
+    const uint32_t mx = __float2uint_rz(fast_round1(amax, mult) - 4194304.0f);   // the difference is exact
     const int shift = (32 - __clz(static_cast<int>(mx))) - (bits - 1);
     return shift < 0 ? 0 : shift;
 }
 
-// Constants of the second rounding for a given shift: u = fma(r1, inv, c) with r1 = 2^23 + |v|.
+// Constants of the second rounding for a given shift.
 __device__ __forceinline__ void fast_round_consts(int shift, float& inv, float& c) {
     inv = __uint_as_float(static_cast<uint32_t>(127 - shift) << 23);   // 2^-shift
-    c = (shift > 0 ? 0.5f : 0.0f) - 8388608.0f * inv;
+    c = (8388608.0f - 4194304.0f * inv) + (shift > 0 ? 0.5f : 0.0f);   // both steps exact
 }
 
-// Quantised magnitude of x (low mantissa byte of the result) for 16-bit-precision x with |x * mult| < 2^23:
-// |v| = floor(|x| * mult + 0.5) and then floor(|v| * 2^-shift + 0.5 * [shift > 0]), each as an exact
-// float32 sum whose round-toward-zero addition of 2^23 leaves the integer in the mantissa.
+// Quantised magnitude of x in the low mantissa byte of the result.
 __device__ __forceinline__ uint32_t fast_magnitude(float x, float mult, float inv, float c) {
-    const float r1 = __fadd_rz(fmaf(fabsf(x), mult, 0.5f), 8388608.0f);
-    return __float_as_uint(__fadd_rz(fmaf(r1, inv, c), 8388608.0f));
+    return __float_as_uint(__fmaf_rz(fast_round1(fabsf(x), mult), inv, c));
 }
 
 }  // namespace bsi
