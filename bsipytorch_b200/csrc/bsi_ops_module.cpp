@@ -13,8 +13,11 @@
 #include <pybind11/stl.h>
 
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <cuda_runtime_api.h>
+#include <unistd.h>
 
 #include <cmath>
 #include <cstdlib>
@@ -33,52 +36,66 @@ namespace py = pybind11;
 namespace {
 
 // ---- environment (bsi_vector_cuda.cpp:254-358, bsi_cuda.cpp:108-143) ----------------------------
-int env_int(const char* name, int fallback) {
-    const char* s = std::getenv(name);
-    return s ? std::atoi(s) : fallback;
-}
-
-int fixed_bits(const char* specific, int fallback) {
-    int v = fallback;
-    if (const char* s = std::getenv(specific)) v = std::atoi(s);
-    else if (const char* g = std::getenv("BSI_FIXED_BITS")) v = std::atoi(g);
-    TORCH_CHECK(v == 0 || (v >= 2 && v <= 8), specific, " must be 0 (variable-slice mode) or in [2, 8], got ", v);
-    return v;
-}
-int bits_queries() { return fixed_bits("BSI_FIXED_BITS_QUERIES", 7); }
-int bits_keys() { return fixed_bits("BSI_FIXED_BITS_KEYS", 6); }
-bool chunk_scale_enabled() { return env_int("BSI_FIXED_CHUNK_SCALE", 1) != 0; }
-bool profile_enabled() { return env_int("BSI_PROFILE", 0) != 0; }
-// BSI_FIXED_CLIP_K (bsi_vector_cuda.cpp:295-307): > 0 caps the magnitude that selects a group's shift at
-// clip_k * mean |v|. The reference reads it once per process; here it is read per call like the other switches.
-float clip_k_from_env() {
-    const char* s = std::getenv("BSI_FIXED_CLIP_K");
-    const float v = s ? std::strtof(s, nullptr) : 0.0f;
-    return v > 0.0f ? v : 0.0f;
-}
-// The builders honour the variable; the fused additions below (single-call layer, packers that write into
-// exchange buffers, re-quantising epilogue) have no clipping variant and refuse to run with it.
-void check_clip(const char* what) {
-    TORCH_CHECK(!(clip_k_from_env() > 0.0f), what, " does not implement BSI_FIXED_CLIP_K > 0 (outlier clipping); "
-                "use the build_bsi_* entry points");
-}
-int engine_from_env() {
-    const char* s = std::getenv("BSI_B200_ENGINE");
-    if (!s || !*s || std::string(s) == "auto") {
-        // BSI_TC_DOT=0 is the reference's switch to its non-tensor-core kernel, re-read on every launch
-        // (bsi_cuda_kernels_dot.cuh:2642); here it selects the CUDA-core (dp4a) engine, which evaluates the
-        // same recurrence, so verify_tc_dot_correctness.py compares two engines as it does in the reference.
-        const char* tc = std::getenv("BSI_TC_DOT");
-        if (tc && *tc && std::atoi(tc) == 0) return BSI_ENGINE_SIMT;
-        return BSI_ENGINE_AUTO;
+// The switches of one call, read in one walk over the environment (a getenv() per switch cost a microsecond per layer
+// call). Every entry point takes its own copy, so a change between two calls is seen, as in the reference.
+struct Env {
+    const char *engine = nullptr, *tc_dot = nullptr, *bits_q = nullptr, *bits_k = nullptr, *bits_any = nullptr,
+               *chunk = nullptr, *profile_s = nullptr, *clip = nullptr, *fp32 = nullptr;
+    Env() {
+        for (char** e = environ; e != nullptr && *e != nullptr; ++e) {
+            const char* v = *e;
+            if (v[0] != 'B' || v[1] != 'S' || v[2] != 'I' || v[3] != '_') continue;
+            take(v, "BSI_B200_ENGINE=", engine) || take(v, "BSI_TC_DOT=", tc_dot) || take(v, "BSI_FIXED_BITS_QUERIES=", bits_q) ||
+                take(v, "BSI_FIXED_BITS_KEYS=", bits_k) || take(v, "BSI_FIXED_BITS=", bits_any) ||
+                take(v, "BSI_FIXED_CHUNK_SCALE=", chunk) || take(v, "BSI_PROFILE=", profile_s) ||
+                take(v, "BSI_FIXED_CLIP_K=", clip) || take(v, "BSI_QUERY_FP32=", fp32);
+        }
     }
-    const std::string v(s);
-    if (v == "tcgen05") return BSI_ENGINE_TCGEN05;
-    if (v == "simt") return BSI_ENGINE_SIMT;
-    if (v == "bmma") return BSI_ENGINE_BMMA;
-    if (v.rfind("tcgen05:", 0) == 0) return 1000 + std::atoi(v.c_str() + 8);  // pinned tile width
-    TORCH_CHECK(false, "BSI_B200_ENGINE must be auto, tcgen05, tcgen05:<64|128|256>, simt or bmma");
-}
+    int bits_queries() const { return fixed_bits("BSI_FIXED_BITS_QUERIES", bits_q, 7); }
+    int bits_keys() const { return fixed_bits("BSI_FIXED_BITS_KEYS", bits_k, 6); }
+    bool chunk_scale() const { return chunk == nullptr || std::atoi(chunk) != 0; }
+    bool profile() const { return profile_s != nullptr && std::atoi(profile_s) != 0; }
+    // BSI_FIXED_CLIP_K (bsi_vector_cuda.cpp:295-307): > 0 caps the magnitude that selects a group's shift at
+    // clip_k * mean |v|. The reference reads it once per process; here it is read per call like the other switches.
+    float clip_k() const {
+        const float v = clip != nullptr ? std::strtof(clip, nullptr) : 0.0f;
+        return v > 0.0f ? v : 0.0f;
+    }
+    // The builders honour the variable; the fused additions below (packers that write into exchange buffers,
+    // re-quantising epilogue) have no clipping variant and refuse to run with it.
+    void check_clip(const char* what) const {
+        TORCH_CHECK(!(clip_k() > 0.0f), what, " does not implement BSI_FIXED_CLIP_K > 0 (outlier clipping); "
+                    "use the build_bsi_* entry points");
+    }
+    int dot_engine() const {
+        if (engine == nullptr || !*engine || std::strcmp(engine, "auto") == 0) {
+            // BSI_TC_DOT=0 is the reference's switch to its non-tensor-core kernel, re-read on every launch
+            // (bsi_cuda_kernels_dot.cuh:2642); here it selects the CUDA-core (dp4a) engine, which evaluates the
+            // same recurrence, so verify_tc_dot_correctness.py compares two engines as it does in the reference.
+            if (tc_dot != nullptr && *tc_dot && std::atoi(tc_dot) == 0) return BSI_ENGINE_SIMT;
+            return BSI_ENGINE_AUTO;
+        }
+        const std::string v(engine);
+        if (v == "tcgen05") return BSI_ENGINE_TCGEN05;
+        if (v == "simt") return BSI_ENGINE_SIMT;
+        if (v == "bmma") return BSI_ENGINE_BMMA;
+        if (v.rfind("tcgen05:", 0) == 0) return 1000 + std::atoi(v.c_str() + 8);  // pinned tile width
+        TORCH_CHECK(false, "BSI_B200_ENGINE must be auto, tcgen05, tcgen05:<64|128|256>, simt or bmma");
+    }
+
+private:
+    static bool take(const char* v, const char* name, const char*& slot) {
+        const size_t n = std::strlen(name);
+        if (std::strncmp(v, name, n) != 0) return false;
+        if (slot == nullptr) slot = v + n;
+        return true;
+    }
+    int fixed_bits(const char* name, const char* specific, int fallback) const {
+        const int v = specific != nullptr ? std::atoi(specific) : (bits_any != nullptr ? std::atoi(bits_any) : fallback);
+        TORCH_CHECK(v == 0 || (v >= 2 && v <= 8), name, " must be 0 (variable-slice mode) or in [2, 8], got ", v);
+        return v;
+    }
+};
 
 void check_status(int rc, const char* what) {
     TORCH_CHECK(rc == BSI_OK, what, " failed: ", bsi_b200_status_string(rc), " (", bsi_b200_last_error(), ")");
@@ -153,22 +170,19 @@ struct PrebuiltBSIKeysCUDA {
     }
 };
 
-// Registers a query batch's chunk sums of squares for the duration of one dot call (the Cauchy-Schwarz side of the
-// exact-integer route); the kernel gets the pointers at launch, so the entry can go when the call returns.
-struct ScopedQueryBounds {
-    const int8_t* a8 = nullptr;
-    explicit ScopedQueryBounds(const PackedBatch& qb) {
-        if (qb.sq_norms.defined() && qb.chunk_mode && qb.q8.defined() && qb.q8.numel() > 0) {
-            a8 = qb.q8.data_ptr<int8_t>();
-            bsi_b200_register_query_bounds(a8, qb.sq_norms.data_ptr<float>(), qb.sq_norms.size(1));
-        }
+// What a dot of queries of `query_bits` bits with `keys` may use to prove its integer route exact; qb: the batch whose
+// chunk sums of squares go with it, if it has them.
+bsi_dot_bounds dot_bounds(const PrebuiltBSIKeysCUDA& keys, int query_bits, const PackedBatch* qb) {
+    bsi_dot_bounds b = {};
+    if (!keys.abs_sum.defined()) return b;
+    b.key_bounds = keys.abs_sum.data_ptr<float>();
+    b.query_abs_max = (query_bits >= 2 && query_bits <= 8) ? (1 << (query_bits - 1)) : 128;
+    if (qb != nullptr && qb->sq_norms.defined() && qb->chunk_mode) {
+        b.query_sq = qb->sq_norms.data_ptr<float>();
+        b.query_sq_stride = qb->sq_norms.size(1);
     }
-    ~ScopedQueryBounds() {
-        if (a8 != nullptr) bsi_b200_unregister_query_bounds(a8);
-    }
-    ScopedQueryBounds(const ScopedQueryBounds&) = delete;
-    ScopedQueryBounds& operator=(const ScopedQueryBounds&) = delete;
-};
+    return b;
+}
 
 struct PrebuiltBSIQueryBatchCUDA {
     PackedBatch b;
@@ -204,10 +218,9 @@ uint64_t g_last_quantize_ns = 0, g_last_pack_ns = 0, g_last_total_ns = 0;
 // Quantise + pack `x` ([rows, d], f32/f16/bf16, CPU or CUDA) in one kernel.
 // lean = true skips the bit slices and slice weights (only the int8 image and the scales are
 // produced): what the fused linear path needs. key_bounds (row mode): receives the [3, rows] bounds of the image.
-PackedBatch pack(const at::Tensor& input, int decimal_places, int bits, bool chunk_mode, bool profile,
+PackedBatch pack(const at::Tensor& input, int decimal_places, int bits, bool chunk_mode, float clip_k, bool profile,
                  bool lean = false, at::Tensor* key_bounds = nullptr) {
     TORCH_CHECK(input.dim() == 2, "expects 2D tensor [rows, d]");
-    const float clip_k = clip_k_from_env();
     const auto dev = work_device(input);
     c10::cuda::CUDAGuard guard(dev);
     at::Tensor x = input.detach();
@@ -345,23 +358,23 @@ PackedBatch pack_variable(const at::Tensor& input, int decimal_places, bool for_
     return b;
 }
 
-void require_fixed_queries(const char* what) {
-    TORCH_CHECK(bits_queries() > 0, what, " needs the fixed-bit query mode (BSI_FIXED_BITS_QUERIES in [2, 8])");
+void require_fixed_queries(const Env& env, const char* what) {
+    TORCH_CHECK(env.bits_queries() > 0, what, " needs the fixed-bit query mode (BSI_FIXED_BITS_QUERIES in [2, 8])");
 }
 
 // Queries get chunk scales when enabled and the word count allows 256-bit chunks
 // (bsi_vector_cuda.cpp:980-994).
-PackedBatch pack_queries(const at::Tensor& q2d, int decimal_places, bool lean = false) {
-    const int bits = bits_queries();
+PackedBatch pack_queries(const Env& env, const at::Tensor& q2d, int decimal_places, bool lean = false) {
+    const int bits = env.bits_queries();
     if (bits == 0) {
         g_last_quantize_ns = g_last_pack_ns = g_last_total_ns = 0;
         return pack_variable(q2d, decimal_places, /*for_keys=*/false);
     }
     const int64_t d = q2d.size(1);
     const int W = d > 0 ? static_cast<int>((d + 63) / 64) : 1;
-    const bool chunk = chunk_scale_enabled() && (W % 4 == 0);
-    const bool profile = profile_enabled() && q2d.is_cuda();
-    PackedBatch b = pack(q2d, decimal_places, bits, chunk, profile, lean);
+    const bool chunk = env.chunk_scale() && (W % 4 == 0);
+    const bool profile = env.profile() && q2d.is_cuda();
+    PackedBatch b = pack(q2d, decimal_places, bits, chunk, env.clip_k(), profile, lean);
     // One fused kernel does quantise and pack; its time is reported as the pack time.
     g_last_quantize_ns = 0;
     g_last_pack_ns = profile ? static_cast<uint64_t>(b.quantize_ms * 1.0e6) : 0;
@@ -379,10 +392,12 @@ size_t batch_mem_bytes(const PackedBatch& b) {
 // ---- builders -------------------------------------------------------------------------------------
 py::tuple build_bsi_keys_cuda(torch::Tensor K, int decimalPlaces, float compress_threshold) {
     TORCH_CHECK(K.dim() == 2, "K must be 2D [num_keys, d]");
-    auto* holder = new PrebuiltBSIKeysCUDA();
-    const int kbits = bits_keys();
+    const Env env;
+    const int kbits = env.bits_keys();
+    auto owned = std::make_unique<PrebuiltBSIKeysCUDA>();
+    auto* holder = owned.get();
     holder->b = kbits == 0 ? pack_variable(K, decimalPlaces, /*for_keys=*/true)
-                           : pack(K, decimalPlaces, kbits, /*chunk_mode=*/false, /*profile=*/false, /*lean=*/false,
+                           : pack(K, decimalPlaces, kbits, /*chunk_mode=*/false, env.clip_k(), /*profile=*/false, /*lean=*/false,
                                   &holder->abs_sum);
     holder->num_keys = K.size(0);
     holder->threshold = compress_threshold;
@@ -391,7 +406,7 @@ py::tuple build_bsi_keys_cuda(torch::Tensor K, int decimalPlaces, float compress
         total_mem_bytes = 0;
         for (int sb : holder->b.row_slices) total_mem_bytes += static_cast<uint64_t>(sb) * holder->b.W * 8;
     }
-    py::capsule cap(holder, "PrebuiltBSIKeysCUDA", [](PyObject* c) {
+    py::capsule cap(owned.release(), "PrebuiltBSIKeysCUDA", [](PyObject* c) {
         delete reinterpret_cast<PrebuiltBSIKeysCUDA*>(PyCapsule_GetPointer(c, "PrebuiltBSIKeysCUDA"));
     });
     return py::make_tuple(cap, total_mem_bytes, holder->num_keys, K.size(1), holder->b.W);
@@ -400,10 +415,10 @@ py::tuple build_bsi_keys_cuda(torch::Tensor K, int decimalPlaces, float compress
 py::capsule build_bsi_queries_cuda_batch_packed(torch::Tensor q2d, int decimalPlaces, float compress_threshold) {
     TORCH_CHECK(q2d.dim() == 2, "q must be 2D [Q, d]");
     (void)compress_threshold;  // ignored by the reference too (bsi_cuda.cpp:350)
-    auto* holder = new PrebuiltBSIQueryBatchCUDA();
-    holder->b = pack_queries(q2d, decimalPlaces);
+    auto holder = std::make_unique<PrebuiltBSIQueryBatchCUDA>();
+    holder->b = pack_queries(Env(), q2d, decimalPlaces);
     holder->mem_bytes = batch_mem_bytes(holder->b);
-    return py::capsule(holder, "PrebuiltBSIQueryBatchCUDA", [](PyObject* c) {
+    return py::capsule(holder.release(), "PrebuiltBSIQueryBatchCUDA", [](PyObject* c) {
         delete reinterpret_cast<PrebuiltBSIQueryBatchCUDA*>(PyCapsule_GetPointer(c, "PrebuiltBSIQueryBatchCUDA"));
     });
 }
@@ -422,7 +437,7 @@ py::capsule row_capsule(const std::shared_ptr<PackedBatch>& parent, int64_t row,
 py::list build_bsi_queries_cuda_batch(torch::Tensor q2d, int decimalPlaces, float compress_threshold) {
     TORCH_CHECK(q2d.dim() == 2, "q must be 2D [Q, d]");
     (void)compress_threshold;
-    auto parent = std::make_shared<PackedBatch>(pack_queries(q2d, decimalPlaces));
+    auto parent = std::make_shared<PackedBatch>(pack_queries(Env(), q2d, decimalPlaces));
     py::list out;
     for (int64_t qi = 0; qi < parent->rows; ++qi) out.append(row_capsule(parent, qi, false));
     return out;
@@ -433,9 +448,10 @@ py::list build_bsi_queries_cuda_batch(torch::Tensor q2d, int decimalPlaces, floa
 py::tuple build_bsi_query_cuda(torch::Tensor q, int decimalPlaces, float compress_threshold) {
     TORCH_CHECK(q.dim() == 1, "q must be 1D [d]");
     (void)compress_threshold;
+    const Env env;
     auto parent = std::make_shared<PackedBatch>(
-        bits_queries() == 0 ? pack_variable(q.unsqueeze(0), decimalPlaces, /*for_keys=*/false)
-                            : pack(q.unsqueeze(0), decimalPlaces, bits_queries(), /*chunk_mode=*/false, /*profile=*/false));
+        env.bits_queries() == 0 ? pack_variable(q.unsqueeze(0), decimalPlaces, /*for_keys=*/false)
+                            : pack(q.unsqueeze(0), decimalPlaces, env.bits_queries(), /*chunk_mode=*/false, env.clip_k(), /*profile=*/false));
     const bool has_negative = q.numel() > 0 && (parent->variable ? parent->slice_weights.lt(0).any().item<bool>()
                                                                  : parent->q8.lt(0).any().item<bool>());
     py::capsule cap = row_capsule(parent, 0, has_negative);
@@ -499,9 +515,10 @@ at::Tensor ewah_decode(const EwahStream& e, int64_t W) {
 // the verbatim words the dot consumes; mem_bytes = compressed + verbatim.
 py::tuple build_bsi_query_cuda_hybrid(torch::Tensor q, int decimalPlaces, double compress_threshold) {
     TORCH_CHECK(q.dim() == 1, "q must be 1D [d]");
+    const Env env;
     auto parent = std::make_shared<PackedBatch>(
-        bits_queries() == 0 ? pack_variable(q.unsqueeze(0), decimalPlaces, /*for_keys=*/false)
-                            : pack(q.unsqueeze(0), decimalPlaces, bits_queries(), /*chunk_mode=*/false, /*profile=*/false));
+        env.bits_queries() == 0 ? pack_variable(q.unsqueeze(0), decimalPlaces, /*for_keys=*/false)
+                            : pack(q.unsqueeze(0), decimalPlaces, env.bits_queries(), /*chunk_mode=*/false, env.clip_k(), /*profile=*/false));
     const bool has_negative = q.numel() > 0 && (parent->variable ? parent->slice_weights.lt(0).any().item<bool>()
                                                                  : parent->q8.lt(0).any().item<bool>());
     auto words2d = parent->words.view({parent->S, parent->W});
@@ -514,7 +531,7 @@ py::tuple build_bsi_query_cuda_hybrid(torch::Tensor q, int decimalPlaces, double
 }
 
 // ---- dot ------------------------------------------------------------------------------------------
-py::tuple run_dot(const PackedBatch& qb, const PrebuiltBSIKeysCUDA& keys, bool want_iacc, at::Tensor* iacc_out) {
+py::tuple run_dot(const Env& env, const PackedBatch& qb, const PrebuiltBSIKeysCUDA& keys, bool want_iacc, at::Tensor* iacc_out) {
     const int64_t Q = qb.rows, R = keys.num_keys;
     same_device(qb.q8, keys.b.q8, "queries and keys");
     c10::cuda::CUDAGuard guard(keys.b.q8.device());
@@ -532,7 +549,7 @@ py::tuple run_dot(const PackedBatch& qb, const PrebuiltBSIKeysCUDA& keys, bool w
     at::Tensor iacc;
     if (want_iacc) iacc = at::empty({Q, R, qb.chunks}, fopt.dtype(at::kInt));
 
-    const bool profile = profile_enabled();
+    const bool profile = env.profile();
     auto stream = at::cuda::getCurrentCUDAStream();
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     float kernel_ms = 0.f;
@@ -541,10 +558,9 @@ py::tuple run_dot(const PackedBatch& qb, const PrebuiltBSIKeysCUDA& keys, bool w
         cudaEventCreate(&e1);
         cudaEventRecord(e0, stream.stream());
     }
-    const int engine = engine_from_env();
+    const int engine = env.dot_engine();
     const int64_t qs_stride = qb.chunk_mode ? qb.chunks : 0;
-    keys.register_bounds(qb.variable ? 8 : qb.S);
-    ScopedQueryBounds query_bounds(qb);
+    const bsi_dot_bounds bounds = dot_bounds(keys, qb.variable ? 8 : qb.S, &qb);
     if (qb.variable || keys.b.variable) {
         TORCH_CHECK(engine != BSI_ENGINE_BMMA, "the b1 mma.sync engine reads fixed-bit slices; variable-slice operands use the int8 engines");
         TORCH_CHECK(!want_iacc, "the per-chunk accumulator dump is defined for the fixed-bit mode");
@@ -557,9 +573,9 @@ py::tuple run_dot(const PackedBatch& qb, const PrebuiltBSIKeysCUDA& keys, bool w
         for (int digit = 0; digit < 2; ++digit) {
             const at::Tensor& a8 = digit == 0 ? qb.q8 : qb.q8_hi;
             at::Tensor& dst = digit == 0 ? out : out_hi;
-            check_status(bsi_b200_dot_i8(a8.data_ptr<int8_t>(), a8.size(1), qb.scales.data_ptr<float>(), 0,
+            check_status(bsi_b200_dot_i8_bounded(a8.data_ptr<int8_t>(), a8.size(1), qb.scales.data_ptr<float>(), 0,
                                          keys.b.q8.data_ptr<int8_t>(), keys.b.q8.size(1), keys.b.scales.data_ptr<float>(),
-                                         Q, R, qb.chunks, 1.0f, dst.data_ptr<float>(), R, nullptr, engine, current_stream()),
+                                         Q, R, qb.chunks, 1.0f, dst.data_ptr<float>(), R, nullptr, engine, &bounds, current_stream()),
                          "bsi_b200_dot_i8");
         }
         out.add_(out_hi, 128.0f).mul_(static_cast<float>(scale_inv));
@@ -572,10 +588,10 @@ py::tuple run_dot(const PackedBatch& qb, const PrebuiltBSIKeysCUDA& keys, bool w
                                         want_iacc ? iacc.data_ptr<int>() : nullptr, current_stream()),
                      "bsi_b200_dot_words");
     } else {
-        check_status(bsi_b200_dot_i8(qb.q8.data_ptr<int8_t>(), qb.q8.size(1), qb.scales.data_ptr<float>(), qs_stride,
+        check_status(bsi_b200_dot_i8_bounded(qb.q8.data_ptr<int8_t>(), qb.q8.size(1), qb.scales.data_ptr<float>(), qs_stride,
                                      keys.b.q8.data_ptr<int8_t>(), keys.b.q8.size(1), keys.b.scales.data_ptr<float>(),
                                      Q, R, qb.chunks, static_cast<float>(scale_inv), out.data_ptr<float>(), R,
-                                     want_iacc ? iacc.data_ptr<int>() : nullptr, engine, current_stream()),
+                                     want_iacc ? iacc.data_ptr<int>() : nullptr, engine, &bounds, current_stream()),
                      "bsi_b200_dot_i8");
     }
     if (profile) {
@@ -597,7 +613,7 @@ py::tuple batch_dot_product_multiquery_cuda_batch_caps(py::capsule query_batch_c
     TORCH_CHECK(keys != nullptr, "Invalid CUDA keys capsule");
     auto* qb = from_capsule<PrebuiltBSIQueryBatchCUDA>(query_batch_cap, "PrebuiltBSIQueryBatchCUDA");
     TORCH_CHECK(qb != nullptr, "Invalid CUDA query-batch capsule");
-    return run_dot(qb->b, *keys, false, nullptr);
+    return run_dot(Env(), qb->b, *keys, false, nullptr);
 }
 
 // Rebuilds a batch from per-row capsules. Rows that are, in order, all the rows of one parent
@@ -657,7 +673,7 @@ py::tuple batch_dot_product_multiquery_cuda_caps(py::list query_caps_list, py::c
     TORCH_CHECK(keys != nullptr, "Invalid CUDA keys capsule");
     TORCH_CHECK(keys->num_keys > 0 && py::len(query_caps_list) > 0, "Empty keys or queries");
     PackedBatch b = batch_from_list(query_caps_list);
-    return run_dot(b, *keys, false, nullptr);
+    return run_dot(Env(), b, *keys, false, nullptr);
 }
 
 // ---- stats ----------------------------------------------------------------------------------------
@@ -708,50 +724,122 @@ std::string cuda_builder_version() { return "BSI_B200_SM100A_V" + std::to_string
 // One call for a whole linear layer: pack x, dot with the keys, cast to x's dtype and add the bias.
 // Same arithmetic as BSIQuantizedLinear.forward (verify_accuracy_bsi.py:118-215) without the
 // capsule round trip, the float32 [Q, R] re-read by two elementwise kernels, or host syncs.
-at::Tensor bsi_linear_forward(torch::Tensor x2d, py::capsule keyset_cuda_cap, c10::optional<torch::Tensor> bias,
-                              int decimalPlaces) {
-    auto* keys = from_capsule<PrebuiltBSIKeysCUDA>(keyset_cuda_cap, "PrebuiltBSIKeysCUDA");
+at::Tensor linear_forward(const Env& env, const at::Tensor& x2d, const PrebuiltBSIKeysCUDA& keys,
+                          const c10::optional<torch::Tensor>& bias, int decimalPlaces) {
     TORCH_CHECK(x2d.dim() == 2 && x2d.is_cuda(), "x must be a 2D CUDA tensor");
-    same_device(x2d, keys->b.q8, "activations and keys");
+    same_device(x2d, keys.b.q8, "activations and keys");
     c10::cuda::CUDAGuard guard(x2d.device());
-    const int engine = engine_from_env();
+    const int engine = env.dot_engine();
+    const int bits = env.bits_queries();
     // two-digit variable-slice queries need two dots and a combine: they take the unfused route below
-    const bool fused = (engine == BSI_ENGINE_AUTO || engine == BSI_ENGINE_TCGEN05) && bits_queries() > 0;
-    PackedBatch qb = pack_queries(x2d, decimalPlaces, /*lean=*/fused);
-    const int64_t Q = qb.rows, R = keys->num_keys;
+    const bool fused = (engine == BSI_ENGINE_AUTO || engine == BSI_ENGINE_TCGEN05) && bits > 0;
+    const int64_t Q = x2d.size(0), D = x2d.size(1), R = keys.num_keys;
     TORCH_CHECK(Q > 0 && R > 0, "Empty queries or keys");
-    TORCH_CHECK(qb.W == keys->b.W, "Word count mismatch between query batch and keys");
-    TORCH_CHECK(qb.decimals == keys->b.decimals, "Decimal mismatch between queries and keys: q=", qb.decimals,
-                " k=", keys->b.decimals);
-    const int total_decimals = qb.decimals + keys->b.decimals;
+    const int W = D > 0 ? static_cast<int>((D + 63) / 64) : 1;
+    TORCH_CHECK(W == keys.b.W, "Word count mismatch between query batch and keys");
+    TORCH_CHECK(decimalPlaces == keys.b.decimals, "Decimal mismatch between queries and keys: q=", decimalPlaces,
+                " k=", keys.b.decimals);
+    const int total_decimals = decimalPlaces + keys.b.decimals;
     const double scale_inv = total_decimals > 0 ? 1.0 / std::pow(10.0, total_decimals) : 1.0;
     at::ScalarType yt = x2d.scalar_type();
     if (!(yt == at::kFloat || yt == at::kHalf || yt == at::kBFloat16)) yt = at::kFloat;
-    at::Tensor y = at::empty({Q, R}, qb.q8.options().dtype(yt));
+    at::Tensor y = at::detail::empty_cuda({Q, R}, yt, x2d.device(), c10::nullopt);
     const float* bptr = nullptr;
     at::Tensor b32;
     if (bias.has_value() && bias->defined()) {
-        b32 = bias->to(y.device(), at::kFloat).contiguous();
+        b32 = *bias;
+        if (b32.scalar_type() != at::kFloat || b32.device() != y.device() || !b32.is_contiguous())
+            b32 = b32.to(y.device(), at::kFloat).contiguous();
         TORCH_CHECK(b32.numel() == R, "bias length mismatch");
         bptr = b32.data_ptr<float>();
     }
     const int code = yt == at::kHalf ? BSI_DTYPE_F16 : (yt == at::kBFloat16 ? BSI_DTYPE_BF16 : BSI_DTYPE_F32);
-    if (fused) {
-        keys->register_bounds(qb.S);
-        ScopedQueryBounds query_bounds(qb);
-        check_status(bsi_b200_linear_i8(qb.q8.data_ptr<int8_t>(), qb.q8.size(1), qb.scales.data_ptr<float>(),
-                                        qb.chunk_mode ? qb.chunks : 0, keys->b.q8.data_ptr<int8_t>(),
-                                        keys->b.q8.size(1), keys->b.scales.data_ptr<float>(), bptr, Q, R, qb.chunks,
-                                        static_cast<float>(scale_inv), y.data_ptr(), R, code, current_stream()),
-                     "bsi_b200_linear_i8");
+    if (!fused || D == 0) {
+        // other engines: float32 dot, then the separate cast + bias kernel
+        PackedBatch qb = pack_queries(env, x2d, decimalPlaces);
+        py::tuple r = run_dot(env, qb, keys, false, nullptr);
+        at::Tensor out = r[0].cast<at::Tensor>();
+        check_status(bsi_b200_cast_bias(out.data_ptr<float>(), R, bptr, Q, R, y.data_ptr(), R, code, current_stream()),
+                     "bsi_b200_cast_bias");
         return y;
     }
-    // other engines: float32 dot, then the separate cast + bias kernel
-    py::tuple r = run_dot(qb, *keys, false, nullptr);
-    at::Tensor out = r[0].cast<at::Tensor>();
-    check_status(bsi_b200_cast_bias(out.data_ptr<float>(), R, bptr, Q, R, y.data_ptr(), R, code, current_stream()),
-                 "bsi_b200_cast_bias");
+    at::Tensor x = x2d;
+    if (x.scalar_type() != yt) x = x.to(yt);
+    if (x.stride(1) != 1 || x.stride(0) < D) x = x.contiguous();
+    const bool chunk = env.chunk_scale() && W % 4 == 0;
+    const float clip_k = env.clip_k();
+    const bool profile = env.profile();
+    const int64_t chunks = (D + 255) / 256, ldx = x.stride(0);
+    if (chunk && !(clip_k > 0.0f) && !profile && decimalPlaces >= 0 && decimalPlaces <= 8 &&
+        engine == BSI_ENGINE_AUTO && bsi_b200_linear_decode_fits(Q, R, D)) {
+        check_status(bsi_b200_linear_decode(x.data_ptr(), code, ldx, D, decimalPlaces, bits, keys.b.q8.data_ptr<int8_t>(),
+                                            keys.b.q8.size(1), keys.b.scales.data_ptr<float>(), bptr, Q, R,
+                                            static_cast<float>(scale_inv), y.data_ptr(), R, BSI_ACT_NONE, current_stream()),
+                     "bsi_b200_linear_decode");
+        return y;
+    }
+    // int8 image, scales and chunk sums of squares share one block that goes back to the allocator (stream-ordered)
+    // when the call returns
+    const int64_t image = Q * chunks * 256, per_row = chunk ? chunks : 1;
+    c10::DataPtr work = c10::cuda::CUDACachingAllocator::get()->allocate(static_cast<size_t>(image + 8 * Q * per_row));
+    int8_t* q8 = static_cast<int8_t*>(work.get());
+    float* scales = reinterpret_cast<float*>(q8 + image);
+    float* sq = chunk ? scales + Q * per_row : nullptr;
+    cudaEvent_t e0 = nullptr, e1 = nullptr;
+    if (profile) {
+        cudaEventCreate(&e0);
+        cudaEventCreate(&e1);
+        cudaEventRecord(e0, at::cuda::getCurrentCUDAStream().stream());
+    }
+    check_status(bsi_b200_quantize_pack_all(x.data_ptr(), code, Q, D, ldx, decimalPlaces, bits, chunk ? 1 : 0, clip_k, nullptr,
+                                            scales, nullptr, q8, chunks * 256, sq, nullptr, nullptr, current_stream()),
+                 "bsi_b200_quantize_pack_all");
+    float pack_ms = 0.f;
+    if (profile) {
+        cudaEventRecord(e1, at::cuda::getCurrentCUDAStream().stream());
+        cudaEventSynchronize(e1);
+        cudaEventElapsedTime(&pack_ms, e0, e1);
+        cudaEventDestroy(e0);
+        cudaEventDestroy(e1);
+    }
+    g_last_quantize_ns = 0;
+    g_last_pack_ns = g_last_total_ns = static_cast<uint64_t>(pack_ms * 1.0e6);
+    bsi_dot_bounds bounds = dot_bounds(keys, bits, nullptr);
+    bounds.query_sq = sq;
+    bounds.query_sq_stride = chunks;
+    check_status(bsi_b200_linear_i8_bounded(q8, chunks * 256, scales, chunk ? chunks : 0, keys.b.q8.data_ptr<int8_t>(),
+                                            keys.b.q8.size(1), keys.b.scales.data_ptr<float>(), bptr, Q, R, chunks,
+                                            static_cast<float>(scale_inv), y.data_ptr(), R, code, BSI_ACT_NONE, &bounds,
+                                            current_stream()),
+                 "bsi_b200_linear_i8_bounded");
     return y;
+}
+
+at::Tensor bsi_linear_forward(torch::Tensor x2d, py::capsule keyset_cuda_cap, c10::optional<torch::Tensor> bias,
+                              int decimalPlaces) {
+    auto* keys = from_capsule<PrebuiltBSIKeysCUDA>(keyset_cuda_cap, "PrebuiltBSIKeysCUDA");
+    return linear_forward(Env(), x2d.detach(), *keys, bias, decimalPlaces);
+}
+
+// BSIQuantizedLinear.forward: any leading dimensions, the result in x's type. None when BSI_PROFILE asks for the two
+// separate entry points. One native call because the same steps in Python cost as much as the launches.
+py::object bsi_layer_forward(const torch::Tensor& x, const py::capsule& keyset_cuda_cap, const c10::optional<torch::Tensor>& bias,
+                             int decimalPlaces) {
+    const Env env;
+    if (env.profile_s != nullptr && std::strcmp(env.profile_s, "0") != 0) return py::none();
+    auto* keys = from_capsule<PrebuiltBSIKeysCUDA>(keyset_cuda_cap, "PrebuiltBSIKeysCUDA");
+    TORCH_CHECK(x.dim() >= 1, "x must have at least one dimension");
+    at::Tensor x2d = x.detach();
+    if (x2d.dim() != 2) x2d = x2d.reshape({-1, x2d.size(-1)});
+    if (env.fp32 != nullptr && std::strcmp(env.fp32, "0") != 0) x2d = x2d.to(at::kFloat);   // verify_accuracy_bsi.py:126
+    at::Tensor y = linear_forward(env, x2d, *keys, bias, decimalPlaces);
+    if (y.scalar_type() != x.scalar_type()) y = y.to(x.scalar_type());
+    if (x.dim() != 2) {
+        std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
+        shape.back() = keys->num_keys;
+        y = y.view(shape);
+    }
+    return py::cast(y);
 }
 
 // Quantise + pack activations (query side: chunk scales) into tensors the caller owns: q8 [rows, >= d]
@@ -760,15 +848,16 @@ at::Tensor bsi_linear_forward(torch::Tensor x2d, py::capsule keyset_cuda_cap, c1
 // that a tensor-parallel layer can pack its own column block straight into the buffer the ranks
 // exchange. d must be a multiple of 256.
 void pack_queries_into(torch::Tensor x2d, torch::Tensor q8, torch::Tensor scales, int decimalPlaces) {
-    require_fixed_queries("pack_queries_into");
+    const Env env;
+    require_fixed_queries(env, "pack_queries_into");
     TORCH_CHECK(x2d.dim() == 2 && x2d.is_cuda(), "x must be a 2D CUDA tensor");
     TORCH_CHECK(q8.dim() == 2 && q8.is_cuda() && q8.scalar_type() == at::kChar && q8.stride(1) == 1, "q8 must be int8 [rows, d]");
     TORCH_CHECK(scales.is_cuda() && scales.scalar_type() == at::kFloat && scales.is_contiguous(), "scales must be contiguous float32");
-    check_clip("pack_queries_into");
+    env.check_clip("pack_queries_into");
     same_device(x2d, q8, "pack_queries_into");
     same_device(x2d, scales, "pack_queries_into");
     c10::cuda::CUDAGuard guard(x2d.device());
-    TORCH_CHECK(chunk_scale_enabled(), "pack_queries_into needs BSI_FIXED_CHUNK_SCALE=1");
+    TORCH_CHECK(env.chunk_scale(), "pack_queries_into needs BSI_FIXED_CHUNK_SCALE=1");
     at::Tensor x = x2d.detach();
     if (!(x.scalar_type() == at::kFloat || x.scalar_type() == at::kHalf || x.scalar_type() == at::kBFloat16))
         x = x.to(at::kFloat);
@@ -779,7 +868,7 @@ void pack_queries_into(torch::Tensor x2d, torch::Tensor q8, torch::Tensor scales
     TORCH_CHECK(scales.numel() == rows * (d / 256), "scales shape mismatch");
     if (rows == 0 || d == 0) return;
     check_status(bsi_b200_quantize_pack(x.data_ptr(), dtype_code(x), rows, d, x.stride(0), decimalPlaces,
-                                        bits_queries(), 1, nullptr, scales.data_ptr<float>(), nullptr,
+                                        env.bits_queries(), 1, nullptr, scales.data_ptr<float>(), nullptr,
                                         q8.data_ptr<int8_t>(), q8.stride(0), current_stream()),
                  "bsi_b200_quantize_pack");
 }
@@ -814,12 +903,13 @@ at::Tensor linear_from_packed(torch::Tensor q8, torch::Tensor scales, py::capsul
         bptr = b32.data_ptr<float>();
     }
     const int code = yt == at::kHalf ? BSI_DTYPE_F16 : (yt == at::kBFloat16 ? BSI_DTYPE_BF16 : BSI_DTYPE_F32);
-    keys->register_bounds(bits_queries());
-    check_status(bsi_b200_linear_i8_act(q8.data_ptr<int8_t>(), q8.stride(0), scales.data_ptr<float>(), chunks,
-                                        keys->b.q8.data_ptr<int8_t>(), keys->b.q8.size(1), keys->b.scales.data_ptr<float>(),
-                                        bptr, Q, R, chunks, static_cast<float>(scale_inv), y.data_ptr(), R, code,
-                                        relu ? BSI_ACT_RELU : BSI_ACT_NONE, current_stream()),
-                 "bsi_b200_linear_i8_act");
+    const bsi_dot_bounds bounds = dot_bounds(*keys, Env().bits_queries(), nullptr);
+    check_status(bsi_b200_linear_i8_bounded(q8.data_ptr<int8_t>(), q8.stride(0), scales.data_ptr<float>(), chunks,
+                                            keys->b.q8.data_ptr<int8_t>(), keys->b.q8.size(1),
+                                            keys->b.scales.data_ptr<float>(), bptr, Q, R, chunks,
+                                            static_cast<float>(scale_inv), y.data_ptr(), R, code,
+                                            relu ? BSI_ACT_RELU : BSI_ACT_NONE, &bounds, current_stream()),
+                 "bsi_b200_linear_i8_bounded");
     return y;
 }
 
@@ -858,12 +948,13 @@ void peer_barrier(std::vector<int64_t> flag_ptrs, int rank, int64_t timeout_ms) 
 // scale_ptrs[i] + 4 * (row * scale_ld + chunk).
 void pack_queries_multi(torch::Tensor x2d, std::vector<int64_t> q8_ptrs, int64_t ld8, std::vector<int64_t> scale_ptrs,
                         int64_t scale_ld, int decimalPlaces) {
-    require_fixed_queries("pack_queries_multi");
+    const Env env;
+    require_fixed_queries(env, "pack_queries_multi");
     TORCH_CHECK(x2d.dim() == 2 && x2d.is_cuda(), "x must be a 2D CUDA tensor");
     TORCH_CHECK(!q8_ptrs.empty() && !scale_ptrs.empty(), "destination lists must not be empty");
     c10::cuda::CUDAGuard guard(x2d.device());   // raw destinations: the caller's own or peer mappings of this device
-    check_clip("pack_queries_multi");
-    TORCH_CHECK(chunk_scale_enabled(), "pack_queries_multi needs BSI_FIXED_CHUNK_SCALE=1");
+    env.check_clip("pack_queries_multi");
+    TORCH_CHECK(env.chunk_scale(), "pack_queries_multi needs BSI_FIXED_CHUNK_SCALE=1");
     at::Tensor x = x2d.detach();
     if (!(x.scalar_type() == at::kFloat || x.scalar_type() == at::kHalf || x.scalar_type() == at::kBFloat16))
         x = x.to(at::kFloat);
@@ -873,7 +964,7 @@ void pack_queries_multi(torch::Tensor x2d, std::vector<int64_t> q8_ptrs, int64_t
     for (int64_t p : q8_ptrs) q.push_back(reinterpret_cast<int8_t*>(static_cast<intptr_t>(p)));
     for (int64_t p : scale_ptrs) sc.push_back(reinterpret_cast<float*>(static_cast<intptr_t>(p)));
     check_status(bsi_b200_quantize_pack_multi(x.data_ptr(), dtype_code(x), x.size(0), x.size(1), x.stride(0), decimalPlaces,
-                                              bits_queries(), static_cast<int>(q.size()), q.data(), ld8,
+                                              env.bits_queries(), static_cast<int>(q.size()), q.data(), ld8,
                                               static_cast<int>(sc.size()), sc.data(), scale_ld, current_stream()),
                  "bsi_b200_quantize_pack_multi");
 }
@@ -908,7 +999,7 @@ void linear_from_packed_scatter(torch::Tensor q8, torch::Tensor scales, py::caps
     std::vector<void*> y;
     for (int64_t p : y_ptrs) y.push_back(reinterpret_cast<void*>(static_cast<intptr_t>(p)));
     const int code = yt == at::kHalf ? BSI_DTYPE_F16 : (yt == at::kBFloat16 ? BSI_DTYPE_BF16 : BSI_DTYPE_F32);
-    keys->register_bounds(bits_queries());
+    keys->register_bounds(Env().bits_queries());
     check_status(bsi_b200_linear_i8_scatter(q8.data_ptr<int8_t>(), q8.stride(0), scales.data_ptr<float>(), chunks,
                                             keys->b.q8.data_ptr<int8_t>(), keys->b.q8.size(1),
                                             keys->b.scales.data_ptr<float>(), bptr, Q, R, chunks,
@@ -924,8 +1015,9 @@ void linear_from_packed_requant(torch::Tensor q8, torch::Tensor scales, py::caps
                                 c10::optional<torch::Tensor> bias, int decimalPlaces, py::object layer_dtype, bool relu,
                                 std::vector<int64_t> q8_ptrs, int64_t ld8, std::vector<int64_t> scale_ptrs,
                                 int64_t scale_ld) {
-    require_fixed_queries("linear_from_packed_requant");
-    check_clip("linear_from_packed_requant");
+    const Env env;
+    require_fixed_queries(env, "linear_from_packed_requant");
+    env.check_clip("linear_from_packed_requant");
     auto* keys = from_capsule<PrebuiltBSIKeysCUDA>(keyset_cuda_cap, "PrebuiltBSIKeysCUDA");
     TORCH_CHECK(q8.dim() == 2 && q8.is_cuda() && q8.scalar_type() == at::kChar && q8.stride(1) == 1, "q8 must be int8 [Q, d]");
     TORCH_CHECK(scales.is_cuda() && scales.scalar_type() == at::kFloat && scales.is_contiguous(), "scales must be contiguous float32");
@@ -953,12 +1045,12 @@ void linear_from_packed_requant(torch::Tensor q8, torch::Tensor scales, py::caps
     std::vector<float*> sd;
     for (int64_t p : q8_ptrs) qd.push_back(reinterpret_cast<int8_t*>(static_cast<intptr_t>(p)));
     for (int64_t p : scale_ptrs) sd.push_back(reinterpret_cast<float*>(static_cast<intptr_t>(p)));
-    keys->register_bounds(bits_queries());
+    keys->register_bounds(Env().bits_queries());
     check_status(bsi_b200_linear_i8_requant(q8.data_ptr<int8_t>(), q8.stride(0), scales.data_ptr<float>(), chunks,
                                             keys->b.q8.data_ptr<int8_t>(), keys->b.q8.size(1),
                                             keys->b.scales.data_ptr<float>(), bptr, Q, R, chunks,
                                             static_cast<float>(scale_inv), yt == at::kHalf ? BSI_DTYPE_F16 : BSI_DTYPE_BF16,
-                                            relu ? BSI_ACT_RELU : BSI_ACT_NONE, decimalPlaces, bits_queries(),
+                                            relu ? BSI_ACT_RELU : BSI_ACT_NONE, decimalPlaces, env.bits_queries(),
                                             static_cast<int>(qd.size()), qd.data(), ld8, sd.data(), scale_ld, current_stream()),
                  "bsi_b200_linear_i8_requant");
 }
@@ -968,7 +1060,8 @@ void linear_from_packed_requant(torch::Tensor q8, torch::Tensor scales, py::caps
 at::Tensor add_layernorm_pack(torch::Tensor x, c10::optional<torch::Tensor> delta, torch::Tensor weight, torch::Tensor bias,
                               double eps, std::vector<int64_t> q8_ptrs, int64_t ld8, std::vector<int64_t> scale_ptrs,
                               int64_t scale_ld, int decimalPlaces) {
-    require_fixed_queries("add_layernorm_pack");
+    const Env env;
+    require_fixed_queries(env, "add_layernorm_pack");
     TORCH_CHECK(x.dim() == 2 && x.is_cuda() && x.is_contiguous(), "x must be a contiguous 2D CUDA tensor");
     TORCH_CHECK(x.scalar_type() == at::kHalf || x.scalar_type() == at::kBFloat16, "x must be float16 or bfloat16");
     TORCH_CHECK(weight.scalar_type() == x.scalar_type() && bias.scalar_type() == x.scalar_type() && weight.is_contiguous() &&
@@ -978,8 +1071,8 @@ at::Tensor add_layernorm_pack(torch::Tensor x, c10::optional<torch::Tensor> delt
     same_device(x, weight, "add_layernorm_pack");
     same_device(x, bias, "add_layernorm_pack");
     c10::cuda::CUDAGuard guard(x.device());
-    check_clip("add_layernorm_pack");
-    TORCH_CHECK(chunk_scale_enabled(), "add_layernorm_pack needs BSI_FIXED_CHUNK_SCALE=1");
+    env.check_clip("add_layernorm_pack");
+    TORCH_CHECK(env.chunk_scale(), "add_layernorm_pack needs BSI_FIXED_CHUNK_SCALE=1");
     const void* dptr = nullptr;
     at::Tensor d;
     if (delta.has_value() && delta->defined()) {
@@ -994,7 +1087,7 @@ at::Tensor add_layernorm_pack(torch::Tensor x, c10::optional<torch::Tensor> delt
     for (int64_t p : scale_ptrs) sc.push_back(reinterpret_cast<float*>(static_cast<intptr_t>(p)));
     check_status(bsi_b200_add_layernorm_pack(x.data_ptr(), dptr, weight.data_ptr(), bias.data_ptr(), static_cast<float>(eps),
                                              dtype_code(x), x.size(0), x.size(1), out.data_ptr(), decimalPlaces,
-                                             bits_queries(), static_cast<int>(q.size()), q.data(), ld8,
+                                             env.bits_queries(), static_cast<int>(q.size()), q.data(), ld8,
                                              static_cast<int>(sc.size()), sc.data(), scale_ld, current_stream()),
                  "bsi_b200_add_layernorm_pack");
     return out;
@@ -1039,7 +1132,7 @@ py::tuple debug_dot_iacc(py::capsule query_batch_cap, py::capsule keyset_cuda_ca
     auto* keys = from_capsule<PrebuiltBSIKeysCUDA>(keyset_cuda_cap, "PrebuiltBSIKeysCUDA");
     auto* qb = from_capsule<PrebuiltBSIQueryBatchCUDA>(query_batch_cap, "PrebuiltBSIQueryBatchCUDA");
     at::Tensor iacc;
-    py::tuple r = run_dot(qb->b, *keys, true, &iacc);
+    py::tuple r = run_dot(Env(), qb->b, *keys, true, &iacc);
     return py::make_tuple(r[0], iacc);
 }
 
@@ -1275,6 +1368,8 @@ PYBIND11_MODULE(bsi_ops, m) {
     m.def("bsi_linear_forward", &bsi_linear_forward, py::arg("x2d"), py::arg("keyset_cuda_cap"),
           py::arg("bias") = py::none(), py::arg("decimal_places") = 2,
           "pack + dot + cast + bias for one linear layer");
+    m.def("bsi_layer_forward", &bsi_layer_forward, py::arg("x"), py::arg("keyset_cuda_cap"), py::arg("bias") = py::none(),
+          py::arg("decimal_places") = 2, "bsi_linear_forward over the last dimension of x, in x's type; None under BSI_PROFILE");
     m.def("pack_queries_into", &pack_queries_into, py::arg("x2d"), py::arg("q8"), py::arg("scales"),
           py::arg("decimal_places"), "Pack activations into caller-owned int8 / chunk-scale tensors");
     m.def("linear_from_packed", &linear_from_packed, py::arg("q8"), py::arg("scales"), py::arg("keyset_cuda_cap"),

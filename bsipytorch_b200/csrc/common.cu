@@ -42,9 +42,31 @@ bool lookup_query_bounds(const void* a8, QueryBounds* out) {
     return true;
 }
 
-bool lookup_key_bounds(const void* k8, KeyBounds* out) {
+bool exact_int_enabled() {
     const char* e = getenv("BSI_B200_EXACT_INT");      // 0 switches the integer accumulation off (A/B comparisons)
-    if (e != nullptr && e[0] == '0') return false;
+    return e == nullptr || e[0] != '0';
+}
+
+bsi_dot_bounds resolve_bounds(const bsi_dot_bounds* given, const void* a8, const void* k8, int64_t R) {
+    bsi_dot_bounds b = {};
+    if (given != nullptr) {
+        if (given->key_bounds != nullptr && exact_int_enabled()) b = *given;
+        return b;
+    }
+    KeyBounds kb = {};
+    if (!lookup_key_bounds(k8, &kb) || kb.rows != R) return b;
+    b.key_bounds = kb.abs_sum;
+    b.query_abs_max = static_cast<int>(kb.query_abs_max);
+    QueryBounds qb = {};
+    if (lookup_query_bounds(a8, &qb)) {
+        b.query_sq = qb.sq_norms;
+        b.query_sq_stride = qb.stride;
+    }
+    return b;
+}
+
+bool lookup_key_bounds(const void* k8, KeyBounds* out) {
+    if (!exact_int_enabled()) return false;
     std::lock_guard<std::mutex> lock(g_bounds_mu);
     auto it = g_bounds.find(k8);
     if (it == g_bounds.end()) return false;

@@ -74,6 +74,9 @@ struct QueryBounds {
     int64_t stride;          // floats per row
 };
 bool lookup_query_bounds(const void* a8, QueryBounds* out);
+bool exact_int_enabled();     // BSI_B200_EXACT_INT is not 0
+// The bounds of one dot: what the caller passes (given != nullptr), else what is registered for the two images.
+bsi_dot_bounds resolve_bounds(const bsi_dot_bounds* given, const void* a8, const void* k8, int64_t R);
 
 // True unless BSI_B200_PDL=0: the dot kernels are launched with programmatic stream serialisation (their set-up
 // may overlap the tail of a dot kernel right before them on the stream).

@@ -10,12 +10,17 @@ namespace bsi {
 
 int dot_i8_tcgen05(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride, const int8_t* k8,
                    int64_t ldk, const float* bw0, int64_t Q, int64_t R, int64_t chunks, float scale_inv,
-                   float* out, int64_t ldo, int32_t* dbg_iacc, int force_bn, cudaStream_t stream);
+                   float* out, int64_t ldo, int32_t* dbg_iacc, int force_bn, const bsi_dot_bounds& bounds, cudaStream_t stream);
 
 int dot_i8_pair(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride, const int8_t* k8, int64_t ldk,
                 const float* bw0, const float* bias, int64_t Q, int64_t R, int64_t chunks, float scale_inv,
                 void* out, int64_t ldo, int y_dtype, int32_t* dbg_iacc, int force_bn, int relu,
-                const ScatterDst* scatter, const RequantDst* requant, cudaStream_t stream);
+                const ScatterDst* scatter, const RequantDst* requant, const bsi_dot_bounds& bounds, cudaStream_t stream);
+
+bool decode_fits(int64_t Q, int64_t R, int64_t chunks);
+int dot_decode(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride, const int8_t* k8, int64_t ldk, const float* bw0,
+               const float* bias, int64_t Q, int64_t R, int64_t chunks, float scale_inv, void* out, int64_t ldo, int y_dtype,
+               int relu, cudaStream_t stream, bool* taken);
 
 int dot_words_bmma(const uint64_t* A, const float* qs, int64_t qs_stride, int Sa, int64_t W,
                    const uint64_t* B, const float* Bw, int Sb, int64_t R, int64_t Q, float scale_inv,
@@ -107,7 +112,16 @@ extern "C" int bsi_b200_dot_i8(const int8_t* a8, int64_t lda, const float* qs, i
                                const int8_t* k8, int64_t ldk, const float* bw0,
                                int64_t Q, int64_t R, int64_t chunks, float scale_inv,
                                float* out, int64_t ldo, int32_t* dbg_iacc, int engine,
-                               bsi_stream_t stream_) {
+                               bsi_stream_t stream) {
+    return bsi_b200_dot_i8_bounded(a8, lda, qs, qs_stride, k8, ldk, bw0, Q, R, chunks, scale_inv, out, ldo, dbg_iacc, engine,
+                                   nullptr, stream);
+}
+
+extern "C" int bsi_b200_dot_i8_bounded(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride,
+                                       const int8_t* k8, int64_t ldk, const float* bw0,
+                                       int64_t Q, int64_t R, int64_t chunks, float scale_inv,
+                                       float* out, int64_t ldo, int32_t* dbg_iacc, int engine,
+                                       const bsi_dot_bounds* bounds, bsi_stream_t stream_) {
     using namespace bsi;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
     if (Q < 0 || R < 0 || chunks < 0) return fail(BSI_ERR_INVALID, "dot_i8: negative size");
@@ -127,10 +141,18 @@ extern "C" int bsi_b200_dot_i8(const int8_t* a8, int64_t lda, const float* qs, i
         force_bn = engine - 1000;
         engine = BSI_ENGINE_TCGEN05;
     }
-    if (engine == BSI_ENGINE_AUTO) engine = BSI_ENGINE_TCGEN05;
+    if (engine == BSI_ENGINE_AUTO) {
+        if (dbg_iacc == nullptr && decode_fits(Q, R, chunks)) {
+            bool taken = false;
+            const int rc = dot_decode(a8, lda, qs, qs_stride, k8, ldk, bw0, nullptr, Q, R, chunks, scale_inv, out, ldo,
+                                      BSI_DTYPE_F32, 0, stream, &taken);
+            if (rc != BSI_OK || taken) return rc;
+        }
+        engine = BSI_ENGINE_TCGEN05;
+    }
     if (engine == BSI_ENGINE_TCGEN05) {
         return dot_i8_tcgen05(a8, lda, qs, qs_stride, k8, ldk, bw0, Q, R, chunks, scale_inv, out, ldo,
-                              dbg_iacc, force_bn, stream);
+                              dbg_iacc, force_bn, resolve_bounds(bounds, a8, k8, R), stream);
     }
     if (engine == BSI_ENGINE_SIMT) {
         if (Q > 0x7fffff00ll || R > 0x7fffff00ll || chunks > 0x400000)
@@ -148,7 +170,15 @@ extern "C" int bsi_b200_dot_i8(const int8_t* a8, int64_t lda, const float* qs, i
 extern "C" int bsi_b200_linear_i8_act(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride,
                                   const int8_t* k8, int64_t ldk, const float* bw0, const float* bias,
                                   int64_t Q, int64_t R, int64_t chunks, float scale_inv,
-                                  void* y, int64_t ldy, int y_dtype, int activation, bsi_stream_t stream_) {
+                                  void* y, int64_t ldy, int y_dtype, int activation, bsi_stream_t stream) {
+    return bsi_b200_linear_i8_bounded(a8, lda, qs, qs_stride, k8, ldk, bw0, bias, Q, R, chunks, scale_inv, y, ldy, y_dtype,
+                                      activation, nullptr, stream);
+}
+
+extern "C" int bsi_b200_linear_i8_bounded(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride,
+                                          const int8_t* k8, int64_t ldk, const float* bw0, const float* bias,
+                                          int64_t Q, int64_t R, int64_t chunks, float scale_inv, void* y, int64_t ldy,
+                                          int y_dtype, int activation, const bsi_dot_bounds* bounds, bsi_stream_t stream_) {
     using namespace bsi;
     if (Q < 0 || R < 0 || chunks < 0) return fail(BSI_ERR_INVALID, "linear_i8: negative size");
     if (Q == 0 || R == 0) return BSI_OK;
@@ -165,8 +195,15 @@ extern "C" int bsi_b200_linear_i8_act(const int8_t* a8, int64_t lda, const float
     if (y_dtype != BSI_DTYPE_F32 && y_dtype != BSI_DTYPE_F16 && y_dtype != BSI_DTYPE_BF16)
         return fail(BSI_ERR_INVALID, "linear_i8: unknown y_dtype");
     if (int rc = require_sm100()) return rc;
+    const int relu = activation == BSI_ACT_RELU ? 1 : 0;
+    if (decode_fits(Q, R, chunks)) {
+        bool taken = false;
+        const int rc = dot_decode(a8, lda, qs, qs_stride, k8, ldk, bw0, bias, Q, R, chunks, scale_inv, y, ldy, y_dtype, relu,
+                                  static_cast<cudaStream_t>(stream_), &taken);
+        if (rc != BSI_OK || taken) return rc;
+    }
     return dot_i8_pair(a8, lda, qs, qs_stride, k8, ldk, bw0, bias, Q, R, chunks, scale_inv, y, ldy, y_dtype,
-                       nullptr, 0, activation == BSI_ACT_RELU ? 1 : 0, nullptr, nullptr, static_cast<cudaStream_t>(stream_));
+                       nullptr, 0, relu, nullptr, nullptr, resolve_bounds(bounds, a8, k8, R), static_cast<cudaStream_t>(stream_));
 }
 
 extern "C" int bsi_b200_linear_i8_scatter(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride,
@@ -204,7 +241,7 @@ extern "C" int bsi_b200_linear_i8_scatter(const int8_t* a8, int64_t lda, const f
     }
     if (int rc = require_sm100()) return rc;
     return dot_i8_pair(a8, lda, qs, qs_stride, k8, ldk, bw0, bias, Q, R, chunks, scale_inv, nullptr, ldy, y_dtype,
-                       nullptr, 0, activation == BSI_ACT_RELU ? 1 : 0, &sc, nullptr, static_cast<cudaStream_t>(stream_));
+                       nullptr, 0, activation == BSI_ACT_RELU ? 1 : 0, &sc, nullptr, resolve_bounds(nullptr, a8, k8, R), static_cast<cudaStream_t>(stream_));
 }
 
 extern "C" int bsi_b200_linear_i8_requant(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride,
@@ -248,7 +285,7 @@ extern "C" int bsi_b200_linear_i8_requant(const int8_t* a8, int64_t lda, const f
     }
     if (int rc = require_sm100()) return rc;
     return dot_i8_pair(a8, lda, qs, qs_stride, k8, ldk, bw0, bias, Q, R, chunks, scale_inv, q8_dst[0], R, layer_dtype,
-                       nullptr, 0, activation == BSI_ACT_RELU ? 1 : 0, nullptr, &rq, static_cast<cudaStream_t>(stream_));
+                       nullptr, 0, activation == BSI_ACT_RELU ? 1 : 0, nullptr, &rq, resolve_bounds(nullptr, a8, k8, R), static_cast<cudaStream_t>(stream_));
 }
 
 extern "C" int bsi_b200_linear_i8(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride,

@@ -29,6 +29,7 @@
 #include <cuda_fp16.h>
 
 #include "common.cuh"
+#include "epilogue.cuh"
 #include "quant_bytes.cuh"
 
 namespace bsi {
@@ -537,7 +538,7 @@ int pick_bn(int64_t Q, int64_t R) {
 int dot_i8_pair(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride, const int8_t* k8, int64_t ldk,
                 const float* bw0, const float* bias, int64_t Q, int64_t R, int64_t chunks, float scale_inv,
                 void* out, int64_t ldo, int y_dtype, int32_t* dbg_iacc, int force_bn, int relu,
-                const ScatterDst* scatter_in, const RequantDst* requant_in, cudaStream_t stream) {
+                const ScatterDst* scatter_in, const RequantDst* requant_in, const bsi_dot_bounds& bounds, cudaStream_t stream) {
     RequantDst requant = {};
     if (requant_in != nullptr) {
         requant = *requant_in;
@@ -557,21 +558,12 @@ int dot_i8_pair(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_strid
     if (Q > 0x7fffff00ll || R > 0x7fffff00ll || chunks > 0x400000)
         return fail(BSI_ERR_UNSUPPORTED, "dot_i8: Q, R or chunks too large");
     const bool any_width = y_dtype == BSI_DTYPE_F32;
-    // bounds registered for this key image switch on the integer accumulation where it is provably exact
-    KeyBounds kb = {};
-    const float* kabs = nullptr;
-    float qabs = 0.0f;
-    const float* qsq = nullptr;
-    int64_t qsq_stride = 0;
-    if (lookup_key_bounds(k8, &kb) && kb.rows == R) {
-        kabs = kb.abs_sum;
-        qabs = kb.query_abs_max;
-        QueryBounds qb = {};
-        if (qs_stride != 0 && lookup_query_bounds(a8, &qb) && qb.stride >= chunks) {
-            qsq = qb.sq_norms;
-            qsq_stride = qb.stride;
-        }
-    }
+    // bounds of the two images switch on the integer accumulation where it is provably exact
+    const float* kabs = bounds.key_bounds;
+    const float qabs = static_cast<float>(bounds.query_abs_max);
+    const bool has_sq = kabs != nullptr && qs_stride != 0 && bounds.query_sq_stride >= chunks;
+    const float* qsq = has_sq ? bounds.query_sq : nullptr;
+    const int64_t qsq_stride = bounds.query_sq_stride;
     int bn = force_bn ? force_bn : pick_bn_pair(Q, R, any_width);
     if (!force_bn && any_width && bn == 256 && kabs != nullptr && qsq != nullptr) {
         // Both sides carry their bounds, so the integer route is likely, and with its cheaper epilogue a single
@@ -629,14 +621,14 @@ int dot_i8_pair(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_strid
 
 int dot_i8_tcgen05(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride, const int8_t* k8,
                    int64_t ldk, const float* bw0, int64_t Q, int64_t R, int64_t chunks, float scale_inv,
-                   float* out, int64_t ldo, int32_t* dbg_iacc, int force_bn, cudaStream_t stream) {
+                   float* out, int64_t ldo, int32_t* dbg_iacc, int force_bn, const bsi_dot_bounds& bounds, cudaStream_t stream) {
     if (Q > 0x7fffff00ll || R > 0x7fffff00ll || chunks > 0x400000)
         return fail(BSI_ERR_UNSUPPORTED, "dot_i8: Q, R or chunks too large");
     // force_bn: 0 = automatic; 64/128/256 = single-CTA tiles; 2064/2128/2256 = paired-CTA tiles.
     const bool want_pair = force_bn ? (force_bn >= 2000) : (Q > 128);
     if (want_pair) {
         return dot_i8_pair(a8, lda, qs, qs_stride, k8, ldk, bw0, nullptr, Q, R, chunks, scale_inv, out, ldo,
-                           BSI_DTYPE_F32, dbg_iacc, force_bn ? force_bn - 2000 : 0, /*relu=*/0, nullptr, nullptr, stream);
+                           BSI_DTYPE_F32, dbg_iacc, force_bn ? force_bn - 2000 : 0, /*relu=*/0, nullptr, nullptr, bounds, stream);
     }
     const int bn = force_bn ? force_bn : pick_bn(Q, R);
     CUtensorMap ma, mb;

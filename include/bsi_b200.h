@@ -228,6 +228,33 @@ int bsi_b200_unregister_query_bounds(const int8_t* a8);
  * last call on this device; synchronises and clears the counter. */
 int bsi_b200_debug_exact_int_tiles(unsigned long long* count_out);
 
+/* The same bounds handed to a dot directly, without the registry (host struct of device pointers; key_bounds NULL: none,
+ * query_sq NULL: no Cauchy-Schwarz bound). bounds == NULL: bsi_b200_dot_i8 / bsi_b200_linear_i8_act. */
+typedef struct bsi_dot_bounds {
+    const float* key_bounds;     /* [3, R], as for bsi_b200_register_key_bounds */
+    const float* query_sq;       /* as for bsi_b200_register_query_bounds */
+    int64_t query_sq_stride;
+    int query_abs_max;
+} bsi_dot_bounds;
+int bsi_b200_dot_i8_bounded(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride,
+                            const int8_t* k8, int64_t ldk, const float* bw0, int64_t Q, int64_t R, int64_t chunks,
+                            float scale_inv, float* out, int64_t ldo, int32_t* dbg_iacc, int engine,
+                            const bsi_dot_bounds* bounds, bsi_stream_t stream);
+int bsi_b200_linear_i8_bounded(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride,
+                               const int8_t* k8, int64_t ldk, const float* bw0, const float* bias,
+                               int64_t Q, int64_t R, int64_t chunks, float scale_inv, void* y, int64_t ldy, int y_dtype,
+                               int activation, const bsi_dot_bounds* bounds, bsi_stream_t stream);
+
+/* A linear layer of a few rows in one launch: the activations x [Q, D] (row stride ldx) are quantised (chunk scales)
+ * by every CTA for itself, dotted with the keys, cast to x's type, bias (float32, may be NULL) and activation applied.
+ * Same values as bsi_b200_quantize_pack (chunk_mode 1) followed by bsi_b200_linear_i8_act. For sizes
+ * bsi_b200_linear_decode_fits accepts (host function, 1 or 0): at most 16 rows and few (row, 256-element chunk) groups. */
+#define BSI_B200_DECODE_FUSED_GROUPS 128
+int bsi_b200_linear_decode_fits(int64_t Q, int64_t R, int64_t D);
+int bsi_b200_linear_decode(const void* x, int x_dtype, int64_t ldx, int64_t D, int decimal_places, int bits,
+                           const int8_t* k8, int64_t ldk, const float* bw0, const float* bias, int64_t Q, int64_t R,
+                           float scale_inv, void* y, int64_t ldy, int activation, bsi_stream_t stream);
+
 /* Linear whose finished output is re-quantised for the next linear inside the epilogue, so that the
  * layer-type [Q, R] matrix is never written: y = activation(cast(out) + cast(bias)) in layer_dtype
  * (BSI_DTYPE_F16 / BF16) is what bsi_b200_linear_i8_act would store; here every 256-column chunk of y

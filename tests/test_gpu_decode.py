@@ -1,0 +1,53 @@
+"""The decode kernel (16 query rows and fewer): same bits as the checker and as the tensor-core tiles."""
+import numpy as np
+import pytest
+import torch
+
+import _capi_helpers as H
+import _inputs
+from bsipytorch_b200 import capi
+from oracle import oracle as o
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+# edges of the splits: query groups of 8, row tiles of 16, more tiles than SMs (two and more per CTA), warps along K
+# (1, 2, 16 chunks and one more), slabs of K (32 chunks at 8 rows, 16 at 16), ragged depth, the first size beyond
+@pytest.mark.parametrize("Q,R,D", [(1, 1, 256), (1, 17, 250), (8, 300, 512), (9, 300, 4096), (16, 5000, 768), (17, 4111, 4352),
+                                   (16, 500, 8192), (16, 2500, 4352), (3, 40, 16384), (5, 2400, 33000)])
+@pytest.mark.parametrize("chunk_mode", [True, False])
+def test_decode_dot_matches_other_engines(Q, R, D, chunk_mode):
+    q, k = _inputs.fc1(Q=Q, R=R, D=D, seed=Q + R + D, dtype=torch.float32)
+    qa = H.quantize_pack(q.to(DEV), 2, 7, chunk_mode)
+    kb = H.quantize_pack(k.to(DEV), 2, 6, False)
+    got = H.dot_i8(qa["q8"], qa["scales"], kb["q8"], kb["scales"], o.scale_inv(2))
+    want = H.dot_i8(qa["q8"], qa["scales"], kb["q8"], kb["scales"], o.scale_inv(2), 3064)
+    assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+    assert capi.device_status() == 0
+
+
+# the one-launch layer: 1 .. 128 (row, chunk) groups per CTA, chunks that need the 64-bit quantiser, ragged depth
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("Q,R,D", [(1, 33, 256), (1, 3000, 4096), (2, 520, 16384), (7, 100, 1000), (8, 2500, 4096), (16, 130, 2048)])
+def test_one_launch_layer_equals_build_and_dot(dtype, Q, R, D):
+    import bsipytorch_b200
+    ops = bsipytorch_b200.bsi_ops
+    assert capi.lib().bsi_b200_linear_decode_fits(Q, R, D) == 1
+    q, k = _inputs.fc1(Q=Q, R=R, D=D, seed=Q + R + D, dtype=torch.float32)
+    if Q > 1:
+        q[1, D // 3] = float("inf")
+        q[1, 5] = float("nan")
+        q[0, D - 1] = 6.0e4
+    x = q.to(dtype).to(DEV)
+    keys = ops.build_bsi_keys_cuda(k.to(DEV), 2)[0]
+    bias = torch.linspace(-1, 1, R, device=DEV)
+    scores = ops.batch_dot_product_multiquery_cuda_batch_caps(ops.build_bsi_queries_cuda_batch_packed(x, 2), keys)[0]
+    for b in (None, bias):
+        want = scores.to(dtype) if b is None else scores.to(dtype) + b.to(dtype)
+        got = ops.bsi_layer_forward(x, keys, b, 2)
+        assert got.dtype == dtype and torch.equal(got, want)
+        strided = torch.zeros(Q, D + 3, dtype=dtype, device=DEV)
+        strided[:, :D] = x
+        assert torch.equal(ops.bsi_layer_forward(strided[:, :D], keys, b, 2), want)     # rows that are not 16-byte aligned
+    assert torch.equal(ops.bsi_layer_forward(x.view(1, Q, D), keys, bias, 2), want.view(1, Q, R))
