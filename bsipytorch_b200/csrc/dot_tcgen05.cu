@@ -30,7 +30,7 @@
 
 #include "common.cuh"
 #include "epilogue.cuh"
-#include "quant_bytes.cuh"
+#include "quantise.cuh"
 
 namespace bsi {
 
@@ -425,6 +425,26 @@ int make_map(CUtensorMap* map, const int8_t* base, int64_t rows, int64_t depth, 
     return BSI_OK;
 }
 
+// The output as destination of bulk stores: [rows, cols] elements of esz bytes, boxes of 32 rows x box_bytes, whose
+// 16-byte pieces are swizzled by row (128- or 64-byte rows).
+int make_out_map(CUtensorMap* map, void* out, int esz, int64_t rows, int64_t cols, int64_t ld, int box_bytes) {
+    EncodeTiledFn fn = encode_tiled_fn();
+    if (fn == nullptr) return fail(BSI_ERR_CUDA, "dot_i8: cuTensorMapEncodeTiled entry point not found");
+    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
+    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld * esz)};
+    const cuuint32_t box[2] = {static_cast<cuuint32_t>(box_bytes / esz), 32u};
+    const cuuint32_t estr[2] = {1, 1};
+    const CUresult r = fn(map, esz == 4 ? CU_TENSOR_MAP_DATA_TYPE_UINT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, out, dims, strides,
+                          box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                          box_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                          CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        set_error("dot_i8: cuTensorMapEncodeTiled failed with CUresult %d", static_cast<int>(r));
+        return BSI_ERR_CUDA;
+    }
+    return BSI_OK;
+}
+
 template <int BN, bool DBG>
 int launch_tile(const CUtensorMap& ma, const CUtensorMap& mb, const float* qs, int64_t qs_stride,
                 const float* bw0, int Q, int R, int chunks, float scale_inv, float* out, int64_t ldo,
@@ -445,12 +465,12 @@ int launch_tile(const CUtensorMap& ma, const CUtensorMap& mb, const float* qs, i
 }
 
 template <int BN, bool DBG, typename OutT, bool REQ = false>
-int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, int vector_store,
+int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo, const CUtensorMap& mt, int vector_store,
                 const float* qs, int64_t qs_stride, const float* bw0, const float* bias, int Q, int R, int chunks,
                 float scale_inv, void* out, int64_t ldo, int32_t* dbg, const ScatterDst& scatter,
                 const RequantDst& requant, const float* k_abs_sum, float q_abs_max, const float* q_sq, int64_t q_sq_stride,
                 cudaStream_t stream) {
-    using C = pair::Cfg<BN>;
+    using C = pair::Cfg<BN, OutT, REQ>;
     static int max_clusters[64] = {0};   // per instantiation
     int dev = 0;
     BSI_CUDA_TRY(cudaGetDevice(&dev));
@@ -483,7 +503,7 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, int vector_store,
     }
     int pairs = tiles_total < resident ? tiles_total : resident;
     cfg.gridDim = dim3(2 * pairs, 1, 1);
-    BSI_CUDA_TRY(cudaLaunchKernelEx(&cfg, pair::dot_i8_tcgen05_pair_kernel<BN, DBG, OutT, REQ>, ma, mb, vector_store, qs,
+    BSI_CUDA_TRY(cudaLaunchKernelEx(&cfg, pair::dot_i8_tcgen05_pair_kernel<BN, DBG, OutT, REQ>, ma, mb, mo, mt, vector_store, qs,
                                     qs_stride, bw0, bias, Q, R, chunks, tiles_m, tiles_total, scale_inv, out, ldo, dbg, scatter, requant,
                                     k_abs_sum, q_abs_max, q_sq, q_sq_stride));
     return check_launch("dot_i8 tcgen05 pair launch");
@@ -587,9 +607,17 @@ int dot_i8_pair(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_strid
     const int vector_store =
         (((reinterpret_cast<uintptr_t>(out) & 15) == 0 && (ldo % per16) == 0 && (R % per16) == 0) ? 1 : 0) |
         (relu ? 2 : 0);   // the kernel's store_flags
+    // bulk stores into the one output matrix; several destinations (scatter) keep plain stores
+    CUtensorMap mo = {}, mt = {};
+    int store_flags = vector_store;
+    if ((vector_store & 1) && scatter.n == 0 && requant.n == 0 && ldo * esz < (1ll << 40)) {
+        if (int rc = make_out_map(&mo, out, esz, Q, R, ldo, 128)) return rc;
+        if (int rc = make_out_map(&mt, out, esz, Q, R, ldo, 64)) return rc;
+        store_flags |= 4;
+    }
     const int q = static_cast<int>(Q), r = static_cast<int>(R), c = static_cast<int>(chunks);
 #define BSI_PAIR_T(BN_, DBG_, T_)                                                                              \
-    launch_pair<BN_, DBG_, T_>(ma, mb, vector_store, qs, qs_stride, bw0, bias, q, r, c, scale_inv, out, ldo,  \
+    launch_pair<BN_, DBG_, T_>(ma, mb, mo, mt, store_flags, qs, qs_stride, bw0, bias, q, r, c, scale_inv, out, ldo,  \
                                dbg_iacc, scatter, requant, kabs, qabs, qsq, qsq_stride, stream)
 #define BSI_PAIR(BN_)                                                                   \
     (y_dtype == BSI_DTYPE_F16    ? BSI_PAIR_T(BN_, false, __half)                       \
@@ -598,9 +626,9 @@ int dot_i8_pair(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_strid
                                  : BSI_PAIR_T(BN_, false, float))
     if (requant.n > 0) {
         if (y_dtype == BSI_DTYPE_F16)
-            return launch_pair<256, false, __half, true>(ma, mb, vector_store, qs, qs_stride, bw0, bias, q, r, c, scale_inv,
+            return launch_pair<256, false, __half, true>(ma, mb, mo, mt, store_flags, qs, qs_stride, bw0, bias, q, r, c, scale_inv,
                                                          out, ldo, nullptr, scatter, requant, kabs, qabs, qsq, qsq_stride, stream);
-        return launch_pair<256, false, __nv_bfloat16, true>(ma, mb, vector_store, qs, qs_stride, bw0, bias, q, r, c,
+        return launch_pair<256, false, __nv_bfloat16, true>(ma, mb, mo, mt, store_flags, qs, qs_stride, bw0, bias, q, r, c,
                                                             scale_inv, out, ldo, nullptr, scatter, requant, kabs, qabs, qsq,
                                                             qsq_stride, stream);
     }

@@ -9,29 +9,29 @@
 //
 // Why persistent: a pair walks over tiles t = pair, pair + P, ... . Barrier/TMEM set-up happens once,
 // the TMA producer runs ahead into the next tile while the epilogue of the current one drains, and
-// the fp32 result leaves through shared memory as coalesced stores that overlap the next tile's MMAs.
+// the result leaves through shared memory as bulk tensor stores that overlap the next tile's MMAs.
 //
 // Tile = 256 query rows x BN key rows, BN any multiple of 32 up to 256 (float32 output; the 16-bit layer
 // epilogues use 64, 128 or 256): tcgen05.mma with M = 256 takes every N that is a multiple of 16.
 //
 // Roles per CTA (12 warps; register budget moved with setmaxnreg):
-//   warps 0, 2, 3 TMA producers, k-blocks round robin (both CTAs; every load signals the LEADER's
-//                 full barrier)
-//   warp 1        MMA issuer (leader CTA only), TMEM alloc/dealloc (both CTAs)
+//   warps 0, 2    TMA producers, k-blocks in turn (both CTAs; every load signals the LEADER's full barrier)
+//   warps 1, 3    MMA issuers, chunks in turn (leader CTA only); warp 1 also TMEM alloc/dealloc (both CTAs)
 //   warps 4..11   epilogue: TMEM -> registers, acc = fmaf(float(I), qs[q][c], acc) per chunk in order;
-//                 at the end of a tile: scale, transpose through smem, coalesced st.global.v4
+//                 at the end of a tile: finish into smem, bulk tensor stores (scatter, ragged rows: plain stores)
 //
 // Barriers (same smem offsets in both CTAs):
 //   full[s]    leader's copy used: 1 arrival (leader producer, expect_tx of BOTH CTAs' bytes)
 //   empty[s]   local in each CTA: tcgen05.commit (multicast to both CTAs) after the stage's MMAs
 //   tfull[b]   local in each CTA: multicast commit after a chunk's 8 MMAs
 //   tempty[b]  leader's copy used: one arrival per epilogue warp of BOTH CTAs (16)
-// The accumulator ring holds 2, 4 or 8 buffers (BN > 128, > 64, = 64): with narrow tiles the MMA issuer runs
-// several chunks ahead of the epilogue, which takes the barrier round trip off the critical path.
-// What bounds a chunk on wide tiles is the epilogue, not the 8 MMAs (1024 cycles at BN = 256): three
-// instructions per accumulator value (integer add, float add, FMA; see int_to_float_exact) at one warp
-// instruction per clock and SM sub-partition, next to TMEM loads that slow down while the tensor pipe
-// reads and writes its accumulators; measured about 1450 cycles per chunk at BN = 256.
+// The accumulator ring holds 2 or 4 buffers (BN > 128, else): with narrow tiles the MMA issuers run several chunks
+// ahead of the epilogue, which takes the barrier round trip off the critical path.
+// What bounds a chunk on wide tiles is the epilogue (about 1100 cycles with integer sums, 1350 with every SM storing;
+// the 8 MMAs take 1024): one or three instructions per accumulator value at one warp instruction per clock and SM
+// sub-partition, next to TMEM loads that slow down while the tensor pipe reads and writes its accumulators. What a tile
+// costs beyond its chunks, the bounds and the store phase, went from 20 to 6 thousand cycles with batched bound loads,
+// key scales and bias in shared memory and bulk stores: 4096 x 16384 x 4096, float16 out: 254 -> 189 us (2.9 POPS).
 // All waits are bounded; a timeout raises the abort flag of both CTAs and every role drains out.
 #pragma once
 
@@ -50,26 +50,33 @@ constexpr long long kWait = 500000000ll;  // ~0.25 s; real waits are microsecond
 
 constexpr int kSmemLimit = 232448;   // 227 KB: the most dynamic shared memory one CTA can opt in to
 
-template <int BN>
+template <int BN, typename OutT, bool REQ>
 struct Cfg {
     static_assert(BN % 32 == 0 && BN >= 64 && BN <= 256, "tile width: a multiple of 32 in [64, 256]");
     static constexpr int kHalfN = BN / 2;                 // key rows each CTA loads
     static constexpr int kABytes = BM * BK;               // 16 KB
     static constexpr int kBBytes = kHalfN * BK;           // 4 .. 16 KB, a multiple of 1 KB (swizzle atom)
     static constexpr int kStageBytes = kABytes + kBBytes;
-    static constexpr int kStoreBytes = kEpiWarps * 4096;  // one 32x32 fp32 block per epilogue warp
+    static constexpr int kStoreBytes = kEpiWarps * 4096;  // one block of 32 rows x 128 bytes per epilogue warp
     static constexpr int kTmemCols = 512;                 // all of TMEM: 1 CTA per SM anyway
-    // accumulator ring: buffers start at multiples of the next power of two >= BN (2, 4 or 8 buffers)
+    // accumulator ring: buffers start at multiples of the next power of two >= BN (2 or 4 buffers)
     static constexpr int kAccStride = BN > 128 ? 256 : (BN > 64 ? 128 : 64);
-    static constexpr int kAccBufs = 512 / kAccStride;
+    static constexpr int kAccBufs = BN > 128 ? 2 : 4;
+    // key scales and bias of the tile's columns
+    static constexpr int kColBytes = BN * (4 + static_cast<int>(sizeof(OutT)));
     // chunk-maximum exchange of the re-quantising epilogue: 2 parities x 8 warps x 32 lanes x 2 bytes + 8 counters
-    static constexpr int kXchgBytes = 2 * kEpiWarps * 32 * 2 + kEpiWarps * 4;
-    static constexpr int kFixedBytes = kStoreBytes + (2 * 9 + 2 * kAccBufs + 1) * 8 + 16 + kXchgBytes + 1024;
+    static constexpr int kXchgBytes = REQ ? 2 * kEpiWarps * 32 * 2 + kEpiWarps * 4 : 0;
+    static constexpr int kFixedBytes = kStoreBytes + (2 * 9 + 2 * kAccBufs + 2) * 8 + 16 + kColBytes + kXchgBytes;
     static constexpr int kFit = (kSmemLimit - kFixedBytes) / kStageBytes;
     static constexpr int kStages = kFit > 9 ? 9 : kFit;   // 6 (BN >= 192), 7, 8, 8, 9 (BN = 64)
-    static constexpr int kBarriers = 2 * kStages + 2 * kAccBufs + 1;
-    static constexpr int kSmemBytes = kStages * kStageBytes + kStoreBytes + kBarriers * 8 + 16 + kXchgBytes + 1024;
+    static constexpr int kBarriers = 2 * kStages + 2 * kAccBufs + 2;
+    static constexpr int kSmemBytes = kStages * kStageBytes + kStoreBytes + kBarriers * 8 + 16 + kColBytes + kXchgBytes;
+    // Two MMA issuers take the chunks in turn. An issuer's wait for a stage could only mistake the previous lap for its
+    // own if that lap's chunk were not drained yet, and the accumulator wait in front of it says that chunk
+    // cc - kAccBufs is.
+    static_assert(kStages / 2 >= kAccBufs, "a ring lap must not be shorter than the accumulator ring");
     static_assert(kStages >= 4 && kSmemBytes <= kSmemLimit, "operand ring does not fit");
+    static_assert(kStages * kStageBytes >= kEpiWarps * 4096 * ((kHalfN * static_cast<int>(sizeof(OutT)) + 127) / 128), "the last tile is staged in the ring");
 };
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
@@ -177,26 +184,92 @@ __device__ __forceinline__ float int_to_float_exact(int32_t v) {
     return __int_as_float(v + 0x4B400000) - 12582912.0f;
 }
 
+// ---- finishing 16 bytes of a row: (acc * w) * scale_inv, + bias, ReLU, in the output type ---------------------------
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+    return static_cast<uint64_t>(__float_as_uint(lo)) | (static_cast<uint64_t>(__float_as_uint(hi)) << 32);
+}
+// The values of two adjacent columns; w0, w1: their key scales.
+__device__ __forceinline__ float2 scaled2(const float* acc, float w0, float w1, uint64_t scale2) {
+    const uint64_t r = mul2(mul2(pack2(acc[0], acc[1]), pack2(w0, w1)), scale2);
+    return make_float2(__uint_as_float(static_cast<uint32_t>(r)), __uint_as_float(static_cast<uint32_t>(r >> 32)));
+}
+// cast, then + cast(bias) with one rounding: a 16-bit add rounds like the float32 add of the two values rounded to 16
+// bits (24 >= 2 * 11 + 2), which is what finish<OutT> computes.
+__device__ __forceinline__ uint32_t finish2(float2 v, uint32_t b2, bool has_bias, bool relu, __half) {
+    __half2 y = __floats2half2_rn(v.x, v.y);
+    if (has_bias) y = __hadd2(y, *reinterpret_cast<const __half2*>(&b2));
+    uint32_t o = *reinterpret_cast<const uint32_t*>(&y);
+    if (relu) o &= ~__hlt2_mask(y, __half2half2(__ushort_as_half(0)));
+    return o;
+}
+__device__ __forceinline__ uint32_t finish2(float2 v, uint32_t b2, bool has_bias, bool relu, __nv_bfloat16) {
+    __nv_bfloat162 y = __floats2bfloat162_rn(v.x, v.y);
+    if (has_bias) y = __hadd2(y, *reinterpret_cast<const __nv_bfloat162*>(&b2));
+    uint32_t o = *reinterpret_cast<const uint32_t*>(&y);
+    if (relu) o &= ~__hlt2_mask(y, __bfloat162bfloat162(__ushort_as_bfloat16(0)));
+    return o;
+}
+// colw / colb: the columns' key scales and bias in shared memory, read by every lane at once.
+template <typename OutT>
+__device__ __forceinline__ uint4 finish16(const float* acc, const float* colw, const OutT* colb, uint64_t scale2, bool has_bias,
+                                          bool relu) {
+    if constexpr (sizeof(OutT) == 4) {
+        const float4 w = *reinterpret_cast<const float4*>(colw);
+        float2 a = scaled2(acc, w.x, w.y, scale2), c = scaled2(acc + 2, w.z, w.w, scale2);
+        if (has_bias) {
+            const float4 b = *reinterpret_cast<const float4*>(colb);
+            a.x += b.x; a.y += b.y; c.x += b.z; c.y += b.w;
+        }
+        return make_uint4(__float_as_uint(relu_if<float>(a.x, relu)), __float_as_uint(relu_if<float>(a.y, relu)),
+                          __float_as_uint(relu_if<float>(c.x, relu)), __float_as_uint(relu_if<float>(c.y, relu)));
+    } else {
+        const float4 w = *reinterpret_cast<const float4*>(colw);
+        const float4 v = *reinterpret_cast<const float4*>(colw + 4);
+        const uint4 b = *reinterpret_cast<const uint4*>(colb);
+        return make_uint4(finish2(scaled2(acc, w.x, w.y, scale2), b.x, has_bias, relu, OutT()),
+                          finish2(scaled2(acc + 2, w.z, w.w, scale2), b.y, has_bias, relu, OutT()),
+                          finish2(scaled2(acc + 4, v.x, v.y, scale2), b.z, has_bias, relu, OutT()),
+                          finish2(scaled2(acc + 6, v.z, v.w, scale2), b.w, has_bias, relu, OutT()));
+    }
+}
+__device__ __forceinline__ float cast_bias(float b, float) { return b; }
+__device__ __forceinline__ __half cast_bias(float b, __half) { return __float2half_rn(b); }
+__device__ __forceinline__ __nv_bfloat16 cast_bias(float b, __nv_bfloat16) { return __float2bfloat16_rn(b); }
+
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];"
+                 ::"l"(map), "r"(src), "r"(x), "r"(y) : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+
 template <int BN, bool DBG, typename OutT, bool REQ = false>
 __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
     const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-    int store_flags,   // bit 0: 16-byte vector stores are possible; bit 1: ReLU on the finished value
+    const __grid_constant__ CUtensorMap map_o, const __grid_constant__ CUtensorMap map_t,   // out in boxes of 32 rows x 128 / 64 bytes
+    int store_flags,   // bit 0: 16-byte pieces of a row are aligned; bit 1: ReLU; bit 2: map_o and map_t are valid
     const float* __restrict__ qs, int64_t qs_stride, const float* __restrict__ bw0,
     const float* __restrict__ bias, int Q, int R, int chunks, int tiles_m, int tiles_total, float scale_inv,
     void* __restrict__ out, int64_t ldo, int32_t* __restrict__ dbg_iacc, const ScatterDst scatter,
     const RequantDst requant, const float* __restrict__ k_abs_sum, float q_abs_max,
     const float* __restrict__ q_sq, int64_t q_sq_stride) {
-    using C = Cfg<BN>;
+    using C = Cfg<BN, OutT, REQ>;
     constexpr int kStages = C::kStages;
     constexpr int kCols = BN / 2;              // accumulator columns per epilogue warp: a multiple of 16
 
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    extern __shared__ __align__(1024) uint8_t smem[];     // swizzled operand tiles start on 1 KB
     uint8_t* store_area = smem + kStages * C::kStageBytes;
     uint64_t* bars = reinterpret_cast<uint64_t*>(store_area + C::kStoreBytes);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + C::kBarriers);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    uint16_t* xchg_vals = reinterpret_cast<uint16_t*>(tmem_slot + 4);                       // [2][kEpiWarps][32]
+    float* colw = reinterpret_cast<float*>(tmem_slot + 4);                                  // [BN]
+    OutT* colb = reinterpret_cast<OutT*>(colw + BN);                                        // [BN]
+    uint16_t* xchg_vals = reinterpret_cast<uint16_t*>(colb + BN);                           // [2][kEpiWarps][32] (REQ)
     volatile uint32_t* xchg_count = reinterpret_cast<volatile uint32_t*>(xchg_vals + 2 * kEpiWarps * 32);   // [kEpiWarps]
 
     // let the next kernel of the stream start its own set-up as soon as every CTA of this grid is running
@@ -209,10 +282,10 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
     constexpr int kAccBufs = C::kAccBufs;
     auto tfull_bar = [&](int b) { return bar_base + 8u * (2 * kStages + b); };
     auto tempty_bar = [&](int b) { return bar_base + 8u * (2 * kStages + kAccBufs + b); };
-    const uint32_t drain_bar = bar_base + 8u * (2 * kStages + 2 * kAccBufs);
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
+    const uint32_t drain_bar = bar_base + 8u * (2 * kStages + 2 * kAccBufs + ((warp >> 1) & 1));   // one per issuer
     const uint32_t rank = cluster_ctarank();
     const bool leader = rank == 0;
     const int pair_id = blockIdx.x >> 1;
@@ -234,7 +307,7 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
             asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
             *abort_flag = 0;
         }
-        if (lane < kEpiWarps) xchg_count[lane] = 0u;
+        if (REQ && lane < kEpiWarps) xchg_count[lane] = 0u;
         for (int i = lane; i < C::kBarriers; i += 32) {
             const bool is_tempty = i >= 2 * kStages + kAccBufs && i < 2 * kStages + 2 * kAccBufs;
             mbar_init(bar_base + 8u * i, is_tempty ? 2 * kEpiWarps : 1);
@@ -245,7 +318,7 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
     // Cluster barrier split around the TMEM allocation: arrive now (thread 0's barrier inits are
     // released by its own arrive), wait after the allocation, so the two latencies overlap.
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    const bool is_producer = warp < kFirstEpiWarp && warp != 1;
+    const bool is_producer = warp == 0 || warp == 2;
     uint32_t tmem_base = 0;
     if (is_producer) {
         // The producers need the barriers of both CTAs, not the accumulator memory: they go on to their
@@ -258,8 +331,8 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
             asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
         }
         tc_fence_before();
-        // warp 1 and the eight epilogue warps: the TMEM address is in shared memory from here on
-        asm volatile("bar.sync 1, %0;" ::"n"((1 + kEpiWarps) * 32) : "memory");
+        // the issuers and the eight epilogue warps: the TMEM address is in shared memory from here on
+        asm volatile("bar.sync 1, %0;" ::"n"((2 + kEpiWarps) * 32) : "memory");
         // both CTAs' barriers are initialised before anyone touches the peer's
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
         tc_fence_after();
@@ -273,13 +346,13 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
 
     if (warp < kFirstEpiWarp) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsLow));
-        if (warp != 1 && lane == 0) {
+        if (is_producer && lane == 0) {
             // ---------------- TMA producers ----------------
             // One thread needs ~450 cycles per k-block (empty wait, expect_tx, two tensor copies), which
-            // is slower than the MMAs consume narrow tiles; warps 0, 2 and 3 therefore take the k-blocks
-            // round robin. Stage s = it % kStages is always filled by the producer that owns `it`.
-            constexpr int kProducers = 3;
-            const int me = warp == 0 ? 0 : warp - 1;
+            // is slower than the MMAs consume narrow tiles; warps 0 and 2 therefore take the k-blocks
+            // in turn. Stage s = it % kStages is always filled by the producer that owns `it`.
+            constexpr int kProducers = 2;
+            const int me = warp >> 1;
             int it = 0;
             bool ok = true;
             for (int tile = pair_id; tile < tiles_total && ok; tile += num_pairs) {
@@ -298,40 +371,44 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                     tma_load_2d_pair(a_dst + C::kABytes, &map_b, kb * BK, row_b, leader_full0 + 8u * s);
                 }
             }
-        } else if (warp == 1 && leader) {
-            // ---------------- MMA issuer (leader CTA) ----------------
+        } else if (!is_producer && leader) {
+            // ---------------- MMA issuers (leader CTA) ----------------
             // The whole warp walks the loop (so that addresses and descriptors stay in the uniform
-            // datapath) and one elected lane issues the tensor-core instructions.
+            // datapath) and one elected lane issues the tensor-core instructions. A chunk costs an issuer about 770
+            // cycles (three barrier waits, eight MMAs, three commits), more than the MMAs of tiles up to 160 columns
+            // take, so warps 1 and 3 issue alternate chunks; they share nothing but the order of the rings.
             constexpr uint32_t idesc = umma_idesc_pair(BN);
-            int it = 0, cc = 0;
+            const int mi = warp >> 1;
+            const int total = ((tiles_total - pair_id + num_pairs - 1) / num_pairs) * chunks;
+            int s = 2 * mi;
+            uint32_t ph = 0;
             bool ok = true;
-            for (int tile = pair_id; tile < tiles_total && ok; tile += num_pairs) {
-                for (int c = 0; c < chunks && ok; ++c, ++cc) {
-                    const int b = cc % kAccBufs;
-                    const uint32_t tph = static_cast<uint32_t>(cc / kAccBufs) & 1u;
-                    if (!wait_or_abort(tempty_bar(b), tph ^ 1u, actx, 3)) { ok = false; break; }
-                    const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(b * C::kAccStride);
+            for (int cc = mi; cc < total && ok; cc += 2) {
+                const int b = cc % kAccBufs;
+                const uint32_t tph = static_cast<uint32_t>(cc / kAccBufs) & 1u;
+                if (!wait_or_abort(tempty_bar(b), tph ^ 1u, actx, 3)) { ok = false; break; }
+                const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(b * C::kAccStride);
 #pragma unroll
-                    for (int half = 0; half < 2; ++half, ++it) {
-                        const int s = it % kStages;
-                        const uint32_t ph = static_cast<uint32_t>(it / kStages) & 1u;
-                        if (!wait_or_abort(full_bar(s), ph, actx, 2)) { ok = false; break; }
-                        tc_fence_after();
-                        const uint32_t a_addr = smem_base + s * C::kStageBytes;
-                        const uint64_t adesc = umma_desc(a_addr);
-                        const uint64_t bdesc = umma_desc(a_addr + C::kABytes);
-                        if (elect_one()) {
+                for (int half = 0; half < 2; ++half) {
+                    if (!wait_or_abort(full_bar(s), ph, actx, 2)) { ok = false; break; }
+                    tc_fence_after();
+                    const uint32_t a_addr = smem_base + s * C::kStageBytes;
+                    const uint64_t adesc = umma_desc(a_addr);
+                    const uint64_t bdesc = umma_desc(a_addr + C::kABytes);
+                    if (elect_one()) {
 #pragma unroll
-                            for (int k = 0; k < BK / UMMA_K; ++k) {
-                                umma_i8_pair(tmem_d, adesc + 2u * k, bdesc + 2u * k, idesc,
-                                             (half | k) != 0 ? 1u : 0u);
-                            }
-                            umma_commit_pair(empty_bar(s));
-                            if (half == 1) umma_commit_pair(tfull_bar(b));
+                        for (int k = 0; k < BK / UMMA_K; ++k) {
+                            umma_i8_pair(tmem_d, adesc + 2u * k, bdesc + 2u * k, idesc,
+                                         (half | k) != 0 ? 1u : 0u);
                         }
-                        __syncwarp();
+                        umma_commit_pair(empty_bar(s));
+                        if (half == 1) umma_commit_pair(tfull_bar(b));
                     }
+                    __syncwarp();
+                    if (++s == kStages) { s = 0; ph ^= 1u; }
                 }
+                s += 2;                                    // the other issuer's chunk
+                if (s >= kStages) { s -= kStages; ph ^= 1u; }
             }
             if (!ok && lane == 0) {
                 umma_commit(drain_bar);
@@ -353,7 +430,8 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
         int cc = 0;
         bool ok = true;
         uint32_t tiles_done = 0;   // tiles this warp has re-quantised (the chunk-maximum exchange counts them)
-        for (int tile = pair_id; tile < tiles_total && ok; tile += num_pairs) {
+        // An aborting warp stays in the loop for its barriers: the four warps of a column half meet at two per tile.
+        for (int tile = pair_id; tile < tiles_total; tile += num_pairs) {
             const int tm = tile % tiles_m;
             const int tn = tile / tiles_m;
             const int row = tm * 256 + static_cast<int>(rank) * BM + quad * 32 + lane;
@@ -362,20 +440,14 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
             const float* qs_row = qs + static_cast<int64_t>(row_ok ? row : 0) * (qs_stride ? qs_stride : 1);
 #pragma unroll
             for (int j = 0; j < kCols; ++j) acc[j] = 0.0f;
-            // Key scales of this warp's columns: lane L keeps columns 4L..4L+3 (of the warp's kCols) in
-            // registers; the load's latency hides behind the mainloop and the store phase fetches them
-            // with shuffles.
-            float bwreg[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            float biasreg[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            if (lane * 4 < kCols) {
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int col = n0 + col0 + lane * 4 + e;
-                    if (col < R) {
-                        bwreg[e] = __ldg(bw0 + col);
-                        if (has_bias) biasreg[e] = __ldg(bias + col);
-                    }
-                }
+            // Key scale and bias of the column this lane puts into shared memory for the store phase: a quarter of the
+            // half's columns per warp, loaded here so that the latency hides behind the main loop.
+            constexpr int kOwn = kCols / 4;
+            const int own = quad * kOwn + lane;
+            float own_w = 0.0f, own_b = 0.0f;
+            if (lane < kOwn && n0 + col0 + own < R) {
+                own_w = __ldg(bw0 + n0 + col0 + own);
+                if (has_bias) own_b = __ldg(bias + n0 + col0 + own);
             }
 
             // Integer accumulation where it provably equals the float32 chain: the chunk terms I_c * 2^shift are
@@ -387,98 +459,85 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
             // available). Where both fail and the query image carries its chunk sums of squares (q_sq), the
             // Cauchy-Schwarz product of the two rows' L2 norms is tried. The test is made for the warp's 32 rows x
             // kCols columns at once, so the branch is uniform; a warp whose bounds all fail runs the float32 chain.
-            bool exact = false;
-            if (k_abs_sum != nullptr) {
-                // largest and summed 2^shift of the row
-                float smax = 0.0f, ssum = 0.0f;
-                if (row_ok) {
-                    if (qs_stride) {
-                        // the row's chunk scales, 16 bytes at a time and four loads in flight where the row allows
-                        int c = 0;
-                        float m0 = 0.0f, m1 = 0.0f, m2 = 0.0f, m3 = 0.0f, t0 = 0.0f, t1 = 0.0f, t2 = 0.0f, t3 = 0.0f;
-                        if ((reinterpret_cast<uintptr_t>(qs_row) & 15) == 0) {
-                            const float4* q4 = reinterpret_cast<const float4*>(qs_row);
-                            for (; c + 16 <= chunks; c += 16) {
-                                const float4 a = __ldg(q4 + (c >> 2)), b4 = __ldg(q4 + (c >> 2) + 1);
-                                const float4 d = __ldg(q4 + (c >> 2) + 2), e4 = __ldg(q4 + (c >> 2) + 3);
-                                m0 = fmaxf(m0, fmaxf(fmaxf(a.x, a.y), fmaxf(a.z, a.w)));
-                                m1 = fmaxf(m1, fmaxf(fmaxf(b4.x, b4.y), fmaxf(b4.z, b4.w)));
-                                m2 = fmaxf(m2, fmaxf(fmaxf(d.x, d.y), fmaxf(d.z, d.w)));
-                                m3 = fmaxf(m3, fmaxf(fmaxf(e4.x, e4.y), fmaxf(e4.z, e4.w)));
-                                t0 += (a.x + a.y) + (a.z + a.w);
-                                t1 += (b4.x + b4.y) + (b4.z + b4.w);
-                                t2 += (d.x + d.y) + (d.z + d.w);
-                                t3 += (e4.x + e4.y) + (e4.z + e4.w);
-                            }
-                            for (; c + 4 <= chunks; c += 4) {
-                                const float4 a = __ldg(q4 + (c >> 2));
-                                m0 = fmaxf(m0, fmaxf(fmaxf(a.x, a.y), fmaxf(a.z, a.w)));
-                                t0 += (a.x + a.y) + (a.z + a.w);
-                            }
-                        }
-                        for (; c < chunks; ++c) {
-                            const float v1 = __ldg(qs_row + c);
-                            m0 = fmaxf(m0, v1);
-                            t0 += v1;
-                        }
-                        smax = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
-                        ssum = (t0 + t1) + (t2 + t3);
-                    } else {
-                        smax = __ldg(qs_row);
-                        ssum = smax * static_cast<float>(chunks);
-                    }
-                }
-                // of the warp's key rows: the largest sum of |k| over a row and over one 256-element chunk
-                float ktot = 0.0f, kchk = 0.0f;
+            // Everything the bounds read is loaded in one go: one after the other, as scalars behind the previous
+            // bound's outcome, they cost 5 to 10 thousand cycles per tile.
+            bool exact = false, small = false;
+            if (k_abs_sum != nullptr && ok) {
+                // of the warp's key rows: the largest sum of |k| over a row and over one chunk, the largest sum of k^2
+                float ktot = 0.0f, kchk = 0.0f, k2 = 0.0f;
                 if (lane * 4 < kCols) {
+                    float kv[12];
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
-                        const int col = n0 + col0 + lane * 4 + e;
-                        if (col < R) {
-                            ktot = fmaxf(ktot, __ldg(k_abs_sum + col));
-                            kchk = fmaxf(kchk, __ldg(k_abs_sum + R + col));
+                        const int col = min(n0 + col0 + lane * 4 + e, R - 1);
+                        kv[e] = __ldg(k_abs_sum + col);
+                        kv[4 + e] = __ldg(k_abs_sum + R + col);
+                        kv[8 + e] = __ldg(k_abs_sum + 2 * static_cast<int64_t>(R) + col);
+                    }
+                    ktot = fmaxf(fmaxf(kv[0], kv[1]), fmaxf(kv[2], kv[3]));
+                    kchk = fmaxf(fmaxf(kv[4], kv[5]), fmaxf(kv[6], kv[7]));
+                    k2 = fmaxf(fmaxf(kv[8], kv[9]), fmaxf(kv[10], kv[11]));
+                }
+                // of the lane's query row: the largest and the summed 2^shift, the sum of squares
+                float smax = 0.0f, ssum = 0.0f, u2 = 0.0f;
+                if (row_ok) {
+                    const float* nrow = q_sq != nullptr ? q_sq + static_cast<int64_t>(row) * q_sq_stride : nullptr;
+                    if (!qs_stride) {
+                        smax = __ldg(qs_row);
+                        ssum = smax * static_cast<float>(chunks);
+                    } else if (((reinterpret_cast<uintptr_t>(qs_row) | reinterpret_cast<uintptr_t>(nrow)) & 15) == 0 && (chunks & 3) == 0) {
+                        constexpr int kAhead = 4;
+                        for (int c = 0; c < chunks; c += 4 * kAhead) {
+                            float4 a[kAhead], n[kAhead];
+#pragma unroll
+                            for (int h = 0; h < kAhead; ++h) {
+                                const bool in = c + 4 * h < chunks;
+                                a[h] = in ? __ldg(reinterpret_cast<const float4*>(qs_row + c) + h) : make_float4(0.f, 0.f, 0.f, 0.f);
+                                n[h] = in && nrow != nullptr ? __ldg(reinterpret_cast<const float4*>(nrow + c) + h) : make_float4(0.f, 0.f, 0.f, 0.f);
+                            }
+#pragma unroll
+                            for (int h = 0; h < kAhead; ++h) {
+                                smax = fmaxf(smax, fmaxf(fmaxf(a[h].x, a[h].y), fmaxf(a[h].z, a[h].w)));
+                                ssum += (a[h].x + a[h].y) + (a[h].z + a[h].w);
+                                u2 += (n[h].x + n[h].y) + (n[h].z + n[h].w);
+                            }
+                        }
+                    } else {
+                        constexpr int kAhead = 8;
+                        for (int c = 0; c < chunks; c += kAhead) {
+                            float a[kAhead], n[kAhead];
+#pragma unroll
+                            for (int h = 0; h < kAhead; ++h) {
+                                a[h] = c + h < chunks ? __ldg(qs_row + c + h) : 0.0f;
+                                n[h] = c + h < chunks && nrow != nullptr ? __ldg(nrow + c + h) : 0.0f;
+                            }
+#pragma unroll
+                            for (int h = 0; h < kAhead; ++h) {
+                                smax = fmaxf(smax, a[h]);
+                                ssum += a[h];
+                                u2 += n[h];
+                            }
                         }
                     }
                 }
                 // non-negative floats order like their bit patterns; an infinity anywhere fails the test
-                const float su = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(smax)));
-                const float tu = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(ssum)));
-                const float ku = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(ktot)));
-                const float cu = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(kchk)));
-                // the sums above round (relative 2^-24 per addition, at most a few hundred additions): 0.999 covers it
-                exact = fminf(su * ku, tu * cu) * q_abs_max < 16777216.0f * 0.999f;
-                if (!exact && q_sq != nullptr) {
-                    // Cauchy-Schwarz: |prefix|^2 <= (sum of squares of the de-shifted query row) x (sum of k^2)
-                    float u2 = 0.0f;
-                    if (row_ok) {
-                        const float* nrow = q_sq + static_cast<int64_t>(row) * q_sq_stride;
-                        float a0 = 0.0f, a1 = 0.0f;
-                        int c = 0;
-                        for (; c + 2 <= chunks; c += 2) {
-                            a0 += __ldg(nrow + c);
-                            a1 += __ldg(nrow + c + 1);
-                        }
-                        if (c < chunks) a0 += __ldg(nrow + c);
-                        u2 = a0 + a1;
-                    }
-                    float k2 = 0.0f;
-                    if (lane * 4 < kCols) {
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const int col = n0 + col0 + lane * 4 + e;
-                            if (col < R) k2 = fmaxf(k2, __ldg(k_abs_sum + 2 * static_cast<int64_t>(R) + col));
-                        }
-                    }
-                    const float u2w = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(u2)));
-                    const float k2w = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(k2)));
-                    exact = u2w * k2w < 281474976710656.0f * 0.999f;      // 2^48
-                }
+                auto most = [](float v) { return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v))); };
+                const float su = most(smax), tu = most(ssum), ku = most(ktot), cu = most(kchk);
+                // the sums above round (relative 2^-24 per addition, at most a few thousand additions): 0.999 covers it
+                const float first = fminf(su * ku, tu * cu) * q_abs_max;
+                const float norm = q_sq != nullptr && qs_stride ? most(u2) * most(k2) : __uint_as_float(0x7f800000u);
+                exact = first < 16777216.0f * 0.999f || norm < 281474976710656.0f * 0.999f;      // 2^24, 2^48
+                small = first < 4194304.0f * 0.999f || norm < 17592186044416.0f * 0.999f;        // 2^22, 2^44
             }
 
+            // the chunk scale of the next chunk is loaded a whole chunk ahead: a scattered load per lane (32 rows) that
+            // would otherwise stand in front of every fold
+            float qnext = __ldg(qs_row);
             for (int c = 0; c < chunks && ok; ++c, ++cc) {
                 const int b = cc % kAccBufs;
                 const uint32_t tph = static_cast<uint32_t>(cc / kAccBufs) & 1u;
-                const float qscale = qs_stride ? __ldg(qs_row + c) : __ldg(qs_row);
+                const float qscale = qnext;
+                if (qs_stride && c + 1 < chunks) qnext = __ldg(qs_row + c + 1);
                 const int qmul = exact ? __float2int_rn(qscale) : 0;
                 if (!wait_or_abort(tfull_bar(b), tph, actx, 4)) { ok = false; break; }
                 tc_fence_after();
@@ -539,27 +598,41 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                     }
                 }
             }
-            if (!ok) break;
+            // the half's key scales and bias into shared memory: behind the first barrier nobody reads the last tile's
+            asm volatile("bar.sync %0, 128;" ::"r"(2 + half) : "memory");
+            if (lane < kOwn) {
+                colw[col0 + own] = own_w;
+                colb[col0 + own] = cast_bias(own_b, OutT());
+            }
+            asm volatile("bar.sync %0, 128;" ::"r"(2 + half) : "memory");
+            if (!ok) continue;
             if (exact) {
-                // the int32 sums (below 2^24 in magnitude) as floats: what the float32 chain would hold
+                // the int32 sums (below 2^24 in magnitude) as floats: what the float32 chain would hold. Below 2^22 by an
+                // integer and a float add, at four times the rate of the conversion instruction.
+                if (small) {
 #pragma unroll
-                for (int j = 0; j < kCols; ++j) acc[j] = static_cast<float>(__float_as_int(acc[j]));
+                    for (int j = 0; j < kCols; ++j) acc[j] = int_to_float_exact(__float_as_int(acc[j]));
+                } else {
+#pragma unroll
+                    for (int j = 0; j < kCols; ++j) acc[j] = static_cast<float>(__float_as_int(acc[j]));
+                }
                 if (lane == 0) atomicAdd(&g_exact_int_tiles, 1ull);
             }
 
             // ---- tile result: out = (acc * bw0[r]) * scale_inv ----
-            // A lane owns a row; 32 x 32 blocks go through this warp's 4 KB of smem (16-byte chunks
-            // XOR-swizzled by row so that both directions are conflict free) and leave as
-            // st.global.v4 with 8 lanes per 128-byte row segment: every store instruction writes
-            // four full 128-byte lines. Plain stores are fire-and-forget, so the warp moves on to
-            // the next tile (or exits) while they drain.
+            // A lane owns a row. Blocks of 32 rows x 128 bytes are finished into shared memory (16-byte pieces swizzled
+            // as the tensor map wants them, which also keeps the banks apart) and leave as one bulk tensor store each,
+            // so that the warp is back in the next tile's main loop while they drain; written with ordinary stores, the
+            // output took half of a tile's time at 16 chunks. A warp has one block of its own; on a CTA's last tile
+            // every block has its place in the operand ring, which nothing reads any more.
             const int row_base = tm * 256 + static_cast<int>(rank) * BM + quad * 32;
             constexpr int E = static_cast<int>(sizeof(OutT));
-            constexpr int kPerChunk = 16 / E;                                   // values per 16-byte chunk
-            constexpr int kRoundCols = (kCols * E >= 128) ? 128 / E : kCols;    // columns staged per round
-            constexpr int kChunks = kRoundCols * E / 16;                        // 8, or 4 for 64-byte rows
-            constexpr int kRounds = kCols / kRoundCols;
-            constexpr int kRowBytes = kChunks * 16;
+            constexpr int kPerChunk = 16 / E;                        // values per 16-byte piece
+            constexpr int kRoundCols = 128 / E;                      // columns per block
+            constexpr int kFull = kCols / kRoundCols;                // whole blocks; then one of 64-byte rows, or none
+            constexpr int kRounds = kFull + (kCols % kRoundCols != 0 ? 1 : 0);
+            static_assert((kCols * E) % 64 == 0, "whole 64-byte pieces of a row");
+            const uint64_t scale2 = pack2(scale_inv, scale_inv);
             if constexpr (REQ) {
                 static_assert(BN == 256 && !DBG && sizeof(OutT) == 2, "re-quantisation: 256-wide tiles, 16-bit layer type");
                 {
@@ -567,19 +640,12 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                     // what the next linear's packer would read; with BN = 256 a tile row is exactly one chunk,
                     // split between this warp and the warp of the other column half. Same integers as the pack
                     // kernel's fast path (the values have 16-bit precision, so the float32 rounding is exact).
-                    uint32_t amax_bits = 0;
+                    RawLane<OutT> y[kCols / 8];
+                    uint32_t amax_bits = 0;                   // pattern of OutT: orders like the magnitude
 #pragma unroll
-                    for (int j = 0; j < kCols; ++j) {
-                        const float w = __shfl_sync(0xffffffffu, bwreg[j & 3], j >> 2);
-                        const float bv = __shfl_sync(0xffffffffu, biasreg[j & 3], j >> 2);
-                        // cast, then add the bias rounded to the layer type (0 without bias: the sum is then the
-                        // value itself), round again: what finish<OutT> computes, without its branch on has_bias
-                        float v = static_cast<float>(static_cast<OutT>((acc[j] * w) * scale_inv));
-                        v = static_cast<float>(static_cast<OutT>(v + static_cast<float>(static_cast<OutT>(bv))));
-                        if (relu && v < 0.0f) v = 0.0f;
-                        acc[j] = v;
-                        amax_bits = max(amax_bits, __float_as_uint(v) & 0x7fffffffu);
-                        if ((j & 15) == 15) asm volatile("" ::: "memory");   // keeps the 128 steps from being interleaved
+                    for (int j = 0; j < kCols / 8; ++j) {
+                        y[j].v[0] = finish16<OutT>(acc + j * 8, colw + col0 + j * 8, colb + col0 + j * 8, scale2, has_bias, relu);
+                        amax_bits = max(amax_bits, y[j].abs_max());
                     }
                     // Largest magnitude of the whole chunk: swap with the partner warp (same rows, other column
                     // half). The value is one of the OutT values, so its 16-bit pattern carries it exactly. Each
@@ -588,8 +654,7 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                     // The wait is bounded like every other wait of the kernel.
                     {
                         const uint32_t par = tiles_done & 1u;
-                        const OutT amax_t = static_cast<OutT>(__uint_as_float(amax_bits));
-                        xchg_vals[(par * kEpiWarps + ew) * 32 + lane] = *reinterpret_cast<const uint16_t*>(&amax_t);
+                        xchg_vals[(par * kEpiWarps + ew) * 32 + lane] = static_cast<uint16_t>(amax_bits);
                         __syncwarp();
                         if (lane == 0) {
                             __threadfence_block();
@@ -606,40 +671,29 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                             }
                         }
                         ok = __all_sync(0xffffffffu, ok);
-                        if (!ok) break;
+                        if (!ok) continue;
                         __threadfence_block();
-                        const uint16_t other = xchg_vals[(par * kEpiWarps + (ew ^ 4)) * 32 + lane];
-                        const OutT other_t = *reinterpret_cast<const OutT*>(&other);
-                        amax_bits = max(amax_bits, __float_as_uint(static_cast<float>(other_t)) & 0x7fffffffu);
+                        amax_bits = max(amax_bits, static_cast<uint32_t>(xchg_vals[(par * kEpiWarps + (ew ^ 4)) * 32 + lane]));
                         ++tiles_done;
                     }
-                    float amax = __uint_as_float(amax_bits);
-                    if (!(amax_bits < 0x7f800000u && amax * requant.mult < 8388608.0f)) {
+                    float amax = RawLane<OutT>::abs_value(amax_bits);
+                    if (!(amax * requant.mult < 8388608.0f)) {      // NaN fails the comparison too
                         // NaN / inf / out of the exact range: not representable on this path; report, store zeros
                         atomicCAS(&g_device_status, 0, 48);
                         amax = 0.0f;
 #pragma unroll
-                        for (int j = 0; j < kCols; ++j) acc[j] = 0.0f;
+                        for (int j = 0; j < kCols / 8; ++j) y[j].v[0] = make_uint4(0u, 0u, 0u, 0u);
                     }
                     const int shift = fast_shift(amax, requant.mult, requant.bits);
-                    float inv, cst;
-                    fast_round_consts(shift, inv, cst);
                     // stage 32 rows x 128 bytes through this warp's 4 KB (16-byte chunks XOR-swizzled by row)
                     uint8_t* dst = my_store + lane * 128;
 #pragma unroll
                     for (int ch = 0; ch < 8; ++ch) {
-                        uint32_t wv[4];
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            const int j = ch * 16 + k * 4;
-                            wv[k] = sign_clamp4(fast_magnitude(acc[j], requant.mult, inv, cst),
-                                                fast_magnitude(acc[j + 1], requant.mult, inv, cst),
-                                                fast_magnitude(acc[j + 2], requant.mult, inv, cst),
-                                                fast_magnitude(acc[j + 3], requant.mult, inv, cst),
-                                                __float_as_uint(acc[j]), __float_as_uint(acc[j + 1]),
-                                                __float_as_uint(acc[j + 2]), __float_as_uint(acc[j + 3]), requant.bits);
-                        }
-                        *reinterpret_cast<uint4*>(dst + ((ch ^ (lane & 7)) << 4)) = make_uint4(wv[0], wv[1], wv[2], wv[3]);
+                        const u64 lo = y[2 * ch].quantise(requant.mult, shift, requant.bits);
+                        const u64 hi = y[2 * ch + 1].quantise(requant.mult, shift, requant.bits);
+                        *reinterpret_cast<uint4*>(dst + ((ch ^ (lane & 7)) << 4)) =
+                            make_uint4(static_cast<uint32_t>(lo), static_cast<uint32_t>(lo >> 32), static_cast<uint32_t>(hi),
+                                       static_cast<uint32_t>(hi >> 32));
                     }
                     __syncwarp();
                     const int cchunk = lane & 7;
@@ -675,103 +729,83 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                 outp = static_cast<OutT*>(scatter.y[d]);
                 row_shift = d * scatter.rows_per_dst;
             }
-            if ((store_flags & 1)) {
-                if constexpr (sizeof(OutT) == 4) {
-                    // float32 output: the raw running sums are transposed first and scaled afterwards, when a
-                    // lane holds four consecutive columns of a row: the key scales (and bias) of those columns
-                    // are four loads per round instead of two shuffles per value (the warp shuffles of the
-                    // other order cost as many cycles as the stores themselves). Rounds of 32 columns, then
-                    // one of 16 when the warp's column count is not a multiple of 32.
-                    float* outf = reinterpret_cast<float*>(outp);
-                    constexpr int kFull = kCols / 32;
-                    constexpr int kRoundsF = kFull + ((kCols % 32) != 0 ? 1 : 0);
+            if (store_flags & 1) {
+                const bool bulk = (store_flags & 4) != 0;
+                const bool last = tile + num_pairs >= tiles_total;
 #pragma unroll
-                    for (int g = 0; g < kRoundsF; ++g) {
-                        const bool tail = g == kFull;
-                        const int nch = tail ? 4 : 8;          // 16-byte pieces per staged row
-                        const int cchunk = lane & (nch - 1);
-                        const int col = n0 + col0 + g * 32 + cchunk * 4;
-                        float w[4], bv[4];
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const bool in = col + e < R;
-                            w[e] = in ? __ldg(bw0 + col + e) : 0.0f;
-                            bv[e] = (in && has_bias) ? __ldg(bias + col + e) : 0.0f;
-                        }
-                        uint8_t* dst = my_store + lane * (nch * 16);
-#pragma unroll
-                        for (int ch = 0; ch < 8; ++ch) {
-                            if (ch < nch) {
-                                const int swz = tail ? (ch ^ ((lane >> 1) & 3)) : (ch ^ (lane & 7));
-                                const int j = g * 32 + ch * 4;
-                                *reinterpret_cast<float4*>(dst + (swz << 4)) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
-                            }
-                        }
+                for (int g = 0; g < kRounds; ++g) {
+                    const bool whole = g < kFull;
+                    const int nch = whole ? 8 : 4;                   // 16-byte pieces per staged row
+                    const int cg = col0 + g * kRoundCols;            // first column of the block in the tile
+                    uint8_t* block = my_store;
+                    if (bulk && last) {
+                        block = smem + (ew * kRounds + g) * 4096;
+                    } else if (bulk) {
+                        if (lane == 0) tma_store_wait_read();
                         __syncwarp();
+                    }
+                    uint8_t* dst = block + lane * (nch * 16);
+#pragma unroll
+                    for (int ch = 0; ch < 8; ++ch) {
+                        if (ch < nch) {
+                            const int swz = whole ? (ch ^ (lane & 7)) : (ch ^ ((lane >> 1) & 3));
+                            const int j = g * kRoundCols + ch * kPerChunk;
+                            *reinterpret_cast<uint4*>(dst + (swz << 4)) =
+                                finish16<OutT>(acc + j, colw + col0 + j, colb + col0 + j, scale2, has_bias, relu);
+                        }
+                    }
+                    if (bulk) {
+                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                        __syncwarp();
+                        if (lane == 0 && row_base < Q && n0 + cg < R)      // rows and columns beyond the matrix are clipped
+                            tma_store_2d(whole ? &map_o : &map_t, smem_u32(block), n0 + cg, row_base);
+                    } else {
+                        __syncwarp();
+                        const int cchunk = lane & (nch - 1);
+                        const int col = n0 + cg + cchunk * kPerChunk;
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {
                             if (i < nch) {
                                 const int rr = i * (32 / nch) + lane / nch;
-                                const int swz = tail ? (cchunk ^ ((rr >> 1) & 3)) : (cchunk ^ (rr & 7));
-                                float4 o = *reinterpret_cast<const float4*>(my_store + rr * (nch * 16) + (swz << 4));
-                                o.x = relu_if<float>(finish<float>((o.x * w[0]) * scale_inv, bv[0], has_bias), relu);
-                                o.y = relu_if<float>(finish<float>((o.y * w[1]) * scale_inv, bv[1], has_bias), relu);
-                                o.z = relu_if<float>(finish<float>((o.z * w[2]) * scale_inv, bv[2], has_bias), relu);
-                                o.w = relu_if<float>(finish<float>((o.w * w[3]) * scale_inv, bv[3], has_bias), relu);
+                                const int swz = whole ? (cchunk ^ (rr & 7)) : (cchunk ^ ((rr >> 1) & 3));
+                                const uint4 o = *reinterpret_cast<const uint4*>(block + rr * (nch * 16) + (swz << 4));
                                 const int grow = row_base + rr;
-                                if (grow < Q && col < R) {   // R is a multiple of 4 on this path
-                                    *reinterpret_cast<float4*>(outf + static_cast<int64_t>(grow - row_shift) * ldo + col) = o;
-                                }
+                                if (grow < Q && col < R)             // R is a multiple of kPerChunk on this path
+                                    *reinterpret_cast<uint4*>(outp + static_cast<int64_t>(grow - row_shift) * ldo + col) = o;
                             }
                         }
                         __syncwarp();
                     }
-                } else {
-                static_assert(kCols % kRoundCols == 0, "this store order needs whole rounds");
-#pragma unroll
-                for (int g = 0; g < kRounds; ++g) {
-                    const int colg = n0 + col0 + g * kRoundCols;
-                    uint8_t* dst = my_store + lane * kRowBytes;
-#pragma unroll
-                    for (int ch = 0; ch < kChunks; ++ch) {
-                        OutT vals[kPerChunk];
-#pragma unroll
-                        for (int e = 0; e < kPerChunk; ++e) {
-                            const int j = g * kRoundCols + ch * kPerChunk + e;
-                            const float w = __shfl_sync(0xffffffffu, bwreg[j & 3], j >> 2);
-                            const float bv = __shfl_sync(0xffffffffu, biasreg[j & 3], j >> 2);
-                            vals[e] = relu_if<OutT>(finish<OutT>((acc[j] * w) * scale_inv, bv, has_bias), relu);
-                        }
-                        const int swz = kChunks == 8 ? (ch ^ (lane & 7)) : (ch ^ ((lane >> 1) & 3));
-                        *reinterpret_cast<uint4*>(dst + (swz << 4)) = *reinterpret_cast<const uint4*>(vals);
-                    }
-                    __syncwarp();
-                    const int cchunk = lane % kChunks;
-                    const int col = colg + cchunk * kPerChunk;
-#pragma unroll
-                    for (int i = 0; i < kChunks; ++i) {
-                        const int rr = i * (32 / kChunks) + lane / kChunks;
-                        const int swz = kChunks == 8 ? (cchunk ^ (rr & 7)) : (cchunk ^ ((rr >> 1) & 3));
-                        const uint4 o = *reinterpret_cast<const uint4*>(my_store + rr * kRowBytes + (swz << 4));
-                        const int grow = row_base + rr;
-                        if (grow < Q && col < R) {   // R is a multiple of kPerChunk on this path
-                            *reinterpret_cast<uint4*>(outp + static_cast<int64_t>(grow - row_shift) * ldo + col) = o;
-                        }
-                    }
-                    __syncwarp();
-                }
                 }
             } else {
-                OutT* orow = outp + static_cast<int64_t>(row_ok ? row - row_shift : 0) * ldo;
+                // Rows that do not start on 16 bytes: blocks of 32 x 32 raw sums through the warp's 4 KB, then a row at
+                // a time with one value per lane, so that a store still covers consecutive addresses.
+                float* stage = reinterpret_cast<float*>(my_store);
+                constexpr int kBlocks = (kCols + 31) / 32;
 #pragma unroll
-                for (int j = 0; j < kCols; ++j) {
+                for (int g = 0; g < kBlocks; ++g) {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j)
+                        if (g * 32 + j < kCols) stage[lane * 32 + (j ^ lane)] = acc[g * 32 + j];
+                    __syncwarp();
+                    const int j = g * 32 + lane;
                     const int col = n0 + col0 + j;
-                    const float w = __shfl_sync(0xffffffffu, bwreg[j & 3], j >> 2);
-                    const float bv = __shfl_sync(0xffffffffu, biasreg[j & 3], j >> 2);
-                    if (row_ok && col < R) orow[col] = relu_if<OutT>(finish<OutT>((acc[j] * w) * scale_inv, bv, has_bias), relu);
+                    const bool in = j < kCols && col < R;
+                    const float w = in ? colw[col0 + j] : 0.0f;
+                    const float bv = in ? static_cast<float>(colb[col0 + j]) : 0.0f;      // finish() narrows it again: no change
+#pragma unroll 4
+                    for (int rr = 0; rr < 32; ++rr) {
+                        const float v = stage[rr * 32 + (lane ^ rr)];
+                        const int grow = row_base + rr;
+                        if (in && grow < Q)
+                            outp[static_cast<int64_t>(grow - row_shift) * ldo + col] =
+                                relu_if<OutT>(finish<OutT>((v * w) * scale_inv, bv, has_bias), relu);
+                    }
+                    __syncwarp();
                 }
             }
         }
+        if (lane == 0) tma_store_wait_read();      // shared memory is read until then
     }
 
     if (threadIdx.x == 0 && *abort_flag) {
