@@ -25,6 +25,7 @@
 #include <filesystem>
 #include <fstream>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -465,33 +466,87 @@ struct EwahStream {
     int64_t total = 0;
 };
 
+// Words of pinned host memory a kernel writes and the host watches. One page for the process, never freed; a caller
+// holds its word alone from take() to give().
+class HostWords {
+public:
+    static volatile uint64_t* take() {
+        std::lock_guard<std::mutex> lock(mutex());
+        auto& f = free_list();
+        static bool made = false;
+        if (!made) {
+            made = true;
+            void* page = nullptr;
+            if (cudaHostAlloc(&page, 64 * kStride, cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
+                for (int i = 0; i < 64; ++i) f.push_back(reinterpret_cast<volatile uint64_t*>(static_cast<char*>(page) + i * kStride));
+            } else {
+                (void)cudaGetLastError();
+            }
+        }
+        if (f.empty()) return nullptr;
+        auto* w = f.back();
+        f.pop_back();
+        return w;
+    }
+    static void give(volatile uint64_t* w) {
+        std::lock_guard<std::mutex> lock(mutex());
+        free_list().push_back(w);
+    }
+
+private:
+    static constexpr size_t kStride = 64;     // a cache line each
+    static std::mutex& mutex() { static std::mutex m; return m; }
+    static std::vector<volatile uint64_t*>& free_list() { static std::vector<volatile uint64_t*> v; return v; }
+};
+
 EwahStream ewah_encode(const at::Tensor& words2d, double threshold) {
     TORCH_CHECK(words2d.dim() == 2 && words2d.scalar_type() == at::kLong && words2d.is_cuda(),
                 "words must be a CUDA int64 tensor [S, W]");
     c10::cuda::CUDAGuard guard(words2d.device());
     auto w = words2d.contiguous();
     const int64_t S = w.size(0), W = w.size(1);
-    auto o64 = at::TensorOptions().dtype(at::kLong).device(w.device());
-    auto o32 = at::TensorOptions().dtype(at::kInt).device(w.device());
+    auto fresh = [&](int64_t n, at::ScalarType t) { return at::detail::empty_cuda({n}, t, w.device(), c10::nullopt); };
     EwahStream e;
-    e.off = at::empty({S}, o64);
-    e.len = at::empty({S}, o32);
-    e.flags = at::empty({S}, o32);
-    auto total = at::zeros({1}, o64);
+    e.off = fresh(S, at::kLong);
+    e.len = fresh(S, at::kInt);
+    e.flags = fresh(S, at::kInt);
     const int64_t capacity = S * (W + 1);  // worst case: every slice verbatim, or alternating words
-    e.stream = at::empty({std::max<int64_t>(capacity, 1)}, o64);
-    auto scratch = at::empty({std::max<int64_t>(bsi_b200_ewah_scratch_bytes(S), 8)},
-                             at::TensorOptions().dtype(at::kByte).device(w.device()));
-    if (S > 0) {
-        check_status(bsi_b200_ewah_encode(reinterpret_cast<const uint64_t*>(w.data_ptr<int64_t>()), S, W, threshold,
-                                          scratch.data_ptr(), scratch.numel(),
-                                          reinterpret_cast<uint64_t*>(e.stream.data_ptr<int64_t>()), capacity,
-                                          reinterpret_cast<uint64_t*>(e.off.data_ptr<int64_t>()),
-                                          e.len.data_ptr<int>(), e.flags.data_ptr<int>(),
-                                          reinterpret_cast<uint64_t*>(total.data_ptr<int64_t>()), current_stream()),
-                     "bsi_b200_ewah_encode");
+    e.stream = fresh(std::max<int64_t>(capacity, 1), at::kLong);
+    if (S == 0) {
+        e.stream = e.stream.narrow(0, 0, 0);
+        return e;
     }
-    e.total = total.item<int64_t>();
+    const int64_t scratch_bytes = std::max<int64_t>(bsi_b200_ewah_scratch_bytes(S), 8);
+    c10::DataPtr scratch = c10::cuda::CUDACachingAllocator::get()->allocate(static_cast<size_t>(scratch_bytes));
+    // The length of the stream comes back through a word of mapped host memory that the second pass writes first, so
+    // that this call returns while the streams are still being written.
+    volatile uint64_t* word = HostWords::take();
+    at::Tensor total_dev;
+    if (word == nullptr) total_dev = fresh(1, at::kLong);
+    else *word = ~0ull;
+    const cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
+    const int rc = bsi_b200_ewah_encode(reinterpret_cast<const uint64_t*>(w.data_ptr<int64_t>()), S, W, threshold, scratch.get(),
+                                        scratch_bytes, reinterpret_cast<uint64_t*>(e.stream.data_ptr<int64_t>()), capacity,
+                                        reinterpret_cast<uint64_t*>(e.off.data_ptr<int64_t>()), e.len.data_ptr<int>(),
+                                        e.flags.data_ptr<int>(),
+                                        word != nullptr ? const_cast<uint64_t*>(word)
+                                                        : reinterpret_cast<uint64_t*>(total_dev.data_ptr<int64_t>()),
+                                        static_cast<bsi_stream_t>(stream));
+    check_status(rc, "bsi_b200_ewah_encode");      // a word whose kernel may still write it is not given back
+    if (word != nullptr) {
+        py::gil_scoped_release unlocked;
+        cudaError_t state = cudaErrorNotReady;
+        for (uint32_t spins = 1; *word == ~0ull; ++spins) {
+            if ((spins & 0xfffu) != 0u) continue;
+            if (state != cudaErrorNotReady) break;             // asked before the last look at the word
+            state = cudaStreamQuery(stream);
+        }
+        TORCH_CHECK(*word != ~0ull, "ewah_encode: the stream ended without a result: ", cudaGetErrorString(state));
+        e.total = static_cast<int64_t>(*word);
+        HostWords::give(word);
+    } else {
+        e.total = total_dev.item<int64_t>();
+    }
     e.stream = e.stream.narrow(0, 0, e.total);
     return e;
 }
@@ -500,7 +555,7 @@ at::Tensor ewah_decode(const EwahStream& e, int64_t W) {
     const int64_t S = e.off.size(0);
     c10::cuda::CUDAGuard guard(e.off.device());
     same_device(e.off, e.stream, "ewah_decode");
-    auto out = at::empty({S, W}, at::TensorOptions().dtype(at::kLong).device(e.off.device()));
+    auto out = at::detail::empty_cuda({S, W}, at::kLong, e.off.device(), c10::nullopt);
     if (S > 0) {
         check_status(bsi_b200_ewah_decode(reinterpret_cast<const uint64_t*>(e.stream.data_ptr<int64_t>()),
                                           reinterpret_cast<const uint64_t*>(e.off.data_ptr<int64_t>()),

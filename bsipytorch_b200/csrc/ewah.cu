@@ -245,27 +245,42 @@ __global__ void __launch_bounds__(1024) ewah_offsets_kernel(const u64* __restric
     exclusive_scan_block(sizes, S, off, total);
 }
 
-// The same scan as the middle kernel of the one-call encoder, launched as a programmatic dependent of the sizes
-// pass: it lets the emit pass start (whose blocks first load their slices, which depend on nothing), then waits
-// for the sizes pass to be complete.
-__global__ void __launch_bounds__(1024) ewah_block_offsets_kernel(const u64* __restrict__ sums, int64_t n,
-                                                                  u64* __restrict__ off, u64* __restrict__ total) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    exclusive_scan_block(sums, n, off, total);
-}
-
-// Decode: lane 0 parses the RLWs in order (bsi_cuda_kernels_ewah.cuh:16-32), the warp fills runs
-// and copies literals together.
+// Decode (bsi_cuda_kernels_ewah.cuh:16-32), one warp per slice: the RLWs are parsed in order by every lane, the warp
+// fills runs and copies literals together. A stream of up to kHeld words is first loaded as a whole, every load in
+// flight at once, and parsed in shared memory; fetched word by word, an RLW and then its literals stood behind each
+// other's latency (28672 slices of 256 words: 31 us). A slice that is one literal run leaves straight from registers.
+constexpr int kHeldTiles = 9;
+constexpr int kHeld = kHeldTiles * 32;      // up to 256 words and some RLWs
 __global__ void __launch_bounds__(kWarpsPerBlock * 32) ewah_decode_kernel(
     const u64* __restrict__ in, const u64* __restrict__ off, const int32_t* __restrict__ len,
     int64_t S, int64_t W, u64* __restrict__ out) {
+    __shared__ u64 held[kWarpsPerBlock][kHeld];
     const int lane = threadIdx.x & 31;
-    const int64_t s = static_cast<int64_t>(blockIdx.x) * kWarpsPerBlock + (threadIdx.x >> 5);
+    const int warp = threadIdx.x >> 5;
+    const int64_t s = static_cast<int64_t>(blockIdx.x) * kWarpsPerBlock + warp;
     if (s >= S) return;
     const u64* src = in + off[s];
     const int64_t in_len = len[s];
     u64* dst = out + s * W;
+    if (in_len <= kHeld) {
+        const int n = static_cast<int>(in_len);
+        u64 v[kHeldTiles];
+#pragma unroll
+        for (int t = 0; t < kHeldTiles; ++t) v[t] = t * 32 + lane < n ? __ldcs(src + t * 32 + lane) : 0ull;
+        const u64 first = __shfl_sync(0xffffffffu, v[0], 0);
+        if (W < kHeld && first == static_cast<u64>(W) << 33 && n == W + 1) {
+#pragma unroll
+            for (int t = 0; t < kHeldTiles; ++t) {
+                const int w = t * 32 + lane - 1;
+                if (w >= 0 && w < W) dst[w] = v[t];
+            }
+            return;
+        }
+#pragma unroll
+        for (int t = 0; t < kHeldTiles; ++t) held[warp][t * 32 + lane] = v[t];
+        __syncwarp();
+        src = held[warp];
+    }
     int64_t idx = 0, o = 0;
     while (idx < in_len && o < W) {
         const u64 rlw = src[idx++];
@@ -431,32 +446,45 @@ __device__ __forceinline__ void load_slice(const u64* __restrict__ base, int64_t
     }
 }
 
-// Pass 1: flag and encoded size of every slice, and the sum of the sizes of each block's 8 slices.
+// Two passes over the slices with `per_block` of them per block, at most kMaxSums blocks whatever S is: the sums of the
+// blocks' encoded sizes are then few enough for every block of the second pass to add up the ones before its own,
+// which a scan kernel between the passes did before (7 us, most of it latency).
+constexpr int kMaxSums = 2048;
+inline int64_t slices_per_block(int64_t S) {
+    const int64_t least = (S + kMaxSums - 1) / kMaxSums;
+    return (least + kWarpsPerBlock - 1) / kWarpsPerBlock * kWarpsPerBlock;
+}
+
+// Pass 1: flag and encoded size of every slice, and the sum of the sizes of each block's slices. Bound by the one read
+// of the slices: popcounts are added up in 32 bits by one reduction, and only slices that compress are walked.
 // TILES = 0 walks the slice in memory (W > 256).
 template <int TILES>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32) ewah_sizes_kernel(
-    const u64* __restrict__ words, int64_t S, int64_t W, double threshold, const FlagCuts cuts,
+    const u64* __restrict__ words, int64_t S, int64_t W, double threshold, const FlagCuts cuts, int64_t per_block,
     int32_t* __restrict__ flags, u64* __restrict__ sizes, u64* __restrict__ block_sums) {
     __shared__ u64 wsize[kWarpsPerBlock];
-    // the scan and the emit pass are launched as programmatic dependents: once every block of this grid runs,
-    // theirs may be scheduled into SMs that fall idle (they wait for this grid's results where they need them)
+    // the emit pass is launched as programmatic dependent: once every block of this grid runs, its blocks may be
+    // scheduled into SMs that fall idle (they wait for this grid's results where they need them)
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    const int64_t s = static_cast<int64_t>(blockIdx.x) * kWarpsPerBlock + warp;
-    u64 n = 0;
-    if (s < S) {
+    const int64_t s0 = static_cast<int64_t>(blockIdx.x) * per_block;
+    const int64_t s1 = s0 + per_block < S ? s0 + per_block : S;
+    u64 mine = 0;
+    for (int64_t s = s0 + warp; s < s1; s += kWarpsPerBlock) {
         const u64* base = words + s * W;
-        u64 local = 0;
         int flag;
+        u64 n;
         if constexpr (TILES > 0) {
             u64 wv[TILES];
             load_slice<TILES>(base, W, lane, wv);
+            uint32_t local = 0;
 #pragma unroll
-            for (int t = 0; t < TILES; ++t) local += static_cast<u64>(__popcll(wv[t]));
-            flag = flag_from(warp_sum_u64(local), W, threshold, cuts);
-            n = encode_slice_regs<false, TILES>(wv, W, flag, nullptr, lane);
+            for (int t = 0; t < TILES; ++t) local += static_cast<uint32_t>(__popcll(wv[t]));
+            flag = flag_from(__reduce_add_sync(0xffffffffu, local), W, threshold, cuts);
+            n = flag ? encode_slice_regs<false, TILES>(wv, W, flag, nullptr, lane) : 1ull + static_cast<u64>(W);
         } else {
+            u64 local = 0;
             for (int64_t w = lane; w < W; w += 32) local += static_cast<u64>(__popcll(base[w]));
             flag = flag_from(warp_sum_u64(local), W, threshold, cuts);
             n = encode_slice<false>(base, W, flag, nullptr, lane);
@@ -465,8 +493,9 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) ewah_sizes_kernel(
             flags[s] = flag;
             sizes[s] = n;
         }
+        mine += n;
     }
-    if (lane == 0) wsize[warp] = n;
+    if (lane == 0) wsize[warp] = mine;
     __syncthreads();
     if (threadIdx.x == 0) {
         u64 t = 0;
@@ -476,42 +505,68 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) ewah_sizes_kernel(
     }
 }
 
-// Pass 3: offsets of the block's slices from the scanned block sums, then the streams.
+// Pass 2: offsets of the block's slices from the sums of the blocks before, then the streams. Block 0 leaves the total
+// as the first thing it does, so that a host that watches it (mapped memory) goes on while the streams are written.
 template <int TILES>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32) ewah_emit_blocks_kernel(
-    const u64* __restrict__ words, int64_t S, int64_t W, const int32_t* __restrict__ flags,
-    const u64* __restrict__ sizes, const u64* __restrict__ block_off, u64 capacity,
-    u64* __restrict__ off, u64* __restrict__ out, int32_t* __restrict__ out_len) {
+    const u64* __restrict__ words, int64_t S, int64_t W, int64_t per_block, const int32_t* __restrict__ flags,
+    const u64* __restrict__ sizes, const u64* __restrict__ block_sums, u64 capacity,
+    u64* __restrict__ off, u64* __restrict__ out, int32_t* __restrict__ out_len, u64* __restrict__ total) {
+    __shared__ u64 wsum[kWarpsPerBlock];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    const int64_t s0 = static_cast<int64_t>(blockIdx.x) * kWarpsPerBlock;
-    const int64_t s = s0 + warp;
-    // The slice itself is input of the whole call: it is loaded before the wait for the two passes before this one
-    // (programmatic dependent launch), so that this read overlaps their tail and the scan.
+    const int64_t s0 = static_cast<int64_t>(blockIdx.x) * per_block;
+    const int64_t s1 = s0 + per_block < S ? s0 + per_block : S;
+    // The slice itself is input of the whole call: the first one is loaded before the wait for the pass before this
+    // one (programmatic dependent launch), so that this read overlaps its tail.
     u64 wv[TILES > 0 ? TILES : 1];
     if constexpr (TILES > 0) {
-        if (s < S) load_slice<TILES>(words + s * W, W, lane, wv);
+        if (s0 + warp < s1) load_slice<TILES>(words + (s0 + warp) * W, W, lane, wv);
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    // every warp adds up the sizes of the block's slices before its own
-    u64 mine = (lane < kWarpsPerBlock && s0 + lane < S) ? sizes[s0 + lane] : 0ull;
-    u64 before = (lane < warp) ? mine : 0ull;
-    before = warp_sum_u64(before);
-    if (s >= S) return;
-    const u64 o = block_off[blockIdx.x] + before;
-    const u64 n_expected = __shfl_sync(0xffffffffu, mine, warp);
-    if (lane == 0) off[s] = o;
-    if (o + n_expected > capacity) {
-        if (lane == 0) out_len[s] = static_cast<int32_t>(n_expected);
-        return;
-    }
-    u64 n;
-    if constexpr (TILES > 0) {
-        n = encode_slice_regs<true, TILES>(wv, W, flags[s], out + o, lane);
+    auto sum_of = [&](unsigned n) {      // of the first n block sums, for every thread of the block
+        u64 t = 0;
+        for (unsigned i = threadIdx.x; i < n; i += kWarpsPerBlock * 32) t += __ldg(block_sums + i);
+        t = warp_sum_u64(t);
+        if (lane == 0) wsum[warp] = t;
+        __syncthreads();
+        t = 0;
+#pragma unroll
+        for (int w = 0; w < kWarpsPerBlock; ++w) t += wsum[w];
+        return t;
+    };
+    u64 base_off = 0;
+    if (blockIdx.x == 0) {
+        const u64 all = sum_of(gridDim.x);
+        if (threadIdx.x == 0 && total != nullptr) {
+            *reinterpret_cast<volatile u64*>(total) = all;
+            __threadfence_system();
+        }
     } else {
-        n = encode_slice<true>(words + s * W, W, flags[s], out + o, lane);
+        base_off = sum_of(blockIdx.x);
     }
-    if (lane == 0) out_len[s] = static_cast<int32_t>(n);
+    for (int64_t g0 = s0; g0 < s1; g0 += kWarpsPerBlock) {
+        const int64_t s = g0 + warp;
+        if constexpr (TILES > 0) {
+            if (g0 != s0 && s < s1) load_slice<TILES>(words + s * W, W, lane, wv);
+        }
+        // every warp adds up the sizes of the group's slices before its own
+        const u64 mine = (lane < kWarpsPerBlock && g0 + lane < s1) ? __ldg(sizes + g0 + lane) : 0ull;
+        const u64 o = base_off + warp_sum_u64(lane < warp ? mine : 0ull);
+        const u64 n_expected = __shfl_sync(0xffffffffu, mine, warp);
+        base_off += warp_sum_u64(mine);
+        if (s >= s1) continue;
+        if (lane == 0) {
+            off[s] = o;
+            out_len[s] = static_cast<int32_t>(n_expected);
+        }
+        if (o + n_expected > capacity) continue;
+        if constexpr (TILES > 0) {
+            encode_slice_regs<true, TILES>(wv, W, __ldg(flags + s), out + o, lane);
+        } else {
+            encode_slice<true>(words + s * W, W, flags[s], out + o, lane);
+        }
+    }
 }
 
 // Launch as a programmatic dependent of the kernel before it in the stream: the kernel may start while that one
@@ -613,7 +668,7 @@ extern "C" int bsi_b200_ewah_decode(const uint64_t* in, const uint64_t* off, con
 }
 
 extern "C" int64_t bsi_b200_ewah_scratch_bytes(int64_t S) {
-    // sizes [S], block sums and block offsets [ceil(S / 8)] each, 3 words for the flag bounds; rounded up generously
+    // sizes [S], at most min(ceil(S / 8), kMaxSums) block sums, 3 words for the flag bounds; rounded up generously
     return S < 0 ? 0 : (2 * S + 16) * static_cast<int64_t>(sizeof(uint64_t));
 }
 
@@ -674,16 +729,17 @@ extern "C" int bsi_b200_ewah_encode(const uint64_t* words, int64_t S, int64_t W,
         return fail(BSI_ERR_INVALID, "ewah_encode: scratch too small or misaligned");
     if (out == nullptr || off == nullptr || out_len == nullptr || flags == nullptr || capacity < 0)
         return fail(BSI_ERR_INVALID, "ewah_encode: null pointer");
-    const int64_t nb = (S + kWarpsPerBlock - 1) / kWarpsPerBlock;
+    const int64_t per_block = slices_per_block(S);
+    const int64_t nb = (S + per_block - 1) / per_block;
     u64* sizes = static_cast<u64*>(scratch);
     u64* block_sums = sizes + S;
-    u64* block_off = block_sums + nb;
-    u64* cut_words = block_off + nb;
+    u64* cut_words = block_sums + nb;
     FlagCuts cuts;
     if (int rc = flag_cuts(W, threshold, cut_words, stream, &cuts)) return rc;
     const u64* w64 = reinterpret_cast<const u64*>(words);
-    const unsigned grid = warp_blocks(S);
-#define BSI_EWAH_SIZES(T) ewah_sizes_kernel<T><<<grid, kWarpsPerBlock * 32, 0, stream>>>(w64, S, W, threshold, cuts, flags, sizes, block_sums)
+    const unsigned grid = static_cast<unsigned>(nb);
+#define BSI_EWAH_SIZES(T) ewah_sizes_kernel<T><<<grid, kWarpsPerBlock * 32, 0, stream>>>(w64, S, W, threshold, cuts, per_block, \
+                                                                                         flags, sizes, block_sums)
     if (W <= 32) BSI_EWAH_SIZES(1);
     else if (W <= 64) BSI_EWAH_SIZES(2);
     else if (W <= 128) BSI_EWAH_SIZES(4);
@@ -691,13 +747,10 @@ extern "C" int bsi_b200_ewah_encode(const uint64_t* words, int64_t S, int64_t W,
     else BSI_EWAH_SIZES(0);
 #undef BSI_EWAH_SIZES
     if (int rc = check_launch("ewah_encode sizes launch")) return rc;
-    BSI_CUDA_TRY(launch_dependent(ewah_block_offsets_kernel, 1u, 1024u, stream, static_cast<const u64*>(block_sums), nb,
-                                  block_off, reinterpret_cast<u64*>(total)));
-    if (int rc = check_launch("ewah_encode offsets launch")) return rc;
 #define BSI_EWAH_EMIT(T) BSI_CUDA_TRY(launch_dependent(ewah_emit_blocks_kernel<T>, grid, kWarpsPerBlock * 32u, stream, \
-        w64, S, W, static_cast<const int32_t*>(flags), static_cast<const u64*>(sizes),                                \
-        static_cast<const u64*>(block_off), static_cast<u64>(capacity), reinterpret_cast<u64*>(off),                  \
-        reinterpret_cast<u64*>(out), out_len))
+        w64, S, W, per_block, static_cast<const int32_t*>(flags), static_cast<const u64*>(sizes),                      \
+        static_cast<const u64*>(block_sums), static_cast<u64>(capacity), reinterpret_cast<u64*>(off),                  \
+        reinterpret_cast<u64*>(out), out_len, reinterpret_cast<u64*>(total)))
     if (W <= 32) BSI_EWAH_EMIT(1);
     else if (W <= 64) BSI_EWAH_EMIT(2);
     else if (W <= 128) BSI_EWAH_EMIT(4);
