@@ -58,10 +58,10 @@ __device__ __forceinline__ u64 transpose8x8(u64 x) {
 // stay inside a half, the third swaps the high nibbles of lo with the low nibbles of hi.
 __device__ __forceinline__ void transpose8x8_halves(uint32_t& lo, uint32_t& hi) {
     uint32_t t;
-    t = (lo ^ (lo >> 7)) & 0x00AA00AAu;  lo = lo ^ t ^ (t << 7);
-    t = (hi ^ (hi >> 7)) & 0x00AA00AAu;  hi = hi ^ t ^ (t << 7);
-    t = (lo ^ (lo >> 14)) & 0x0000CCCCu; lo = lo ^ t ^ (t << 14);
-    t = (hi ^ (hi >> 14)) & 0x0000CCCCu; hi = hi ^ t ^ (t << 14);
+    t = (lo ^ (lo >> 7)) & 0x00AA00AAu;  lo ^= t * 0x81u;       // t ^ (t << 7) on the multiplier: the logic pipe is the
+    t = (hi ^ (hi >> 7)) & 0x00AA00AAu;  hi ^= t * 0x81u;       // one these kernels fill
+    t = (lo ^ (lo >> 14)) & 0x0000CCCCu; lo ^= t * 0x4001u;
+    t = (hi ^ (hi >> 14)) & 0x0000CCCCu; hi ^= t * 0x4001u;
     t = (lo ^ (hi << 4)) & 0xF0F0F0F0u;
     lo ^= t;
     hi ^= t >> 4;
@@ -729,6 +729,7 @@ __global__ void __launch_bounds__(256, CPW * RawLane<T>::kVecs <= 2 ? 4 : (CPW *
     const float mult = static_cast<float>(dec_mult);
     int shift = fast_group_shift(RawLane<T>::abs_value(amax_bits), mult, bits);
     const bool fast = shift >= 0;
+    const bool clamp = fast && needs_clamp(RawLane<T>::abs_value(amax_bits), mult, shift, bits);
     if (!fast) shift = generic_row_shift<T>(xr, chunks, D, dec_scale, dec_mult, bits, vec_ok, lane);
 
     int asum = 0, amax_chunk = 0, qsum = 0;
@@ -738,7 +739,7 @@ __global__ void __launch_bounds__(256, CPW * RawLane<T>::kVecs <= 2 ? 4 : (CPW *
         if (row_ok && chunk < chunks) {
             u64 packed;
             if (fast) {
-                packed = raw[i].quantise(mult, shift, bits);
+                packed = clamp ? raw[i].template quantise<true>(mult, shift, bits) : raw[i].template quantise<false>(mult, shift, bits);
             } else {
                 packed = generic_row_chunk<T>(xr, chunk, D, dec_scale, dec_mult, bits, vec_ok, lane, shift);
             }

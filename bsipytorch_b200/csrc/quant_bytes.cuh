@@ -15,24 +15,26 @@ __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
 }
 
 // u0..u3 carry the unsigned quantised magnitudes of four elements in their low bytes (0 .. 2^(bits-1)), m is 0xff in
-// the bytes of the negative ones. Clamps positives to 2^(bits-1)-1, negates the negatives and returns the four
-// two's-complement bytes.
+// the bytes of the negative ones. Clamps positives to 2^(bits-1)-1 (kClamp: some may be beyond), negates the negatives
+// and returns the four two's-complement bytes.
+template <bool kClamp>
 __device__ __forceinline__ uint32_t mask_clamp4(uint32_t u0, uint32_t u1, uint32_t u2, uint32_t u3, uint32_t m, int bits) {
-    const uint32_t top = 0x01010101u << (bits - 1);
     uint32_t w = __byte_perm(__byte_perm(u0, u1, 0x0040), __byte_perm(u2, u3, 0x0040), 0x5410);   // the low bytes
-    // positive 2^(bits-1) -> 2^(bits-1) - 1 (the byte is exactly `top` there, so the borrow stays inside it)
-    const uint32_t over = w & ~m & top;
-    w -= over >> (bits - 1);
-    // negate the bytes under m: (~b + 1) per byte, the carry kept inside the byte by adding in 7 bits
-    const uint32_t x = w ^ m;
-    const uint32_t t = (x & 0x7f7f7f7fu) + (m & 0x01010101u);
-    return t ^ (x & 0x80808080u);
+    if (kClamp) {
+        // positive 2^(bits-1) -> 2^(bits-1) - 1 (the byte is exactly `top` there, so the borrow stays inside it)
+        const uint32_t over = w & ~m & (0x01010101u << (bits - 1));
+        w -= over >> (bits - 1);
+    }
+    // negate the bytes under m: (~b + 1) per byte, the carry kept inside the byte by adding in 7 bits. Without a
+    // magnitude of 128 the top bit of w ^ m is m's.
+    const uint32_t t = ((w ^ m) & 0x7f7f7f7fu) + (m & 0x01010101u);
+    return kClamp ? t ^ ((w ^ m) & 0x80808080u) : t ^ (m & 0x80808080u);
 }
 
 // The same with the signs in bit 31 of s0..s3 (e.g. the float bit patterns).
 __device__ __forceinline__ uint32_t sign_clamp4(uint32_t u0, uint32_t u1, uint32_t u2, uint32_t u3, uint32_t s0,
                                                 uint32_t s1, uint32_t s2, uint32_t s3, int bits) {
-    return mask_clamp4(u0, u1, u2, u3, prmt(prmt(s0, s1, 0x00fbu), prmt(s2, s3, 0x00fbu), 0x5410u), bits);
+    return mask_clamp4<true>(u0, u1, u2, u3, prmt(prmt(s0, s1, 0x00fbu), prmt(s2, s3, 0x00fbu), 0x5410u), bits);
 }
 
 // The reference's two roundings, |v| = floor(|x| * 10^dp + 0.5) and (|v| + [shift > 0] * 2^(shift-1)) >> shift, as two
@@ -55,6 +57,13 @@ __device__ __forceinline__ int fast_shift(float amax, float mult, int bits) {
 __device__ __forceinline__ void fast_round_consts(int shift, float& inv, float& c) {
     inv = __uint_as_float(static_cast<uint32_t>(127 - shift) << 23);   // 2^-shift
     c = (8388608.0f - 4194304.0f * inv) + (shift > 0 ? 0.5f : 0.0f);   // both steps exact
+}
+
+// Whether a group with largest magnitude amax holds values beyond the clamp, i.e. amax itself rounds to 2^(bits-1).
+__device__ __forceinline__ bool needs_clamp(float amax, float mult, int shift, int bits) {
+    float inv, c;
+    fast_round_consts(shift, inv, c);
+    return (__float_as_uint(__fmaf_rz(fast_round1(amax, mult), inv, c)) & 0xffu) >> (bits - 1) != 0u;
 }
 
 // Quantised magnitude of x in the low mantissa byte of the result.

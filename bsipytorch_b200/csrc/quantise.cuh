@@ -176,6 +176,8 @@ struct RawLane {
         else return __uint_as_float(bits << 16);
     }
     // The 8 values quantised with the group's shift, one byte each.
+    // kClamp = false where the group needs none (needs_clamp).
+    template <bool kClamp = true>
     __device__ __forceinline__ u64 quantise(float mult, int shift, int bits) const {
         float inv, c;
         fast_round_consts(shift, inv, c);
@@ -184,7 +186,7 @@ struct RawLane {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const uint32_t p = h == 0 ? v[0].x : v[0].z, q = h == 0 ? v[0].y : v[0].w;
-                w[h] = mask_clamp4(mag(p, 0, mult, inv, c), mag(p, 1, mult, inv, c), mag(q, 0, mult, inv, c),
+                w[h] = mask_clamp4<kClamp>(mag(p, 0, mult, inv, c), mag(p, 1, mult, inv, c), mag(q, 0, mult, inv, c),
                                    mag(q, 1, mult, inv, c), prmt(p, q, 0xfdb9u), bits);
             }
             return static_cast<u64>(w[0]) | (static_cast<u64>(w[1]) << 32);
@@ -193,9 +195,9 @@ struct RawLane {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const uint4& a = v[h == 0 ? 0 : kVecs - 1];
-                w[h] = sign_clamp4(fast_magnitude(__uint_as_float(a.x), mult, inv, c), fast_magnitude(__uint_as_float(a.y), mult, inv, c),
-                                   fast_magnitude(__uint_as_float(a.z), mult, inv, c), fast_magnitude(__uint_as_float(a.w), mult, inv, c),
-                                   a.x, a.y, a.z, a.w, bits);
+                w[h] = mask_clamp4<kClamp>(fast_magnitude(__uint_as_float(a.x), mult, inv, c), fast_magnitude(__uint_as_float(a.y), mult, inv, c),
+                                           fast_magnitude(__uint_as_float(a.z), mult, inv, c), fast_magnitude(__uint_as_float(a.w), mult, inv, c),
+                                           prmt(prmt(a.x, a.y, 0x00fbu), prmt(a.z, a.w, 0x00fbu), 0x5410u), bits);
             }
             return static_cast<u64>(w[0]) | (static_cast<u64>(w[1]) << 32);
         }
@@ -220,9 +222,12 @@ __device__ __forceinline__ int fast_group_shift(float amax, float mult, int bits
 // One chunk per warp: false when it needs the generic path. Same integers as that path, far fewer instructions.
 template <typename T>
 __device__ __forceinline__ bool fast_quantise(const RawLane<T>& r, float mult, int bits, int& shift, u64& packed) {
-    shift = fast_group_shift(RawLane<T>::abs_value(__reduce_max_sync(0xffffffffu, r.abs_max())), mult, bits);
+    const float amax = RawLane<T>::abs_value(__reduce_max_sync(0xffffffffu, r.abs_max()));
+    shift = fast_group_shift(amax, mult, bits);
     if (shift < 0) return false;
-    packed = r.quantise(mult, shift, bits);
+    // one group in a hundred or so has a value at the clamp: the others skip its steps
+    if (needs_clamp(amax, mult, shift, bits)) packed = r.template quantise<true>(mult, shift, bits);
+    else packed = r.template quantise<false>(mult, shift, bits);
     return true;
 }
 
