@@ -647,15 +647,15 @@ __global__ void __launch_bounds__(256) quantize_pack_row_kernel(
     }
 }
 
-// What a dot's exactness test needs of one 256-element chunk of keys: sum of |k| and sum of k^2 over the warp's bytes.
-__device__ __forceinline__ void chunk_sums(u64 packed, int& abs_sum, int& sq_sum) {
+// What a dot's exactness test needs of one 256-element chunk of keys: the sum of |k| over the warp's bytes; the lane's
+// part of the sum of k^2 is added to lane_sq.
+__device__ __forceinline__ void chunk_sums(u64 packed, int& abs_sum, int& lane_sq) {
     const uint32_t lo = static_cast<uint32_t>(packed), hi = static_cast<uint32_t>(packed >> 32);
     // +-1 per byte by its sign: k * sign(k) = |k|
     const int slo = static_cast<int>(prmt(lo, lo, 0xba98u) | 0x01010101u), shi = static_cast<int>(prmt(hi, hi, 0xba98u) | 0x01010101u);
     const int a = __dp4a(static_cast<int>(hi), shi, __dp4a(static_cast<int>(lo), slo, 0));
-    const int q = __dp4a(static_cast<int>(hi), static_cast<int>(hi), __dp4a(static_cast<int>(lo), static_cast<int>(lo), 0));
+    lane_sq = __dp4a(static_cast<int>(hi), static_cast<int>(hi), __dp4a(static_cast<int>(lo), static_cast<int>(lo), lane_sq));
     abs_sum = __reduce_add_sync(0xffffffffu, a);
-    sq_sum = __reduce_add_sync(0xffffffffu, q);
 }
 
 // One chunk of a row on the 64-bit path with the row's shift; returns the lane's bytes.
@@ -695,7 +695,7 @@ __device__ __noinline__ int generic_row_shift(const T* xr, int64_t chunks, int64
 // Bound by HBM: 4 bytes in and 1 + bits / 8 out per element (float32). A row with NaN, inf or |x * 10^dp| beyond the
 // fast range is redone from memory on the 64-bit path, every warp finding the shift for itself.
 template <typename T, int CPW>
-__global__ void __launch_bounds__(256, CPW * RawLane<T>::kVecs <= 2 ? 4 : (CPW * RawLane<T>::kVecs <= 4 ? 3 : 2)) quantize_pack_row_fast_kernel(
+__global__ void __launch_bounds__(256, CPW * RawLane<T>::kVecs <= 4 ? 4 : 2) quantize_pack_row_fast_kernel(
     const T* __restrict__ x, int64_t rows, int64_t D, int64_t ldx, double dec_scale, uint32_t dec_mult, int bits,
     int chunks, int64_t W, int wpr_log2, u64* __restrict__ words, float* __restrict__ scales,
     int32_t* __restrict__ shifts, int8_t* __restrict__ q8, int64_t ld8, int vec_ok, float* __restrict__ slice_weights,
@@ -733,6 +733,12 @@ __global__ void __launch_bounds__(256, CPW * RawLane<T>::kVecs <= 2 ? 4 : (CPW *
     if (!fast) shift = generic_row_shift<T>(xr, chunks, D, dec_scale, dec_mult, bits, vec_ok, lane);
 
     int asum = 0, amax_chunk = 0, qsum = 0;
+    const int s0 = first_slice(lane);
+    int8_t* q8_out = q8 + row * ld8 + sub * 256 + lane * 8;
+    // half word (lane / 4) % 2 of the lane's word in slice s0, and in the slice after it
+    uint32_t* w_out = reinterpret_cast<uint32_t*>(words + (row * bits + s0) * W + sub * 4 + (lane >> 3)) + ((lane >> 2) & 1);
+    uint32_t* w_out1 = w_out + 2 * W;
+    const int words_left = static_cast<int>(W) - sub * 4 - (lane >> 3);      // the lane's word exists while this is positive
 #pragma unroll
     for (int i = 0; i < CPW; ++i) {
         const int chunk = sub + i * wpr;
@@ -743,28 +749,24 @@ __global__ void __launch_bounds__(256, CPW * RawLane<T>::kVecs <= 2 ? 4 : (CPW *
             } else {
                 packed = generic_row_chunk<T>(xr, chunk, D, dec_scale, dec_mult, bits, vec_ok, lane, shift);
             }
-            if (q8 != nullptr) *reinterpret_cast<u64*>(q8 + row * ld8 + chunk * 256 + lane * 8) = packed;
+            if (q8 != nullptr) *reinterpret_cast<u64*>(q8_out + i * wpr * 256) = packed;
             if (words != nullptr) {
                 uint32_t w0, w1;
                 slice_pieces(packed, lane, w0, w1);
-                const int64_t word = static_cast<int64_t>(chunk) * 4 + (lane >> 3);
-                if (word < W) {
-                    const int s0 = first_slice(lane);
-                    // half word (lane / 4) % 2 of the lane's word in slice s0
-                    uint32_t* dst = reinterpret_cast<uint32_t*>(words + (row * bits + s0) * W + word) + ((lane >> 2) & 1);
-                    if (s0 < bits) *dst = w0;
-                    if (s0 + 1 < bits) dst[2 * W] = w1;
+                if (words_left > i * wpr * 4) {
+                    if (s0 < bits) w_out[i * wpr * 8] = w0;
+                    if (s0 + 1 < bits) w_out1[i * wpr * 8] = w1;
                 }
             }
             if (bounds != nullptr) {
-                int a, q;
-                chunk_sums(packed, a, q);
+                int a;
+                chunk_sums(packed, a, qsum);
                 asum += a;
-                qsum += q;
                 amax_chunk = max(amax_chunk, a);
             }
         }
     }
+    if (bounds != nullptr) qsum = __reduce_add_sync(0xffffffffu, qsum);
     const float scale = static_cast<float>(1ull << shift);
     if (row_ok && sub == 0) {
         if (lane == 0) {
@@ -804,10 +806,10 @@ __global__ void __launch_bounds__(256) key_bounds_kernel(const int8_t* __restric
     int amax_chunk = 0;
 #pragma unroll 4
     for (int64_t c = 0; c < chunks; ++c) {
-        int a, q;
+        int a, q = 0;
         chunk_sums(__ldg(src + c * 32), a, q);
         asum += a;
-        qsum += q;
+        qsum += __reduce_add_sync(0xffffffffu, q);
         amax_chunk = max(amax_chunk, a);
     }
     if (lane == 0) {
