@@ -464,12 +464,12 @@ int launch_tile(const CUtensorMap& ma, const CUtensorMap& mb, const float* qs, i
     return check_launch("dot_i8 tcgen05 launch");
 }
 
-template <int BN, bool DBG, typename OutT, bool REQ = false>
+template <int BN, bool DBG, typename OutT, bool REQ = false, int SPLIT = 1>
 int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo, const CUtensorMap& mt, int vector_store,
                 const float* qs, int64_t qs_stride, const float* bw0, const float* bias, int Q, int R, int chunks,
                 float scale_inv, void* out, int64_t ldo, int32_t* dbg, const ScatterDst& scatter,
                 const RequantDst& requant, const float* k_abs_sum, float q_abs_max, const float* q_sq, int64_t q_sq_stride,
-                cudaStream_t stream) {
+                cudaStream_t stream, int* max_clusters_out = nullptr /* only asks how many clusters fit at once */) {
     using C = pair::Cfg<BN, OutT, REQ>;
     static int max_clusters[64] = {0};   // per instantiation
     int dev = 0;
@@ -480,7 +480,7 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap&
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.x = 2 * SPLIT;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     // programmatic dependent launch: this kernel's set-up may overlap the tail of the kernel before it
@@ -494,16 +494,20 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap&
     int resident = 0;
     if (dev >= 0 && dev < 64) resident = max_clusters[dev];
     if (resident == 0) {
-        BSI_CUDA_TRY(cudaFuncSetAttribute(pair::dot_i8_tcgen05_pair_kernel<BN, DBG, OutT, REQ>,
+        BSI_CUDA_TRY(cudaFuncSetAttribute(pair::dot_i8_tcgen05_pair_kernel<BN, DBG, OutT, REQ, SPLIT>,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
-        cfg.gridDim = dim3(2 * (sm_count() / 2), 1, 1);
-        BSI_CUDA_TRY(cudaOccupancyMaxActiveClusters(&resident, pair::dot_i8_tcgen05_pair_kernel<BN, DBG, OutT, REQ>, &cfg));
+        cfg.gridDim = dim3(2 * SPLIT * (sm_count() / (2 * SPLIT)), 1, 1);
+        BSI_CUDA_TRY(cudaOccupancyMaxActiveClusters(&resident, pair::dot_i8_tcgen05_pair_kernel<BN, DBG, OutT, REQ, SPLIT>, &cfg));
         if (resident <= 0) return fail(BSI_ERR_CUDA, "dot_i8: no cluster of 2 CTAs fits on this device");
         if (dev >= 0 && dev < 64) max_clusters[dev] = resident;
     }
-    int pairs = tiles_total < resident ? tiles_total : resident;
-    cfg.gridDim = dim3(2 * pairs, 1, 1);
-    BSI_CUDA_TRY(cudaLaunchKernelEx(&cfg, pair::dot_i8_tcgen05_pair_kernel<BN, DBG, OutT, REQ>, ma, mb, mo, mt, vector_store, qs,
+    if (max_clusters_out != nullptr) {
+        *max_clusters_out = resident;
+        return BSI_OK;
+    }
+    const int clusters = SPLIT > 1 || tiles_total < resident ? tiles_total : resident;
+    cfg.gridDim = dim3(2 * SPLIT * clusters, 1, 1);
+    BSI_CUDA_TRY(cudaLaunchKernelEx(&cfg, pair::dot_i8_tcgen05_pair_kernel<BN, DBG, OutT, REQ, SPLIT>, ma, mb, mo, mt, vector_store, qs,
                                     qs_stride, bw0, bias, Q, R, chunks, tiles_m, tiles_total, scale_inv, out, ldo, dbg, scatter, requant,
                                     k_abs_sum, q_abs_max, q_sq, q_sq_stride));
     return check_launch("dot_i8 tcgen05 pair launch");
@@ -532,24 +536,47 @@ int pick_bn_pair(int64_t Q, int64_t R, bool any_width) {
     return best;
 }
 
-// Picks the key-tile width: the widest tile wins unless a narrower one fills more SMs.
-int pick_bn(int64_t Q, int64_t R) {
-    const int sms = sm_count();
-    const int64_t mt = (Q + BM - 1) / BM;
-    const int cand[3] = {256, 128, 64};
-    const double eff[3] = {1.0, 0.9, 0.67};  // narrower tiles re-read A more often per MMA
-    int best = 256;
-    double best_cost = 1e300;
-    for (int i = 0; i < 3; ++i) {
-        const int64_t tiles = mt * ((R + cand[i] - 1) / cand[i]);
-        const int64_t waves = (tiles + sms - 1) / sms;
-        const double cost = static_cast<double>(waves) * cand[i] / eff[i];
-        if (cost < best_cost * 0.999) {
-            best_cost = cost;
-            best = cand[i];
+// How many clusters of 2 * SPLIT CTAs run at once (one CTA per SM whatever the tile width); 0 when the query fails.
+template <int SPLIT>
+int resident_clusters() {
+    static int cached[64] = {0};
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    if (cached[dev] == 0) {
+        const CUtensorMap none = {};
+        if (launch_pair<64, false, float, false, SPLIT>(none, none, none, none, 0, nullptr, 0, nullptr, nullptr, 0, 0, 1, 0.0f, nullptr, 0,
+                                                        nullptr, ScatterDst{}, RequantDst{}, nullptr, 0.0f, nullptr, 0, nullptr, &n) != BSI_OK)
+            n = 0;
+        cached[dev] = n > 0 ? n : -1;
+    }
+    return cached[dev] > 0 ? cached[dev] : 0;
+}
+
+// Split along K or not, and the tile width to split at: *bn and the number of parts, 1 for no split. A chunk of a tile
+// costs max(780, 420 + 3.85 bn) cycles (measured on 512 x 2048 x 8192 at widths 64 .. 256); filling the ring and storing
+// about 7000; the vote and the exchange of a split about 4500 more. A split takes one wave of clusters and has to save
+// an eighth.
+int pick_split(int64_t Q, int64_t R, int64_t chunks, int unsplit_bn, int* bn) {
+    auto per_chunk = [](int w) { const double c = 420.0 + 3.85 * w; return c > 780.0 ? c : 780.0; };
+    const int64_t mt = (Q + 255) / 256, pairs = sm_count() / 2;
+    const int64_t tiles = mt * ((R + unsplit_bn - 1) / unsplit_bn);
+    const int64_t waves = (tiles + pairs - 1) / pairs;
+    double best = 0.875 * (static_cast<double>(waves * chunks) * per_chunk(unsplit_bn) + 7000.0);
+    int parts = 1;
+    if (waves > 1) return 1;
+    for (int s = 2; s <= 4; s *= 2) {
+        const int64_t room = s == 2 ? resident_clusters<2>() : resident_clusters<4>();
+        for (int w = 256; w >= 64; w /= 2) {
+            if (mt * ((R + w - 1) / w) > room) continue;
+            const double cost = static_cast<double>((chunks + s - 1) / s) * per_chunk(w) + 11500.0;
+            if (cost < best) {
+                best = cost;
+                parts = s;
+                *bn = w;
+            }
         }
     }
-    return best;
+    return parts;
 }
 
 }  // namespace
@@ -593,6 +620,9 @@ int dot_i8_pair(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_strid
         const int64_t t256 = mt * ((R + 255) / 256), t224 = mt * ((R + 223) / 224);
         if (t256 <= pairs && t224 <= pairs && t224 > t256) bn = 224;
     }
+    // only with bounds (a split adds integers), one plain destination, and no accumulator dump
+    const bool may_split = !force_bn && kabs != nullptr && dbg_iacc == nullptr && scatter.n == 0;
+    const int parts = may_split ? pick_split(Q, R, chunks, bn, &bn) : 1;
     if (bn < 64 || bn > 256 || (bn & 31) != 0 || (!any_width && (bn & (bn - 1)) != 0))
         return fail(BSI_ERR_INVALID, "dot_i8: tile width must be a multiple of 32 in [64, 256] (64, 128 or 256 for 16-bit outputs)");
     if (dbg_iacc != nullptr && y_dtype != BSI_DTYPE_F32)
@@ -616,6 +646,19 @@ int dot_i8_pair(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_strid
         store_flags |= 4;
     }
     const int q = static_cast<int>(Q), r = static_cast<int>(R), c = static_cast<int>(chunks);
+    if (parts > 1) {
+#define BSI_SPLIT_T(BN_, S_, T_)                                                                                            \
+    launch_pair<BN_, false, T_, false, S_>(ma, mb, mo, mt, store_flags, qs, qs_stride, bw0, bias, q, r, c, scale_inv, out, ldo, \
+                                           nullptr, scatter, requant, kabs, qabs, qsq, qsq_stride, stream)
+#define BSI_SPLIT(BN_, S_)                                                    \
+    (y_dtype == BSI_DTYPE_F16    ? BSI_SPLIT_T(BN_, S_, __half)               \
+     : y_dtype == BSI_DTYPE_BF16 ? BSI_SPLIT_T(BN_, S_, __nv_bfloat16)        \
+                                 : BSI_SPLIT_T(BN_, S_, float))
+        if (parts == 2) return bn == 256 ? BSI_SPLIT(256, 2) : (bn == 128 ? BSI_SPLIT(128, 2) : BSI_SPLIT(64, 2));
+        return bn == 256 ? BSI_SPLIT(256, 4) : (bn == 128 ? BSI_SPLIT(128, 4) : BSI_SPLIT(64, 4));
+#undef BSI_SPLIT
+#undef BSI_SPLIT_T
+    }
 #define BSI_PAIR_T(BN_, DBG_, T_)                                                                              \
     launch_pair<BN_, DBG_, T_>(ma, mb, mo, mt, store_flags, qs, qs_stride, bw0, bias, q, r, c, scale_inv, out, ldo,  \
                                dbg_iacc, scatter, requant, kabs, qabs, qsq, qsq_stride, stream)
@@ -653,12 +696,12 @@ int dot_i8_tcgen05(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_st
     if (Q > 0x7fffff00ll || R > 0x7fffff00ll || chunks > 0x400000)
         return fail(BSI_ERR_UNSUPPORTED, "dot_i8: Q, R or chunks too large");
     // force_bn: 0 = automatic; 64/128/256 = single-CTA tiles; 2064/2128/2256 = paired-CTA tiles.
-    const bool want_pair = force_bn ? (force_bn >= 2000) : (Q > 128);
+    const bool want_pair = force_bn == 0 || force_bn >= 2000;
     if (want_pair) {
         return dot_i8_pair(a8, lda, qs, qs_stride, k8, ldk, bw0, nullptr, Q, R, chunks, scale_inv, out, ldo,
                            BSI_DTYPE_F32, dbg_iacc, force_bn ? force_bn - 2000 : 0, /*relu=*/0, nullptr, nullptr, bounds, stream);
     }
-    const int bn = force_bn ? force_bn : pick_bn(Q, R);
+    const int bn = force_bn;
     CUtensorMap ma, mb;
     if (int rc = make_map(&ma, a8, Q, chunks * 256, lda, BM)) return rc;
     if (int rc = make_map(&mb, k8, R, chunks * 256, ldk, bn)) return rc;

@@ -32,6 +32,12 @@
 // sub-partition, next to TMEM loads that slow down while the tensor pipe reads and writes its accumulators. What a tile
 // costs beyond its chunks, the bounds and the store phase, went from 20 to 6 thousand cycles with batched bound loads,
 // key scales and bias in shared memory and bulk stores: 4096 x 16384 x 4096, float16 out: 254 -> 189 us (2.9 POPS).
+// Split along K (SPLIT = 2 or 4): where the tiles leave most SMs idle, a cluster of SPLIT pairs shares one tile, each
+// with a part of the chunks. The chunk terms are integers, so where the bounds of the integer route hold for every warp
+// of the tile (the cluster votes before the first MMA) the parts add up in any order to the float32 chain's bits: every
+// warp sends its sums through distributed shared memory to the pair that owns the columns, which adds and stores them.
+// If a bound fails anywhere, pair 0 does the whole tile on its own with the chain in order, as an unsplit kernel would.
+// 512 x 2048 x 8192 (16 tiles of 256 x 256, 4 pairs each): 18.5 -> SPLIT_US us.
 // All waits are bounded; a timeout raises the abort flag of both CTAs and every role drains out.
 #pragma once
 
@@ -138,8 +144,7 @@ __device__ __forceinline__ void umma_i8_pair(uint32_t tmem_d, uint64_t adesc, ui
 }
 
 // Arrives on the barrier at this smem offset in BOTH CTAs of the pair once all earlier MMAs are done.
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
-    const uint16_t mask = 3;
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar, uint16_t mask) {   // mask: the pair's two CTAs of the cluster
     asm volatile(
         "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
         ::"r"(bar), "h"(mask)
@@ -248,7 +253,7 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t sr
 }
 __device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 
-template <int BN, bool DBG, typename OutT, bool REQ = false>
+template <int BN, bool DBG, typename OutT, bool REQ = false, int SPLIT = 1>
 __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
     const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
     const __grid_constant__ CUtensorMap map_o, const __grid_constant__ CUtensorMap map_t,   // out in boxes of 32 rows x 128 / 64 bytes
@@ -286,18 +291,26 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const uint32_t drain_bar = bar_base + 8u * (2 * kStages + 2 * kAccBufs + ((warp >> 1) & 1));   // one per issuer
-    const uint32_t rank = cluster_ctarank();
+    const uint32_t crank = cluster_ctarank();
+    const uint32_t rank = crank & 1u;                     // within the pair
+    const uint32_t lead = crank & ~1u;                    // the pair's leader CTA
+    const int part = static_cast<int>(crank >> 1);        // of the chunks (SPLIT > 1)
+    const uint16_t pair_mask = static_cast<uint16_t>(3u << lead);
     const bool leader = rank == 0;
-    const int pair_id = blockIdx.x >> 1;
-    const int num_pairs = gridDim.x >> 1;
-    const int num_kb = chunks * 2;
+    const int pair_id = static_cast<int>(blockIdx.x) / (2 * SPLIT);
+    const int num_pairs = static_cast<int>(gridDim.x) / (2 * SPLIT);     // split: one tile per cluster
+    const int per_part = (chunks + SPLIT - 1) / SPLIT;
+    const int c_lo = SPLIT > 1 ? min(part * per_part, chunks) : 0;
+    const int my_chunks = SPLIT > 1 ? min(c_lo + per_part, chunks) - c_lo : chunks;
+    int num_kb = my_chunks * 2;
+    volatile int* vote = reinterpret_cast<volatile int*>(tmem_slot + 2);   // some warp of the cluster has no bound
     const bool has_bias = bias != nullptr;
     const bool relu = (store_flags & 2) != 0;
 
-    const uint32_t leader_full0 = map_to_cta(full_bar(0), 0);
+    const uint32_t leader_full0 = map_to_cta(full_bar(0), lead);
     AbortCtx actx;
     actx.flag = abort_flag;
-    actx.peer_flag = map_to_cta(smem_u32(const_cast<int*>(abort_flag)), rank ^ 1u);
+    actx.peer_flag = map_to_cta(smem_u32(const_cast<int*>(abort_flag)), crank ^ 1u);
 
     if (warp == 0) {
         // one barrier per lane: full[s], empty[s], tfull[b] and drain count 1 arrival, tempty[b] one per epilogue
@@ -306,6 +319,7 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
             asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
             asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
             *abort_flag = 0;
+            *vote = 0;
         }
         if (REQ && lane < kEpiWarps) xchg_count[lane] = 0u;
         for (int i = lane; i < C::kBarriers; i += 32) {
@@ -346,32 +360,45 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
 
     if (warp < kFirstEpiWarp) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsLow));
-        if (is_producer && lane == 0) {
+        if (is_producer) {
             // ---------------- TMA producers ----------------
             // One thread needs ~450 cycles per k-block (empty wait, expect_tx, two tensor copies), which
             // is slower than the MMAs consume narrow tiles; warps 0 and 2 therefore take the k-blocks
             // in turn. Stage s = it % kStages is always filled by the producer that owns `it`.
             constexpr int kProducers = 2;
             const int me = warp >> 1;
-            int it = 0;
             bool ok = true;
-            for (int tile = pair_id; tile < tiles_total && ok; tile += num_pairs) {
-                const int tm = tile % tiles_m;
-                const int tn = tile / tiles_m;
-                const int row_a = tm * 256 + static_cast<int>(rank) * BM;
-                const int row_b = tn * BN + static_cast<int>(rank) * C::kHalfN;
-                for (int kb = 0; kb < num_kb; ++kb, ++it) {
-                    if (it % kProducers != me) continue;
-                    const int s = it % kStages;
-                    const uint32_t ph = static_cast<uint32_t>(it / kStages) & 1u;
-                    if (!wait_or_abort(empty_bar(s), ph ^ 1u, actx, 1)) { ok = false; break; }
-                    if (leader) mbar_expect_tx(full_bar(s), 2u * C::kStageBytes);
-                    const uint32_t a_dst = smem_base + s * C::kStageBytes;
-                    tma_load_2d_pair(a_dst, &map_a, kb * BK, row_a, leader_full0 + 8u * s);
-                    tma_load_2d_pair(a_dst + C::kABytes, &map_b, kb * BK, row_b, leader_full0 + 8u * s);
-                }
+            auto load = [&](int it, int kb, int tm, int tn) {
+                const int s = it % kStages;
+                const uint32_t ph = static_cast<uint32_t>(it / kStages) & 1u;
+                if (!wait_or_abort(empty_bar(s), ph ^ 1u, actx, 1)) return false;
+                if (leader) mbar_expect_tx(full_bar(s), 2u * C::kStageBytes);
+                const uint32_t a_dst = smem_base + s * C::kStageBytes;
+                tma_load_2d_pair(a_dst, &map_a, (c_lo * 2 + kb) * BK, tm * 256 + static_cast<int>(rank) * BM, leader_full0 + 8u * s);
+                tma_load_2d_pair(a_dst + C::kABytes, &map_b, (c_lo * 2 + kb) * BK, tn * BN + static_cast<int>(rank) * C::kHalfN,
+                                 leader_full0 + 8u * s);
+                return true;
+            };
+            int done = 0;
+            if constexpr (SPLIT > 1) {
+                // the first ring round goes out before the vote: it is the part's own beginning either way
+                done = min(kStages, num_kb);
+                if (lane == 0)
+                    for (int it = me; it < done && ok; it += kProducers) ok = load(it, it, pair_id % tiles_m, pair_id / tiles_m);
+                __syncwarp();
+                cluster_sync_all();
+                if (*vote) num_kb = part == 0 ? 2 * chunks : done;
             }
-        } else if (!is_producer && leader) {
+            if (lane == 0) {
+                int it = 0;
+                for (int tile = pair_id; tile < tiles_total && ok; tile += num_pairs)
+                    for (int kb = 0; kb < num_kb && ok; ++kb, ++it)
+                        if (it >= done && it % kProducers == me) ok = load(it, kb, tile % tiles_m, tile / tiles_m);
+            }
+            __syncwarp();
+        } else {
+            if constexpr (SPLIT > 1) cluster_sync_all();
+            if (leader) {
             // ---------------- MMA issuers (leader CTA) ----------------
             // The whole warp walks the loop (so that addresses and descriptors stay in the uniform
             // datapath) and one elected lane issues the tensor-core instructions. A chunk costs an issuer about 770
@@ -379,7 +406,16 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
             // take, so warps 1 and 3 issue alternate chunks; they share nothing but the order of the rings.
             constexpr uint32_t idesc = umma_idesc_pair(BN);
             const int mi = warp >> 1;
-            const int total = ((tiles_total - pair_id + num_pairs - 1) / num_pairs) * chunks;
+            int total = ((tiles_total - pair_id + num_pairs - 1) / num_pairs) * my_chunks;
+            if constexpr (SPLIT > 1) {
+                if (*vote) {
+                    total = part == 0 ? chunks : 0;
+                    // this part's copies are in flight for nothing: they have to land before the CTAs go
+                    if (part != 0 && mi == 0)
+                        for (int st = 0; st < min(kStages, num_kb); ++st)
+                            if (!wait_or_abort(full_bar(st), 0, actx, 2)) break;
+                }
+            }
             int s = 2 * mi;
             uint32_t ph = 0;
             bool ok = true;
@@ -401,8 +437,8 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                             umma_i8_pair(tmem_d, adesc + 2u * k, bdesc + 2u * k, idesc,
                                          (half | k) != 0 ? 1u : 0u);
                         }
-                        umma_commit_pair(empty_bar(s));
-                        if (half == 1) umma_commit_pair(tfull_bar(b));
+                        umma_commit_pair(empty_bar(s), pair_mask);
+                        if (half == 1) umma_commit_pair(tfull_bar(b), pair_mask);
                     }
                     __syncwarp();
                     if (++s == kStages) { s = 0; ph ^= 1u; }
@@ -415,6 +451,12 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                 const long long t0 = clock64();
                 while (!mbar_try(drain_bar, 0) && clock64() - t0 < kWait / 64) {}
             }
+            __syncwarp();
+            }
+        }
+        if constexpr (SPLIT > 1) {      // the two barriers around the exchange of sums
+            cluster_sync_all();
+            cluster_sync_all();
         }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsHigh));
@@ -424,7 +466,7 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
         const int half = ew >> 2;              // which half of the BN columns
         const int col0 = half * kCols;
         uint8_t* my_store = store_area + ew * 4096;
-        const uint32_t leader_tempty0 = map_to_cta(tempty_bar(0), 0);
+        const uint32_t leader_tempty0 = map_to_cta(tempty_bar(0), lead);
 
         float acc[kCols];
         int cc = 0;
@@ -520,8 +562,13 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                         }
                     }
                 }
-                // non-negative floats order like their bit patterns; an infinity anywhere fails the test
-                auto most = [](float v) { return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v))); };
+                // an infinity anywhere fails the test. By shuffles: as redux.sync the maximum left out some lanes in the split
+                // instantiations (nvcc 12.9), which a row that breaks the bounds on lane 22 showed.
+                auto most = [](float v) {
+#pragma unroll
+                    for (int d = 16; d > 0; d >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, d));
+                    return v;
+                };
                 const float su = most(smax), tu = most(ssum), ku = most(ktot), cu = most(kchk);
                 // the sums above round (relative 2^-24 per addition, at most a few thousand additions): 0.999 covers it
                 const float first = fminf(su * ku, tu * cu) * q_abs_max;
@@ -530,14 +577,26 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                 small = first < 4194304.0f * 0.999f || norm < 17592186044416.0f * 0.999f;        // 2^22, 2^44
             }
 
+            int n_chunks = my_chunks;
+            bool whole_tile = SPLIT == 1;      // this pair does all chunks and stores all columns
+            if constexpr (SPLIT > 1) {
+                if (!exact && lane < 2 * SPLIT)
+                    store_flag_cluster(map_to_cta(smem_u32(const_cast<int*>(vote)), static_cast<uint32_t>(lane)), 1);
+                __syncwarp();
+                cluster_sync_all();
+                if (*vote) {
+                    whole_tile = part == 0;
+                    n_chunks = part == 0 ? chunks : 0;
+                }
+            }
             // the chunk scale of the next chunk is loaded a whole chunk ahead: a scattered load per lane (32 rows) that
             // would otherwise stand in front of every fold
-            float qnext = __ldg(qs_row);
-            for (int c = 0; c < chunks && ok; ++c, ++cc) {
+            float qnext = qs_stride ? __ldg(qs_row + min(c_lo, chunks - 1)) : __ldg(qs_row);
+            for (int c = 0; c < n_chunks && ok; ++c, ++cc) {
                 const int b = cc % kAccBufs;
                 const uint32_t tph = static_cast<uint32_t>(cc / kAccBufs) & 1u;
                 const float qscale = qnext;
-                if (qs_stride && c + 1 < chunks) qnext = __ldg(qs_row + c + 1);
+                if (qs_stride && c + 1 < n_chunks) qnext = __ldg(qs_row + c_lo + c + 1);
                 const int qmul = exact ? __float2int_rn(qscale) : 0;
                 if (!wait_or_abort(tfull_bar(b), tph, actx, 4)) { ok = false; break; }
                 tc_fence_after();
@@ -597,6 +656,76 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                         }
                     }
                 }
+            }
+            if constexpr (SPLIT > 1) {
+                constexpr int kShare = kCols / SPLIT;        // columns of this warp that each pair stores
+                constexpr int kWide = kShare < 32 ? kShare : 32;
+                const bool add_up = *vote == 0;
+                __syncwarp();
+                cluster_sync_all();          // the operand rings of all CTAs are free
+                // [warp][source][4 columns][lane]: 512 bytes per 4 columns, written and read without bank conflicts
+                const uint32_t slots = smem_base + static_cast<uint32_t>(ew * (SPLIT - 1) * kShare * 128 + lane * 16);
+                if (add_up && ok) {
+#pragma unroll
+                    for (int q = 0; q < SPLIT; ++q) {
+                        if (q != part) {
+                            const uint32_t dst = map_to_cta(slots, static_cast<uint32_t>(2 * q) + rank) +
+                                                 static_cast<uint32_t>((part < q ? part : part - 1) * kShare * 128);
+#pragma unroll
+                            for (int j = 0; j < kShare; j += 4)
+                                asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};"
+                                             ::"r"(dst + j * 128), "r"(__float_as_int(acc[q * kShare + j])), "r"(__float_as_int(acc[q * kShare + j + 1])),
+                                               "r"(__float_as_int(acc[q * kShare + j + 2])), "r"(__float_as_int(acc[q * kShare + j + 3])) : "memory");
+                        }
+                    }
+                }
+                cluster_sync_all();          // every part's sums have arrived
+                if (add_up) {
+                    if (!ok) continue;
+                    int sum[kShare];
+#pragma unroll
+                    for (int q = 0; q < SPLIT; ++q) {
+                        if (q == part) {
+#pragma unroll
+                            for (int j = 0; j < kShare; ++j) sum[j] = __float_as_int(acc[q * kShare + j]);
+                        }
+                    }
+#pragma unroll
+                    for (int q = 0; q < SPLIT - 1; ++q) {
+#pragma unroll
+                        for (int j = 0; j < kShare; j += 4) {
+                            const int4 v = *reinterpret_cast<const int4*>(smem + ew * (SPLIT - 1) * kShare * 128 + lane * 16 + (q * kShare + j) * 128);
+                            sum[j] += v.x; sum[j + 1] += v.y; sum[j + 2] += v.z; sum[j + 3] += v.w;
+                        }
+                    }
+                    if (lane == 0) atomicAdd(&g_exact_int_tiles, 1ull);
+                    // blocks of 32 rows x kWide columns through the warp's 4 KB, then stores of kWide adjacent columns
+                    float* stage = reinterpret_cast<float*>(my_store);
+                    OutT* o = static_cast<OutT*>(out);
+                    const int first_row = tm * 256 + static_cast<int>(rank) * BM + quad * 32;
+                    const int cj = lane & (kWide - 1);
+#pragma unroll
+                    for (int g = 0; g < kShare / kWide; ++g) {
+                        const int col = n0 + col0 + part * kShare + g * kWide + cj;
+                        const float w = col < R ? __ldg(bw0 + col) : 0.0f;
+                        const float bv = col < R && has_bias ? __ldg(bias + col) : 0.0f;
+#pragma unroll
+                        for (int j = 0; j < kWide; ++j)
+                            stage[lane * kWide + (j ^ (lane & (kWide - 1)))] = small ? int_to_float_exact(sum[g * kWide + j]) : static_cast<float>(sum[g * kWide + j]);
+                        __syncwarp();
+#pragma unroll 8
+                        for (int i = 0; i < kWide; ++i) {
+                            const int rr = i * (32 / kWide) + lane / kWide;
+                            const float v = stage[rr * kWide + (cj ^ (rr & (kWide - 1)))];
+                            if (first_row + rr < Q && col < R)
+                                o[static_cast<int64_t>(first_row + rr) * ldo + col] =
+                                    relu_if<OutT>(finish<OutT>((v * w) * scale_inv, bv, has_bias), relu);
+                        }
+                        __syncwarp();
+                    }
+                    continue;
+                }
+                if (!whole_tile) continue;
             }
             // the half's key scales and bias into shared memory: behind the first barrier nobody reads the last tile's
             asm volatile("bar.sync %0, 128;" ::"r"(2 + half) : "memory");

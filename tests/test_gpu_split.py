@@ -1,0 +1,56 @@
+"""Dots split along K over a cluster of CTA pairs: same bits as the float32 chain of the CUDA-core engine, with the bounds
+holding everywhere and with one row that breaks them (the cluster then falls back to one pair)."""
+import ctypes as C
+
+import pytest
+import torch
+
+import _capi_helpers as H
+import _inputs
+from bsipytorch_b200 import capi
+from oracle import oracle as o
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+class _Bounds(C.Structure):
+    _fields_ = [("key_bounds", C.c_void_p), ("query_sq", C.c_void_p), ("query_sq_stride", C.c_int64), ("query_abs_max", C.c_int)]
+
+
+# sizes whose widths and parts differ: 256 and 128 columns in 2 and 4 parts, 64 columns (a share of 8 or 16 columns per
+# warp); chunk counts that do not divide, a part without chunks; ragged rows and columns
+@pytest.mark.parametrize("broken", [False, True])
+@pytest.mark.parametrize("Q,R,D", [(512, 2048, 8192), (512, 2040, 4352), (300, 1111, 5000), (40, 500, 8192), (129, 64, 1280), (256, 1500, 2304),
+                                   (33, 65, 16384)])
+def test_split_dot_and_layer(Q, R, D, broken):
+    q, k = _inputs.fc1(Q=Q, R=R, D=D, seed=Q + R + D, dtype=torch.float32)
+    if broken:
+        q[Q // 2] *= 3.0e4
+    chunks, ld = (D + 255) // 256, (D + 255) // 256 * 256
+    kb = H.quantize_pack(k.to(DEV), 2, 6, False)
+    x = q.to(DEV)
+    q8 = torch.empty(Q, ld, dtype=torch.int8, device=DEV)
+    scales, norms = torch.empty(Q, chunks, device=DEV), torch.empty(Q, chunks, device=DEV)
+    bounds = torch.empty(3, R, device=DEV)
+    L = capi.lib()
+    capi.check(L.bsi_b200_quantize_pack_all(capi.ptr(x), capi.DTYPE_F32, Q, D, D, 2, 7, 1, C.c_float(0.0), None, capi.ptr(scales), None,
+                                            capi.ptr(q8), ld, capi.ptr(norms), None, None, capi.stream_ptr()))
+    capi.check(L.bsi_b200_key_bounds(capi.ptr(kb["q8"]), ld, R, chunks, capi.ptr(bounds), capi.stream_ptr()))
+    want = H.dot_i8(q8, scales, kb["q8"], kb["scales"], o.scale_inv(2), capi.ENGINE_SIMT)
+    given = _Bounds(bounds.data_ptr(), norms.data_ptr(), chunks, 64)
+    capi.exact_int_tiles()
+    out = torch.full((Q, R), float("nan"), device=DEV)
+    inv = C.c_float(float(o.scale_inv(2)))
+    capi.check(L.bsi_b200_dot_i8_bounded(capi.ptr(q8), ld, capi.ptr(scales), chunks, capi.ptr(kb["q8"]), ld, capi.ptr(kb["scales"]), Q, R,
+                                         chunks, inv, capi.ptr(out), R, None, 0, C.byref(given), capi.stream_ptr()))
+    assert torch.equal(out.view(torch.int32), want.view(torch.int32))
+    assert capi.exact_int_tiles() > 0 or broken
+    bias = torch.linspace(-1, 1, R, device=DEV)
+    for dtype in (torch.float16, torch.bfloat16):
+        y = torch.full((Q, R), float("nan"), dtype=dtype, device=DEV)
+        capi.check(L.bsi_b200_linear_i8_bounded(capi.ptr(q8), ld, capi.ptr(scales), chunks, capi.ptr(kb["q8"]), ld, capi.ptr(kb["scales"]),
+                                                capi.ptr(bias), Q, R, chunks, inv, capi.ptr(y), R, H._DT[dtype], 1, C.byref(given),
+                                                capi.stream_ptr()))
+        assert torch.equal(y, torch.relu(want.to(dtype) + bias.to(dtype)))
+    assert capi.device_status() == 0
