@@ -470,7 +470,7 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap&
                 float scale_inv, void* out, int64_t ldo, int32_t* dbg, const ScatterDst& scatter,
                 const RequantDst& requant, const float* k_abs_sum, float q_abs_max, const float* q_sq, int64_t q_sq_stride,
                 cudaStream_t stream, int* max_clusters_out = nullptr /* only asks how many clusters fit at once */) {
-    using C = pair::Cfg<BN, OutT, REQ>;
+    using C = pair::Cfg<BN, OutT, REQ, SPLIT>;
     static int max_clusters[64] = {0};   // per instantiation
     int dev = 0;
     BSI_CUDA_TRY(cudaGetDevice(&dev));
@@ -552,25 +552,26 @@ int resident_clusters() {
     return cached[dev] > 0 ? cached[dev] : 0;
 }
 
-// Split along K or not, and the tile width to split at: *bn and the number of parts, 1 for no split. A chunk of a tile
-// costs max(780, 420 + 3.85 bn) cycles (measured on 512 x 2048 x 8192 at widths 64 .. 256); filling the ring and storing
-// about 7000; the vote and the exchange of a split about 4500 more. A split takes one wave of clusters and has to save
-// an eighth.
+// Split along K or not, and the tile width to split at: *bn and the number of parts, 1 for no split. The costs are cycles
+// fitted to runs of 2 .. 64 chunks at widths 64, 128 and 256: 820 + 1.3 bn per chunk, and beside the chunks 7000 + 25 bn
+// without a split, 7500 + 55 bn with two parts, 12000 + 47 bn with four (clusters of eight start later). A split takes one
+// wave of clusters (33 of four CTAs and 15 of eight fit) and has to save a fifteenth.
 int pick_split(int64_t Q, int64_t R, int64_t chunks, int unsplit_bn, int* bn) {
-    auto per_chunk = [](int w) { const double c = 420.0 + 3.85 * w; return c > 780.0 ? c : 780.0; };
     const int64_t mt = (Q + 255) / 256, pairs = sm_count() / 2;
-    const int64_t tiles = mt * ((R + unsplit_bn - 1) / unsplit_bn);
-    const int64_t waves = (tiles + pairs - 1) / pairs;
-    double best = 0.875 * (static_cast<double>(waves * chunks) * per_chunk(unsplit_bn) + 7000.0);
+    if (mt * ((R + unsplit_bn - 1) / unsplit_bn) > pairs) return 1;
+    auto cost = [&](int w, double fixed, double per_column, int64_t parts) {
+        return fixed + per_column * w + static_cast<double>((chunks + parts - 1) / parts) * (820.0 + 1.3 * w);
+    };
+    double best = 0.93 * cost(unsplit_bn, 7000.0, 25.0, 1);
     int parts = 1;
-    if (waves > 1) return 1;
+    if (cost(64, 7500.0, 55.0, 4) >= best) return 1;       // not even the cheapest one: no need to ask the driver
     for (int s = 2; s <= 4; s *= 2) {
         const int64_t room = s == 2 ? resident_clusters<2>() : resident_clusters<4>();
         for (int w = 256; w >= 64; w /= 2) {
             if (mt * ((R + w - 1) / w) > room) continue;
-            const double cost = static_cast<double>((chunks + s - 1) / s) * per_chunk(w) + 11500.0;
-            if (cost < best) {
-                best = cost;
+            const double c = s == 2 ? cost(w, 7500.0, 55.0, 2) : cost(w, 12000.0, 47.0, 4);
+            if (c < best) {
+                best = c;
                 parts = s;
                 *bn = w;
             }

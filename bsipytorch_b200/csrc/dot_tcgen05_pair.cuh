@@ -37,7 +37,7 @@
 // of the tile (the cluster votes before the first MMA) the parts add up in any order to the float32 chain's bits: every
 // warp sends its sums through distributed shared memory to the pair that owns the columns, which adds and stores them.
 // If a bound fails anywhere, pair 0 does the whole tile on its own with the chain in order, as an unsplit kernel would.
-// 512 x 2048 x 8192 (16 tiles of 256 x 256, 4 pairs each): 18.5 -> SPLIT_US us.
+// 512 x 2048 x 8192 (32 tiles of 256 x 128, 2 pairs each): 20.5 -> 18.5 us; 64 x 512 x 16384: 33.8 -> 15.9 us.
 // All waits are bounded; a timeout raises the abort flag of both CTAs and every role drains out.
 #pragma once
 
@@ -56,7 +56,7 @@ constexpr long long kWait = 500000000ll;  // ~0.25 s; real waits are microsecond
 
 constexpr int kSmemLimit = 232448;   // 227 KB: the most dynamic shared memory one CTA can opt in to
 
-template <int BN, typename OutT, bool REQ>
+template <int BN, typename OutT, bool REQ, int SPLIT>
 struct Cfg {
     static_assert(BN % 32 == 0 && BN >= 64 && BN <= 256, "tile width: a multiple of 32 in [64, 256]");
     static constexpr int kHalfN = BN / 2;                 // key rows each CTA loads
@@ -72,16 +72,18 @@ struct Cfg {
     static constexpr int kColBytes = BN * (4 + static_cast<int>(sizeof(OutT)));
     // chunk-maximum exchange of the re-quantising epilogue: 2 parities x 8 warps x 32 lanes x 2 bytes + 8 counters
     static constexpr int kXchgBytes = REQ ? 2 * kEpiWarps * 32 * 2 + kEpiWarps * 4 : 0;
-    static constexpr int kFixedBytes = kStoreBytes + (2 * 9 + 2 * kAccBufs + 2) * 8 + 16 + kColBytes + kXchgBytes;
+    static constexpr int kSumBars = SPLIT > 1 ? kEpiWarps : 0;      // arrival of the other parts' sums, per epilogue warp
+    static constexpr int kFixedBytes = kStoreBytes + (2 * 9 + 2 * kAccBufs + 2 + kSumBars) * 8 + 16 + kColBytes + kXchgBytes;
     static constexpr int kFit = (kSmemLimit - kFixedBytes) / kStageBytes;
     static constexpr int kStages = kFit > 9 ? 9 : kFit;   // 6 (BN >= 192), 7, 8, 8, 9 (BN = 64)
-    static constexpr int kBarriers = 2 * kStages + 2 * kAccBufs + 2;
+    static constexpr int kBarriers = 2 * kStages + 2 * kAccBufs + 2 + kSumBars;
     static constexpr int kSmemBytes = kStages * kStageBytes + kStoreBytes + kBarriers * 8 + 16 + kColBytes + kXchgBytes;
     // Two MMA issuers take the chunks in turn. An issuer's wait for a stage could only mistake the previous lap for its
     // own if that lap's chunk were not drained yet, and the accumulator wait in front of it says that chunk
     // cc - kAccBufs is.
     static_assert(kStages / 2 >= kAccBufs, "a ring lap must not be shorter than the accumulator ring");
     static_assert(kStages >= 4 && kSmemBytes <= kSmemLimit, "operand ring does not fit");
+    static_assert(2 * kEpiWarps * (SPLIT - 1) * (kHalfN / SPLIT) * 128 <= kStages * kStageBytes, "sums to send and received fit the ring");
     static_assert(kStages * kStageBytes >= kEpiWarps * 4096 * ((kHalfN * static_cast<int>(sizeof(OutT)) + 127) / 128), "the last tile is staged in the ring");
 };
 
@@ -253,6 +255,186 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t sr
 }
 __device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 
+__device__ __forceinline__ float most4(float4 v) { return fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)); }
+__device__ __forceinline__ float most4(float v) { return v; }
+__device__ __forceinline__ float sum4(float4 v) { return (v.x + v.y) + (v.z + v.w); }
+__device__ __forceinline__ float sum4(float v) { return v; }
+template <typename V>
+__device__ __forceinline__ V zero_of();
+template <>
+__device__ __forceinline__ float4 zero_of<float4>() { return make_float4(0.0f, 0.0f, 0.0f, 0.0f); }
+template <>
+__device__ __forceinline__ float zero_of<float>() { return 0.0f; }
+
+// Over 32 rows of per-chunk scales (and sums of squares; norms may be null), `units` vectors V each: the largest scale,
+// the largest sum of a row's scales, the largest sum of a row's squares, spread over the lanes (the caller takes the
+// maximum over them). Neighbouring lanes read neighbouring vectors of a row and add up by shuffles: with a row per lane
+// every load touched 32 lines, 7 thousand cycles for 64 chunks.
+template <typename V>
+__device__ __forceinline__ void row_stats(const float* __restrict__ qs, int64_t qs_stride, const float* __restrict__ norms, int64_t n_stride,
+                                          int first_row, int Q, int units, float& smax, float& ssum, float& u2) {
+    constexpr int kMost = sizeof(V) == 16 ? 8 : 32;      // lanes on a row at most
+    constexpr int kRows = 4;                             // rows per lane group in flight
+    const int lane = threadIdx.x & 31;
+    int lg = 0;
+    while ((1 << lg) < units && (1 << lg) < kMost) ++lg;
+    const int group = 1 << lg, sub = lane & (group - 1);
+    for (int it = 0; it < group; it += kRows) {
+        float m[kRows], t[kRows], n[kRows];
+#pragma unroll
+        for (int h = 0; h < kRows; ++h) m[h] = t[h] = n[h] = 0.0f;
+        for (int u0 = 0; u0 < units; u0 += group) {
+            V a[kRows], b[kRows];
+#pragma unroll
+            for (int h = 0; h < kRows; ++h) {
+                const int r = first_row + (((it + h) << 5) >> lg) + (lane >> lg);
+                const bool in = it + h < group && u0 + sub < units && r < Q;
+                a[h] = in ? __ldg(reinterpret_cast<const V*>(qs + r * qs_stride) + u0 + sub) : zero_of<V>();
+                b[h] = in && norms != nullptr ? __ldg(reinterpret_cast<const V*>(norms + r * n_stride) + u0 + sub) : zero_of<V>();
+            }
+#pragma unroll
+            for (int h = 0; h < kRows; ++h) {
+                m[h] = fmaxf(m[h], most4(a[h]));
+                t[h] += sum4(a[h]);
+                n[h] += sum4(b[h]);
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < kRows; ++h) {
+            for (int d = 1; d < group; d <<= 1) {
+                t[h] += __shfl_xor_sync(0xffffffffu, t[h], d);
+                n[h] += __shfl_xor_sync(0xffffffffu, n[h], d);
+            }
+            smax = fmaxf(smax, m[h]);
+            ssum = fmaxf(ssum, t[h]);
+            u2 = fmaxf(u2, n[h]);
+        }
+    }
+}
+
+// The same for one row per lane: kAhead vectors of each array in flight.
+template <typename V, int kAhead>
+__device__ __forceinline__ void row_of_lane(const float* __restrict__ qs_row, const float* __restrict__ n_row, int units, float& smax,
+                                            float& ssum, float& u2) {
+    for (int c = 0; c < units; c += kAhead) {
+        V a[kAhead], n[kAhead];
+#pragma unroll
+        for (int h = 0; h < kAhead; ++h) {
+            a[h] = c + h < units ? __ldg(reinterpret_cast<const V*>(qs_row) + c + h) : zero_of<V>();
+            n[h] = c + h < units && n_row != nullptr ? __ldg(reinterpret_cast<const V*>(n_row) + c + h) : zero_of<V>();
+        }
+#pragma unroll
+        for (int h = 0; h < kAhead; ++h) {
+            smax = fmaxf(smax, most4(a[h]));
+            ssum += sum4(a[h]);
+            u2 += sum4(n[h]);
+        }
+    }
+}
+
+// 16-byte-aligned blocks a warp's kCols columns make: of 128-byte rows, the last one of 64-byte rows where that is left
+template <typename OutT, int kCols>
+__host__ __device__ constexpr int kBlocks() {
+    return (kCols * static_cast<int>(sizeof(OutT)) + 127) / 128;
+}
+
+// Stores 32 rows (lane = row) x kCols finished columns: out = (acc * w) * scale_inv + bias, ReLU.
+// A lane owns a row. Blocks of 32 rows x 128 bytes are finished into shared memory (16-byte pieces swizzled as the
+// tensor map wants them, which also keeps the banks apart) and leave as one bulk tensor store each, so that the warp is
+// back in the next tile's main loop while they drain; written with ordinary stores, the output took half of a tile's
+// time at 16 chunks. A warp has one block of its own; places != nullptr (a CTA's last tile, when nothing reads the operand
+// ring any more) gives every block its own place.
+template <typename OutT, int kCols>
+__device__ __forceinline__ void store_columns(const float (&acc)[kCols], uint8_t* places, uint8_t* own, const float* colw, const OutT* colb,
+                                              const CUtensorMap& map_o, const CUtensorMap& map_t, OutT* __restrict__ outp, int64_t ldo,
+                                              int row_shift, int row_base, int Q, int col, int R, float scale_inv, bool has_bias, bool relu,
+                                              int store_flags) {
+    const int lane = threadIdx.x & 31;
+    constexpr int E = static_cast<int>(sizeof(OutT));
+    constexpr int kPerChunk = 16 / E;                        // values per 16-byte piece
+    constexpr int kRoundCols = 128 / E;                      // columns per block
+    constexpr int kFull = kCols / kRoundCols;                // whole blocks; then one of 64-byte rows, or none
+    constexpr int kRounds = kBlocks<OutT, kCols>();
+    const uint64_t scale2 = pack2(scale_inv, scale_inv);
+    if ((store_flags & 1) && (kCols * E) % 64 == 0) {
+        const bool bulk = (store_flags & 4) != 0;
+#pragma unroll
+        for (int g = 0; g < kRounds; ++g) {
+            const bool whole = g < kFull;
+            const int nch = whole ? 8 : 4;                   // 16-byte pieces per staged row
+            const int cg = g * kRoundCols;
+            uint8_t* block = places != nullptr ? places + g * 4096 : own;
+            if (bulk && places == nullptr) {
+                if (lane == 0) tma_store_wait_read();
+                __syncwarp();
+            }
+            uint8_t* dst = block + lane * (nch * 16);
+#pragma unroll
+            for (int ch = 0; ch < 8; ++ch) {
+                if (ch < nch) {
+                    const int swz = whole ? (ch ^ (lane & 7)) : (ch ^ ((lane >> 1) & 3));
+                    const int j = cg + ch * kPerChunk;
+                    if (j < kCols)
+                        *reinterpret_cast<uint4*>(dst + (swz << 4)) = finish16<OutT>(acc + j, colw + j, colb + j, scale2, has_bias, relu);
+                }
+            }
+            if (bulk) {
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0 && row_base < Q && col + cg < R)      // rows and columns beyond the matrix are clipped
+                    tma_store_2d(whole ? &map_o : &map_t, smem_u32(block), col + cg, row_base);
+            } else {
+                __syncwarp();
+                const int cchunk = lane & (nch - 1);
+                const int c = col + cg + cchunk * kPerChunk;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    if (i < nch) {
+                        const int rr = i * (32 / nch) + lane / nch;
+                        const int swz = whole ? (cchunk ^ (rr & 7)) : (cchunk ^ ((rr >> 1) & 3));
+                        const uint4 o = *reinterpret_cast<const uint4*>(block + rr * (nch * 16) + (swz << 4));
+                        const int grow = row_base + rr;
+                        if (grow < Q && c < R)               // R is a multiple of kPerChunk on this path
+                            *reinterpret_cast<uint4*>(outp + static_cast<int64_t>(grow - row_shift) * ldo + c) = o;
+                    }
+                }
+                __syncwarp();
+            }
+        }
+        return;
+    }
+    // Rows that do not start on 16 bytes, shares narrower than 64 bytes: blocks of 32 rows x kWide raw sums through the
+    // warp's 4 KB, then kWide adjacent columns of 32 / kWide rows at a time, so that a store covers consecutive addresses.
+    constexpr int kWide = kCols < 32 ? (kCols & -kCols) : 32;
+    if (store_flags & 4) {
+        if (lane == 0) tma_store_wait_read();
+        __syncwarp();
+    }
+    float* stage = reinterpret_cast<float*>(own);
+    const int cj = lane & (kWide - 1);
+#pragma unroll
+    for (int g = 0; g < (kCols + kWide - 1) / kWide; ++g) {
+#pragma unroll
+        for (int j = 0; j < kWide; ++j)
+            if (g * kWide + j < kCols) stage[lane * kWide + (j ^ (lane & (kWide - 1)))] = acc[g * kWide + j];
+        __syncwarp();
+        const int j = g * kWide + cj;
+        const bool in = j < kCols && col + j < R;
+        const float w = in ? colw[j] : 0.0f;
+        const float bv = in ? static_cast<float>(colb[j]) : 0.0f;      // finish() narrows it again: no change
+        OutT* o = outp + static_cast<int64_t>(row_base - row_shift + lane / kWide) * ldo + col + j;
+        const int rows = in ? Q - row_base - lane / kWide : 0;         // this lane's rows are 32 / kWide apart
+#pragma unroll 8
+        for (int i = 0; i < kWide; ++i) {
+            const int rr = i * (32 / kWide) + lane / kWide;
+            const float v = stage[rr * kWide + (cj ^ (rr & (kWide - 1)))];
+            if (i * (32 / kWide) < rows) *o = relu_if<OutT>(finish<OutT>((v * w) * scale_inv, bv, has_bias), relu);
+            o += (32 / kWide) * ldo;
+        }
+        __syncwarp();
+    }
+}
+
 template <int BN, bool DBG, typename OutT, bool REQ = false, int SPLIT = 1>
 __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
     const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
@@ -263,7 +445,7 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
     void* __restrict__ out, int64_t ldo, int32_t* __restrict__ dbg_iacc, const ScatterDst scatter,
     const RequantDst requant, const float* __restrict__ k_abs_sum, float q_abs_max,
     const float* __restrict__ q_sq, int64_t q_sq_stride) {
-    using C = Cfg<BN, OutT, REQ>;
+    using C = Cfg<BN, OutT, REQ, SPLIT>;
     constexpr int kStages = C::kStages;
     constexpr int kCols = BN / 2;              // accumulator columns per epilogue warp: a multiple of 16
 
@@ -454,10 +636,7 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
             __syncwarp();
             }
         }
-        if constexpr (SPLIT > 1) {      // the two barriers around the exchange of sums
-            cluster_sync_all();
-            cluster_sync_all();
-        }
+        if constexpr (SPLIT > 1) cluster_sync_all();      // the operand rings are free
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsHigh));
         // ---------------- epilogue ----------------
@@ -520,46 +699,24 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                     kchk = fmaxf(fmaxf(kv[4], kv[5]), fmaxf(kv[6], kv[7]));
                     k2 = fmaxf(fmaxf(kv[8], kv[9]), fmaxf(kv[10], kv[11]));
                 }
-                // of the lane's query row: the largest and the summed 2^shift, the sum of squares
+                // of the warp's query rows: the largest and the largest summed 2^shift of a row, the largest sum of squares
                 float smax = 0.0f, ssum = 0.0f, u2 = 0.0f;
-                if (row_ok) {
-                    const float* nrow = q_sq != nullptr ? q_sq + static_cast<int64_t>(row) * q_sq_stride : nullptr;
-                    if (!qs_stride) {
-                        smax = __ldg(qs_row);
-                        ssum = smax * static_cast<float>(chunks);
-                    } else if (((reinterpret_cast<uintptr_t>(qs_row) | reinterpret_cast<uintptr_t>(nrow)) & 15) == 0 && (chunks & 3) == 0) {
-                        constexpr int kAhead = 4;
-                        for (int c = 0; c < chunks; c += 4 * kAhead) {
-                            float4 a[kAhead], n[kAhead];
-#pragma unroll
-                            for (int h = 0; h < kAhead; ++h) {
-                                const bool in = c + 4 * h < chunks;
-                                a[h] = in ? __ldg(reinterpret_cast<const float4*>(qs_row + c) + h) : make_float4(0.f, 0.f, 0.f, 0.f);
-                                n[h] = in && nrow != nullptr ? __ldg(reinterpret_cast<const float4*>(nrow + c) + h) : make_float4(0.f, 0.f, 0.f, 0.f);
-                            }
-#pragma unroll
-                            for (int h = 0; h < kAhead; ++h) {
-                                smax = fmaxf(smax, fmaxf(fmaxf(a[h].x, a[h].y), fmaxf(a[h].z, a[h].w)));
-                                ssum += (a[h].x + a[h].y) + (a[h].z + a[h].w);
-                                u2 += (n[h].x + n[h].y) + (n[h].z + n[h].w);
-                            }
-                        }
-                    } else {
-                        constexpr int kAhead = 8;
-                        for (int c = 0; c < chunks; c += kAhead) {
-                            float a[kAhead], n[kAhead];
-#pragma unroll
-                            for (int h = 0; h < kAhead; ++h) {
-                                a[h] = c + h < chunks ? __ldg(qs_row + c + h) : 0.0f;
-                                n[h] = c + h < chunks && nrow != nullptr ? __ldg(nrow + c + h) : 0.0f;
-                            }
-#pragma unroll
-                            for (int h = 0; h < kAhead; ++h) {
-                                smax = fmaxf(smax, a[h]);
-                                ssum += a[h];
-                                u2 += n[h];
-                            }
-                        }
+                const int first_row = row - lane;
+                const float* norms = qs_stride ? q_sq : nullptr;
+                if (!qs_stride) {
+                    if (row_ok) smax = __ldg(qs_row);
+                    ssum = smax * static_cast<float>(chunks);
+                } else {
+                    const bool vec = (chunks & 3) == 0 && (qs_stride & 3) == 0 && (q_sq_stride & 3) == 0 &&
+                                     ((reinterpret_cast<uintptr_t>(qs) | reinterpret_cast<uintptr_t>(norms)) & 15) == 0;
+                    if (chunks > 16) {
+                        if (vec) row_stats<float4>(qs, qs_stride, norms, q_sq_stride, first_row, Q, chunks / 4, smax, ssum, u2);
+                        else row_stats<float>(qs, qs_stride, norms, q_sq_stride, first_row, Q, chunks, smax, ssum, u2);
+                    } else if (row_ok) {
+                        // few chunks: a row per lane, everything in one go or two
+                        const float* nrow = norms != nullptr ? norms + static_cast<int64_t>(row) * q_sq_stride : nullptr;
+                        if (vec) row_of_lane<float4, 4>(qs_row, nrow, chunks / 4, smax, ssum, u2);
+                        else row_of_lane<float, 8>(qs_row, nrow, chunks, smax, ssum, u2);
                     }
                 }
                 // an infinity anywhere fails the test. By shuffles: as redux.sync the maximum left out some lanes in the split
@@ -657,29 +814,49 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                     }
                 }
             }
+            // the half's key scales and bias into shared memory: behind the first barrier nobody reads the last tile's
+            asm volatile("bar.sync %0, 128;" ::"r"(2 + half) : "memory");
+            if (lane < kOwn) {
+                colw[col0 + own] = own_w;
+                colb[col0 + own] = cast_bias(own_b, OutT());
+            }
+            asm volatile("bar.sync %0, 128;" ::"r"(2 + half) : "memory");
             if constexpr (SPLIT > 1) {
                 constexpr int kShare = kCols / SPLIT;        // columns of this warp that each pair stores
-                constexpr int kWide = kShare < 32 ? kShare : 32;
                 const bool add_up = *vote == 0;
                 __syncwarp();
                 cluster_sync_all();          // the operand rings of all CTAs are free
-                // [warp][source][4 columns][lane]: 512 bytes per 4 columns, written and read without bank conflicts
-                const uint32_t slots = smem_base + static_cast<uint32_t>(ew * (SPLIT - 1) * kShare * 128 + lane * 16);
+                // Sums to send and sums received, both [warp][slot][4 columns][lane] in the ring: 512 bytes per 4 columns,
+                // no bank conflicts. A share travels as one bulk copy; stored to the other CTA's shared memory by the
+                // lanes, the exchange of a 256-column tile took 8 us.
+                constexpr int kShareBytes = kShare * 128, kSlotBytes = (SPLIT - 1) * kShareBytes;
+                const uint32_t sum_bar = bar_base + 8u * (2 * kStages + 2 * kAccBufs + 2 + ew);
+                uint8_t* to_send = smem + ew * kSlotBytes;
+                uint8_t* received = smem + (kEpiWarps + ew) * kSlotBytes;
                 if (add_up && ok) {
+                    if (lane == 0) mbar_expect_tx(sum_bar, kSlotBytes);
 #pragma unroll
                     for (int q = 0; q < SPLIT; ++q) {
                         if (q != part) {
-                            const uint32_t dst = map_to_cta(slots, static_cast<uint32_t>(2 * q) + rank) +
-                                                 static_cast<uint32_t>((part < q ? part : part - 1) * kShare * 128);
+                            uint8_t* mine = to_send + (q < part ? q : q - 1) * kShareBytes + lane * 16;
 #pragma unroll
                             for (int j = 0; j < kShare; j += 4)
-                                asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};"
-                                             ::"r"(dst + j * 128), "r"(__float_as_int(acc[q * kShare + j])), "r"(__float_as_int(acc[q * kShare + j + 1])),
-                                               "r"(__float_as_int(acc[q * kShare + j + 2])), "r"(__float_as_int(acc[q * kShare + j + 3])) : "memory");
+                                *reinterpret_cast<float4*>(mine + j * 128) = make_float4(acc[q * kShare + j], acc[q * kShare + j + 1],
+                                                                                         acc[q * kShare + j + 2], acc[q * kShare + j + 3]);
                         }
                     }
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    __syncwarp();
+                    if (lane < SPLIT && lane != part) {
+                        const uint32_t cta = static_cast<uint32_t>(2 * lane) + rank;
+                        asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                                     ::"r"(map_to_cta(smem_u32(received), cta) + static_cast<uint32_t>((part < lane ? part : part - 1) * kShareBytes)),
+                                     "r"(smem_u32(to_send) + static_cast<uint32_t>((lane < part ? lane : lane - 1) * kShareBytes)), "r"(kShareBytes),
+                                     "r"(map_to_cta(sum_bar, cta)) : "memory");
+                    }
+                    __syncwarp();
+                    ok = wait_or_abort(sum_bar, 0, actx, 6);
                 }
-                cluster_sync_all();          // every part's sums have arrived
                 if (add_up) {
                     if (!ok) continue;
                     int sum[kShare];
@@ -694,46 +871,22 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                     for (int q = 0; q < SPLIT - 1; ++q) {
 #pragma unroll
                         for (int j = 0; j < kShare; j += 4) {
-                            const int4 v = *reinterpret_cast<const int4*>(smem + ew * (SPLIT - 1) * kShare * 128 + lane * 16 + (q * kShare + j) * 128);
+                            const int4 v = *reinterpret_cast<const int4*>(received + lane * 16 + (q * kShare + j) * 128);
                             sum[j] += v.x; sum[j + 1] += v.y; sum[j + 2] += v.z; sum[j + 3] += v.w;
                         }
                     }
                     if (lane == 0) atomicAdd(&g_exact_int_tiles, 1ull);
-                    // blocks of 32 rows x kWide columns through the warp's 4 KB, then stores of kWide adjacent columns
-                    float* stage = reinterpret_cast<float*>(my_store);
-                    OutT* o = static_cast<OutT*>(out);
-                    const int first_row = tm * 256 + static_cast<int>(rank) * BM + quad * 32;
-                    const int cj = lane & (kWide - 1);
+                    float val[kShare];
 #pragma unroll
-                    for (int g = 0; g < kShare / kWide; ++g) {
-                        const int col = n0 + col0 + part * kShare + g * kWide + cj;
-                        const float w = col < R ? __ldg(bw0 + col) : 0.0f;
-                        const float bv = col < R && has_bias ? __ldg(bias + col) : 0.0f;
-#pragma unroll
-                        for (int j = 0; j < kWide; ++j)
-                            stage[lane * kWide + (j ^ (lane & (kWide - 1)))] = small ? int_to_float_exact(sum[g * kWide + j]) : static_cast<float>(sum[g * kWide + j]);
-                        __syncwarp();
-#pragma unroll 8
-                        for (int i = 0; i < kWide; ++i) {
-                            const int rr = i * (32 / kWide) + lane / kWide;
-                            const float v = stage[rr * kWide + (cj ^ (rr & (kWide - 1)))];
-                            if (first_row + rr < Q && col < R)
-                                o[static_cast<int64_t>(first_row + rr) * ldo + col] =
-                                    relu_if<OutT>(finish<OutT>((v * w) * scale_inv, bv, has_bias), relu);
-                        }
-                        __syncwarp();
-                    }
+                    for (int j = 0; j < kShare; ++j) val[j] = small ? int_to_float_exact(sum[j]) : static_cast<float>(sum[j]);
+                    const int cs = col0 + part * kShare;
+                    store_columns<OutT, kShare>(val, nullptr, my_store, colw + cs, colb + cs, map_o, map_t, static_cast<OutT*>(out), ldo, 0,
+                                                tm * 256 + static_cast<int>(rank) * BM + quad * 32, Q, n0 + cs, R, scale_inv, has_bias, relu,
+                                                store_flags);
                     continue;
                 }
                 if (!whole_tile) continue;
             }
-            // the half's key scales and bias into shared memory: behind the first barrier nobody reads the last tile's
-            asm volatile("bar.sync %0, 128;" ::"r"(2 + half) : "memory");
-            if (lane < kOwn) {
-                colw[col0 + own] = own_w;
-                colb[col0 + own] = cast_bias(own_b, OutT());
-            }
-            asm volatile("bar.sync %0, 128;" ::"r"(2 + half) : "memory");
             if (!ok) continue;
             if (exact) {
                 // the int32 sums (below 2^24 in magnitude) as floats: what the float32 chain would hold. Below 2^22 by an
@@ -749,19 +902,7 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
             }
 
             // ---- tile result: out = (acc * bw0[r]) * scale_inv ----
-            // A lane owns a row. Blocks of 32 rows x 128 bytes are finished into shared memory (16-byte pieces swizzled
-            // as the tensor map wants them, which also keeps the banks apart) and leave as one bulk tensor store each,
-            // so that the warp is back in the next tile's main loop while they drain; written with ordinary stores, the
-            // output took half of a tile's time at 16 chunks. A warp has one block of its own; on a CTA's last tile
-            // every block has its place in the operand ring, which nothing reads any more.
             const int row_base = tm * 256 + static_cast<int>(rank) * BM + quad * 32;
-            constexpr int E = static_cast<int>(sizeof(OutT));
-            constexpr int kPerChunk = 16 / E;                        // values per 16-byte piece
-            constexpr int kRoundCols = 128 / E;                      // columns per block
-            constexpr int kFull = kCols / kRoundCols;                // whole blocks; then one of 64-byte rows, or none
-            constexpr int kRounds = kFull + (kCols % kRoundCols != 0 ? 1 : 0);
-            static_assert((kCols * E) % 64 == 0, "whole 64-byte pieces of a row");
-            const uint64_t scale2 = pack2(scale_inv, scale_inv);
             if constexpr (REQ) {
                 static_assert(BN == 256 && !DBG && sizeof(OutT) == 2, "re-quantisation: 256-wide tiles, 16-bit layer type");
                 {
@@ -769,6 +910,7 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                     // what the next linear's packer would read; with BN = 256 a tile row is exactly one chunk,
                     // split between this warp and the warp of the other column half. Same integers as the pack
                     // kernel's fast path (the values have 16-bit precision, so the float32 rounding is exact).
+                    const uint64_t scale2 = pack2(scale_inv, scale_inv);
                     RawLane<OutT> y[kCols / 8];
                     uint32_t amax_bits = 0;                   // pattern of OutT: orders like the magnitude
 #pragma unroll
@@ -858,81 +1000,10 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                 outp = static_cast<OutT*>(scatter.y[d]);
                 row_shift = d * scatter.rows_per_dst;
             }
-            if (store_flags & 1) {
-                const bool bulk = (store_flags & 4) != 0;
-                const bool last = tile + num_pairs >= tiles_total;
-#pragma unroll
-                for (int g = 0; g < kRounds; ++g) {
-                    const bool whole = g < kFull;
-                    const int nch = whole ? 8 : 4;                   // 16-byte pieces per staged row
-                    const int cg = col0 + g * kRoundCols;            // first column of the block in the tile
-                    uint8_t* block = my_store;
-                    if (bulk && last) {
-                        block = smem + (ew * kRounds + g) * 4096;
-                    } else if (bulk) {
-                        if (lane == 0) tma_store_wait_read();
-                        __syncwarp();
-                    }
-                    uint8_t* dst = block + lane * (nch * 16);
-#pragma unroll
-                    for (int ch = 0; ch < 8; ++ch) {
-                        if (ch < nch) {
-                            const int swz = whole ? (ch ^ (lane & 7)) : (ch ^ ((lane >> 1) & 3));
-                            const int j = g * kRoundCols + ch * kPerChunk;
-                            *reinterpret_cast<uint4*>(dst + (swz << 4)) =
-                                finish16<OutT>(acc + j, colw + col0 + j, colb + col0 + j, scale2, has_bias, relu);
-                        }
-                    }
-                    if (bulk) {
-                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                        __syncwarp();
-                        if (lane == 0 && row_base < Q && n0 + cg < R)      // rows and columns beyond the matrix are clipped
-                            tma_store_2d(whole ? &map_o : &map_t, smem_u32(block), n0 + cg, row_base);
-                    } else {
-                        __syncwarp();
-                        const int cchunk = lane & (nch - 1);
-                        const int col = n0 + cg + cchunk * kPerChunk;
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            if (i < nch) {
-                                const int rr = i * (32 / nch) + lane / nch;
-                                const int swz = whole ? (cchunk ^ (rr & 7)) : (cchunk ^ ((rr >> 1) & 3));
-                                const uint4 o = *reinterpret_cast<const uint4*>(block + rr * (nch * 16) + (swz << 4));
-                                const int grow = row_base + rr;
-                                if (grow < Q && col < R)             // R is a multiple of kPerChunk on this path
-                                    *reinterpret_cast<uint4*>(outp + static_cast<int64_t>(grow - row_shift) * ldo + col) = o;
-                            }
-                        }
-                        __syncwarp();
-                    }
-                }
-            } else {
-                // Rows that do not start on 16 bytes: blocks of 32 x 32 raw sums through the warp's 4 KB, then a row at
-                // a time with one value per lane, so that a store still covers consecutive addresses.
-                float* stage = reinterpret_cast<float*>(my_store);
-                constexpr int kBlocks = (kCols + 31) / 32;
-#pragma unroll
-                for (int g = 0; g < kBlocks; ++g) {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j)
-                        if (g * 32 + j < kCols) stage[lane * 32 + (j ^ lane)] = acc[g * 32 + j];
-                    __syncwarp();
-                    const int j = g * 32 + lane;
-                    const int col = n0 + col0 + j;
-                    const bool in = j < kCols && col < R;
-                    const float w = in ? colw[col0 + j] : 0.0f;
-                    const float bv = in ? static_cast<float>(colb[col0 + j]) : 0.0f;      // finish() narrows it again: no change
-#pragma unroll 4
-                    for (int rr = 0; rr < 32; ++rr) {
-                        const float v = stage[rr * 32 + (lane ^ rr)];
-                        const int grow = row_base + rr;
-                        if (in && grow < Q)
-                            outp[static_cast<int64_t>(grow - row_shift) * ldo + col] =
-                                relu_if<OutT>(finish<OutT>((v * w) * scale_inv, bv, has_bias), relu);
-                    }
-                    __syncwarp();
-                }
-            }
+            const bool last = tile + num_pairs >= tiles_total;
+            store_columns<OutT, kCols>(acc, (store_flags & 4) && last ? smem + ew * kBlocks<OutT, kCols>() * 4096 : nullptr, my_store, colw + col0,
+                                       colb + col0, map_o, map_t, outp, ldo, row_shift, row_base, Q, n0 + col0, R, scale_inv, has_bias, relu,
+                                       store_flags);
         }
         if (lane == 0) tma_store_wait_read();      // shared memory is read until then
     }
