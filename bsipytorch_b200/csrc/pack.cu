@@ -238,6 +238,10 @@ __global__ void __launch_bounds__(256, BSI_PACK_MIN_BLOCKS) quantize_pack_chunk_
     const T* __restrict__ x, FastGeom g, double dec_scale, uint32_t dec_mult, int bits,
     u64* __restrict__ words, float* __restrict__ scales, int32_t* __restrict__ shifts, int8_t* __restrict__ q8,
     int vec_ok, float* __restrict__ sq_norms, float* __restrict__ slice_weights) {
+    // Launched as a programmatic dependent, and letting its own dependents go at once: a dot sets up its barriers and
+    // tensor memory while this kernel runs, and reads its results behind griddepcontrol.wait.
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     __shared__ uint32_t slow_queue[8][kSlowQueue];
     constexpr int kDepth = sizeof(T) == 2 ? 4 : 2;
     const int lane = threadIdx.x & 31;
@@ -945,8 +949,17 @@ int launch_chunk_fast(const T* x, const PackArgs& a) {
     g.W = static_cast<uint32_t>(a.W);
     g.row_bytes = static_cast<uint32_t>(a.bits * a.W * 8);
     g.slice_bytes = static_cast<uint32_t>(a.W * 8);
-    quantize_pack_chunk_fast_kernel<T, kDense, kWords, kQ8><<<static_cast<unsigned>(blocks), 256, 0, a.stream>>>(
-        x, g, a.dec_scale, a.dec_mult, a.bits, a.words, a.scales, a.shifts, a.q8, a.vec_ok, a.sq_norms, a.slice_weights);
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = dim3(static_cast<unsigned>(blocks), 1, 1);
+    cfg.blockDim = dim3(256, 1, 1);
+    cfg.stream = a.stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 1 : 0;
+    BSI_CUDA_TRY(cudaLaunchKernelEx(&cfg, quantize_pack_chunk_fast_kernel<T, kDense, kWords, kQ8>, x, g, a.dec_scale, a.dec_mult,
+                                    a.bits, a.words, a.scales, a.shifts, a.q8, a.vec_ok, a.sq_norms, a.slice_weights));
     return BSI_OK;
 }
 
