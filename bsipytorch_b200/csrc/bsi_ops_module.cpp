@@ -779,45 +779,27 @@ std::string cuda_builder_version() { return "BSI_B200_SM100A_V" + std::to_string
 // One call for a whole linear layer: pack x, dot with the keys, cast to x's dtype and add the bias.
 // Same arithmetic as BSIQuantizedLinear.forward (verify_accuracy_bsi.py:118-215) without the
 // capsule round trip, the float32 [Q, R] re-read by two elementwise kernels, or host syncs.
-at::Tensor linear_forward(const Env& env, const at::Tensor& x2d, const PrebuiltBSIKeysCUDA& keys,
-                          const c10::optional<torch::Tensor>& bias, int decimalPlaces) {
+// Several layers that read the same activations (`n` of them: query, key and value projections) share one packing.
+struct LinearTo {
+    const PrebuiltBSIKeysCUDA* keys;
+    const c10::optional<torch::Tensor>* bias;
+    at::Tensor y;
+};
+void linear_forward(const Env& env, const at::Tensor& x2d, int decimalPlaces, bool relu, LinearTo* to, int n) {
     TORCH_CHECK(x2d.dim() == 2 && x2d.is_cuda(), "x must be a 2D CUDA tensor");
-    same_device(x2d, keys.b.q8, "activations and keys");
     c10::cuda::CUDAGuard guard(x2d.device());
     const int engine = env.dot_engine();
     const int bits = env.bits_queries();
     // two-digit variable-slice queries need two dots and a combine: they take the unfused route below
     const bool fused = (engine == BSI_ENGINE_AUTO || engine == BSI_ENGINE_TCGEN05) && bits > 0;
-    const int64_t Q = x2d.size(0), D = x2d.size(1), R = keys.num_keys;
-    TORCH_CHECK(Q > 0 && R > 0, "Empty queries or keys");
+    const int64_t Q = x2d.size(0), D = x2d.size(1);
     const int W = D > 0 ? static_cast<int>((D + 63) / 64) : 1;
-    TORCH_CHECK(W == keys.b.W, "Word count mismatch between query batch and keys");
-    TORCH_CHECK(decimalPlaces == keys.b.decimals, "Decimal mismatch between queries and keys: q=", decimalPlaces,
-                " k=", keys.b.decimals);
-    const int total_decimals = decimalPlaces + keys.b.decimals;
-    const double scale_inv = total_decimals > 0 ? 1.0 / std::pow(10.0, total_decimals) : 1.0;
+    const int total_decimals = 2 * decimalPlaces;
+    const float scale_inv = static_cast<float>(total_decimals > 0 ? 1.0 / std::pow(10.0, total_decimals) : 1.0);
     at::ScalarType yt = x2d.scalar_type();
     if (!(yt == at::kFloat || yt == at::kHalf || yt == at::kBFloat16)) yt = at::kFloat;
-    at::Tensor y = at::detail::empty_cuda({Q, R}, yt, x2d.device(), c10::nullopt);
-    const float* bptr = nullptr;
-    at::Tensor b32;
-    if (bias.has_value() && bias->defined()) {
-        b32 = *bias;
-        if (b32.scalar_type() != at::kFloat || b32.device() != y.device() || !b32.is_contiguous())
-            b32 = b32.to(y.device(), at::kFloat).contiguous();
-        TORCH_CHECK(b32.numel() == R, "bias length mismatch");
-        bptr = b32.data_ptr<float>();
-    }
     const int code = yt == at::kHalf ? BSI_DTYPE_F16 : (yt == at::kBFloat16 ? BSI_DTYPE_BF16 : BSI_DTYPE_F32);
-    if (!fused || D == 0) {
-        // other engines: float32 dot, then the separate cast + bias kernel
-        PackedBatch qb = pack_queries(env, x2d, decimalPlaces);
-        py::tuple r = run_dot(env, qb, keys, false, nullptr);
-        at::Tensor out = r[0].cast<at::Tensor>();
-        check_status(bsi_b200_cast_bias(out.data_ptr<float>(), R, bptr, Q, R, y.data_ptr(), R, code, current_stream()),
-                     "bsi_b200_cast_bias");
-        return y;
-    }
+    const int act = relu ? BSI_ACT_RELU : BSI_ACT_NONE;
     at::Tensor x = x2d;
     if (x.scalar_type() != yt) x = x.to(yt);
     if (x.stride(1) != 1 || x.stride(0) < D) x = x.contiguous();
@@ -825,49 +807,89 @@ at::Tensor linear_forward(const Env& env, const at::Tensor& x2d, const PrebuiltB
     const float clip_k = env.clip_k();
     const bool profile = env.profile();
     const int64_t chunks = (D + 255) / 256, ldx = x.stride(0);
-    if (chunk && !(clip_k > 0.0f) && !profile && decimalPlaces >= 0 && decimalPlaces <= 8 &&
-        engine == BSI_ENGINE_AUTO && bsi_b200_linear_decode_fits(Q, R, D)) {
-        check_status(bsi_b200_linear_decode(x.data_ptr(), code, ldx, D, decimalPlaces, bits, keys.b.q8.data_ptr<int8_t>(),
-                                            keys.b.q8.size(1), keys.b.scales.data_ptr<float>(), bptr, Q, R,
-                                            static_cast<float>(scale_inv), y.data_ptr(), R, BSI_ACT_NONE, current_stream()),
-                     "bsi_b200_linear_decode");
-        return y;
-    }
+    const bool one_launch = chunk && !(clip_k > 0.0f) && !profile && decimalPlaces >= 0 && decimalPlaces <= 8 && engine == BSI_ENGINE_AUTO;
     // int8 image, scales and chunk sums of squares share one block that goes back to the allocator (stream-ordered)
     // when the call returns
-    const int64_t image = Q * chunks * 256, per_row = chunk ? chunks : 1;
-    c10::DataPtr work = c10::cuda::CUDACachingAllocator::get()->allocate(static_cast<size_t>(image + 8 * Q * per_row));
-    int8_t* q8 = static_cast<int8_t*>(work.get());
-    float* scales = reinterpret_cast<float*>(q8 + image);
-    float* sq = chunk ? scales + Q * per_row : nullptr;
-    cudaEvent_t e0 = nullptr, e1 = nullptr;
-    if (profile) {
-        cudaEventCreate(&e0);
-        cudaEventCreate(&e1);
-        cudaEventRecord(e0, at::cuda::getCurrentCUDAStream().stream());
+    c10::DataPtr work;
+    int8_t* q8 = nullptr;
+    float *scales = nullptr, *sq = nullptr;
+    for (int i = 0; i < n; ++i) {
+        const PrebuiltBSIKeysCUDA& keys = *to[i].keys;
+        const int64_t R = keys.num_keys;
+        same_device(x2d, keys.b.q8, "activations and keys");
+        TORCH_CHECK(Q > 0 && R > 0, "Empty queries or keys");
+        TORCH_CHECK(W == keys.b.W, "Word count mismatch between query batch and keys");
+        TORCH_CHECK(decimalPlaces == keys.b.decimals, "Decimal mismatch between queries and keys: q=", decimalPlaces,
+                    " k=", keys.b.decimals);
+        at::Tensor& y = to[i].y;
+        y = at::detail::empty_cuda({Q, R}, yt, x2d.device(), c10::nullopt);
+        const float* bptr = nullptr;
+        at::Tensor b32;
+        if (to[i].bias->has_value() && (*to[i].bias)->defined()) {
+            b32 = **to[i].bias;
+            if (b32.scalar_type() != at::kFloat || b32.device() != y.device() || !b32.is_contiguous())
+                b32 = b32.to(y.device(), at::kFloat).contiguous();
+            TORCH_CHECK(b32.numel() == R, "bias length mismatch");
+            bptr = b32.data_ptr<float>();
+        }
+        if (!fused || D == 0) {
+            // other engines: float32 dot, then the separate cast + bias kernel
+            PackedBatch qb = pack_queries(env, x2d, decimalPlaces);
+            py::tuple r = run_dot(env, qb, keys, false, nullptr);
+            at::Tensor out = r[0].cast<at::Tensor>();
+            check_status(bsi_b200_cast_bias(out.data_ptr<float>(), R, bptr, Q, R, y.data_ptr(), R, code, current_stream()),
+                         "bsi_b200_cast_bias");
+            if (relu) y.relu_();
+            continue;
+        }
+        if (one_launch && bsi_b200_linear_decode_fits(Q, R, D)) {
+            check_status(bsi_b200_linear_decode(x.data_ptr(), code, ldx, D, decimalPlaces, bits, keys.b.q8.data_ptr<int8_t>(),
+                                                keys.b.q8.size(1), keys.b.scales.data_ptr<float>(), bptr, Q, R, scale_inv,
+                                                y.data_ptr(), R, act, current_stream()),
+                         "bsi_b200_linear_decode");
+            continue;
+        }
+        if (q8 == nullptr) {
+            const int64_t image = Q * chunks * 256, per_row = chunk ? chunks : 1;
+            work = c10::cuda::CUDACachingAllocator::get()->allocate(static_cast<size_t>(image + 8 * Q * per_row));
+            q8 = static_cast<int8_t*>(work.get());
+            scales = reinterpret_cast<float*>(q8 + image);
+            sq = chunk ? scales + Q * per_row : nullptr;
+            cudaEvent_t e0 = nullptr, e1 = nullptr;
+            if (profile) {
+                cudaEventCreate(&e0);
+                cudaEventCreate(&e1);
+                cudaEventRecord(e0, at::cuda::getCurrentCUDAStream().stream());
+            }
+            check_status(bsi_b200_quantize_pack_all(x.data_ptr(), code, Q, D, ldx, decimalPlaces, bits, chunk ? 1 : 0, clip_k, nullptr,
+                                                    scales, nullptr, q8, chunks * 256, sq, nullptr, nullptr, current_stream()),
+                         "bsi_b200_quantize_pack_all");
+            float pack_ms = 0.f;
+            if (profile) {
+                cudaEventRecord(e1, at::cuda::getCurrentCUDAStream().stream());
+                cudaEventSynchronize(e1);
+                cudaEventElapsedTime(&pack_ms, e0, e1);
+                cudaEventDestroy(e0);
+                cudaEventDestroy(e1);
+            }
+            g_last_quantize_ns = 0;
+            g_last_pack_ns = g_last_total_ns = static_cast<uint64_t>(pack_ms * 1.0e6);
+        }
+        bsi_dot_bounds bounds = dot_bounds(keys, bits, nullptr);
+        bounds.query_sq = sq;
+        bounds.query_sq_stride = chunks;
+        check_status(bsi_b200_linear_i8_bounded(q8, chunks * 256, scales, chunk ? chunks : 0, keys.b.q8.data_ptr<int8_t>(),
+                                                keys.b.q8.size(1), keys.b.scales.data_ptr<float>(), bptr, Q, R, chunks, scale_inv,
+                                                y.data_ptr(), R, code, act, &bounds, current_stream()),
+                     "bsi_b200_linear_i8_bounded");
     }
-    check_status(bsi_b200_quantize_pack_all(x.data_ptr(), code, Q, D, ldx, decimalPlaces, bits, chunk ? 1 : 0, clip_k, nullptr,
-                                            scales, nullptr, q8, chunks * 256, sq, nullptr, nullptr, current_stream()),
-                 "bsi_b200_quantize_pack_all");
-    float pack_ms = 0.f;
-    if (profile) {
-        cudaEventRecord(e1, at::cuda::getCurrentCUDAStream().stream());
-        cudaEventSynchronize(e1);
-        cudaEventElapsedTime(&pack_ms, e0, e1);
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-    }
-    g_last_quantize_ns = 0;
-    g_last_pack_ns = g_last_total_ns = static_cast<uint64_t>(pack_ms * 1.0e6);
-    bsi_dot_bounds bounds = dot_bounds(keys, bits, nullptr);
-    bounds.query_sq = sq;
-    bounds.query_sq_stride = chunks;
-    check_status(bsi_b200_linear_i8_bounded(q8, chunks * 256, scales, chunk ? chunks : 0, keys.b.q8.data_ptr<int8_t>(),
-                                            keys.b.q8.size(1), keys.b.scales.data_ptr<float>(), bptr, Q, R, chunks,
-                                            static_cast<float>(scale_inv), y.data_ptr(), R, code, BSI_ACT_NONE, &bounds,
-                                            current_stream()),
-                 "bsi_b200_linear_i8_bounded");
-    return y;
+}
+
+at::Tensor linear_forward(const Env& env, const at::Tensor& x2d, const PrebuiltBSIKeysCUDA& keys,
+                          const c10::optional<torch::Tensor>& bias, int decimalPlaces, bool relu = false) {
+    LinearTo to{&keys, &bias, at::Tensor()};
+    linear_forward(env, x2d, decimalPlaces, relu, &to, 1);
+    return to.y;
 }
 
 at::Tensor bsi_linear_forward(torch::Tensor x2d, py::capsule keyset_cuda_cap, c10::optional<torch::Tensor> bias,
@@ -895,6 +917,46 @@ py::object bsi_layer_forward(const torch::Tensor& x, const py::capsule& keyset_c
         y = y.view(shape);
     }
     return py::cast(y);
+}
+
+// One OPT decoder layer (pre-LN attention, ReLU MLP) whose six linears are BSI layers: the same ATen operators in the
+// same order as the module's Python forward and the BSI layers' own kernels, so the same bits. In Python the layer costs
+// 170 us of host time against 75 us of kernels (1024 tokens of OPT-125M). The query, key and value projections read one
+// packed image, and fc1's ReLU runs in its epilogue. linears: (key set, bias, decimal places) of q, k, v, out, fc1, fc2.
+// None where the environment asks for the layers' other forms.
+py::object opt_layer_forward(const torch::Tensor& x, const py::tuple& norms, const py::tuple& linears, int64_t heads) {
+    const Env env;
+    if ((env.profile_s != nullptr && std::strcmp(env.profile_s, "0") != 0) ||
+        (env.fp32 != nullptr && std::strcmp(env.fp32, "0") != 0) || env.bits_queries() == 0)
+        return py::none();
+    TORCH_CHECK(x.dim() == 3 && x.is_cuda(), "x must be a [batch, tokens, hidden] CUDA tensor");
+    const int64_t B = x.size(0), T = x.size(1), H = x.size(2);
+    if (B * T == 0) return py::none();
+    c10::cuda::CUDAGuard guard(x.device());
+    const PrebuiltBSIKeysCUDA* keys[6];
+    c10::optional<torch::Tensor> bias[6];
+    int dp[6];
+    for (int i = 0; i < 6; ++i) {
+        const py::tuple l = linears[i].cast<py::tuple>();
+        keys[i] = from_capsule<PrebuiltBSIKeysCUDA>(l[0].cast<py::capsule>(), "PrebuiltBSIKeysCUDA");
+        if (!l[1].is_none()) bias[i] = l[1].cast<torch::Tensor>();
+        dp[i] = l[2].cast<int>();
+    }
+    if (dp[0] != dp[1] || dp[0] != dp[2]) return py::none();
+    auto norm = [&](const at::Tensor& t, int first) {
+        return at::layer_norm(t, {H}, norms[first].cast<torch::Tensor>(), norms[first + 1].cast<torch::Tensor>(), norms[first + 2].cast<double>());
+    };
+    auto flat = [](const at::Tensor& t) { return t.reshape({-1, t.size(-1)}); };
+    auto split = [&](const at::Tensor& t) { return t.view({B, T, heads, H / heads}).transpose(1, 2); };
+    LinearTo qkv[3] = {{keys[0], &bias[0], at::Tensor()}, {keys[1], &bias[1], at::Tensor()}, {keys[2], &bias[2], at::Tensor()}};
+    linear_forward(env, flat(norm(x, 0)), dp[0], false, qkv, 3);
+    // query scaled in the model's type, attention with unit scaling: the order HuggingFace's OPT uses
+    const at::Tensor q = qkv[0].y.mul(std::pow(static_cast<double>(H / heads), -0.5));
+    const at::Tensor a = at::scaled_dot_product_attention(split(q), split(qkv[1].y), split(qkv[2].y), {}, 0.0, true, 1.0);
+    const at::Tensor o = linear_forward(env, flat(a.transpose(1, 2).reshape({B, T, H})), *keys[3], bias[3], dp[3]);
+    const at::Tensor mid = x.add(o.view({B, T, H}));
+    const at::Tensor f = linear_forward(env, flat(norm(mid, 3)), *keys[4], bias[4], dp[4], /*relu=*/true);
+    return py::cast(mid.add(linear_forward(env, f, *keys[5], bias[5], dp[5]).view({B, T, H})));
 }
 
 // Quantise + pack activations (query side: chunk scales) into tensors the caller owns: q8 [rows, >= d]
@@ -1425,6 +1487,8 @@ PYBIND11_MODULE(bsi_ops, m) {
           "pack + dot + cast + bias for one linear layer");
     m.def("bsi_layer_forward", &bsi_layer_forward, py::arg("x"), py::arg("keyset_cuda_cap"), py::arg("bias") = py::none(),
           py::arg("decimal_places") = 2, "bsi_linear_forward over the last dimension of x, in x's type; None under BSI_PROFILE");
+    m.def("opt_layer_forward", &opt_layer_forward, py::arg("x"), py::arg("norms"), py::arg("linears"), py::arg("heads"),
+          "One OPT decoder layer over BSI linears; None where the environment asks for another form of the layers");
     m.def("pack_queries_into", &pack_queries_into, py::arg("x2d"), py::arg("q8"), py::arg("scales"),
           py::arg("decimal_places"), "Pack activations into caller-owned int8 / chunk-scale tensors");
     m.def("linear_from_packed", &linear_from_packed, py::arg("q8"), py::arg("scales"), py::arg("keyset_cuda_cap"),

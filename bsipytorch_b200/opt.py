@@ -18,6 +18,8 @@ import torch
 import torch.nn.functional as F
 from torch import nn
 
+from .linear import BSIQuantizedLinear, _ops
+
 
 @dataclass
 class OPTConfig:
@@ -83,8 +85,41 @@ class OPTDecoderLayer(nn.Module):
         self.final_layer_norm = nn.LayerNorm(cfg.hidden_size)
 
     def forward(self, x):
+        y = self._native(x)
+        if y is not None:
+            return y
         x = x + self.self_attn(self.self_attn_layer_norm(x))
         return x + self.fc2(F.relu(self.fc1(self.final_layer_norm(x))))
+
+    def _native(self, x):
+        """The layer as one extension call where all six linears are fused BSI layers and nobody looks in between (no
+        gradients, no hooks); None otherwise. Same operators, same bits: what it saves is the Python between them."""
+        if torch.is_grad_enabled() or not x.is_cuda or x.dtype not in (torch.float16, torch.bfloat16, torch.float32):
+            return None
+        mods = self._modules
+        attn = mods["self_attn"]
+        inner = attn._modules
+        linears = (inner["q_proj"], inner["k_proj"], inner["v_proj"], inner["out_proj"], mods["fc1"], mods["fc2"])
+        norms = (mods["self_attn_layer_norm"], mods["final_layer_norm"])
+        if type(attn) is not OPTAttention:
+            return None
+        for m in linears:
+            if type(m) is not BSIQuantizedLinear or not m.fused:
+                return None
+        for m in norms:
+            if type(m) is not nn.LayerNorm:
+                return None
+        for m in (attn, *linears, *norms):
+            if m._forward_hooks or m._forward_pre_hooks:
+                return None
+        p0, p1 = norms[0]._parameters, norms[1]._parameters
+        y = _ops().opt_layer_forward(x, (p0["weight"], p0["bias"], norms[0].eps, p1["weight"], p1["bias"], norms[1].eps),
+                                     tuple((m._bsi_keys_cuda, m._buffers["bias"], m.decimalPlaces) for m in linears), attn.num_heads)
+        if y is not None:
+            n = x.shape[0] * x.shape[1]
+            for m in linears:
+                m.count(n)
+        return y
 
 
 class OPTDecoder(nn.Module):
@@ -161,7 +196,6 @@ def build_opt_bsi(name: str = "opt-125m", dtype=torch.float16, device="cuda", se
                   compress_threshold: float = 0.5, rank: int = 0, world: int = 1, group=None, keep_dense: bool = False):
     """Random-init OPT with BSI linears, built layer by layer so that the dense weights of a large
     model never sit in memory all at once. world > 1 shards every BSI linear along its output rows."""
-    from .linear import BSIQuantizedLinear
     from .sharded import BSIShardedLinear
 
     cfg = CONFIGS[name] if isinstance(name, str) else name
