@@ -784,6 +784,7 @@ struct LinearTo {
     const PrebuiltBSIKeysCUDA* keys;
     const c10::optional<torch::Tensor>* bias;
     at::Tensor y;
+    double factor = 1.0;      // of the whole finished output; 1: none
 };
 void linear_forward(const Env& env, const at::Tensor& x2d, int decimalPlaces, bool relu, LinearTo* to, int n) {
     TORCH_CHECK(x2d.dim() == 2 && x2d.is_cuda(), "x must be a 2D CUDA tensor");
@@ -822,6 +823,10 @@ void linear_forward(const Env& env, const at::Tensor& x2d, int decimalPlaces, bo
         TORCH_CHECK(decimalPlaces == keys.b.decimals, "Decimal mismatch between queries and keys: q=", decimalPlaces,
                     " k=", keys.b.decimals);
         at::Tensor& y = to[i].y;
+        // a factor rides in the epilogue for whole groups of 8 columns
+        const int64_t scaled = to[i].factor != 1.0 && R % 8 == 0 && fused && D > 0 ? R : 0;
+        const float factor = static_cast<float>(to[i].factor);
+        auto rest = [&] { if (to[i].factor != 1.0 && scaled == 0) y = y.mul(to[i].factor); };
         y = at::detail::empty_cuda({Q, R}, yt, x2d.device(), c10::nullopt);
         const float* bptr = nullptr;
         at::Tensor b32;
@@ -840,13 +845,15 @@ void linear_forward(const Env& env, const at::Tensor& x2d, int decimalPlaces, bo
             check_status(bsi_b200_cast_bias(out.data_ptr<float>(), R, bptr, Q, R, y.data_ptr(), R, code, current_stream()),
                          "bsi_b200_cast_bias");
             if (relu) y.relu_();
+            rest();
             continue;
         }
         if (one_launch && bsi_b200_linear_decode_fits(Q, R, D)) {
             check_status(bsi_b200_linear_decode(x.data_ptr(), code, ldx, D, decimalPlaces, bits, keys.b.q8.data_ptr<int8_t>(),
                                                 keys.b.q8.size(1), keys.b.scales.data_ptr<float>(), bptr, Q, R, scale_inv,
-                                                y.data_ptr(), R, act, current_stream()),
+                                                y.data_ptr(), R, act, scaled, factor, current_stream()),
                          "bsi_b200_linear_decode");
+            rest();
             continue;
         }
         if (q8 == nullptr) {
@@ -880,14 +887,15 @@ void linear_forward(const Env& env, const at::Tensor& x2d, int decimalPlaces, bo
         bounds.query_sq_stride = chunks;
         check_status(bsi_b200_linear_i8_bounded(q8, chunks * 256, scales, chunk ? chunks : 0, keys.b.q8.data_ptr<int8_t>(),
                                                 keys.b.q8.size(1), keys.b.scales.data_ptr<float>(), bptr, Q, R, chunks, scale_inv,
-                                                y.data_ptr(), R, code, act, &bounds, current_stream()),
+                                                y.data_ptr(), R, code, act, scaled, factor, &bounds, current_stream()),
                      "bsi_b200_linear_i8_bounded");
+        rest();
     }
 }
 
 at::Tensor linear_forward(const Env& env, const at::Tensor& x2d, const PrebuiltBSIKeysCUDA& keys,
                           const c10::optional<torch::Tensor>& bias, int decimalPlaces, bool relu = false) {
-    LinearTo to{&keys, &bias, at::Tensor()};
+    LinearTo to{&keys, &bias, at::Tensor(), 1.0};
     linear_forward(env, x2d, decimalPlaces, relu, &to, 1);
     return to.y;
 }
@@ -948,11 +956,12 @@ py::object opt_layer_forward(const torch::Tensor& x, const py::tuple& norms, con
     };
     auto flat = [](const at::Tensor& t) { return t.reshape({-1, t.size(-1)}); };
     auto split = [&](const at::Tensor& t) { return t.view({B, T, heads, H / heads}).transpose(1, 2); };
-    LinearTo qkv[3] = {{keys[0], &bias[0], at::Tensor()}, {keys[1], &bias[1], at::Tensor()}, {keys[2], &bias[2], at::Tensor()}};
+    LinearTo qkv[3] = {{keys[0], &bias[0], at::Tensor(), std::pow(static_cast<double>(H / heads), -0.5)},
+                       {keys[1], &bias[1], at::Tensor(), 1.0},
+                       {keys[2], &bias[2], at::Tensor(), 1.0}};
     linear_forward(env, flat(norm(x, 0)), dp[0], false, qkv, 3);
     // query scaled in the model's type, attention with unit scaling: the order HuggingFace's OPT uses
-    const at::Tensor q = qkv[0].y.mul(std::pow(static_cast<double>(H / heads), -0.5));
-    const at::Tensor a = at::scaled_dot_product_attention(split(q), split(qkv[1].y), split(qkv[2].y), {}, 0.0, true, 1.0);
+    const at::Tensor a = at::scaled_dot_product_attention(split(qkv[0].y), split(qkv[1].y), split(qkv[2].y), {}, 0.0, true, 1.0);
     const at::Tensor o = linear_forward(env, flat(a.transpose(1, 2).reshape({B, T, H})), *keys[3], bias[3], dp[3]);
     const at::Tensor mid = x.add(o.view({B, T, H}));
     const at::Tensor f = linear_forward(env, flat(norm(mid, 3)), *keys[4], bias[4], dp[4], /*relu=*/true);
@@ -994,7 +1003,8 @@ void pack_queries_into(torch::Tensor x2d, torch::Tensor q8, torch::Tensor scales
 // `out_dtype`, bias added, optionally ReLU. q8 [Q, d] int8 (row stride a multiple of 16), scales
 // [Q, d/256] float32 contiguous.
 at::Tensor linear_from_packed(torch::Tensor q8, torch::Tensor scales, py::capsule keyset_cuda_cap,
-                              c10::optional<torch::Tensor> bias, int decimalPlaces, py::object out_dtype, bool relu) {
+                              c10::optional<torch::Tensor> bias, int decimalPlaces, py::object out_dtype, bool relu,
+                              int64_t scaled_columns, double factor) {
     auto* keys = from_capsule<PrebuiltBSIKeysCUDA>(keyset_cuda_cap, "PrebuiltBSIKeysCUDA");
     TORCH_CHECK(q8.dim() == 2 && q8.is_cuda() && q8.scalar_type() == at::kChar && q8.stride(1) == 1, "q8 must be int8 [Q, d]");
     TORCH_CHECK(scales.is_cuda() && scales.scalar_type() == at::kFloat && scales.is_contiguous(), "scales must be contiguous float32");
@@ -1025,7 +1035,8 @@ at::Tensor linear_from_packed(torch::Tensor q8, torch::Tensor scales, py::capsul
                                             keys->b.q8.data_ptr<int8_t>(), keys->b.q8.size(1),
                                             keys->b.scales.data_ptr<float>(), bptr, Q, R, chunks,
                                             static_cast<float>(scale_inv), y.data_ptr(), R, code,
-                                            relu ? BSI_ACT_RELU : BSI_ACT_NONE, &bounds, current_stream()),
+                                            relu ? BSI_ACT_RELU : BSI_ACT_NONE, scaled_columns, static_cast<float>(factor), &bounds,
+                                            current_stream()),
                  "bsi_b200_linear_i8_bounded");
     return y;
 }
@@ -1493,7 +1504,9 @@ PYBIND11_MODULE(bsi_ops, m) {
           py::arg("decimal_places"), "Pack activations into caller-owned int8 / chunk-scale tensors");
     m.def("linear_from_packed", &linear_from_packed, py::arg("q8"), py::arg("scales"), py::arg("keyset_cuda_cap"),
           py::arg("bias"), py::arg("decimal_places"), py::arg("out_dtype"), py::arg("relu") = false,
-          "Dot of packed activations with a key set, cast + bias (+ ReLU) fused");
+          py::arg("scaled_columns") = 0, py::arg("factor") = 1.0,
+          "Dot of packed activations with a key set, cast + bias (+ ReLU) fused; the first scaled_columns output columns (a "
+          "multiple of 8) times factor");
     m.def("peer_alloc", &peer_alloc, py::arg("nbytes"), "Zero-filled device buffer other local processes can map: (uint8 tensor, handle bytes)");
     m.def("peer_open", &peer_open, py::arg("handle"), "Map a peer's buffer; returns its device address here");
     m.def("peer_close", &peer_close, py::arg("ptr"));

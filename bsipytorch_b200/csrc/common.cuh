@@ -61,6 +61,13 @@ struct RequantDst {
     float* scales[BSI_B200_MAX_PEERS];   // already offset to this linear's first output chunk
 };
 
+// What happens to a finished output value: ReLU, and a factor for the first scaled_cols columns (a multiple of 8).
+struct Finishing {
+    int relu;
+    int scaled_cols;
+    float factor;
+};
+
 // Bounds registered for a key image (bsi_b200_register_key_bounds): with them a dot can tell, per tile, that every
 // prefix of a chunk sum stays below 2^24 in magnitude, where integer accumulation gives the float32 chain's bits.
 struct KeyBounds {

@@ -14,13 +14,13 @@ int dot_i8_tcgen05(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_st
 
 int dot_i8_pair(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride, const int8_t* k8, int64_t ldk,
                 const float* bw0, const float* bias, int64_t Q, int64_t R, int64_t chunks, float scale_inv,
-                void* out, int64_t ldo, int y_dtype, int32_t* dbg_iacc, int force_bn, int relu,
+                void* out, int64_t ldo, int y_dtype, int32_t* dbg_iacc, int force_bn, const Finishing& fin,
                 const ScatterDst* scatter, const RequantDst* requant, const bsi_dot_bounds& bounds, cudaStream_t stream);
 
 bool decode_fits(int64_t Q, int64_t R, int64_t chunks);
 int dot_decode(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride, const int8_t* k8, int64_t ldk, const float* bw0,
                const float* bias, int64_t Q, int64_t R, int64_t chunks, float scale_inv, void* out, int64_t ldo, int y_dtype,
-               int relu, cudaStream_t stream, bool* taken);
+               const Finishing& fin, cudaStream_t stream, bool* taken);
 
 int dot_words_bmma(const uint64_t* A, const float* qs, int64_t qs_stride, int Sa, int64_t W,
                    const uint64_t* B, const float* Bw, int Sb, int64_t R, int64_t Q, float scale_inv,
@@ -145,7 +145,7 @@ extern "C" int bsi_b200_dot_i8_bounded(const int8_t* a8, int64_t lda, const floa
         if (dbg_iacc == nullptr && decode_fits(Q, R, chunks)) {
             bool taken = false;
             const int rc = dot_decode(a8, lda, qs, qs_stride, k8, ldk, bw0, nullptr, Q, R, chunks, scale_inv, out, ldo,
-                                      BSI_DTYPE_F32, 0, stream, &taken);
+                                      BSI_DTYPE_F32, Finishing{}, stream, &taken);
             if (rc != BSI_OK || taken) return rc;
         }
         engine = BSI_ENGINE_TCGEN05;
@@ -172,13 +172,14 @@ extern "C" int bsi_b200_linear_i8_act(const int8_t* a8, int64_t lda, const float
                                   int64_t Q, int64_t R, int64_t chunks, float scale_inv,
                                   void* y, int64_t ldy, int y_dtype, int activation, bsi_stream_t stream) {
     return bsi_b200_linear_i8_bounded(a8, lda, qs, qs_stride, k8, ldk, bw0, bias, Q, R, chunks, scale_inv, y, ldy, y_dtype,
-                                      activation, nullptr, stream);
+                                      activation, 0, 1.0f, nullptr, stream);
 }
 
 extern "C" int bsi_b200_linear_i8_bounded(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride,
                                           const int8_t* k8, int64_t ldk, const float* bw0, const float* bias,
                                           int64_t Q, int64_t R, int64_t chunks, float scale_inv, void* y, int64_t ldy,
-                                          int y_dtype, int activation, const bsi_dot_bounds* bounds, bsi_stream_t stream_) {
+                                          int y_dtype, int activation, int64_t scaled_cols, float factor,
+                                          const bsi_dot_bounds* bounds, bsi_stream_t stream_) {
     using namespace bsi;
     if (Q < 0 || R < 0 || chunks < 0) return fail(BSI_ERR_INVALID, "linear_i8: negative size");
     if (Q == 0 || R == 0) return BSI_OK;
@@ -195,15 +196,17 @@ extern "C" int bsi_b200_linear_i8_bounded(const int8_t* a8, int64_t lda, const f
     if (y_dtype != BSI_DTYPE_F32 && y_dtype != BSI_DTYPE_F16 && y_dtype != BSI_DTYPE_BF16)
         return fail(BSI_ERR_INVALID, "linear_i8: unknown y_dtype");
     if (int rc = require_sm100()) return rc;
-    const int relu = activation == BSI_ACT_RELU ? 1 : 0;
+    if (scaled_cols < 0 || scaled_cols > R || (scaled_cols & 7) != 0)
+        return fail(BSI_ERR_INVALID, "linear_i8: scaled_cols must be a multiple of 8 in [0, R]");
+    const Finishing fin{activation == BSI_ACT_RELU ? 1 : 0, static_cast<int>(scaled_cols), factor};
     if (decode_fits(Q, R, chunks)) {
         bool taken = false;
-        const int rc = dot_decode(a8, lda, qs, qs_stride, k8, ldk, bw0, bias, Q, R, chunks, scale_inv, y, ldy, y_dtype, relu,
+        const int rc = dot_decode(a8, lda, qs, qs_stride, k8, ldk, bw0, bias, Q, R, chunks, scale_inv, y, ldy, y_dtype, fin,
                                   static_cast<cudaStream_t>(stream_), &taken);
         if (rc != BSI_OK || taken) return rc;
     }
     return dot_i8_pair(a8, lda, qs, qs_stride, k8, ldk, bw0, bias, Q, R, chunks, scale_inv, y, ldy, y_dtype,
-                       nullptr, 0, relu, nullptr, nullptr, resolve_bounds(bounds, a8, k8, R), static_cast<cudaStream_t>(stream_));
+                       nullptr, 0, fin, nullptr, nullptr, resolve_bounds(bounds, a8, k8, R), static_cast<cudaStream_t>(stream_));
 }
 
 extern "C" int bsi_b200_linear_i8_scatter(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride,
@@ -241,7 +244,7 @@ extern "C" int bsi_b200_linear_i8_scatter(const int8_t* a8, int64_t lda, const f
     }
     if (int rc = require_sm100()) return rc;
     return dot_i8_pair(a8, lda, qs, qs_stride, k8, ldk, bw0, bias, Q, R, chunks, scale_inv, nullptr, ldy, y_dtype,
-                       nullptr, 0, activation == BSI_ACT_RELU ? 1 : 0, &sc, nullptr, resolve_bounds(nullptr, a8, k8, R), static_cast<cudaStream_t>(stream_));
+                       nullptr, 0, Finishing{activation == BSI_ACT_RELU ? 1 : 0, 0, 1.0f}, &sc, nullptr, resolve_bounds(nullptr, a8, k8, R), static_cast<cudaStream_t>(stream_));
 }
 
 extern "C" int bsi_b200_linear_i8_requant(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride,
@@ -285,7 +288,7 @@ extern "C" int bsi_b200_linear_i8_requant(const int8_t* a8, int64_t lda, const f
     }
     if (int rc = require_sm100()) return rc;
     return dot_i8_pair(a8, lda, qs, qs_stride, k8, ldk, bw0, bias, Q, R, chunks, scale_inv, q8_dst[0], R, layer_dtype,
-                       nullptr, 0, activation == BSI_ACT_RELU ? 1 : 0, nullptr, &rq, resolve_bounds(nullptr, a8, k8, R), static_cast<cudaStream_t>(stream_));
+                       nullptr, 0, Finishing{activation == BSI_ACT_RELU ? 1 : 0, 0, 1.0f}, nullptr, &rq, resolve_bounds(nullptr, a8, k8, R), static_cast<cudaStream_t>(stream_));
 }
 
 extern "C" int bsi_b200_linear_i8(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride,

@@ -52,7 +52,7 @@ struct DecodeArgs {
     float scale_inv;
     void* out;
     int64_t ldo;
-    int relu;
+    Finishing fin;
 };
 
 __device__ __forceinline__ uint4 ld_stream(const int8_t* p) {
@@ -245,7 +245,8 @@ __global__ void __launch_bounds__(kThreads, 1) dot_decode_kernel(const DecodeArg
                 if (!last) *keep = acc;
                 else if (row < p.R)
                     static_cast<OutT*>(p.out)[q * p.ldo + row] =
-                        relu_if<OutT>(finish<OutT>((acc * w) * p.scale_inv, bv, p.bias != nullptr), p.relu != 0);
+                        scaled_if<OutT>(relu_if<OutT>(finish<OutT>((acc * w) * p.scale_inv, bv, p.bias != nullptr), p.fin.relu != 0),
+                                        row < p.fin.scaled_cols, p.fin.factor);
             }
         }
     }
@@ -309,11 +310,11 @@ bool decode_fits(int64_t Q, int64_t R, int64_t chunks) {
 
 int dot_decode(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride, const int8_t* k8, int64_t ldk, const float* bw0,
                const float* bias, int64_t Q, int64_t R, int64_t chunks, float scale_inv, void* out, int64_t ldo, int y_dtype,
-               int relu, cudaStream_t stream, bool* taken) {
+               const Finishing& fin, cudaStream_t stream, bool* taken) {
     DecodeArgs a = {};
     a.a8 = a8; a.lda = lda; a.qs = qs; a.qs_stride = qs_stride; a.k8 = k8; a.ldk = ldk; a.bw0 = bw0; a.bias = bias;
     a.Q = static_cast<int>(Q); a.R = static_cast<int>(R); a.chunks = static_cast<int>(chunks);
-    a.scale_inv = scale_inv; a.out = out; a.ldo = ldo; a.relu = relu;
+    a.scale_inv = scale_inv; a.out = out; a.ldo = ldo; a.fin = fin;
     const int nt = Q <= 8 ? 1 : 2;
     unsigned grid = 0;
     const int smem = plan_decode(&a, nt, &grid);
@@ -332,7 +333,8 @@ int dot_decode(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride
 
 extern "C" int bsi_b200_linear_decode(const void* x, int x_dtype, int64_t ldx, int64_t D, int decimal_places, int bits,
                                       const int8_t* k8, int64_t ldk, const float* bw0, const float* bias, int64_t Q, int64_t R,
-                                      float scale_inv, void* y, int64_t ldy, int activation, bsi_stream_t stream_) {
+                                      float scale_inv, void* y, int64_t ldy, int activation, int64_t scaled_cols, float factor,
+                                      bsi_stream_t stream_) {
     using namespace bsi;
     if (Q < 0 || R < 0 || D <= 0 || ldx < D) return fail(BSI_ERR_INVALID, "linear_decode: bad sizes");
     if (Q == 0 || R == 0) return BSI_OK;
@@ -344,6 +346,7 @@ extern "C" int bsi_b200_linear_decode(const void* x, int x_dtype, int64_t ldx, i
     if (bits < 2 || bits > 8) return fail(BSI_ERR_UNSUPPORTED, "linear_decode: bits must be in [2, 8]");
     if (decimal_places < 0 || decimal_places > 8) return fail(BSI_ERR_UNSUPPORTED, "linear_decode: decimal_places must be in [0, 8]");
     if (activation != BSI_ACT_NONE && activation != BSI_ACT_RELU) return fail(BSI_ERR_INVALID, "linear_decode: unknown activation");
+    if (scaled_cols < 0 || scaled_cols > R) return fail(BSI_ERR_INVALID, "linear_decode: bad scaled_cols");
     if (x_dtype != BSI_DTYPE_F32 && x_dtype != BSI_DTYPE_F16 && x_dtype != BSI_DTYPE_BF16)
         return fail(BSI_ERR_INVALID, "linear_decode: unknown x_dtype");
     if (!bsi_b200_linear_decode_fits(Q, R, D)) return fail(BSI_ERR_UNSUPPORTED, "linear_decode: too many query chunks for this form");
@@ -351,7 +354,8 @@ extern "C" int bsi_b200_linear_decode(const void* x, int x_dtype, int64_t ldx, i
     DecodeArgs a = {};
     a.x = x; a.ldx = ldx; a.D = D; a.bits = bits; a.k8 = k8; a.ldk = ldk; a.bw0 = bw0; a.bias = bias;
     a.Q = static_cast<int>(Q); a.R = static_cast<int>(R); a.chunks = static_cast<int>(chunks);
-    a.scale_inv = scale_inv; a.out = y; a.ldo = ldy; a.relu = activation == BSI_ACT_RELU ? 1 : 0;
+    a.scale_inv = scale_inv; a.out = y; a.ldo = ldy;
+    a.fin = Finishing{activation == BSI_ACT_RELU ? 1 : 0, static_cast<int>(scaled_cols), factor};
     a.dec_mult = 1;
     for (int i = 0; i < decimal_places; ++i) a.dec_mult *= 10u;
     a.dec_scale = static_cast<double>(a.dec_mult);

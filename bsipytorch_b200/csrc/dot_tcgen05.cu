@@ -468,7 +468,7 @@ template <int BN, bool DBG, typename OutT, bool REQ = false, int SPLIT = 1>
 int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo, const CUtensorMap& mt, int vector_store,
                 const float* qs, int64_t qs_stride, const float* bw0, const float* bias, int Q, int R, int chunks,
                 float scale_inv, void* out, int64_t ldo, int32_t* dbg, const ScatterDst& scatter,
-                const RequantDst& requant, const float* k_abs_sum, float q_abs_max, const float* q_sq, int64_t q_sq_stride,
+                const RequantDst& requant, const Finishing& fin, const float* k_abs_sum, float q_abs_max, const float* q_sq, int64_t q_sq_stride,
                 cudaStream_t stream, int* max_clusters_out = nullptr /* only asks how many clusters fit at once */) {
     using C = pair::Cfg<BN, OutT, REQ, SPLIT>;
     static int max_clusters[64] = {0};   // per instantiation
@@ -509,7 +509,7 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap&
     cfg.gridDim = dim3(2 * SPLIT * clusters, 1, 1);
     BSI_CUDA_TRY(cudaLaunchKernelEx(&cfg, pair::dot_i8_tcgen05_pair_kernel<BN, DBG, OutT, REQ, SPLIT>, ma, mb, mo, mt, vector_store, qs,
                                     qs_stride, bw0, bias, Q, R, chunks, tiles_m, tiles_total, scale_inv, out, ldo, dbg, scatter, requant,
-                                    k_abs_sum, q_abs_max, q_sq, q_sq_stride));
+                                    fin, k_abs_sum, q_abs_max, q_sq, q_sq_stride));
     return check_launch("dot_i8 tcgen05 pair launch");
 }
 
@@ -545,7 +545,7 @@ int resident_clusters() {
     if (cached[dev] == 0) {
         const CUtensorMap none = {};
         if (launch_pair<64, false, float, false, SPLIT>(none, none, none, none, 0, nullptr, 0, nullptr, nullptr, 0, 0, 1, 0.0f, nullptr, 0,
-                                                        nullptr, ScatterDst{}, RequantDst{}, nullptr, 0.0f, nullptr, 0, nullptr, &n) != BSI_OK)
+                                                        nullptr, ScatterDst{}, RequantDst{}, Finishing{}, nullptr, 0.0f, nullptr, 0, nullptr, &n) != BSI_OK)
             n = 0;
         cached[dev] = n > 0 ? n : -1;
     }
@@ -585,7 +585,7 @@ int pick_split(int64_t Q, int64_t R, int64_t chunks, int unsplit_bn, int* bn) {
 // Paired-CTA engine with the output type and the bias chosen at run time (y_dtype: BSI_DTYPE_*).
 int dot_i8_pair(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride, const int8_t* k8, int64_t ldk,
                 const float* bw0, const float* bias, int64_t Q, int64_t R, int64_t chunks, float scale_inv,
-                void* out, int64_t ldo, int y_dtype, int32_t* dbg_iacc, int force_bn, int relu,
+                void* out, int64_t ldo, int y_dtype, int32_t* dbg_iacc, int force_bn, const Finishing& fin,
                 const ScatterDst* scatter_in, const RequantDst* requant_in, const bsi_dot_bounds& bounds, cudaStream_t stream) {
     RequantDst requant = {};
     if (requant_in != nullptr) {
@@ -637,7 +637,7 @@ int dot_i8_pair(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_strid
     const int per16 = 16 / esz;
     const int vector_store =
         (((reinterpret_cast<uintptr_t>(out) & 15) == 0 && (ldo % per16) == 0 && (R % per16) == 0) ? 1 : 0) |
-        (relu ? 2 : 0);   // the kernel's store_flags
+        (fin.relu ? 2 : 0);   // the kernel's store_flags
     // bulk stores into the one output matrix; several destinations (scatter) keep plain stores
     CUtensorMap mo = {}, mt = {};
     int store_flags = vector_store;
@@ -650,7 +650,7 @@ int dot_i8_pair(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_strid
     if (parts > 1) {
 #define BSI_SPLIT_T(BN_, S_, T_)                                                                                            \
     launch_pair<BN_, false, T_, false, S_>(ma, mb, mo, mt, store_flags, qs, qs_stride, bw0, bias, q, r, c, scale_inv, out, ldo, \
-                                           nullptr, scatter, requant, kabs, qabs, qsq, qsq_stride, stream)
+                                           nullptr, scatter, requant, fin, kabs, qabs, qsq, qsq_stride, stream)
 #define BSI_SPLIT(BN_, S_)                                                    \
     (y_dtype == BSI_DTYPE_F16    ? BSI_SPLIT_T(BN_, S_, __half)               \
      : y_dtype == BSI_DTYPE_BF16 ? BSI_SPLIT_T(BN_, S_, __nv_bfloat16)        \
@@ -662,7 +662,7 @@ int dot_i8_pair(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_strid
     }
 #define BSI_PAIR_T(BN_, DBG_, T_)                                                                              \
     launch_pair<BN_, DBG_, T_>(ma, mb, mo, mt, store_flags, qs, qs_stride, bw0, bias, q, r, c, scale_inv, out, ldo,  \
-                               dbg_iacc, scatter, requant, kabs, qabs, qsq, qsq_stride, stream)
+                               dbg_iacc, scatter, requant, fin, kabs, qabs, qsq, qsq_stride, stream)
 #define BSI_PAIR(BN_)                                                                   \
     (y_dtype == BSI_DTYPE_F16    ? BSI_PAIR_T(BN_, false, __half)                       \
      : y_dtype == BSI_DTYPE_BF16 ? BSI_PAIR_T(BN_, false, __nv_bfloat16)                \
@@ -671,9 +671,9 @@ int dot_i8_pair(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_strid
     if (requant.n > 0) {
         if (y_dtype == BSI_DTYPE_F16)
             return launch_pair<256, false, __half, true>(ma, mb, mo, mt, store_flags, qs, qs_stride, bw0, bias, q, r, c, scale_inv,
-                                                         out, ldo, nullptr, scatter, requant, kabs, qabs, qsq, qsq_stride, stream);
+                                                         out, ldo, nullptr, scatter, requant, fin, kabs, qabs, qsq, qsq_stride, stream);
         return launch_pair<256, false, __nv_bfloat16, true>(ma, mb, mo, mt, store_flags, qs, qs_stride, bw0, bias, q, r, c,
-                                                            scale_inv, out, ldo, nullptr, scatter, requant, kabs, qabs, qsq,
+                                                            scale_inv, out, ldo, nullptr, scatter, requant, fin, kabs, qabs, qsq,
                                                             qsq_stride, stream);
     }
 #define BSI_PAIR_F32(BN_) (dbg_iacc ? BSI_PAIR_T(BN_, true, float) : BSI_PAIR_T(BN_, false, float))
@@ -700,7 +700,7 @@ int dot_i8_tcgen05(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_st
     const bool want_pair = force_bn == 0 || force_bn >= 2000;
     if (want_pair) {
         return dot_i8_pair(a8, lda, qs, qs_stride, k8, ldk, bw0, nullptr, Q, R, chunks, scale_inv, out, ldo,
-                           BSI_DTYPE_F32, dbg_iacc, force_bn ? force_bn - 2000 : 0, /*relu=*/0, nullptr, nullptr, bounds, stream);
+                           BSI_DTYPE_F32, dbg_iacc, force_bn ? force_bn - 2000 : 0, Finishing{}, nullptr, nullptr, bounds, stream);
     }
     const int bn = force_bn;
     CUtensorMap ma, mb;

@@ -244,6 +244,24 @@ __device__ __forceinline__ uint4 finish16(const float* acc, const float* colw, c
                           finish2(scaled2(acc + 6, v.z, v.w, scale2), b.w, has_bias, relu, OutT()));
     }
 }
+// 16 bytes of finished values times a factor, rounded to the output type again.
+__device__ __forceinline__ uint4 times(uint4 o, float factor, float) {
+    return make_uint4(__float_as_uint(__uint_as_float(o.x) * factor), __float_as_uint(__uint_as_float(o.y) * factor),
+                      __float_as_uint(__uint_as_float(o.z) * factor), __float_as_uint(__uint_as_float(o.w) * factor));
+}
+__device__ __forceinline__ uint32_t times2(uint32_t v, float factor, __half) {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&v));
+    const __half2 y = __floats2half2_rn(f.x * factor, f.y * factor);
+    return *reinterpret_cast<const uint32_t*>(&y);
+}
+__device__ __forceinline__ uint32_t times2(uint32_t v, float factor, __nv_bfloat16) {
+    const __nv_bfloat162 y = __floats2bfloat162_rn(__uint_as_float(v << 16) * factor, __uint_as_float(v & 0xffff0000u) * factor);
+    return *reinterpret_cast<const uint32_t*>(&y);
+}
+template <typename OutT>
+__device__ __forceinline__ uint4 times(uint4 o, float factor, OutT t) {
+    return make_uint4(times2(o.x, factor, t), times2(o.y, factor, t), times2(o.z, factor, t), times2(o.w, factor, t));
+}
 __device__ __forceinline__ float cast_bias(float b, float) { return b; }
 __device__ __forceinline__ __half cast_bias(float b, __half) { return __float2half_rn(b); }
 __device__ __forceinline__ __nv_bfloat16 cast_bias(float b, __nv_bfloat16) { return __float2bfloat16_rn(b); }
@@ -348,7 +366,7 @@ template <typename OutT, int kCols>
 __device__ __forceinline__ void store_columns(const float (&acc)[kCols], uint8_t* places, uint8_t* own, const float* colw, const OutT* colb,
                                               const CUtensorMap& map_o, const CUtensorMap& map_t, OutT* __restrict__ outp, int64_t ldo,
                                               int row_shift, int row_base, int Q, int col, int R, float scale_inv, bool has_bias, bool relu,
-                                              int store_flags) {
+                                              const Finishing& fin, int store_flags) {
     const int lane = threadIdx.x & 31;
     constexpr int E = static_cast<int>(sizeof(OutT));
     constexpr int kPerChunk = 16 / E;                        // values per 16-byte piece
@@ -376,6 +394,13 @@ __device__ __forceinline__ void store_columns(const float (&acc)[kCols], uint8_t
                     const int j = cg + ch * kPerChunk;
                     if (j < kCols)
                         *reinterpret_cast<uint4*>(dst + (swz << 4)) = finish16<OutT>(acc + j, colw + j, colb + j, scale2, has_bias, relu);
+                }
+            }
+            if (col + cg < fin.scaled_cols) {      // a second look at the lane's own row, so that other blocks pay one branch
+                for (int ch = 0; ch < nch; ++ch) {
+                    if (col + cg + ch * kPerChunk >= fin.scaled_cols) break;
+                    uint4* o = reinterpret_cast<uint4*>(dst + ((whole ? (ch ^ (lane & 7)) : (ch ^ ((lane >> 1) & 3))) << 4));
+                    *o = times(*o, fin.factor, OutT());
                 }
             }
             if (bulk) {
@@ -428,7 +453,8 @@ __device__ __forceinline__ void store_columns(const float (&acc)[kCols], uint8_t
         for (int i = 0; i < kWide; ++i) {
             const int rr = i * (32 / kWide) + lane / kWide;
             const float v = stage[rr * kWide + (cj ^ (rr & (kWide - 1)))];
-            if (i * (32 / kWide) < rows) *o = relu_if<OutT>(finish<OutT>((v * w) * scale_inv, bv, has_bias), relu);
+            if (i * (32 / kWide) < rows)
+                *o = scaled_if<OutT>(relu_if<OutT>(finish<OutT>((v * w) * scale_inv, bv, has_bias), relu), col + j < fin.scaled_cols, fin.factor);
             o += (32 / kWide) * ldo;
         }
         __syncwarp();
@@ -443,7 +469,7 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
     const float* __restrict__ qs, int64_t qs_stride, const float* __restrict__ bw0,
     const float* __restrict__ bias, int Q, int R, int chunks, int tiles_m, int tiles_total, float scale_inv,
     void* __restrict__ out, int64_t ldo, int32_t* __restrict__ dbg_iacc, const ScatterDst scatter,
-    const RequantDst requant, const float* __restrict__ k_abs_sum, float q_abs_max,
+    const RequantDst requant, const Finishing fin, const float* __restrict__ k_abs_sum, float q_abs_max,
     const float* __restrict__ q_sq, int64_t q_sq_stride) {
     using C = Cfg<BN, OutT, REQ, SPLIT>;
     constexpr int kStages = C::kStages;
@@ -882,7 +908,7 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                     const int cs = col0 + part * kShare;
                     store_columns<OutT, kShare>(val, nullptr, my_store, colw + cs, colb + cs, map_o, map_t, static_cast<OutT*>(out), ldo, 0,
                                                 tm * 256 + static_cast<int>(rank) * BM + quad * 32, Q, n0 + cs, R, scale_inv, has_bias, relu,
-                                                store_flags);
+                                                fin, store_flags);
                     continue;
                 }
                 if (!whole_tile) continue;
@@ -1003,7 +1029,7 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
             const bool last = tile + num_pairs >= tiles_total;
             store_columns<OutT, kCols>(acc, (store_flags & 4) && last ? smem + ew * kBlocks<OutT, kCols>() * 4096 : nullptr, my_store, colw + col0,
                                        colb + col0, map_o, map_t, outp, ldo, row_shift, row_base, Q, n0 + col0, R, scale_inv, has_bias, relu,
-                                       store_flags);
+                                       fin, store_flags);
         }
         if (lane == 0) tma_store_wait_read();      // shared memory is read until then
     }

@@ -33,5 +33,12 @@ __device__ __forceinline__ OutT relu_if(OutT v, bool relu) {
     return (relu && static_cast<float>(v) < 0.0f) ? static_cast<OutT>(0.0f) : v;
 }
 
+// The finished value times a factor, rounded to the output type again: what a separate elementwise multiplication of the
+// layer's output by a scalar computes (OPT's query scaling).
+template <typename OutT>
+__device__ __forceinline__ OutT scaled_if(OutT v, bool on, float factor) {
+    return on ? static_cast<OutT>(static_cast<float>(v) * factor) : v;
+}
+
 }  // namespace
 }  // namespace bsi

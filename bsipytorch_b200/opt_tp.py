@@ -61,6 +61,10 @@ class BsiDeviceOps:
     def linear(self, q8, scales, keys, bias, out_dtype, relu=False):
         return self.m.linear_from_packed(q8, scales, keys, bias, self.dp, out_dtype, relu)
 
+    def linear_scaled(self, q8, scales, keys, bias, out_dtype, columns, factor):
+        """linear whose first `columns` output columns (a multiple of 8) are multiplied by `factor` in the epilogue."""
+        return self.m.linear_from_packed(q8, scales, keys, bias, self.dp, out_dtype, False, columns, factor)
+
     def add_ln_pack(self, x, delta, ln, q8_ptrs, ld8, scale_ptrs, scale_ld):
         """x + delta (delta may be None), LayerNorm `ln` of the sum, packed to the given addresses; returns the sum."""
         return self.m.add_layernorm_pack(x, delta, ln.weight, ln.bias, ln.eps, q8_ptrs, ld8, scale_ptrs, scale_ld, self.dp)
@@ -241,11 +245,20 @@ class TPDecoderLayer(nn.Module):
         return recv.view(G, Q // G, Rl).permute(1, 0, 2).reshape(Q // G, G * Rl)
 
     # -- forward ---------------------------------------------------------------------------------
+    def _qkv(self, q8, sc):
+        """[Q, 3 * H/G], the query block scaled in the model's type (HuggingFace's OPT scales it before an attention with
+        unit scaling): in the epilogue on the extension, where the separate pass over a strided block cost 42 us."""
+        Hl, factor = self.h_hi - self.h_lo, self.head_dim ** -0.5
+        if isinstance(self.ops, BsiDeviceOps) and Hl % 8 == 0:
+            return self.ops.linear_scaled(q8, sc, self.keys_qkv, self.bias_qkv, self.dtype, Hl, factor)
+        qkv = self.ops.linear(q8, sc, self.keys_qkv, self.bias_qkv, self.dtype)
+        qkv[:, :Hl] *= factor
+        return qkv
+
     def _attention(self, qkv, B, T):
         Hl, nh, hd = self.h_hi - self.h_lo, self.local_heads, self.head_dim
         q, k, v = (qkv[:, i * Hl:(i + 1) * Hl].view(B, T, nh, hd).transpose(1, 2) for i in range(3))
-        # query scaled in the model's type, attention with unit scaling: the order HuggingFace's OPT uses
-        attn = F.scaled_dot_product_attention(q * hd ** -0.5, k, v, is_causal=True, scale=1.0)   # [B, nh, T, hd]
+        attn = F.scaled_dot_product_attention(q, k, v, is_causal=True, scale=1.0)   # [B, nh, T, hd]
         return attn.transpose(1, 2).reshape(B * T, Hl)
 
     def forward_peer(self, x_loc, delta, B, T, px: "PeerExchange"):
@@ -274,7 +287,7 @@ class TPDecoderLayer(nn.Module):
             px.barrier()
 
         x_loc = ln_rows_to_all(x_loc, delta, self.self_attn_layer_norm)
-        qkv = ops.linear(px.R_q8, px.R_sc, self.keys_qkv, self.bias_qkv, dt)          # [Q, 3 * H/G]
+        qkv = self._qkv(px.R_q8, px.R_sc)
         attn = self._attention(qkv, B, T)
         px.pack_to_all(attn, ops.dp, "C1_q8", "C1_sc", g * Hl, g * (Hl // 256) * 4, H, hc, px.Q)
         to_owner(px.C1_q8, px.C1_sc, self.keys_out, self.bias_out)
@@ -312,7 +325,7 @@ class TPDecoderLayer(nn.Module):
             return x, q8, sc
 
         x_loc, q8, sc = ln_pack(x_loc, delta, self.self_attn_layer_norm)
-        qkv = ops.linear(q8, sc, self.keys_qkv, self.bias_qkv, dt)                   # [Q, 3 * H/G]
+        qkv = self._qkv(q8, sc)
         attn = self._attention(qkv, B, T)
         q8, sc = self._pack_gather_cols(attn)
         o = ops.linear(q8, sc, self.keys_out, self.bias_out, dt)                      # [Q, H/G]

@@ -243,7 +243,10 @@ int bsi_b200_dot_i8_bounded(const int8_t* a8, int64_t lda, const float* qs, int6
 int bsi_b200_linear_i8_bounded(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride,
                                const int8_t* k8, int64_t ldk, const float* bw0, const float* bias,
                                int64_t Q, int64_t R, int64_t chunks, float scale_inv, void* y, int64_t ldy, int y_dtype,
-                               int activation, const bsi_dot_bounds* bounds, bsi_stream_t stream);
+                               int activation, int64_t scaled_cols, float factor, const bsi_dot_bounds* bounds,
+                               bsi_stream_t stream);
+/* (scaled_cols, a multiple of 8: the finished values of the first scaled_cols columns are multiplied by factor and
+ * rounded to the output type once more, as y[:, :scaled_cols] * factor does; 0: none.) */
 
 /* A linear layer of a few rows in one launch: the activations x [Q, D] (row stride ldx) are quantised (chunk scales)
  * by every CTA for itself, dotted with the keys, cast to x's type, bias (float32, may be NULL) and activation applied.
@@ -253,7 +256,8 @@ int bsi_b200_linear_i8_bounded(const int8_t* a8, int64_t lda, const float* qs, i
 int bsi_b200_linear_decode_fits(int64_t Q, int64_t R, int64_t D);
 int bsi_b200_linear_decode(const void* x, int x_dtype, int64_t ldx, int64_t D, int decimal_places, int bits,
                            const int8_t* k8, int64_t ldk, const float* bw0, const float* bias, int64_t Q, int64_t R,
-                           float scale_inv, void* y, int64_t ldy, int activation, bsi_stream_t stream);
+                           float scale_inv, void* y, int64_t ldy, int activation, int64_t scaled_cols, float factor,
+                           bsi_stream_t stream);
 
 /* Linear whose finished output is re-quantised for the next linear inside the epilogue, so that the
  * layer-type [Q, R] matrix is never written: y = activation(cast(out) + cast(bias)) in layer_dtype

@@ -50,7 +50,10 @@ def test_split_dot_and_layer(Q, R, D, broken):
     for dtype in (torch.float16, torch.bfloat16):
         y = torch.full((Q, R), float("nan"), dtype=dtype, device=DEV)
         capi.check(L.bsi_b200_linear_i8_bounded(capi.ptr(q8), ld, capi.ptr(scales), chunks, capi.ptr(kb["q8"]), ld, capi.ptr(kb["scales"]),
-                                                capi.ptr(bias), Q, R, chunks, inv, capi.ptr(y), R, H._DT[dtype], 1, C.byref(given),
+                                                capi.ptr(bias), Q, R, chunks, inv, capi.ptr(y), R, H._DT[dtype], 1, R // 16 * 8, C.c_float(0.3),
+                                                C.byref(given),
                                                 capi.stream_ptr()))
-        assert torch.equal(y, torch.relu(want.to(dtype) + bias.to(dtype)))
+        z = torch.relu(want.to(dtype) + bias.to(dtype))
+        z[:, : R // 16 * 8] *= 0.3
+        assert torch.equal(y, z)
     assert capi.device_status() == 0
