@@ -699,7 +699,7 @@ __device__ __noinline__ int generic_row_shift(const T* xr, int64_t chunks, int64
 // Bound by HBM: 4 bytes in and 1 + bits / 8 out per element (float32). A row with NaN, inf or |x * 10^dp| beyond the
 // fast range is redone from memory on the 64-bit path, every warp finding the shift for itself.
 template <typename T, int CPW>
-__global__ void __launch_bounds__(256, CPW * RawLane<T>::kVecs <= 4 ? 4 : 2) quantize_pack_row_fast_kernel(
+__global__ void __launch_bounds__(256, CPW * RawLane<T>::kVecs <= 8 ? 4 : 2) quantize_pack_row_fast_kernel(
     const T* __restrict__ x, int64_t rows, int64_t D, int64_t ldx, double dec_scale, uint32_t dec_mult, int bits,
     int chunks, int64_t W, int wpr_log2, u64* __restrict__ words, float* __restrict__ scales,
     int32_t* __restrict__ shifts, int8_t* __restrict__ q8, int64_t ld8, int vec_ok, float* __restrict__ slice_weights,
@@ -971,8 +971,9 @@ int launch_slice_weights(const float* scales, const PackArgs& a) {
 }
 
 // Row mode: the register-resident kernel for rows of up to 64 chunks (8 warps x 8 chunks), decimal_places in [0, 8]
-// and no clipping; the two-pass 64-bit kernel otherwise. Rows of fewer than 8 chunks share a block:
-// as many warps per row as it has chunks (rounded up to a power of two), then chunks per warp.
+// and no clipping; the two-pass 64-bit kernel otherwise. As few warps on a row (1, 2, 4 or 8) as leave each four chunks at
+// most, more than that only on the longest rows: what a row costs beside its chunks is paid per warp (16384 x 4096
+// float32: 96 us with 8 warps of 2 chunks, 84 us with 4 of 4; 4096 x 768: 9.2 us with 4 warps of 1, 7.2 us with 2 of 2).
 template <typename T>
 int launch_row(const T* x, const PackArgs& a) {
     if (a.dec_mult == 0u || a.clip_k > 0.0f || a.chunks > 64) {
@@ -990,7 +991,7 @@ int launch_row(const T* x, const PackArgs& a) {
         return BSI_OK;
     }
     int wpr_log2 = 0;
-    while (wpr_log2 < 3 && (1 << wpr_log2) < a.chunks) ++wpr_log2;
+    while (wpr_log2 < 3 && ((a.chunks + (1 << wpr_log2) - 1) >> wpr_log2) > 4) ++wpr_log2;
     const int64_t per_block = 8 >> wpr_log2;
     const unsigned grid = static_cast<unsigned>((a.rows + per_block - 1) / per_block);
     const int cpw = static_cast<int>((a.chunks + (1 << wpr_log2) - 1) >> wpr_log2);

@@ -10,8 +10,8 @@ from oracle import oracle as o
 pytestmark = pytest.mark.gpu
 
 
-# edges of the kernel's splits: one warp per row up to 256 elements, 8 warps from 5 chunks on, then 2, 4, 8 chunks per
-# warp, and the two-pass kernel from 16385 elements; ragged tails of a lane, a word and a chunk
+# edges of the kernel's splits: one warp per row up to 4 chunks, then 2, 4 and 8, 8 chunks per warp from 33 chunks on, and
+# the two-pass kernel from 16385 elements; ragged tails of a lane, a word and a chunk
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("rows,D", [(9, 1), (5, 255), (17, 256), (6, 257), (3, 1023), (3, 2048), (2, 2049), (2, 4103), (2, 8200),
                                     (2, 16384), (2, 16385)])
