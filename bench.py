@@ -325,9 +325,9 @@ def run_hbm(args, rank, world, local_rank):
         step(0)
         torch.cuda.synchronize()
         stream_words = int(total.item())
-        # flags pass reads the words once, the size pass the compressible slices again, emit reads all and writes the stream
+        # the sizes pass and the emit pass read the words once each, emit writes the stream
         bytes_step = 2 * S * W * 8 + stream_words * 8 + S * 24
-        launches, kernel = 4, "ewah_flags_kernel + ewah_size_kernel + ewah_offsets_kernel + ewah_emit_kernel"
+        launches, kernel = 2, "ewah_sizes_kernel + ewah_emit_blocks_kernel"
         extra = {"stream_words": stream_words, "input_words": S * W}
     else:
         lean = spec["lean"]

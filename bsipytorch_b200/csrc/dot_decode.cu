@@ -372,9 +372,12 @@ extern "C" int bsi_b200_linear_decode(const void* x, int x_dtype, int64_t ldx, i
 #undef BSI_DECODE_FUSED
 }
 
-// Every CTA quantises all Q x chunks groups (16 warps; 128 groups add 3.4 us to 4096 x 4096), so the one-launch form ends
-// where that costs more than a packing kernel and its launch.
+// Every CTA quantises all Q x chunks groups (16 warps; 128 groups add 3.4 us to 4096 x 4096), which a packing kernel does
+// once, in about 1 us beside the dot's set-up. Small key sets take the one launch up to 128 groups all the same: there
+// the host's second launch (3 us) is the longer part; sets of 32 MB and more, which keep the GPU busy for longer than the
+// host needs, up to 32 groups (8 rows of 4096 x 16384: 19.0 us in one launch, 16.5 us in two).
 extern "C" int bsi_b200_linear_decode_fits(int64_t Q, int64_t R, int64_t D) {
     const int64_t chunks = (D + 255) / 256;
-    return Q >= 1 && Q <= 16 && R <= (1 << 27) && Q * chunks <= BSI_B200_DECODE_FUSED_GROUPS ? 1 : 0;
+    const int64_t most = R * chunks * 256 >= (32 << 20) ? 32 : BSI_B200_DECODE_FUSED_GROUPS;
+    return Q >= 1 && Q <= 16 && R <= (1 << 27) && Q * chunks <= most ? 1 : 0;
 }

@@ -29,7 +29,8 @@ def test_decode_dot_matches_other_engines(Q, R, D, chunk_mode):
 
 # the one-launch layer: 1 .. 128 (row, chunk) groups per CTA, chunks that need the 64-bit quantiser, ragged depth
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
-@pytest.mark.parametrize("Q,R,D", [(1, 33, 256), (1, 3000, 4096), (2, 520, 16384), (7, 100, 1000), (8, 2500, 4096), (16, 130, 2048)])
+@pytest.mark.parametrize("Q,R,D", [(1, 33, 256), (1, 3000, 4096), (2, 520, 16384), (7, 100, 1000), (8, 2500, 4096), (16, 130, 2048),
+                                   (2, 8192, 4096), (8, 8191, 4096)])
 def test_one_launch_layer_equals_build_and_dot(dtype, Q, R, D):
     import bsipytorch_b200
     ops = bsipytorch_b200.bsi_ops
@@ -51,3 +52,15 @@ def test_one_launch_layer_equals_build_and_dot(dtype, Q, R, D):
         strided[:, :D] = x
         assert torch.equal(ops.bsi_layer_forward(strided[:, :D], keys, b, 2), want)     # rows that are not 16-byte aligned
     assert torch.equal(ops.bsi_layer_forward(x.view(1, Q, D), keys, bias, 2), want.view(1, Q, R))
+
+
+# 32 MB of keys: beyond 32 groups the rows are packed by a launch of their own
+def test_one_launch_rule_at_large_key_sets():
+    fits = capi.lib().bsi_b200_linear_decode_fits
+    assert [fits(2, 8192, 4096), fits(3, 8192, 4096), fits(8, 8191, 4096), fits(9, 8191, 4096)] == [1, 0, 1, 0]
+    x, k = _inputs.fc1(Q=3, R=8192, D=4096, seed=3, dtype=torch.float32)
+    import bsipytorch_b200
+    ops = bsipytorch_b200.bsi_ops
+    keys = ops.build_bsi_keys_cuda(k.to(DEV), 2)[0]
+    both = ops.bsi_layer_forward(x.to(DEV), keys, None, 2)
+    assert torch.equal(both[:2], ops.bsi_layer_forward(x[:2].to(DEV), keys, None, 2))
