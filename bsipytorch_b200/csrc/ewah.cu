@@ -348,32 +348,32 @@ __device__ __forceinline__ int flag_from(u64 count, int64_t W, double threshold,
     return compress_flag(count, W, threshold);
 }
 
-// encode_slice on a slice held in registers: wv[t] is this lane's word of tile t (word index 32 t + lane).
+// encode_slice on a slice held in registers: wv[t] is this lane's word of tile t (word index 32 t + lane). Positions and
+// counts fit 32 bits here (W <= 256), which halves the registers of the walk.
 template <bool EMIT, int TILES>
-__device__ __forceinline__ u64 encode_slice_regs(const u64 (&wv)[TILES], int64_t W, int compress,
-                                                 u64* __restrict__ out, int lane) {
+__device__ __forceinline__ uint32_t encode_slice_regs(const u64 (&wv)[TILES], int W, int compress, u64* __restrict__ out, int lane) {
     if (!compress) {
         if (EMIT) {
             if (lane == 0) out[0] = static_cast<u64>(W) << 33;
 #pragma unroll
             for (int t = 0; t < TILES; ++t) {
-                const int64_t w = t * 32 + lane;
+                const int w = t * 32 + lane;
                 if (w < W) out[1 + w] = wv[t];
             }
         }
-        return 1ull + static_cast<u64>(W);
+        return 1u + static_cast<uint32_t>(W);
     }
+    auto rlw = [](int bit, int run_len, int lit_count) {
+        return static_cast<u64>(bit) | (static_cast<u64>(run_len) << 1) | (static_cast<u64>(lit_count) << 33);
+    };
     const unsigned below = (1u << lane) - 1u;
-    u64 seg_base = 0, lit_base = 0;
-    int prev_type = 2;
-    int64_t open_w0 = 0;
-    u64 open_lit0 = 0;
-    int open_bit = 0, open_isfill = 0;
+    int seg_base = 0, lit_base = 0, prev_type = 2;
+    int open_w0 = 0, open_lit0 = 0, open_type = 2;      // the open segment: first word, literals before it, its fill
 #pragma unroll
     for (int t = 0; t < TILES; ++t) {
-        const int64_t tile = t * 32;
+        const int tile = t * 32;
         if (tile < W) {
-            const int64_t w = tile + lane;
+            const int w = tile + lane;
             const bool valid = w < W;
             const u64 word = valid ? wv[t] : 1ull;
             const int type = (word == 0ull) ? 0 : ((word == ~0ull) ? 1 : 2);
@@ -384,82 +384,68 @@ __device__ __forceinline__ u64 encode_slice_regs(const u64 (&wv)[TILES], int64_t
             const unsigned S = __ballot_sync(0xffffffffu, start);
             const unsigned L = __ballot_sync(0xffffffffu, lit);
             if (EMIT) {
-                const u64 lit_here = lit_base + __popc(L & below);
-                if (lit) {
-                    const u64 segs_incl = seg_base + __popc(S & (below | (1u << lane)));
-                    out[segs_incl + lit_here] = word;
-                }
+                const int lit_here = lit_base + __popc(L & below);
+                if (lit) out[seg_base + __popc(S & (below | (1u << lane))) + lit_here] = word;
                 const unsigned prior = S & below;
                 const int p = prior ? (31 - __clz(prior)) : 0;
                 const int p_type = __shfl_sync(0xffffffffu, type, p);
                 if (start && w != 0) {
-                    int64_t w0;
-                    u64 lit0, pos;
-                    int bit, isfill;
-                    if (prior) {
-                        w0 = tile + p;
-                        lit0 = lit_base + __popc(L & ((1u << p) - 1u));
-                        pos = seg_base + __popc(S & ((1u << p) - 1u)) + lit0;
-                        bit = (p_type == 1);
-                        isfill = (p_type != 2);
-                    } else {
-                        w0 = open_w0;
-                        lit0 = open_lit0;
-                        pos = (seg_base - 1) + lit0;
-                        bit = open_bit;
-                        isfill = open_isfill;
-                    }
-                    const u64 lit_count = lit_here - lit0;
-                    const u64 run_len = isfill ? (static_cast<u64>(w - w0) - lit_count) : 0ull;
-                    out[pos] = static_cast<u64>(bit) | ((run_len & 0xFFFFFFFFull) << 1) | (lit_count << 33);
+                    const int w0 = prior ? tile + p : open_w0;
+                    const int lit0 = prior ? lit_base + __popc(L & ((1u << p) - 1u)) : open_lit0;
+                    const int pos = lit0 + seg_base + (prior ? __popc(S & ((1u << p) - 1u)) : -1);
+                    const int of = prior ? p_type : open_type;
+                    const int lit_count = lit_here - lit0;
+                    out[pos] = rlw(of == 1, of != 2 ? w - w0 - lit_count : 0, lit_count);
                 }
             }
             if (S) {
                 const int p = 31 - __clz(S);
-                const int p_type = __shfl_sync(0xffffffffu, type, p);
+                open_type = __shfl_sync(0xffffffffu, type, p);
                 open_w0 = tile + p;
                 open_lit0 = lit_base + __popc(L & ((1u << p) - 1u));
-                open_bit = (p_type == 1);
-                open_isfill = (p_type != 2);
             }
             seg_base += __popc(S);
             lit_base += __popc(L);
-            const int last = (W - tile) >= 32 ? 31 : static_cast<int>(W - tile - 1);
-            prev_type = __shfl_sync(0xffffffffu, type, last);
+            prev_type = __shfl_sync(0xffffffffu, type, W - tile >= 32 ? 31 : W - tile - 1);
         }
     }
     if (EMIT && lane == 0 && seg_base > 0) {
-        const u64 lit_count = lit_base - open_lit0;
-        const u64 run_len = open_isfill ? (static_cast<u64>(W - open_w0) - lit_count) : 0ull;
-        out[(seg_base - 1) + open_lit0] =
-            static_cast<u64>(open_bit) | ((run_len & 0xFFFFFFFFull) << 1) | (lit_count << 33);
+        const int lit_count = lit_base - open_lit0;
+        out[seg_base - 1 + open_lit0] = rlw(open_type == 1, open_type != 2 ? W - open_w0 - lit_count : 0, lit_count);
     }
-    return seg_base + lit_base;
+    return static_cast<uint32_t>(seg_base + lit_base);
 }
 
 template <int TILES>
-__device__ __forceinline__ void load_slice(const u64* __restrict__ base, int64_t W, int lane, u64 (&wv)[TILES]) {
+__device__ __forceinline__ void load_slice(const u64* __restrict__ base, int W, bool there, int lane, u64 (&wv)[TILES]) {
 #pragma unroll
     for (int t = 0; t < TILES; ++t) {
-        const int64_t w = t * 32 + lane;
-        wv[t] = w < W ? __ldg(base + w) : 0ull;
+        const int w = t * 32 + lane;
+        wv[t] = there && w < W ? __ldg(base + w) : 0ull;
     }
 }
 
 // Two passes over the slices with `per_block` of them per block, at most kMaxSums blocks whatever S is: the sums of the
 // blocks' encoded sizes are then few enough for every block of the second pass to add up the ones before its own,
 // which a scan kernel between the passes did before (7 us, most of it latency).
+// How many: slices of more than 128 words (registers for two of them per warp: 3 blocks per SM) take one wave of blocks,
+// so that a warp streams through its slices with loads always in flight, instead of four waves that each began with
+// a wait for memory and for the sums (28672 slices of 256 words, 86 % literals: 43.2 -> 31.2 us); two
+// waves up to 128 words, where more and shorter blocks fit; below, as many blocks as the sums allow.
 constexpr int kMaxSums = 2048;
-inline int64_t slices_per_block(int64_t S) {
-    const int64_t least = (S + kMaxSums - 1) / kMaxSums;
+template <int TILES>
+constexpr int kBlocksPerSm = TILES > 4 ? 3 : TILES > 0 ? 4 : 5;
+inline int64_t slices_per_block(int64_t S, int64_t W) {
+    const int64_t blocks = W <= 64 || W > 256 ? kMaxSums : (W <= 128 ? 888 : 444);
+    const int64_t least = (S + blocks - 1) / blocks;
     return (least + kWarpsPerBlock - 1) / kWarpsPerBlock * kWarpsPerBlock;
 }
 
 // Pass 1: flag and encoded size of every slice, and the sum of the sizes of each block's slices. Bound by the one read
-// of the slices: popcounts are added up in 32 bits by one reduction, and only slices that compress are walked.
-// TILES = 0 walks the slice in memory (W > 256).
+// of the slices: popcounts are added up in 32 bits by one reduction, only slices that compress are walked, and a warp
+// has its next slice in flight while it counts one (two register sets). TILES = 0 walks the slice in memory (W > 256).
 template <int TILES>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32) ewah_sizes_kernel(
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, kBlocksPerSm<TILES>) ewah_sizes_kernel(
     const u64* __restrict__ words, int64_t S, int64_t W, double threshold, const FlagCuts cuts, int64_t per_block,
     int32_t* __restrict__ flags, u64* __restrict__ sizes, u64* __restrict__ block_sums) {
     __shared__ u64 wsize[kWarpsPerBlock];
@@ -471,29 +457,45 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) ewah_sizes_kernel(
     const int64_t s0 = static_cast<int64_t>(blockIdx.x) * per_block;
     const int64_t s1 = s0 + per_block < S ? s0 + per_block : S;
     u64 mine = 0;
-    for (int64_t s = s0 + warp; s < s1; s += kWarpsPerBlock) {
-        const u64* base = words + s * W;
-        int flag;
-        u64 n;
-        if constexpr (TILES > 0) {
-            u64 wv[TILES];
-            load_slice<TILES>(base, W, lane, wv);
+    if constexpr (TILES > 0) {
+        const int n_words = static_cast<int>(W);
+        const int count = static_cast<int>(s1 - s0);
+        const u64* base = words + s0 * W;
+        u64 even[TILES], odd[TILES];
+        auto load = [&](int i, u64 (&wv)[TILES]) { load_slice<TILES>(base + static_cast<int64_t>(i) * W, n_words, i < count, lane, wv); };
+        auto one = [&](int i, const u64 (&wv)[TILES]) {
+            if (i >= count) return;
             uint32_t local = 0;
 #pragma unroll
             for (int t = 0; t < TILES; ++t) local += static_cast<uint32_t>(__popcll(wv[t]));
-            flag = flag_from(__reduce_add_sync(0xffffffffu, local), W, threshold, cuts);
-            n = flag ? encode_slice_regs<false, TILES>(wv, W, flag, nullptr, lane) : 1ull + static_cast<u64>(W);
-        } else {
+            const int flag = flag_from(__reduce_add_sync(0xffffffffu, local), W, threshold, cuts);
+            const uint32_t n = encode_slice_regs<false, TILES>(wv, n_words, flag, nullptr, lane);
+            if (lane == 0) {
+                flags[s0 + i] = flag;
+                sizes[s0 + i] = n;
+            }
+            mine += n;
+        };
+        load(warp, even);
+        for (int i = warp; i < count; i += 2 * kWarpsPerBlock) {
+            load(i + kWarpsPerBlock, odd);
+            one(i, even);
+            load(i + 2 * kWarpsPerBlock, even);
+            one(i + kWarpsPerBlock, odd);
+        }
+    } else {
+        for (int64_t s = s0 + warp; s < s1; s += kWarpsPerBlock) {
+            const u64* base = words + s * W;
             u64 local = 0;
             for (int64_t w = lane; w < W; w += 32) local += static_cast<u64>(__popcll(base[w]));
-            flag = flag_from(warp_sum_u64(local), W, threshold, cuts);
-            n = encode_slice<false>(base, W, flag, nullptr, lane);
+            const int flag = flag_from(warp_sum_u64(local), W, threshold, cuts);
+            const u64 n = encode_slice<false>(base, W, flag, nullptr, lane);
+            if (lane == 0) {
+                flags[s] = flag;
+                sizes[s] = n;
+            }
+            mine += n;
         }
-        if (lane == 0) {
-            flags[s] = flag;
-            sizes[s] = n;
-        }
-        mine += n;
     }
     if (lane == 0) wsize[warp] = mine;
     __syncthreads();
@@ -508,7 +510,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) ewah_sizes_kernel(
 // Pass 2: offsets of the block's slices from the sums of the blocks before, then the streams. Block 0 leaves the total
 // as the first thing it does, so that a host that watches it (mapped memory) goes on while the streams are written.
 template <int TILES>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32) ewah_emit_blocks_kernel(
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, kBlocksPerSm<TILES>) ewah_emit_blocks_kernel(
     const u64* __restrict__ words, int64_t S, int64_t W, int64_t per_block, const int32_t* __restrict__ flags,
     const u64* __restrict__ sizes, const u64* __restrict__ block_sums, u64 capacity,
     u64* __restrict__ off, u64* __restrict__ out, int32_t* __restrict__ out_len, u64* __restrict__ total) {
@@ -517,12 +519,17 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) ewah_emit_blocks_kernel(
     const int warp = threadIdx.x >> 5;
     const int64_t s0 = static_cast<int64_t>(blockIdx.x) * per_block;
     const int64_t s1 = s0 + per_block < S ? s0 + per_block : S;
-    // The slice itself is input of the whole call: the first one is loaded before the wait for the pass before this
-    // one (programmatic dependent launch), so that this read overlaps its tail.
-    u64 wv[TILES > 0 ? TILES : 1];
-    if constexpr (TILES > 0) {
-        if (s0 + warp < s1) load_slice<TILES>(words + (s0 + warp) * W, W, lane, wv);
-    }
+    const int count = static_cast<int>(s1 - s0);
+    const int n_words = static_cast<int>(W);
+    // The slices themselves are input of the whole call: the first one is loaded before the wait for the pass before
+    // this one (programmatic dependent launch), so that this read overlaps its tail.
+    constexpr int kRegs = TILES > 0 ? TILES : 1;
+    u64 even[kRegs], odd[kRegs];
+    auto load = [&](int i, u64 (&wv)[kRegs]) {
+        if constexpr (TILES > 0)
+            load_slice<TILES>(words + (s0 + i) * W, n_words, i < count, lane, wv);
+    };
+    load(warp, even);
     asm volatile("griddepcontrol.wait;" ::: "memory");
     auto sum_of = [&](unsigned n) {      // of the first n block sums, for every thread of the block
         u64 t = 0;
@@ -545,27 +552,50 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) ewah_emit_blocks_kernel(
     } else {
         base_off = sum_of(blockIdx.x);
     }
-    for (int64_t g0 = s0; g0 < s1; g0 += kWarpsPerBlock) {
-        const int64_t s = g0 + warp;
+    // sizes of a group of kWarpsPerBlock slices, one per lane (with the flag of the lane's slice in bit 63), fetched a
+    // group ahead like the slices
+    auto group = [&](int g) -> u64 {
+        if (lane >= kWarpsPerBlock || g + lane >= count) return 0ull;
+        return __ldg(sizes + s0 + g + lane) | static_cast<u64>(__ldg(flags + s0 + g + lane)) << 63;
+    };
+    auto one = [&](int g, u64 size_flag, const u64 (&wv)[kRegs]) {
+        const int64_t s = s0 + g + warp;
+        const u64 size = size_flag & ~(1ull << 63);
+        u64 o, n_expected;
         if constexpr (TILES > 0) {
-            if (g0 != s0 && s < s1) load_slice<TILES>(words + s * W, W, lane, wv);
+            const uint32_t n = static_cast<uint32_t>(size);
+            o = base_off + __reduce_add_sync(0xffffffffu, lane < warp ? n : 0u);
+            n_expected = __shfl_sync(0xffffffffu, n, warp);
+            base_off += __reduce_add_sync(0xffffffffu, n);
+        } else {
+            o = base_off + warp_sum_u64(lane < warp ? size : 0ull);
+            n_expected = __shfl_sync(0xffffffffu, size, warp);
+            base_off += warp_sum_u64(size);
         }
-        // every warp adds up the sizes of the group's slices before its own
-        const u64 mine = (lane < kWarpsPerBlock && g0 + lane < s1) ? __ldg(sizes + g0 + lane) : 0ull;
-        const u64 o = base_off + warp_sum_u64(lane < warp ? mine : 0ull);
-        const u64 n_expected = __shfl_sync(0xffffffffu, mine, warp);
-        base_off += warp_sum_u64(mine);
-        if (s >= s1) continue;
+        const int flag = __shfl_sync(0xffffffffu, static_cast<int>(size_flag >> 63), warp);
+        if (g + warp >= count) return;
         if (lane == 0) {
             off[s] = o;
             out_len[s] = static_cast<int32_t>(n_expected);
         }
-        if (o + n_expected > capacity) continue;
-        if constexpr (TILES > 0) {
-            encode_slice_regs<true, TILES>(wv, W, __ldg(flags + s), out + o, lane);
-        } else {
-            encode_slice<true>(words + s * W, W, flags[s], out + o, lane);
-        }
+        if (o + n_expected > capacity) return;
+        if constexpr (TILES > 0)
+            encode_slice_regs<true, TILES>(wv, n_words, flag, out + o, lane);
+        else
+            encode_slice<true>(words + s * W, W, flag, out + o, lane);
+    };
+    if constexpr (TILES == 0) {
+        for (int g = 0; g < count; g += kWarpsPerBlock) one(g, group(g), even);
+        return;
+    }
+    u64 here = group(0);
+    for (int g = 0; g < count; g += 2 * kWarpsPerBlock) {
+        u64 next = group(g + kWarpsPerBlock);
+        load(g + kWarpsPerBlock + warp, odd);
+        one(g, here, even);
+        here = group(g + 2 * kWarpsPerBlock);
+        load(g + 2 * kWarpsPerBlock + warp, even);
+        if (g + kWarpsPerBlock < count) one(g + kWarpsPerBlock, next, odd);
     }
 }
 
@@ -729,7 +759,7 @@ extern "C" int bsi_b200_ewah_encode(const uint64_t* words, int64_t S, int64_t W,
         return fail(BSI_ERR_INVALID, "ewah_encode: scratch too small or misaligned");
     if (out == nullptr || off == nullptr || out_len == nullptr || flags == nullptr || capacity < 0)
         return fail(BSI_ERR_INVALID, "ewah_encode: null pointer");
-    const int64_t per_block = slices_per_block(S);
+    const int64_t per_block = slices_per_block(S, W);
     const int64_t nb = (S + per_block - 1) / per_block;
     u64* sizes = static_cast<u64*>(scratch);
     u64* block_sums = sizes + S;
