@@ -784,7 +784,8 @@ struct LinearTo {
     const PrebuiltBSIKeysCUDA* keys;
     const c10::optional<torch::Tensor>* bias;
     at::Tensor y;
-    double factor = 1.0;      // of the whole finished output; 1: none
+    double factor = 1.0;      // of the first `scaled_cols` finished columns (0: of all); 1: none
+    int64_t scaled_cols = 0;
 };
 void linear_forward(const Env& env, const at::Tensor& x2d, int decimalPlaces, bool relu, LinearTo* to, int n) {
     TORCH_CHECK(x2d.dim() == 2 && x2d.is_cuda(), "x must be a 2D CUDA tensor");
@@ -824,9 +825,10 @@ void linear_forward(const Env& env, const at::Tensor& x2d, int decimalPlaces, bo
                     " k=", keys.b.decimals);
         at::Tensor& y = to[i].y;
         // a factor rides in the epilogue for whole groups of 8 columns
-        const int64_t scaled = to[i].factor != 1.0 && R % 8 == 0 && fused && D > 0 ? R : 0;
+        const int64_t cols = to[i].scaled_cols > 0 ? to[i].scaled_cols : R;
+        const int64_t scaled = to[i].factor != 1.0 && cols % 8 == 0 && fused && D > 0 ? cols : 0;
         const float factor = static_cast<float>(to[i].factor);
-        auto rest = [&] { if (to[i].factor != 1.0 && scaled == 0) y = y.mul(to[i].factor); };
+        auto rest = [&] { if (to[i].factor != 1.0 && scaled == 0) y.narrow(1, 0, cols).mul_(to[i].factor); };
         y = at::detail::empty_cuda({Q, R}, yt, x2d.device(), c10::nullopt);
         const float* bptr = nullptr;
         at::Tensor b32;
@@ -927,12 +929,72 @@ py::object bsi_layer_forward(const torch::Tensor& x, const py::capsule& keyset_c
     return py::cast(y);
 }
 
+// Key sets of layers that read the same activations, laid behind one another in one image, so that one dot serves them
+// all: three dots of 1024 x 768 x 768 leave most of the GPU's SM pairs idle (36 tiles of 256 x 64 each). The members go
+// on as views of the joint image. Meant for models under construction: nothing may be running on the members.
+// keys: capsules, biases: their bias tensors. (joint capsule, joint bias or None, [the members' biases as views of it]),
+// or None where the sets cannot be joined.
+py::object join_key_sets(const py::list& keys, const py::list& biases) {
+    const size_t n = keys.size();
+    TORCH_CHECK(n > 0 && biases.size() == n, "one bias (or None) per key set");
+    std::vector<PrebuiltBSIKeysCUDA*> sets;
+    std::vector<at::Tensor> q8, scales, sums, bias;
+    for (size_t i = 0; i < n; ++i) {
+        auto* k = from_capsule<PrebuiltBSIKeysCUDA>(keys[i].cast<py::capsule>(), "PrebuiltBSIKeysCUDA");
+        const PackedBatch &b = k->b, &first = i == 0 ? b : sets[0]->b;
+        if (b.variable || b.chunk_mode || b.q8_hi.defined() || !b.q8.defined() || !b.q8.is_contiguous() || !k->abs_sum.defined() ||
+            b.q8.size(0) != k->num_keys || b.scales.numel() != k->num_keys || k->num_keys % 8 != 0 || b.d != first.d ||
+            b.S != first.S || b.decimals != first.decimals || b.q8.size(1) != first.q8.size(1) || b.q8.device() != first.q8.device())
+            return py::none();
+        if (!biases[i].is_none()) {
+            bias.push_back(biases[i].cast<at::Tensor>());
+            const at::Tensor& t = bias.back();
+            if (t.scalar_type() != at::kFloat || t.device() != b.q8.device() || !t.is_contiguous() || t.numel() != k->num_keys) return py::none();
+        }
+        sets.push_back(k);
+        q8.push_back(b.q8);
+        scales.push_back(b.scales.reshape({-1}));
+        sums.push_back(k->abs_sum);
+    }
+    if (!bias.empty() && bias.size() != n) return py::none();
+    c10::cuda::CUDAGuard guard(q8[0].device());
+    auto joint = std::make_unique<PrebuiltBSIKeysCUDA>();
+    joint->threshold = sets[0]->threshold;
+    joint->b.S = sets[0]->b.S;
+    joint->b.W = sets[0]->b.W;
+    joint->b.d = sets[0]->b.d;
+    joint->b.chunks = sets[0]->b.chunks;
+    joint->b.decimals = sets[0]->b.decimals;
+    joint->b.q8 = at::cat(q8, 0);
+    joint->b.scales = at::cat(scales, 0);
+    joint->abs_sum = at::cat(sums, 1);
+    joint->num_keys = joint->b.rows = joint->b.q8.size(0);
+    const at::Tensor all = bias.empty() ? at::Tensor() : at::cat(bias, 0);
+    // the members' old images return to the allocator below
+    C10_CUDA_CHECK(cudaDeviceSynchronize());
+    py::list views;
+    int64_t row = 0;
+    for (size_t i = 0; i < n; ++i) {
+        const int64_t rows = sets[i]->num_keys;
+        bsi_b200_unregister_key_bounds(sets[i]->b.q8.data_ptr<int8_t>());
+        sets[i]->b.q8 = joint->b.q8.narrow(0, row, rows);
+        if (all.defined()) views.append(py::cast(all.narrow(0, row, rows)));
+        row += rows;
+    }
+    py::capsule cap(joint.release(), "PrebuiltBSIKeysCUDA",
+                    [](PyObject* c) { delete reinterpret_cast<PrebuiltBSIKeysCUDA*>(PyCapsule_GetPointer(c, "PrebuiltBSIKeysCUDA")); });
+    return py::make_tuple(cap, all.defined() ? py::cast(all) : py::object(py::none()), views);
+}
+
 // One OPT decoder layer (pre-LN attention, ReLU MLP) whose six linears are BSI layers: the same ATen operators in the
 // same order as the module's Python forward and the BSI layers' own kernels, so the same bits. In Python the layer costs
 // 170 us of host time against 75 us of kernels (1024 tokens of OPT-125M). The query, key and value projections read one
-// packed image, and fc1's ReLU runs in its epilogue. linears: (key set, bias, decimal places) of q, k, v, out, fc1, fc2.
+// packed image, and one joint image of keys where joint, the (key set, bias) that join_key_sets made of the three, still is
+// what their layers hold; fc1's ReLU runs in its epilogue. linears: (key set, bias, decimal places) of q, k, v, out, fc1,
+// fc2.
 // None where the environment asks for the layers' other forms.
-py::object opt_layer_forward(const torch::Tensor& x, const py::tuple& norms, const py::tuple& linears, int64_t heads) {
+py::object opt_layer_forward(const torch::Tensor& x, const py::tuple& norms, const py::tuple& linears, int64_t heads,
+                             const py::object& joint) {
     const Env env;
     if ((env.profile_s != nullptr && std::strcmp(env.profile_s, "0") != 0) ||
         (env.fp32 != nullptr && std::strcmp(env.fp32, "0") != 0) || env.bits_queries() == 0)
@@ -956,12 +1018,39 @@ py::object opt_layer_forward(const torch::Tensor& x, const py::tuple& norms, con
     };
     auto flat = [](const at::Tensor& t) { return t.reshape({-1, t.size(-1)}); };
     auto split = [&](const at::Tensor& t) { return t.view({B, T, heads, H / heads}).transpose(1, 2); };
-    LinearTo qkv[3] = {{keys[0], &bias[0], at::Tensor(), std::pow(static_cast<double>(H / heads), -0.5)},
-                       {keys[1], &bias[1], at::Tensor(), 1.0},
-                       {keys[2], &bias[2], at::Tensor(), 1.0}};
-    linear_forward(env, flat(norm(x, 0)), dp[0], false, qkv, 3);
+    const double scaling = std::pow(static_cast<double>(H / heads), -0.5);
+    const PrebuiltBSIKeysCUDA* all = nullptr;
+    c10::optional<torch::Tensor> all_bias;
+    if (!joint.is_none()) {
+        const py::tuple t = joint.cast<py::tuple>();
+        all = from_capsule<PrebuiltBSIKeysCUDA>(t[0].cast<py::capsule>(), "PrebuiltBSIKeysCUDA");
+        if (!t[1].is_none()) all_bias = t[1].cast<torch::Tensor>();
+        bool same = all->num_keys == 3 * H;
+        for (int i = 0; i < 3 && same; ++i) {
+            same = keys[i]->num_keys == H && keys[i]->b.q8.data_ptr() == all->b.q8.data_ptr<int8_t>() + i * H * all->b.q8.size(1) &&
+                   bias[i].has_value() == all_bias.has_value();
+            if (same && all_bias.has_value())
+                same = bias[i]->scalar_type() == at::kFloat && bias[i]->numel() == H && bias[i]->is_contiguous() &&
+                       bias[i]->data_ptr() == all_bias->data_ptr<float>() + i * H;
+        }
+        if (!same) all = nullptr;
+    }
+    at::Tensor q, k, v;
+    if (all != nullptr) {
+        LinearTo to{all, &all_bias, at::Tensor(), scaling, H};
+        linear_forward(env, flat(norm(x, 0)), dp[0], false, &to, 1);
+        q = to.y.narrow(1, 0, H);
+        k = to.y.narrow(1, H, H);
+        v = to.y.narrow(1, 2 * H, H);
+    } else {
+        LinearTo qkv[3] = {{keys[0], &bias[0], at::Tensor(), scaling}, {keys[1], &bias[1], at::Tensor()}, {keys[2], &bias[2], at::Tensor()}};
+        linear_forward(env, flat(norm(x, 0)), dp[0], false, qkv, 3);
+        q = qkv[0].y;
+        k = qkv[1].y;
+        v = qkv[2].y;
+    }
     // query scaled in the model's type, attention with unit scaling: the order HuggingFace's OPT uses
-    const at::Tensor a = at::scaled_dot_product_attention(split(qkv[0].y), split(qkv[1].y), split(qkv[2].y), {}, 0.0, true, 1.0);
+    const at::Tensor a = at::scaled_dot_product_attention(split(q), split(k), split(v), {}, 0.0, true, 1.0);
     const at::Tensor o = linear_forward(env, flat(a.transpose(1, 2).reshape({B, T, H})), *keys[3], bias[3], dp[3]);
     const at::Tensor mid = x.add(o.view({B, T, H}));
     const at::Tensor f = linear_forward(env, flat(norm(mid, 3)), *keys[4], bias[4], dp[4], /*relu=*/true);
@@ -1498,7 +1587,10 @@ PYBIND11_MODULE(bsi_ops, m) {
           "pack + dot + cast + bias for one linear layer");
     m.def("bsi_layer_forward", &bsi_layer_forward, py::arg("x"), py::arg("keyset_cuda_cap"), py::arg("bias") = py::none(),
           py::arg("decimal_places") = 2, "bsi_linear_forward over the last dimension of x, in x's type; None under BSI_PROFILE");
+    m.def("join_key_sets", &join_key_sets, py::arg("keys"), py::arg("biases"),
+          "Key sets over the same inputs laid into one image: (joint key set, joint bias, biases as views) or None");
     m.def("opt_layer_forward", &opt_layer_forward, py::arg("x"), py::arg("norms"), py::arg("linears"), py::arg("heads"),
+          py::arg("joint") = py::none(),
           "One OPT decoder layer over BSI linears; None where the environment asks for another form of the layers");
     m.def("pack_queries_into", &pack_queries_into, py::arg("x2d"), py::arg("q8"), py::arg("scales"),
           py::arg("decimal_places"), "Pack activations into caller-owned int8 / chunk-scale tensors");

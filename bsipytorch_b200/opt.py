@@ -114,12 +114,27 @@ class OPTDecoderLayer(nn.Module):
                 return None
         p0, p1 = norms[0]._parameters, norms[1]._parameters
         y = _ops().opt_layer_forward(x, (p0["weight"], p0["bias"], norms[0].eps, p1["weight"], p1["bias"], norms[1].eps),
-                                     tuple((m._bsi_keys_cuda, m._buffers["bias"], m.decimalPlaces) for m in linears), attn.num_heads)
+                                     tuple((m._bsi_keys_cuda, m._buffers["bias"], m.decimalPlaces) for m in linears), attn.num_heads,
+                                     self.__dict__.get("_joint"))
         if y is not None:
             n = x.shape[0] * x.shape[1]
             for m in linears:
                 m.count(n)
         return y
+
+
+    def join_projections(self):
+        """Lay the key sets of q, k and v into one image, so that one dot serves all three (_native uses it as long as the
+        three layers hold the key sets and biases joined here). For a model under construction: nothing may be running."""
+        inner = self.self_attn._modules
+        layers = [inner[n] for n in ("q_proj", "k_proj", "v_proj")]
+        if any(type(m) is not BSIQuantizedLinear for m in layers):
+            return
+        joint = _ops().join_key_sets([m._bsi_keys_cuda for m in layers], [m._buffers["bias"] for m in layers])
+        if joint is not None:
+            self.__dict__["_joint"] = joint[:2]
+            for m, bias in zip(layers, joint[2]):
+                m._buffers["bias"] = bias
 
 
 class OPTDecoder(nn.Module):
@@ -248,6 +263,7 @@ def build_opt_bsi(name: str = "opt-125m", dtype=torch.float16, device="cuda", se
                 new = BSIQuantizedLinear(lin, decimalPlaces=decimal_places, compress_threshold=compress_threshold)
             setattr(owner, lname, new)
             del lin
+        layer.join_projections()
     model.eval()
     if keep_dense:
         model._dense_weights = dense
