@@ -1003,6 +1003,9 @@ py::object opt_layer_forward(const torch::Tensor& x, const py::tuple& norms, con
     const int64_t B = x.size(0), T = x.size(1), H = x.size(2);
     if (B * T == 0) return py::none();
     c10::cuda::CUDAGuard guard(x.device());
+    // nothing here is recorded for gradients: the operators skip the dispatcher's autograd and view-tracking layers, which
+    // cost 9 us of a layer's 77 us of host time
+    const at::AutoDispatchBelowADInplaceOrView below;
     const PrebuiltBSIKeysCUDA* keys[6];
     c10::optional<torch::Tensor> bias[6];
     int dp[6];
