@@ -916,6 +916,7 @@ py::object bsi_layer_forward(const torch::Tensor& x, const py::capsule& keyset_c
     if (env.profile_s != nullptr && std::strcmp(env.profile_s, "0") != 0) return py::none();
     auto* keys = from_capsule<PrebuiltBSIKeysCUDA>(keyset_cuda_cap, "PrebuiltBSIKeysCUDA");
     TORCH_CHECK(x.dim() >= 1, "x must have at least one dimension");
+    const at::AutoDispatchBelowADInplaceOrView below;       // nothing here is recorded for gradients
     at::Tensor x2d = x.detach();
     if (x2d.dim() != 2) x2d = x2d.reshape({-1, x2d.size(-1)});
     if (env.fp32 != nullptr && std::strcmp(env.fp32, "0") != 0) x2d = x2d.to(at::kFloat);   // verify_accuracy_bsi.py:126
