@@ -216,6 +216,11 @@ void same_device(const at::Tensor& a, const at::Tensor& b, const char* what) {
 
 uint64_t g_last_quantize_ns = 0, g_last_pack_ns = 0, g_last_total_ns = 0;
 
+// Uninitialised CUDA tensor straight from the allocator: at::empty passes the dispatcher first, half a microsecond each.
+at::Tensor fresh(at::IntArrayRef sizes, at::ScalarType type, at::Device dev) {
+    return at::detail::empty_cuda(sizes, type, dev, c10::nullopt);
+}
+
 // Quantise + pack `x` ([rows, d], f32/f16/bf16, CPU or CUDA) in one kernel.
 // lean = true skips the bit slices and slice weights (only the int8 image and the scales are
 // produced): what the fused linear path needs. key_bounds (row mode): receives the [3, rows] bounds of the image.
@@ -224,6 +229,7 @@ PackedBatch pack(const at::Tensor& input, int decimal_places, int bits, bool chu
     TORCH_CHECK(input.dim() == 2, "expects 2D tensor [rows, d]");
     const auto dev = work_device(input);
     c10::cuda::CUDAGuard guard(dev);
+    const at::AutoDispatchBelowADInplaceOrView below;       // nothing here is recorded for gradients
     at::Tensor x = input.detach();
     if (!(x.scalar_type() == at::kFloat || x.scalar_type() == at::kHalf || x.scalar_type() == at::kBFloat16))
         x = x.to(at::kFloat);
@@ -248,13 +254,13 @@ PackedBatch pack(const at::Tensor& input, int decimal_places, int bits, bool chu
     }
     // the kernels write every element: partial last words and padding columns of the image as zeros
     if (!lean) {
-        b.words = at::empty({b.rows, bits, b.W}, opt(at::kLong));
-        b.slice_weights = at::empty({b.rows, bits}, opt(at::kFloat));
+        b.words = fresh({b.rows, bits, b.W}, at::kLong, dev);
+        b.slice_weights = fresh({b.rows, bits}, at::kFloat, dev);
     }
-    b.scales = chunk_mode ? at::empty({b.rows, b.chunks}, opt(at::kFloat)) : at::empty({b.rows}, opt(at::kFloat));
-    b.q8 = at::empty({b.rows, ld8}, opt(at::kChar));
-    if (chunk_mode) b.sq_norms = at::empty({b.rows, b.chunks}, opt(at::kFloat));
-    if (key_bounds != nullptr) *key_bounds = at::empty({3, b.rows}, opt(at::kFloat));
+    b.scales = chunk_mode ? fresh({b.rows, b.chunks}, at::kFloat, dev) : fresh({b.rows}, at::kFloat, dev);
+    b.q8 = fresh({b.rows, ld8}, at::kChar, dev);
+    if (chunk_mode) b.sq_norms = fresh({b.rows, b.chunks}, at::kFloat, dev);
+    if (key_bounds != nullptr) *key_bounds = fresh({3, b.rows}, at::kFloat, dev);
 
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     auto stream = at::cuda::getCurrentCUDAStream();
@@ -600,7 +606,7 @@ py::tuple run_dot(const Env& env, const PackedBatch& qb, const PrebuiltBSIKeysCU
     const double scale_inv = total_decimals > 0 ? 1.0 / std::pow(10.0, total_decimals) : 1.0;  // bsi_cuda.cpp:710-711
 
     auto fopt = at::TensorOptions().dtype(at::kFloat).device(qb.q8.device());
-    at::Tensor out = at::empty({Q, R}, fopt);
+    at::Tensor out = fresh({Q, R}, at::kFloat, keys.b.q8.device());
     at::Tensor iacc;
     if (want_iacc) iacc = at::empty({Q, R, qb.chunks}, fopt.dtype(at::kInt));
 
