@@ -1099,9 +1099,10 @@ py::object opt_layer_forward(const torch::Tensor& x, const py::tuple& norms, con
     // query scaled in the model's type, attention with unit scaling: the order HuggingFace's OPT uses
     const at::Tensor a = at::scaled_dot_product_attention(split(q), split(k), split(v), {}, 0.0, true, 1.0);
     const at::Tensor o = linear_forward(env, flat(a.transpose(1, 2).reshape({B, T, H})), *keys[3], bias[3], dp[3]);
-    const at::Tensor mid = x.add(o.view({B, T, H}));
+    // residual sums into the linears' own outputs: the same sums, without an allocation
+    const at::Tensor mid = o.view({B, T, H}).add_(x);
     const at::Tensor f = linear_forward(env, flat(norm(mid, 3)), *keys[4], bias[4], dp[4], /*relu=*/true);
-    return py::cast(mid.add(linear_forward(env, f, *keys[5], bias[5], dp[5]).view({B, T, H})));
+    return py::cast(linear_forward(env, f, *keys[5], bias[5], dp[5]).view({B, T, H}).add_(mid));
 }
 
 // Quantise + pack activations (query side: chunk scales) into tensors the caller owns: q8 [rows, >= d]
