@@ -12,6 +12,7 @@
 #include <torch/extension.h>
 #include <pybind11/stl.h>
 
+#include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDACachingAllocator.h>
@@ -1036,12 +1037,13 @@ py::object join_key_sets(const py::list& keys, const py::list& biases) {
 // packed image, and one joint image of keys where joint, the (key set, bias) that join_key_sets made of the three, still is
 // what their layers hold; fc1's ReLU runs in its epilogue. linears: (key set, bias, decimal places) of q, k, v, out, fc1,
 // fc2.
-// None where the environment asks for the layers' other forms.
+// None where the environment asks for the layers' other forms, and under autocast: there every operator chooses its own
+// type, and a float32 residual stream stays float32 beside 16-bit attention.
 py::object opt_layer_forward(const torch::Tensor& x, const py::tuple& norms, const py::tuple& linears, int64_t heads,
                              const py::object& joint) {
     const Env env;
     if ((env.profile_s != nullptr && std::strcmp(env.profile_s, "0") != 0) ||
-        (env.fp32 != nullptr && std::strcmp(env.fp32, "0") != 0) || env.bits_queries() == 0)
+        (env.fp32 != nullptr && std::strcmp(env.fp32, "0") != 0) || env.bits_queries() == 0 || at::autocast::is_autocast_enabled(at::kCUDA))
         return py::none();
     TORCH_CHECK(x.dim() == 3 && x.is_cuda(), "x must be a [batch, tokens, hidden] CUDA tensor");
     const int64_t B = x.size(0), T = x.size(1), H = x.size(2);

@@ -24,3 +24,27 @@ def test_native_layer_equals_module_calls(dtype, B, T):
         want = layer(x)
         hook.remove()
     assert torch.equal(got, want)
+
+
+def _layer(dtype=torch.float32):
+    cfg = opt.OPTConfig(vocab_size=500, hidden_size=512, num_hidden_layers=1, num_attention_heads=8, ffn_dim=1280, name="small")
+    layer = opt.build_opt_bsi(cfg, dtype=dtype, seed=3).model.decoder.layers[0]
+    return layer, torch.randn(2, 37, 512, generator=torch.Generator().manual_seed(37)).to(dtype).cuda()
+
+
+def _module_calls(layer, x):
+    """The layer's modules called one by one."""
+    x = x + layer.self_attn(layer.self_attn_layer_norm(x))
+    return x + layer.fc2(torch.relu(layer.fc1(layer.final_layer_norm(x))))
+
+
+# float32 residuals beside 16-bit attention: the sum is float32, and values beyond float16 stay finite
+@pytest.mark.parametrize("low", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_layer_under_autocast_equals_module_calls(dtype, low):
+    layer, x = _layer(dtype)
+    if dtype == torch.float32:
+        x[0, 3, 5] = 1.0e5
+    with torch.no_grad(), torch.autocast("cuda", low):
+        got, want = layer(x), _module_calls(layer, x)
+    assert got.dtype == want.dtype and torch.equal(got, want) and bool(got.isfinite().all())
