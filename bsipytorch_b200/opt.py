@@ -17,6 +17,7 @@ from dataclasses import dataclass
 import torch
 import torch.nn.functional as F
 from torch import nn
+from torch.nn.modules import module as nn_module
 
 from .linear import BSIQuantizedLinear, _ops
 
@@ -95,6 +96,8 @@ class OPTDecoderLayer(nn.Module):
         """The layer as one extension call where all six linears are fused BSI layers and nobody looks in between (no
         gradients, no hooks); None otherwise. Same operators, same bits: what it saves is the Python between them."""
         if torch.is_grad_enabled() or not x.is_cuda or x.dtype not in (torch.float16, torch.bfloat16, torch.float32):
+            return None
+        if nn_module._global_forward_hooks or nn_module._global_forward_pre_hooks:      # hooks on every module
             return None
         # the modules' own dictionaries: nn.Module's attribute lookups and a method call per counter cost 2 us of a 70 us layer
         mods = self._modules

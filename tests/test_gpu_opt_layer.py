@@ -48,3 +48,16 @@ def test_layer_under_autocast_equals_module_calls(dtype, low):
     with torch.no_grad(), torch.autocast("cuda", low):
         got, want = layer(x), _module_calls(layer, x)
     assert got.dtype == want.dtype and torch.equal(got, want) and bool(got.isfinite().all())
+
+
+# hooks on every module see the ten modules of a layer
+def test_global_hooks_fire_for_every_module():
+    module = torch.nn.modules.module
+    layer, x = _layer()
+    for register in (module.register_module_forward_hook, module.register_module_forward_pre_hook):
+        seen = []
+        hook = register(lambda m, *a: seen.append(m))
+        with torch.no_grad():
+            layer(x)
+        hook.remove()
+        assert len(seen) == 10 and {id(m) for m in seen} == {id(m) for m in layer.modules()}
