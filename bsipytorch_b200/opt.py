@@ -94,7 +94,8 @@ class OPTDecoderLayer(nn.Module):
 
     def _native(self, x):
         """The layer as one extension call where all six linears are fused BSI layers and nobody looks in between (no
-        gradients, no hooks); None otherwise. Same operators, same bits: what it saves is the Python between them."""
+        gradients, no hooks, no forward replaced on an instance); None otherwise. Same operators, same bits: what it saves is
+        the Python between them."""
         if torch.is_grad_enabled() or not x.is_cuda or x.dtype not in (torch.float16, torch.bfloat16, torch.float32):
             return None
         if nn_module._global_forward_hooks or nn_module._global_forward_pre_hooks:      # hooks on every module
@@ -105,16 +106,16 @@ class OPTDecoderLayer(nn.Module):
         if type(attn) is not OPTAttention or type(norm0) is not nn.LayerNorm or type(norm1) is not nn.LayerNorm:
             return None
         a, n0, n1 = attn.__dict__, norm0.__dict__, norm1.__dict__
-        if (a["_forward_hooks"] or a["_forward_pre_hooks"] or n0["_forward_hooks"] or n0["_forward_pre_hooks"]
-                or n1["_forward_hooks"] or n1["_forward_pre_hooks"]):
-            return None
+        for d in (a, n0, n1):
+            if d["_forward_hooks"] or d["_forward_pre_hooks"] or "forward" in d:      # a forward of the instance's own
+                return None
         inner = a["_modules"]
         owners, linears = [], []
         for m in (inner["q_proj"], inner["k_proj"], inner["v_proj"], inner["out_proj"], mods["fc1"], mods["fc2"]):
             if type(m) is not BSIQuantizedLinear:
                 return None
             d = m.__dict__
-            if not d["fused"] or d["_forward_hooks"] or d["_forward_pre_hooks"]:
+            if not d["fused"] or d["_forward_hooks"] or d["_forward_pre_hooks"] or "forward" in d:
                 return None
             owners.append(d)
             linears.append((d["_bsi_keys_cuda"], d["_buffers"]["bias"], d["decimalPlaces"]))

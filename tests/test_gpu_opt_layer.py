@@ -61,3 +61,15 @@ def test_global_hooks_fire_for_every_module():
             layer(x)
         hook.remove()
         assert len(seen) == 10 and {id(m) for m in seen} == {id(m) for m in layer.modules()}
+
+
+# wrappers that replace a module's forward on the instance
+@pytest.mark.parametrize("name", ["self_attn", "self_attn_layer_norm", "self_attn.k_proj", "fc1"])
+def test_forward_replaced_on_an_instance_is_called(name):
+    layer, x = _layer()
+    module, seen = layer.get_submodule(name), []
+    own = module.forward
+    module.forward = lambda x: (seen.append(1), own(x))[1]
+    with torch.no_grad():
+        layer(x)
+    assert seen == [1]
