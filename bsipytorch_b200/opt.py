@@ -18,6 +18,8 @@ import torch
 import torch.nn.functional as F
 from torch import nn
 from torch.nn.modules import module as nn_module
+from torch.overrides import _get_current_function_mode_stack
+from torch.utils._device import DeviceContext
 
 from .linear import BSIQuantizedLinear, _ops
 
@@ -94,11 +96,14 @@ class OPTDecoderLayer(nn.Module):
 
     def _native(self, x):
         """The layer as one extension call where all six linears are fused BSI layers and nobody looks in between (no
-        gradients, no hooks, no forward replaced on an instance); None otherwise. Same operators, same bits: what it saves is
-        the Python between them."""
-        if torch.is_grad_enabled() or not x.is_cuda or x.dtype not in (torch.float16, torch.bfloat16, torch.float32):
+        gradients, no hooks, no forward replaced on an instance, no tensor subclass or function mode); None otherwise. Same
+        operators, same bits: what it saves is the Python between them."""
+        if type(x) is not torch.Tensor or torch.is_grad_enabled() or not x.is_cuda or x.dtype not in (torch.float16, torch.bfloat16, torch.float32):
             return None
         if nn_module._global_forward_hooks or nn_module._global_forward_pre_hooks:      # hooks on every module
+            return None
+        # a mode that sees every function (a default device is one too, and asks for nothing here)
+        if torch._C._is_torch_function_mode_enabled() and any(type(m) is not DeviceContext for m in _get_current_function_mode_stack()):
             return None
         # the modules' own dictionaries: nn.Module's attribute lookups and a method call per counter cost 2 us of a 70 us layer
         mods = self._modules

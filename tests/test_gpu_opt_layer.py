@@ -73,3 +73,30 @@ def test_forward_replaced_on_an_instance_is_called(name):
     with torch.no_grad():
         layer(x)
     assert seen == [1]
+
+
+class _Tagged(torch.Tensor):
+    pass
+
+
+class _Recorder(torch.overrides.TorchFunctionMode):
+    def __init__(self):
+        super().__init__()
+        self.names = []
+
+    def __torch_function__(self, func, types, args=(), kwargs=None):
+        self.names.append(getattr(func, "__name__", ""))
+        return func(*args, **(kwargs or {}))
+
+
+def test_tensor_subclasses_and_function_modes_see_the_layer():
+    layer, x = _layer()
+    with torch.no_grad():
+        want = layer(x)
+        tagged = layer(x.as_subclass(_Tagged))
+        with _Recorder() as mode:
+            got = layer(x)
+        with torch.device("cuda"):                 # a default device changes nothing
+            assert layer._native(x) is not None
+    assert type(tagged) is _Tagged and torch.equal(tagged.as_subclass(torch.Tensor), want) and torch.equal(got, want)
+    assert mode.names.count("layer_norm") == 2 and "scaled_dot_product_attention" in mode.names
