@@ -1037,8 +1037,9 @@ py::object join_key_sets(const py::list& keys, const py::list& biases) {
 // packed image, and one joint image of keys where joint, the (key set, bias) that join_key_sets made of the three, still is
 // what their layers hold; fc1's ReLU runs in its epilogue. linears: (key set, bias, decimal places) of q, k, v, out, fc1,
 // fc2.
-// None where the environment asks for the layers' other forms, and under autocast: there every operator chooses its own
-// type, and a float32 residual stream stays float32 beside 16-bit attention.
+// None where the environment asks for the layers' other forms, where x carries a forward-mode tangent (the residual sums
+// pass it on), and under autocast: there every operator chooses its own type, and a float32 residual stream stays float32
+// beside 16-bit attention.
 py::object opt_layer_forward(const torch::Tensor& x, const py::tuple& norms, const py::tuple& linears, int64_t heads,
                              const py::object& joint) {
     const Env env;
@@ -1047,7 +1048,7 @@ py::object opt_layer_forward(const torch::Tensor& x, const py::tuple& norms, con
         return py::none();
     TORCH_CHECK(x.dim() == 3 && x.is_cuda(), "x must be a [batch, tokens, hidden] CUDA tensor");
     const int64_t B = x.size(0), T = x.size(1), H = x.size(2);
-    if (B * T == 0) return py::none();
+    if (B * T == 0 || x._fw_grad(0).defined()) return py::none();
     c10::cuda::CUDAGuard guard(x.device());
     // nothing here is recorded for gradients: the operators skip the dispatcher's autograd and view-tracking layers, which
     // cost 9 us of a layer's 77 us of host time

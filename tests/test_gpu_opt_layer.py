@@ -1,6 +1,7 @@
 """The decoder layer as one extension call against the same modules called one by one: same bits, same counters."""
 import pytest
 import torch
+import torch.autograd.forward_ad as forward_ad
 
 from bsipytorch_b200 import opt
 
@@ -100,3 +101,11 @@ def test_tensor_subclasses_and_function_modes_see_the_layer():
             assert layer._native(x) is not None
     assert type(tagged) is _Tagged and torch.equal(tagged.as_subclass(torch.Tensor), want) and torch.equal(got, want)
     assert mode.names.count("layer_norm") == 2 and "scaled_dot_product_attention" in mode.names
+
+
+def test_residual_sums_pass_forward_tangents_on():
+    layer, x = _layer()
+    tangent = torch.full_like(x, 2.0)
+    with torch.no_grad(), forward_ad.dual_level():
+        y = forward_ad.unpack_dual(layer(forward_ad.make_dual(x, tangent)))
+    assert torch.equal(y.tangent, tangent)          # the linears detach: what is left is the residual stream's
