@@ -1064,7 +1064,8 @@ py::object opt_layer_forward(const torch::Tensor& x, const py::tuple& norms, con
     }
     if (dp[0] != dp[1] || dp[0] != dp[2]) return py::none();
     auto norm = [&](const at::Tensor& t, int first) {
-        return at::layer_norm(t, {H}, norms[first].cast<torch::Tensor>(), norms[first + 1].cast<torch::Tensor>(), norms[first + 2].cast<double>());
+        using Affine = c10::optional<torch::Tensor>;      // None: a LayerNorm without that parameter
+        return at::layer_norm(t, {H}, norms[first].cast<Affine>(), norms[first + 1].cast<Affine>(), norms[first + 2].cast<double>());
     };
     auto flat = [](const at::Tensor& t) { return t.reshape({-1, t.size(-1)}); };
     auto split = [&](const at::Tensor& t) { return t.view({B, T, heads, H / heads}).transpose(1, 2); };

@@ -125,6 +125,8 @@ class OPTDecoderLayer(nn.Module):
             owners.append(d)
             linears.append((d["_bsi_keys_cuda"], d["_buffers"]["bias"], d["decimalPlaces"]))
         p0, p1 = n0["_parameters"], n1["_parameters"]
+        if not ("weight" in p0 and "bias" in p0 and "weight" in p1 and "bias" in p1) or len(n0["normalized_shape"]) + len(n1["normalized_shape"]) != 2:
+            return None
         y = _ops().opt_layer_forward(x, (p0["weight"], p0["bias"], n0["eps"], p1["weight"], p1["bias"], n1["eps"]), tuple(linears),
                                      a["num_heads"], self.__dict__.get("_joint"))
         if y is not None:

@@ -109,3 +109,18 @@ def test_residual_sums_pass_forward_tangents_on():
     with torch.no_grad(), forward_ad.dual_level():
         y = forward_ad.unpack_dual(layer(forward_ad.make_dual(x, tangent)))
     assert torch.equal(y.tangent, tangent)          # the linears detach: what is left is the residual stream's
+
+
+# LayerNorms without weight, without bias, over more than the last dimension, with a weight that is a buffer
+@pytest.mark.parametrize("form", ["plain", "no bias", "two dimensions", "buffer"])
+def test_layer_norms_of_other_forms(form):
+    layer, x = _layer()
+    norm = {"plain": lambda: torch.nn.LayerNorm(512, elementwise_affine=False), "no bias": lambda: torch.nn.LayerNorm(512, bias=False),
+            "two dimensions": lambda: torch.nn.LayerNorm((37, 512)), "buffer": lambda: torch.nn.LayerNorm(512)}[form]().cuda()
+    if form == "buffer":
+        weight = norm.weight.detach() * 3.0
+        del norm.weight
+        norm.register_buffer("weight", weight)
+    layer.final_layer_norm = norm
+    with torch.no_grad():
+        assert torch.equal(layer(x), _module_calls(layer, x))
