@@ -72,7 +72,8 @@ class BSIQuantizedLinear(nn.Module):
 
     def forward(self, x):
         ops = _ops()
-        bias = self._buffers["bias"]
+        buffers = self._buffers                                  # half a microsecond less than nn.Module's attribute lookup
+        bias = buffers["bias"] if "bias" in buffers else self.bias
         out = ops.bsi_layer_forward(x, self._bsi_keys_cuda, bias, self.decimalPlaces) if self.fused else None
         if out is None:                                          # unfused layer, or BSI_PROFILE set
             shape, dtype = x.shape, x.dtype

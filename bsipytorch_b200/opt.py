@@ -123,7 +123,8 @@ class OPTDecoderLayer(nn.Module):
             if not d["fused"] or d["_forward_hooks"] or d["_forward_pre_hooks"] or "forward" in d:
                 return None
             owners.append(d)
-            linears.append((d["_bsi_keys_cuda"], d["_buffers"]["bias"], d["decimalPlaces"]))
+            buffers = d["_buffers"]
+            linears.append((d["_bsi_keys_cuda"], buffers["bias"] if "bias" in buffers else m.bias, d["decimalPlaces"]))
         p0, p1 = n0["_parameters"], n1["_parameters"]
         if not ("weight" in p0 and "bias" in p0 and "weight" in p1 and "bias" in p1) or len(n0["normalized_shape"]) + len(n1["normalized_shape"]) != 2:
             return None

@@ -124,3 +124,14 @@ def test_layer_norms_of_other_forms(form):
     layer.final_layer_norm = norm
     with torch.no_grad():
         assert torch.equal(layer(x), _module_calls(layer, x))
+
+
+def test_bias_set_as_a_parameter():
+    layer, x = _layer()
+    with torch.no_grad():
+        want, linear = layer(x), layer.fc1(x)
+        for m in (layer.self_attn.q_proj, layer.fc1):
+            m.bias = torch.nn.Parameter(m.bias.clone())
+        assert torch.equal(layer(x), want) and torch.equal(layer.fc1(x), linear)
+        layer.fc1.fused = False
+        assert torch.equal(layer.fc1(x), linear)
