@@ -849,10 +849,11 @@ void linear_forward(const Env& env, const at::Tensor& x2d, int decimalPlaces, bo
     at::Tensor x = x2d;
     if (x.scalar_type() != yt) x = x.to(yt);
     if (x.stride(1) != 1 || x.stride(0) < D) x = x.contiguous();
+    const int64_t ldx = Q == 1 ? D : x.stride(0);      // a single row is contiguous whatever its row stride says
     const bool chunk = env.chunk_scale() && W % 4 == 0;
     const float clip_k = env.clip_k();
     const bool profile = env.profile();
-    const int64_t chunks = (D + 255) / 256, ldx = x.stride(0);
+    const int64_t chunks = (D + 255) / 256;
     const bool one_launch = chunk && !(clip_k > 0.0f) && !profile && decimalPlaces >= 0 && decimalPlaces <= 8 && engine == BSI_ENGINE_AUTO;
     // int8 image, scales and chunk sums of squares share one block that goes back to the allocator (stream-ordered)
     // when the call returns

@@ -64,3 +64,20 @@ def test_one_launch_rule_at_large_key_sets():
     keys = ops.build_bsi_keys_cuda(k.to(DEV), 2)[0]
     both = ops.bsi_layer_forward(x.to(DEV), keys, None, 2)
     assert torch.equal(both[:2], ops.bsi_layer_forward(x[:2].to(DEV), keys, None, 2))
+
+
+# a single row has any row stride: a transposed column (1), one of several columns, a broadcast row (0), the last of many
+@pytest.mark.parametrize("D,R", [(512, 300), (16384, 8192)])
+def test_one_row_of_any_row_stride(D, R):
+    import bsipytorch_b200
+    ops = bsipytorch_b200.bsi_ops
+    x, k = _inputs.fc1(Q=1, R=R, D=D, seed=D, dtype=torch.float32)
+    x = x.to(DEV)
+    keys = ops.build_bsi_keys_cuda(k.to(DEV), 2)[0]
+    want = ops.bsi_layer_forward(x.clone(), keys, None, 2)
+    column = x.clone().view(D, 1)
+    assert column.t().stride() == (1, 1)
+    for row in (column.t(), torch.cat([column, column], 1)[:, 1:].t(), x.view(1, 1, D).expand(1, 1, D),
+                x.as_strided((1, D), (0, 1)), torch.cat([x + 1.0, x])[1:], x.as_strided((1, D), (1 << 40, 1))):
+        for call in (ops.bsi_layer_forward, lambda *a: ops.bsi_linear_forward(a[0].reshape(1, D), *a[1:])):
+            assert torch.equal(call(row, keys, None, 2).view(1, R), want)
