@@ -69,6 +69,10 @@ struct Env {
         TORCH_CHECK(!(clip_k() > 0.0f), what, " does not implement BSI_FIXED_CLIP_K > 0 (outlier clipping); "
                     "use the build_bsi_* entry points");
     }
+    // Whether the choice of the dot's engine is left to the library. linear_from_packed runs on the tensor cores either way.
+    bool engine_free() const {
+        return (engine == nullptr || !*engine || std::strcmp(engine, "auto") == 0) && !(tc_dot != nullptr && *tc_dot && std::atoi(tc_dot) == 0);
+    }
     int dot_engine() const {
         if (engine == nullptr || !*engine || std::strcmp(engine, "auto") == 0) {
             // BSI_TC_DOT=0 is the reference's switch to its non-tensor-core kernel, re-read on every launch
@@ -932,10 +936,10 @@ void linear_forward(const Env& env, const at::Tensor& x2d, int decimalPlaces, bo
         bsi_dot_bounds bounds = dot_bounds(keys, bits, nullptr);
         bounds.query_sq = sq;
         bounds.query_sq_stride = chunks;
-        check_status(bsi_b200_linear_i8_bounded(q8, chunks * 256, scales, chunk ? chunks : 0, keys.b.q8.data_ptr<int8_t>(),
-                                                keys.b.q8.size(1), keys.b.scales.data_ptr<float>(), bptr, Q, R, chunks, scale_inv,
-                                                y.data_ptr(), R, code, act, scaled, factor, &bounds, current_stream()),
-                     "bsi_b200_linear_i8_bounded");
+        check_status(bsi_b200_linear_i8_engine(q8, chunks * 256, scales, chunk ? chunks : 0, keys.b.q8.data_ptr<int8_t>(),
+                                               keys.b.q8.size(1), keys.b.scales.data_ptr<float>(), bptr, Q, R, chunks, scale_inv,
+                                               y.data_ptr(), R, code, act, scaled, factor, &bounds, engine, current_stream()),
+                     "bsi_b200_linear_i8_engine");
         rest();
     }
 }
@@ -1172,14 +1176,15 @@ at::Tensor linear_from_packed(torch::Tensor q8, torch::Tensor scales, py::capsul
         bptr = b32.data_ptr<float>();
     }
     const int code = yt == at::kHalf ? BSI_DTYPE_F16 : (yt == at::kBFloat16 ? BSI_DTYPE_BF16 : BSI_DTYPE_F32);
-    const bsi_dot_bounds bounds = dot_bounds(*keys, Env().bits_queries(), nullptr);
-    check_status(bsi_b200_linear_i8_bounded(q8.data_ptr<int8_t>(), q8.stride(0), scales.data_ptr<float>(), chunks,
-                                            keys->b.q8.data_ptr<int8_t>(), keys->b.q8.size(1),
-                                            keys->b.scales.data_ptr<float>(), bptr, Q, R, chunks,
-                                            static_cast<float>(scale_inv), y.data_ptr(), R, code,
-                                            relu ? BSI_ACT_RELU : BSI_ACT_NONE, scaled_columns, static_cast<float>(factor), &bounds,
-                                            current_stream()),
-                 "bsi_b200_linear_i8_bounded");
+    const Env env;
+    const bsi_dot_bounds bounds = dot_bounds(*keys, env.bits_queries(), nullptr);
+    check_status(bsi_b200_linear_i8_engine(q8.data_ptr<int8_t>(), q8.stride(0), scales.data_ptr<float>(), chunks,
+                                           keys->b.q8.data_ptr<int8_t>(), keys->b.q8.size(1),
+                                           keys->b.scales.data_ptr<float>(), bptr, Q, R, chunks,
+                                           static_cast<float>(scale_inv), y.data_ptr(), R, code,
+                                           relu ? BSI_ACT_RELU : BSI_ACT_NONE, scaled_columns, static_cast<float>(factor), &bounds,
+                                           env.engine_free() ? BSI_ENGINE_AUTO : BSI_ENGINE_TCGEN05, current_stream()),
+                 "bsi_b200_linear_i8_engine");
     return y;
 }
 

@@ -179,7 +179,16 @@ extern "C" int bsi_b200_linear_i8_bounded(const int8_t* a8, int64_t lda, const f
                                           const int8_t* k8, int64_t ldk, const float* bw0, const float* bias,
                                           int64_t Q, int64_t R, int64_t chunks, float scale_inv, void* y, int64_t ldy,
                                           int y_dtype, int activation, int64_t scaled_cols, float factor,
-                                          const bsi_dot_bounds* bounds, bsi_stream_t stream_) {
+                                          const bsi_dot_bounds* bounds, bsi_stream_t stream) {
+    return bsi_b200_linear_i8_engine(a8, lda, qs, qs_stride, k8, ldk, bw0, bias, Q, R, chunks, scale_inv, y, ldy, y_dtype,
+                                     activation, scaled_cols, factor, bounds, BSI_ENGINE_AUTO, stream);
+}
+
+extern "C" int bsi_b200_linear_i8_engine(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride,
+                                         const int8_t* k8, int64_t ldk, const float* bw0, const float* bias,
+                                         int64_t Q, int64_t R, int64_t chunks, float scale_inv, void* y, int64_t ldy,
+                                         int y_dtype, int activation, int64_t scaled_cols, float factor,
+                                         const bsi_dot_bounds* bounds, int engine, bsi_stream_t stream_) {
     using namespace bsi;
     if (Q < 0 || R < 0 || chunks < 0) return fail(BSI_ERR_INVALID, "linear_i8: negative size");
     if (Q == 0 || R == 0) return BSI_OK;
@@ -195,11 +204,13 @@ extern "C" int bsi_b200_linear_i8_bounded(const int8_t* a8, int64_t lda, const f
         return fail(BSI_ERR_INVALID, "linear_i8: unknown activation");
     if (y_dtype != BSI_DTYPE_F32 && y_dtype != BSI_DTYPE_F16 && y_dtype != BSI_DTYPE_BF16)
         return fail(BSI_ERR_INVALID, "linear_i8: unknown y_dtype");
+    if (engine != BSI_ENGINE_AUTO && engine != BSI_ENGINE_TCGEN05)
+        return fail(BSI_ERR_INVALID, "linear_i8: engine must be AUTO or TCGEN05");
     if (int rc = require_sm100()) return rc;
     if (scaled_cols < 0 || scaled_cols > R || (scaled_cols & 7) != 0)
         return fail(BSI_ERR_INVALID, "linear_i8: scaled_cols must be a multiple of 8 in [0, R]");
     const Finishing fin{activation == BSI_ACT_RELU ? 1 : 0, static_cast<int>(scaled_cols), factor};
-    if (decode_fits(Q, R, chunks)) {
+    if (engine == BSI_ENGINE_AUTO && decode_fits(Q, R, chunks)) {
         bool taken = false;
         const int rc = dot_decode(a8, lda, qs, qs_stride, k8, ldk, bw0, bias, Q, R, chunks, scale_inv, y, ldy, y_dtype, fin,
                                   static_cast<cudaStream_t>(stream_), &taken);

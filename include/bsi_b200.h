@@ -44,7 +44,7 @@ enum { BSI_DTYPE_F32 = 0, BSI_DTYPE_F16 = 1, BSI_DTYPE_BF16 = 2 };
 
 /* Dot engines. */
 enum {
-    BSI_ENGINE_AUTO = 0,    /* tcgen05 */
+    BSI_ENGINE_AUTO = 0,    /* tcgen05; the key-streaming kernel for 16 query rows and fewer */
     BSI_ENGINE_TCGEN05 = 1, /* int8 recombination, tcgen05.mma kind::i8, TMEM accumulators, TMA */
     BSI_ENGINE_SIMT = 2,    /* dp4a on the CUDA cores (cross-check engine) */
     BSI_ENGINE_BMMA = 3     /* mma.sync b1 AND+POPC directly on the slice words */
@@ -245,6 +245,12 @@ int bsi_b200_linear_i8_bounded(const int8_t* a8, int64_t lda, const float* qs, i
                                int64_t Q, int64_t R, int64_t chunks, float scale_inv, void* y, int64_t ldy, int y_dtype,
                                int activation, int64_t scaled_cols, float factor, const bsi_dot_bounds* bounds,
                                bsi_stream_t stream);
+/* The same on a pinned engine: BSI_ENGINE_AUTO, or BSI_ENGINE_TCGEN05 for the tensor-core tiles at any number of rows. */
+int bsi_b200_linear_i8_engine(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride,
+                              const int8_t* k8, int64_t ldk, const float* bw0, const float* bias,
+                              int64_t Q, int64_t R, int64_t chunks, float scale_inv, void* y, int64_t ldy, int y_dtype,
+                              int activation, int64_t scaled_cols, float factor, const bsi_dot_bounds* bounds,
+                              int engine, bsi_stream_t stream);
 /* (scaled_cols, a multiple of 8: the finished values of the first scaled_cols columns are multiplied by factor and
  * rounded to the output type once more, as y[:, :scaled_cols] * factor does; 0: none.) */
 

@@ -81,3 +81,23 @@ def test_one_row_of_any_row_stride(D, R):
                 x.as_strided((1, D), (0, 1)), torch.cat([x + 1.0, x])[1:], x.as_strided((1, D), (1 << 40, 1))):
         for call in (ops.bsi_layer_forward, lambda *a: ops.bsi_linear_forward(a[0].reshape(1, D), *a[1:])):
             assert torch.equal(call(row, keys, None, 2).view(1, R), want)
+
+
+# a pinned tensor-core engine holds for layers of few rows too: the tiles count themselves, the key-streaming kernel does not
+def test_pinned_engine_is_not_replaced(monkeypatch):
+    import bsipytorch_b200
+    ops = bsipytorch_b200.bsi_ops
+    x, k = _inputs.c1(Q=8, R=300, D=512)
+    x = x.to(DEV)
+    keys = ops.build_bsi_keys_cuda(k.to(DEV), 2)[0]
+    packed = torch.empty(8, 512, dtype=torch.int8, device=DEV), torch.empty(8, 2, device=DEV)
+    ops.pack_queries_into(x, *packed, 2)
+    calls = (lambda: ops.bsi_layer_forward(x, keys, None, 2), lambda: ops.linear_from_packed(*packed, keys, None, 2, torch.float32))
+    for call in calls:
+        capi.exact_int_tiles()
+        free = call()
+        assert capi.exact_int_tiles() == 0
+        monkeypatch.setenv("BSI_B200_ENGINE", "tcgen05")
+        pinned = call()
+        monkeypatch.delenv("BSI_B200_ENGINE")
+        assert capi.exact_int_tiles() > 0 and torch.equal(free, pinned)
