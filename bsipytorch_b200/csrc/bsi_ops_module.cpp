@@ -904,6 +904,7 @@ void linear_forward(const Env& env, const at::Tensor& x2d, int decimalPlaces, bo
                                                 keys.b.q8.size(1), keys.b.scales.data_ptr<float>(), bptr, Q, R, scale_inv,
                                                 y.data_ptr(), R, act, scaled, factor, current_stream()),
                          "bsi_b200_linear_decode");
+            g_last_quantize_ns = g_last_pack_ns = g_last_total_ns = 0;      // no pack of its own to report
             rest();
             continue;
         }

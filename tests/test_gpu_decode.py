@@ -101,3 +101,18 @@ def test_pinned_engine_is_not_replaced(monkeypatch):
         pinned = call()
         monkeypatch.delenv("BSI_B200_ENGINE")
         assert capi.exact_int_tiles() > 0 and torch.equal(free, pinned)
+
+
+# the profile of the last build is that of the last call: a one-launch layer has none
+def test_one_launch_layer_leaves_no_old_profile(monkeypatch):
+    import bsipytorch_b200
+    ops = bsipytorch_b200.bsi_ops
+    x, k = _inputs.c1(Q=8, R=300, D=512)
+    x = x.to(DEV)
+    keys = ops.build_bsi_keys_cuda(k.to(DEV), 2)[0]
+    monkeypatch.setenv("BSI_PROFILE", "1")
+    ops.bsi_linear_forward(x, keys, None, 2)
+    assert ops.get_last_query_build_profile_cuda()[2] > 0
+    monkeypatch.delenv("BSI_PROFILE")
+    ops.bsi_linear_forward(x, keys, None, 2)
+    assert ops.get_last_query_build_profile_cuda() == (0, 0, 0)
