@@ -567,7 +567,9 @@ EwahStream ewah_encode(const at::Tensor& words2d, double threshold) {
     const int64_t scratch_bytes = std::max<int64_t>(bsi_b200_ewah_scratch_bytes(S), 8);
     c10::DataPtr scratch = c10::cuda::CUDACachingAllocator::get()->allocate(static_cast<size_t>(scratch_bytes));
     // The length of the stream comes back through a word of mapped host memory that the second pass writes first, so
-    // that this call returns while the streams are still being written.
+    // that this call returns while the streams are still being written: they are ordered on the current stream like any
+    // operator's results, and the slices, which may belong to another stream, are marked as in use on this one.
+    c10::cuda::CUDACachingAllocator::recordStream(words2d.storage().data_ptr(), at::cuda::getCurrentCUDAStream());
     volatile uint64_t* word = HostWords::take();
     at::Tensor total_dev;
     if (word == nullptr) total_dev = fresh(1, at::kLong);

@@ -1,6 +1,8 @@
 """Streaming encoder: every way the slices of a block and its warps can run out, against the checker."""
 import pytest
+import torch
 
+import bsipytorch_b200
 from test_gpu_ewah import _compare, _structured
 
 pytestmark = pytest.mark.gpu
@@ -12,3 +14,19 @@ pytestmark = pytest.mark.gpu
                                  (16385, 33), (50, 256)])
 def test_encoder_at_block_edges(S, W):
     _compare(_structured(S, W, S + W), 0.5)
+
+
+# The call returns while the slices are still being read: slices that belong to another stream are not reused until the
+# stream of the call is done with them.
+def test_slices_of_another_stream_outlive_the_call():
+    other = torch.cuda.Stream()
+    words = torch.randint(-5, 5, (4096, 64), device="cuda")
+    torch.cuda.synchronize()
+    with torch.cuda.stream(other):
+        bsipytorch_b200.bsi_ops.ewah_encode_words(words, 0.2)
+        torch.cuda._sleep(200_000_000)          # a tenth of a second of work behind the encoder
+    address = words.data_ptr()
+    del words
+    again = torch.empty(4096, 64, dtype=torch.int64, device="cuda")
+    assert not other.query() and again.data_ptr() != address
+    torch.cuda.synchronize()
