@@ -582,7 +582,9 @@ EwahStream ewah_encode(const at::Tensor& words2d, double threshold) {
                                         word != nullptr ? const_cast<uint64_t*>(word)
                                                         : reinterpret_cast<uint64_t*>(total_dev.data_ptr<int64_t>()),
                                         static_cast<bsi_stream_t>(stream));
-    check_status(rc, "bsi_b200_ewah_encode");      // a word whose kernel may still write it is not given back
+    // refused before any launch: the word is free again. One that a kernel may still write is not given back.
+    if (word != nullptr && rc != BSI_OK && rc != BSI_ERR_CUDA) HostWords::give(word);
+    check_status(rc, "bsi_b200_ewah_encode");
     if (word != nullptr) {
         py::gil_scoped_release unlocked;
         cudaError_t state = cudaErrorNotReady;

@@ -30,3 +30,18 @@ def test_slices_of_another_stream_outlive_the_call():
     again = torch.empty(4096, 64, dtype=torch.int64, device="cuda")
     assert not other.query() and again.data_ptr() != address
     torch.cuda.synchronize()
+
+
+# Refused calls do not use up the words of host memory the encoder reports through: it still returns without a
+# synchronising call of torch's (which the fallback without a word makes).
+def test_refused_calls_leave_the_encoder_as_it_was():
+    ops = bsipytorch_b200.bsi_ops
+    empty, words = torch.zeros(8, 0, dtype=torch.int64, device="cuda"), torch.randint(-5, 5, (64, 64), device="cuda")
+    for _ in range(70):
+        with pytest.raises(RuntimeError):
+            ops.ewah_encode_words(empty, 0.2)
+    torch.cuda.set_sync_debug_mode("error")
+    try:
+        ops.ewah_encode_words(words, 0.2)
+    finally:
+        torch.cuda.set_sync_debug_mode("default")
