@@ -12,6 +12,7 @@ the reference.
 """
 from __future__ import annotations
 
+import weakref
 from dataclasses import dataclass
 
 import torch
@@ -147,6 +148,12 @@ class OPTDecoderLayer(nn.Module):
         joint = _ops().join_key_sets([m._bsi_keys_cuda for m in layers], [m._buffers["bias"] for m in layers])
         if joint is not None:
             self.__dict__["_joint"] = joint[:2]
+            this = weakref.ref(self)
+
+            def drop(_):            # a projection was replaced: the joint image would only keep its memory
+                if this() is not None:
+                    this().__dict__.pop("_joint", None)
+            self.__dict__["_joined"] = [weakref.ref(m, drop) for m in layers]
             for m, bias in zip(layers, joint[2]):
                 m._buffers["bias"] = bias
 

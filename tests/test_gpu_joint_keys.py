@@ -32,3 +32,14 @@ def test_joint_projections(dtype, B, T, H):
         changed = layer(x)
         layer.__dict__.pop("_joint")
         assert torch.equal(changed, layer(x)) and not torch.equal(changed, got)
+
+
+# replaced projections take the joint image with them (key sets loaded into a model that was built with joined ones)
+def test_joint_image_goes_with_its_projections():
+    cfg = opt.OPTConfig(vocab_size=300, hidden_size=1024, num_hidden_layers=1, num_attention_heads=16, ffn_dim=1024, name="small")
+    layer = opt.build_opt_bsi(cfg, dtype=torch.float16, seed=5).model.decoder.layers[0]
+    held = torch.cuda.memory_allocated()
+    for name in ("q_proj", "k_proj", "v_proj"):
+        setattr(layer.self_attn, name, torch.nn.Identity())
+    words, image = 3 * 1024 * 6 * 16 * 8, 3 * 1024 * 1024
+    assert held - torch.cuda.memory_allocated() >= words + image
