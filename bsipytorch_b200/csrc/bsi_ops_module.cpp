@@ -14,12 +14,15 @@
 
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CUDAEvent.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <cuda_runtime_api.h>
 #include <unistd.h>
 
+#include <atomic>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -149,6 +152,8 @@ struct PackedBatch {
     float quantize_ms = 0.f;
 };
 
+constexpr int64_t kFewRows = 16;     // dots of more rows have no use for BSI_KEYS_COMPLETE
+
 struct PrebuiltBSIKeysCUDA {
     PackedBatch b;
     int64_t num_keys = 0;
@@ -168,6 +173,34 @@ struct PrebuiltBSIKeysCUDA {
                                          abs_sum.data_ptr<float>(), current_stream()),
                      "bsi_b200_key_bounds");
     }
+    // BSI_KEYS_COMPLETE once the host has seen that everything in front of an earlier dot on these keys is done, their build
+    // included; 0 before that. Called in front of a dot of few rows, on its stream. The event is that of the second such
+    // dot outside a capture: 3 us of host time that neither a build nor a first pass pays.
+    int complete() const {
+        if (!done_.load(std::memory_order_acquire)) {
+            std::lock_guard<std::mutex> lock(mutex_);
+            c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);    // a query may fall into another's capture
+            if (!event_.isCreated()) {
+                if (used_ && c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None)
+                    event_.record(at::cuda::getCurrentCUDAStream());
+                used_ = true;
+                return 0;
+            }
+            if (!event_.query()) return 0;
+            done_.store(true, std::memory_order_release);
+        }
+        return BSI_KEYS_COMPLETE;
+    }
+    bool is_complete() const { return done_.load(std::memory_order_acquire); }
+    void set_complete() { done_.store(true, std::memory_order_release); }       // after a synchronisation
+
+private:
+    mutable std::atomic<bool> done_{false};
+    mutable std::mutex mutex_;
+    mutable at::cuda::CUDAEvent event_;
+    mutable bool used_ = false;
+
+public:
     // Called before every dot on these keys: the bound depends on the width of the queries of that dot.
     void register_bounds(int query_bits) const {
         if (!abs_sum.defined()) return;
@@ -668,6 +701,7 @@ py::tuple run_dot(const Env& env, const PackedBatch& qb, const PrebuiltBSIKeysCU
     const int engine = env.dot_engine();
     const int64_t qs_stride = qb.chunk_mode ? qb.chunks : 0;
     const bsi_dot_bounds bounds = dot_bounds(keys, qb.variable ? 8 : qb.S, &qb);
+    const int complete = Q <= kFewRows ? keys.complete() : 0;
     if (qb.variable || keys.b.variable) {
         TORCH_CHECK(engine != BSI_ENGINE_BMMA, "the b1 mma.sync engine reads fixed-bit slices; variable-slice operands use the int8 engines");
         TORCH_CHECK(!want_iacc, "the per-chunk accumulator dump is defined for the fixed-bit mode");
@@ -682,7 +716,8 @@ py::tuple run_dot(const Env& env, const PackedBatch& qb, const PrebuiltBSIKeysCU
             at::Tensor& dst = digit == 0 ? out : out_hi;
             check_status(bsi_b200_dot_i8_bounded(a8.data_ptr<int8_t>(), a8.size(1), qb.scales.data_ptr<float>(), 0,
                                          keys.b.q8.data_ptr<int8_t>(), keys.b.q8.size(1), keys.b.scales.data_ptr<float>(),
-                                         Q, R, qb.chunks, 1.0f, dst.data_ptr<float>(), R, nullptr, engine, &bounds, current_stream()),
+                                         Q, R, qb.chunks, 1.0f, dst.data_ptr<float>(), R, nullptr, engine | complete, &bounds,
+                                         current_stream()),
                          "bsi_b200_dot_i8");
         }
         out.add_(out_hi, 128.0f).mul_(static_cast<float>(scale_inv));
@@ -698,7 +733,7 @@ py::tuple run_dot(const Env& env, const PackedBatch& qb, const PrebuiltBSIKeysCU
         check_status(bsi_b200_dot_i8_bounded(qb.q8.data_ptr<int8_t>(), qb.q8.size(1), qb.scales.data_ptr<float>(), qs_stride,
                                      keys.b.q8.data_ptr<int8_t>(), keys.b.q8.size(1), keys.b.scales.data_ptr<float>(),
                                      Q, R, qb.chunks, static_cast<float>(scale_inv), out.data_ptr<float>(), R,
-                                     want_iacc ? iacc.data_ptr<int>() : nullptr, engine, &bounds, current_stream()),
+                                     want_iacc ? iacc.data_ptr<int>() : nullptr, engine | complete, &bounds, current_stream()),
                      "bsi_b200_dot_i8");
     }
     if (profile) {
@@ -904,10 +939,10 @@ void linear_forward(const Env& env, const at::Tensor& x2d, int decimalPlaces, bo
             continue;
         }
         if (one_launch && bsi_b200_linear_decode_fits(Q, R, D)) {
-            check_status(bsi_b200_linear_decode(x.data_ptr(), code, ldx, D, decimalPlaces, bits, keys.b.q8.data_ptr<int8_t>(),
-                                                keys.b.q8.size(1), keys.b.scales.data_ptr<float>(), bptr, Q, R, scale_inv,
-                                                y.data_ptr(), R, act, scaled, factor, current_stream()),
-                         "bsi_b200_linear_decode");
+            check_status(bsi_b200_linear_decode_engine(x.data_ptr(), code, ldx, D, decimalPlaces, bits, keys.b.q8.data_ptr<int8_t>(),
+                                                       keys.b.q8.size(1), keys.b.scales.data_ptr<float>(), bptr, Q, R, scale_inv,
+                                                       y.data_ptr(), R, act, scaled, factor, keys.complete(), current_stream()),
+                         "bsi_b200_linear_decode_engine");
             g_last_quantize_ns = g_last_pack_ns = g_last_total_ns = 0;      // no pack of its own to report
             rest();
             continue;
@@ -943,7 +978,8 @@ void linear_forward(const Env& env, const at::Tensor& x2d, int decimalPlaces, bo
         bounds.query_sq_stride = chunks;
         check_status(bsi_b200_linear_i8_engine(q8, chunks * 256, scales, chunk ? chunks : 0, keys.b.q8.data_ptr<int8_t>(),
                                                keys.b.q8.size(1), keys.b.scales.data_ptr<float>(), bptr, Q, R, chunks, scale_inv,
-                                               y.data_ptr(), R, code, act, scaled, factor, &bounds, engine, current_stream()),
+                                               y.data_ptr(), R, code, act, scaled, factor, &bounds,
+                                               engine | (Q <= kFewRows ? keys.complete() : 0), current_stream()),
                      "bsi_b200_linear_i8_engine");
         rest();
     }
@@ -1027,12 +1063,14 @@ py::object join_key_sets(const py::list& keys, const py::list& biases) {
     const at::Tensor all = bias.empty() ? at::Tensor() : at::cat(bias, 0);
     // the members' old images return to the allocator below
     C10_CUDA_CHECK(cudaDeviceSynchronize());
+    joint->set_complete();
     py::list views;
     int64_t row = 0;
     for (size_t i = 0; i < n; ++i) {
         const int64_t rows = sets[i]->num_keys;
         bsi_b200_unregister_key_bounds(sets[i]->b.q8.data_ptr<int8_t>());
         sets[i]->b.q8 = joint->b.q8.narrow(0, row, rows);
+        sets[i]->set_complete();
         if (all.defined()) views.append(py::cast(all.narrow(0, row, rows)));
         row += rows;
     }
@@ -1188,7 +1226,9 @@ at::Tensor linear_from_packed(torch::Tensor q8, torch::Tensor scales, py::capsul
                                            keys->b.scales.data_ptr<float>(), bptr, Q, R, chunks,
                                            static_cast<float>(scale_inv), y.data_ptr(), R, code,
                                            relu ? BSI_ACT_RELU : BSI_ACT_NONE, scaled_columns, static_cast<float>(factor), &bounds,
-                                           env.engine_free() ? BSI_ENGINE_AUTO : BSI_ENGINE_TCGEN05, current_stream()),
+                                           (env.engine_free() ? BSI_ENGINE_AUTO : BSI_ENGINE_TCGEN05) |
+                                               (Q <= kFewRows ? keys->complete() : 0),
+                                           current_stream()),
                  "bsi_b200_linear_i8_engine");
     return y;
 }
@@ -1393,7 +1433,8 @@ py::dict debug_query_batch_tensors(py::capsule cap) {
 py::dict debug_keys_tensors(py::capsule cap) {
     auto* keys = from_capsule<PrebuiltBSIKeysCUDA>(cap, "PrebuiltBSIKeysCUDA");
     py::dict d = debug_batch(keys->b);
-    if (keys->abs_sum.defined()) d["abs_sum"] = keys->abs_sum;   // [2, R]: what register_key_bounds is given
+    if (keys->abs_sum.defined()) d["abs_sum"] = keys->abs_sum;   // [3, R]: what register_key_bounds is given
+    d["complete"] = keys->is_complete();
     return d;
 }
 py::dict debug_query_tensors(py::capsule cap) {

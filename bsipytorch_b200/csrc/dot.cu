@@ -20,7 +20,7 @@ int dot_i8_pair(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_strid
 bool decode_fits(int64_t Q, int64_t R, int64_t chunks);
 int dot_decode(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride, const int8_t* k8, int64_t ldk, const float* bw0,
                const float* bias, int64_t Q, int64_t R, int64_t chunks, float scale_inv, void* out, int64_t ldo, int y_dtype,
-               const Finishing& fin, cudaStream_t stream, bool* taken);
+               const Finishing& fin, bool keys_complete, cudaStream_t stream, bool* taken);
 
 int dot_words_bmma(const uint64_t* A, const float* qs, int64_t qs_stride, int Sa, int64_t W,
                    const uint64_t* B, const float* Bw, int Sb, int64_t R, int64_t Q, float scale_inv,
@@ -136,6 +136,8 @@ extern "C" int bsi_b200_dot_i8_bounded(const int8_t* a8, int64_t lda, const floa
     if (qs_stride != 0 && qs_stride < chunks) return fail(BSI_ERR_INVALID, "dot_i8: qs_stride < chunks");
     if (int rc = require_sm100()) return rc;
 
+    const bool keys_complete = (engine & BSI_KEYS_COMPLETE) != 0;
+    engine &= ~BSI_KEYS_COMPLETE;
     int force_bn = 0;
     if (engine >= 1000) {  // 1000 + tile width: test hook to pin the tcgen05 tile shape
         force_bn = engine - 1000;
@@ -145,7 +147,7 @@ extern "C" int bsi_b200_dot_i8_bounded(const int8_t* a8, int64_t lda, const floa
         if (dbg_iacc == nullptr && decode_fits(Q, R, chunks)) {
             bool taken = false;
             const int rc = dot_decode(a8, lda, qs, qs_stride, k8, ldk, bw0, nullptr, Q, R, chunks, scale_inv, out, ldo,
-                                      BSI_DTYPE_F32, Finishing{}, stream, &taken);
+                                      BSI_DTYPE_F32, Finishing{}, keys_complete, stream, &taken);
             if (rc != BSI_OK || taken) return rc;
         }
         engine = BSI_ENGINE_TCGEN05;
@@ -204,6 +206,8 @@ extern "C" int bsi_b200_linear_i8_engine(const int8_t* a8, int64_t lda, const fl
         return fail(BSI_ERR_INVALID, "linear_i8: unknown activation");
     if (y_dtype != BSI_DTYPE_F32 && y_dtype != BSI_DTYPE_F16 && y_dtype != BSI_DTYPE_BF16)
         return fail(BSI_ERR_INVALID, "linear_i8: unknown y_dtype");
+    const bool keys_complete = (engine & BSI_KEYS_COMPLETE) != 0;
+    engine &= ~BSI_KEYS_COMPLETE;
     if (engine != BSI_ENGINE_AUTO && engine != BSI_ENGINE_TCGEN05)
         return fail(BSI_ERR_INVALID, "linear_i8: engine must be AUTO or TCGEN05");
     if (int rc = require_sm100()) return rc;
@@ -213,7 +217,7 @@ extern "C" int bsi_b200_linear_i8_engine(const int8_t* a8, int64_t lda, const fl
     if (engine == BSI_ENGINE_AUTO && decode_fits(Q, R, chunks)) {
         bool taken = false;
         const int rc = dot_decode(a8, lda, qs, qs_stride, k8, ldk, bw0, bias, Q, R, chunks, scale_inv, y, ldy, y_dtype, fin,
-                                  static_cast<cudaStream_t>(stream_), &taken);
+                                  keys_complete, static_cast<cudaStream_t>(stream_), &taken);
         if (rc != BSI_OK || taken) return rc;
     }
     return dot_i8_pair(a8, lda, qs, qs_stride, k8, ldk, bw0, bias, Q, R, chunks, scale_inv, y, ldy, y_dtype,

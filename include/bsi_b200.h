@@ -47,7 +47,12 @@ enum {
     BSI_ENGINE_AUTO = 0,    /* tcgen05; the key-streaming kernel for 16 query rows and fewer */
     BSI_ENGINE_TCGEN05 = 1, /* int8 recombination, tcgen05.mma kind::i8, TMEM accumulators, TMA */
     BSI_ENGINE_SIMT = 2,    /* dp4a on the CUDA cores (cross-check engine) */
-    BSI_ENGINE_BMMA = 3     /* mma.sync b1 AND+POPC directly on the slice words */
+    BSI_ENGINE_BMMA = 3,    /* mma.sync b1 AND+POPC directly on the slice words */
+    /* Or'ed into an engine argument: the key image is complete, that is, the host has seen (by an event or by
+     * synchronising) that whatever wrote k8 is done, and nothing writes it before the dot is. The dots start while the
+     * kernel before them on the stream still runs; told this, the key-streaming kernel reads its first keys at once
+     * instead of behind that kernel. */
+    BSI_KEYS_COMPLETE = 0x10000
 };
 
 typedef void* bsi_stream_t; /* cudaStream_t */
@@ -264,6 +269,11 @@ int bsi_b200_linear_decode(const void* x, int x_dtype, int64_t ldx, int64_t D, i
                            const int8_t* k8, int64_t ldk, const float* bw0, const float* bias, int64_t Q, int64_t R,
                            float scale_inv, void* y, int64_t ldy, int activation, int64_t scaled_cols, float factor,
                            bsi_stream_t stream);
+/* engine: BSI_ENGINE_AUTO, with or without BSI_KEYS_COMPLETE. */
+int bsi_b200_linear_decode_engine(const void* x, int x_dtype, int64_t ldx, int64_t D, int decimal_places, int bits,
+                                  const int8_t* k8, int64_t ldk, const float* bw0, const float* bias, int64_t Q, int64_t R,
+                                  float scale_inv, void* y, int64_t ldy, int activation, int64_t scaled_cols, float factor,
+                                  int engine, bsi_stream_t stream);
 
 /* Linear whose finished output is re-quantised for the next linear inside the epilogue, so that the
  * layer-type [Q, R] matrix is never written: y = activation(cast(out) + cast(bias)) in layer_dtype

@@ -116,3 +116,38 @@ def test_one_launch_layer_leaves_no_old_profile(monkeypatch):
     monkeypatch.delenv("BSI_PROFILE")
     ops.bsi_linear_forward(x, keys, None, 2)
     assert ops.get_last_query_build_profile_cuda() == (0, 0, 0)
+
+
+# The kernel may read keys ahead of the kernel before it only once the host has seen the key set's build done; a call right
+# behind the build, or recorded in a graph, does not count as having seen it.
+@pytest.mark.parametrize("Q", [4, 16])
+def test_keys_count_as_complete_only_when_seen(Q):
+    import bsipytorch_b200
+    ops = bsipytorch_b200.bsi_ops
+    x, k = _inputs.fc1(Q=Q, R=700, D=4096, seed=Q, dtype=torch.float32)
+    x, k = x.to(DEV), k.to(DEV)
+    want = ops.bsi_layer_forward(x, ops.build_bsi_keys_cuda(k, 2)[0], None, 2)
+    complete = lambda keys: ops.debug_keys_tensors(keys)["complete"]      # noqa: E731
+    torch.cuda.synchronize()
+    torch.cuda._sleep(200_000_000)
+    keys = ops.build_bsi_keys_cuda(k, 2)[0]
+    passes = [ops.bsi_layer_forward(x, keys, None, 2) for _ in range(3)]
+    assert not complete(keys)
+    torch.cuda.synchronize()
+    passes.append(ops.bsi_layer_forward(x, keys, None, 2))
+    assert complete(keys)
+    assert all(torch.equal(y, want) for y in passes)
+    keys = ops.build_bsi_keys_cuda(k, 2)[0]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = ops.bsi_layer_forward(x, keys, None, 2)
+    assert not complete(keys)
+    graph.replay()
+    assert torch.equal(captured, want)
+    queries = ops.build_bsi_queries_cuda_batch_packed(x, 2)
+    for _ in range(3):
+        assert torch.equal(ops.batch_dot_product_multiquery_cuda_batch_caps(queries, keys)[0], want)
+        torch.cuda.synchronize()
+    with torch.cuda.graph(torch.cuda.CUDAGraph()):                        # the question may be asked inside a capture
+        ops.bsi_layer_forward(x, keys, None, 2)
+    assert complete(keys)
