@@ -92,4 +92,15 @@ bool pdl_enabled();
 // Reads and clears the status word of the peer barrier kernels (0 = clean, 64 + p = gave up waiting for rank p).
 int take_peer_status(int* v);
 
+// For kernels that start while the kernels in front of them on the stream still run (programmatic dependent launch): the
+// pointer, behind griddepcontrol.wait, to something those may have written. Loads through it are ordinary coherent ones
+// behind the wait. __ldg, and a const __restrict__ parameter, which the compiler treats alike, are no choice there:
+// ld.global.nc is for memory that nobody writes while the kernel is resident, and may be moved over the wait.
+template <typename T>
+__device__ __forceinline__ const T* behind_wait(const T* p) {
+    size_t g = __cvta_generic_to_global(p);
+    asm volatile("" : "+l"(g) :: "memory");
+    return static_cast<const T*>(__cvta_global_to_generic(g));
+}
+
 }  // namespace bsi

@@ -58,7 +58,7 @@ struct DecodeArgs {
 
 __device__ __forceinline__ uint4 ld_stream(const int8_t* p) {
     uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.L2::256B.v4.u32 {%0, %1, %2, %3}, [%4];"
+    asm volatile("ld.global.L1::no_allocate.L2::256B.v4.u32 {%0, %1, %2, %3}, [%4];"
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }
@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(kThreads, 1) dot_decode_kernel(const DecodeArg
                     const int u = min(u0 + h * kWarps, total - 1);
                     const int q = u / len, c = u - q * len;
                     const int64_t col = static_cast<int64_t>(c0 + c) * 256 + lane * 8;
-                    const XT* row = static_cast<const XT*>(p.x) + q * p.ldx;
+                    const XT* row = behind_wait(static_cast<const XT*>(p.x)) + q * p.ldx;
                     const int64_t left = p.D - col;
                     if (left >= 8 && ((reinterpret_cast<uintptr_t>(row + col) & 15) == 0)) r[h].load(row + col);
                     else r[h].load_tail(row + (left > 0 ? col : 0), left);
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(kThreads, 1) dot_decode_kernel(const DecodeArg
                 for (int h = 0; h < kAhead; ++h) {
                     const int i = min(i0 + h * kThreads, total - 1), qc = i >> 4;
                     const int q = qc / len, c = qc - q * len;
-                    v[h] = *reinterpret_cast<const uint4*>(p.a8 + q * p.lda + static_cast<int64_t>(c0 + c) * 256 + (i & 15) * 16);
+                    v[h] = *reinterpret_cast<const uint4*>(behind_wait(p.a8) + q * p.lda + static_cast<int64_t>(c0 + c) * 256 + (i & 15) * 16);
                 }
 #pragma unroll
                 for (int h = 0; h < kAhead; ++h) {
@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(kThreads, 1) dot_decode_kernel(const DecodeArg
             }
             for (int i = threadIdx.x; i < p.Q * len; i += kThreads) {
                 const int q = i / len, c = i - q * len;
-                qsc[q * p.slab + c] = p.qs_stride ? p.qs[q * p.qs_stride + c0 + c] : p.qs[q];
+                qsc[q * p.slab + c] = behind_wait(p.qs)[p.qs_stride ? q * p.qs_stride + c0 + c : q];
             }
         }
         __syncthreads();
@@ -241,8 +241,8 @@ __global__ void __launch_bounds__(kThreads, 1) dot_decode_kernel(const DecodeArg
                 const bool last = s + 1 == p.slabs;
                 float w = 0.0f, bv = 0.0f;
                 if (last && row < p.R) {
-                    w = __ldg(p.bw0 + row);
-                    if (p.bias != nullptr) bv = __ldg(p.bias + row);
+                    w = behind_wait(p.bw0)[row];
+                    if (p.bias != nullptr) bv = behind_wait(p.bias)[row];
                 }
                 float* keep = accs + (static_cast<int64_t>(it) * p.rt * p.Q + rq) * 16 + key;
                 float acc = s > 0 ? *keep : 0.0f;

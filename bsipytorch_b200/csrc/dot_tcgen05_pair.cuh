@@ -289,7 +289,7 @@ __device__ __forceinline__ float zero_of<float>() { return 0.0f; }
 // maximum over them). Neighbouring lanes read neighbouring vectors of a row and add up by shuffles: with a row per lane
 // every load touched 32 lines, 7 thousand cycles for 64 chunks.
 template <typename V>
-__device__ __forceinline__ void row_stats(const float* __restrict__ qs, int64_t qs_stride, const float* __restrict__ norms, int64_t n_stride,
+__device__ __forceinline__ void row_stats(const float* qs, int64_t qs_stride, const float* norms, int64_t n_stride,
                                           int first_row, int Q, int units, float& smax, float& ssum, float& u2) {
     constexpr int kMost = sizeof(V) == 16 ? 8 : 32;      // lanes on a row at most
     constexpr int kRows = 4;                             // rows per lane group in flight
@@ -307,8 +307,8 @@ __device__ __forceinline__ void row_stats(const float* __restrict__ qs, int64_t 
             for (int h = 0; h < kRows; ++h) {
                 const int r = first_row + (((it + h) << 5) >> lg) + (lane >> lg);
                 const bool in = it + h < group && u0 + sub < units && r < Q;
-                a[h] = in ? __ldg(reinterpret_cast<const V*>(qs + r * qs_stride) + u0 + sub) : zero_of<V>();
-                b[h] = in && norms != nullptr ? __ldg(reinterpret_cast<const V*>(norms + r * n_stride) + u0 + sub) : zero_of<V>();
+                a[h] = in ? reinterpret_cast<const V*>(qs + r * qs_stride)[u0 + sub] : zero_of<V>();
+                b[h] = in && norms != nullptr ? reinterpret_cast<const V*>(norms + r * n_stride)[u0 + sub] : zero_of<V>();
             }
 #pragma unroll
             for (int h = 0; h < kRows; ++h) {
@@ -332,14 +332,14 @@ __device__ __forceinline__ void row_stats(const float* __restrict__ qs, int64_t 
 
 // The same for one row per lane: kAhead vectors of each array in flight.
 template <typename V, int kAhead>
-__device__ __forceinline__ void row_of_lane(const float* __restrict__ qs_row, const float* __restrict__ n_row, int units, float& smax,
+__device__ __forceinline__ void row_of_lane(const float* qs_row, const float* n_row, int units, float& smax,
                                             float& ssum, float& u2) {
     for (int c = 0; c < units; c += kAhead) {
         V a[kAhead], n[kAhead];
 #pragma unroll
         for (int h = 0; h < kAhead; ++h) {
-            a[h] = c + h < units ? __ldg(reinterpret_cast<const V*>(qs_row) + c + h) : zero_of<V>();
-            n[h] = c + h < units && n_row != nullptr ? __ldg(reinterpret_cast<const V*>(n_row) + c + h) : zero_of<V>();
+            a[h] = c + h < units ? reinterpret_cast<const V*>(qs_row)[c + h] : zero_of<V>();
+            n[h] = c + h < units && n_row != nullptr ? reinterpret_cast<const V*>(n_row)[c + h] : zero_of<V>();
         }
 #pragma unroll
         for (int h = 0; h < kAhead; ++h) {
@@ -684,7 +684,7 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
             const int row = tm * 256 + static_cast<int>(rank) * BM + quad * 32 + lane;
             const int n0 = tn * BN;
             const bool row_ok = row < Q;
-            const float* qs_row = qs + static_cast<int64_t>(row_ok ? row : 0) * (qs_stride ? qs_stride : 1);
+            const float* qs_row = behind_wait(qs) + static_cast<int64_t>(row_ok ? row : 0) * (qs_stride ? qs_stride : 1);
 #pragma unroll
             for (int j = 0; j < kCols; ++j) acc[j] = 0.0f;
             // Key scale and bias of the column this lane puts into shared memory for the store phase: a quarter of the
@@ -693,8 +693,8 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
             const int own = quad * kOwn + lane;
             float own_w = 0.0f, own_b = 0.0f;
             if (lane < kOwn && n0 + col0 + own < R) {
-                own_w = __ldg(bw0 + n0 + col0 + own);
-                if (has_bias) own_b = __ldg(bias + n0 + col0 + own);
+                own_w = behind_wait(bw0)[n0 + col0 + own];
+                if (has_bias) own_b = behind_wait(bias)[n0 + col0 + own];
             }
 
             // Integer accumulation where it provably equals the float32 chain: the chunk terms I_c * 2^shift are
@@ -711,15 +711,16 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
             bool exact = false, small = false;
             if (k_abs_sum != nullptr && ok) {
                 // of the warp's key rows: the largest sum of |k| over a row and over one chunk, the largest sum of k^2
+                const float* k_sums = behind_wait(k_abs_sum);
                 float ktot = 0.0f, kchk = 0.0f, k2 = 0.0f;
                 if (lane * 4 < kCols) {
                     float kv[12];
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
                         const int col = min(n0 + col0 + lane * 4 + e, R - 1);
-                        kv[e] = __ldg(k_abs_sum + col);
-                        kv[4 + e] = __ldg(k_abs_sum + R + col);
-                        kv[8 + e] = __ldg(k_abs_sum + 2 * static_cast<int64_t>(R) + col);
+                        kv[e] = k_sums[col];
+                        kv[4 + e] = k_sums[R + col];
+                        kv[8 + e] = k_sums[2 * static_cast<int64_t>(R) + col];
                     }
                     ktot = fmaxf(fmaxf(kv[0], kv[1]), fmaxf(kv[2], kv[3]));
                     kchk = fmaxf(fmaxf(kv[4], kv[5]), fmaxf(kv[6], kv[7]));
@@ -728,16 +729,16 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                 // of the warp's query rows: the largest and the largest summed 2^shift of a row, the largest sum of squares
                 float smax = 0.0f, ssum = 0.0f, u2 = 0.0f;
                 const int first_row = row - lane;
-                const float* norms = qs_stride ? q_sq : nullptr;
+                const float* norms = qs_stride && q_sq != nullptr ? behind_wait(q_sq) : nullptr;
                 if (!qs_stride) {
-                    if (row_ok) smax = __ldg(qs_row);
+                    if (row_ok) smax = *qs_row;
                     ssum = smax * static_cast<float>(chunks);
                 } else {
                     const bool vec = (chunks & 3) == 0 && (qs_stride & 3) == 0 && (q_sq_stride & 3) == 0 &&
                                      ((reinterpret_cast<uintptr_t>(qs) | reinterpret_cast<uintptr_t>(norms)) & 15) == 0;
                     if (chunks > 16) {
-                        if (vec) row_stats<float4>(qs, qs_stride, norms, q_sq_stride, first_row, Q, chunks / 4, smax, ssum, u2);
-                        else row_stats<float>(qs, qs_stride, norms, q_sq_stride, first_row, Q, chunks, smax, ssum, u2);
+                        if (vec) row_stats<float4>(behind_wait(qs), qs_stride, norms, q_sq_stride, first_row, Q, chunks / 4, smax, ssum, u2);
+                        else row_stats<float>(behind_wait(qs), qs_stride, norms, q_sq_stride, first_row, Q, chunks, smax, ssum, u2);
                     } else if (row_ok) {
                         // few chunks: a row per lane, everything in one go or two
                         const float* nrow = norms != nullptr ? norms + static_cast<int64_t>(row) * q_sq_stride : nullptr;
@@ -774,12 +775,12 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
             }
             // the chunk scale of the next chunk is loaded a whole chunk ahead: a scattered load per lane (32 rows) that
             // would otherwise stand in front of every fold
-            float qnext = qs_stride ? __ldg(qs_row + min(c_lo, chunks - 1)) : __ldg(qs_row);
+            float qnext = qs_row[qs_stride ? min(c_lo, chunks - 1) : 0];
             for (int c = 0; c < n_chunks && ok; ++c, ++cc) {
                 const int b = cc % kAccBufs;
                 const uint32_t tph = static_cast<uint32_t>(cc / kAccBufs) & 1u;
                 const float qscale = qnext;
-                if (qs_stride && c + 1 < n_chunks) qnext = __ldg(qs_row + c_lo + c + 1);
+                if (qs_stride && c + 1 < n_chunks) qnext = qs_row[c_lo + c + 1];
                 const int qmul = exact ? __float2int_rn(qscale) : 0;
                 if (!wait_or_abort(tfull_bar(b), tph, actx, 4)) { ok = false; break; }
                 tc_fence_after();

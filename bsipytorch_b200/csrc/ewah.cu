@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, kBlocksPerSm<TILES>) ewah
     asm volatile("griddepcontrol.wait;" ::: "memory");
     auto sum_of = [&](unsigned n) {      // of the first n block sums, for every thread of the block
         u64 t = 0;
-        for (unsigned i = threadIdx.x; i < n; i += kWarpsPerBlock * 32) t += __ldg(block_sums + i);
+        for (unsigned i = threadIdx.x; i < n; i += kWarpsPerBlock * 32) t += behind_wait(block_sums)[i];
         t = warp_sum_u64(t);
         if (lane == 0) wsum[warp] = t;
         __syncthreads();
@@ -556,7 +556,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, kBlocksPerSm<TILES>) ewah
     // group ahead like the slices
     auto group = [&](int g) -> u64 {
         if (lane >= kWarpsPerBlock || g + lane >= count) return 0ull;
-        return __ldg(sizes + s0 + g + lane) | static_cast<u64>(__ldg(flags + s0 + g + lane)) << 63;
+        return behind_wait(sizes)[s0 + g + lane] | static_cast<u64>(behind_wait(flags)[s0 + g + lane]) << 63;
     };
     auto one = [&](int g, u64 size_flag, const u64 (&wv)[kRegs]) {
         const int64_t s = s0 + g + warp;

@@ -97,7 +97,7 @@ __device__ __forceinline__ void emit_chunk(const long long (&v)[8], int shift, i
 // One (row, chunk) unit on the generic path (any decimal_places, any magnitude, NaN/inf, any layout):
 // 64-bit integers and 64-bit offsets throughout.
 template <typename T>
-__device__ __forceinline__ void generic_unit(const T* __restrict__ x, int64_t unit, int64_t D, int64_t ldx,
+__device__ __forceinline__ void generic_unit(const T* x, int64_t unit, int64_t D, int64_t ldx,
                                              double dec_scale, uint32_t dec_mult, int bits, int64_t chunks, int64_t W,
                                              u64* __restrict__ words, float* __restrict__ scales,
                                              int32_t* __restrict__ shifts, int8_t* __restrict__ q8, int64_t ld8,
@@ -235,13 +235,14 @@ constexpr int kSlowQueue = 8;   // units per warp that may wait for the generic 
 // a unit's element offset is unit * 256 and no lane ever needs the scalar tail loads.
 template <typename T, bool kDense, bool kWords, bool kQ8>
 __global__ void __launch_bounds__(256, BSI_PACK_MIN_BLOCKS) quantize_pack_chunk_fast_kernel(
-    const T* __restrict__ x, FastGeom g, double dec_scale, uint32_t dec_mult, int bits,
+    const T* x, FastGeom g, double dec_scale, uint32_t dec_mult, int bits,
     u64* __restrict__ words, float* __restrict__ scales, int32_t* __restrict__ shifts, int8_t* __restrict__ q8,
     int vec_ok, float* __restrict__ sq_norms, float* __restrict__ slice_weights) {
     // Launched as a programmatic dependent, and letting its own dependents go at once: a dot sets up its barriers and
     // tensor memory while this kernel runs, and reads its results behind griddepcontrol.wait.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    x = behind_wait(x);
     __shared__ uint32_t slow_queue[8][kSlowQueue];
     constexpr int kDepth = sizeof(T) == 2 ? 4 : 2;
     const int lane = threadIdx.x & 31;

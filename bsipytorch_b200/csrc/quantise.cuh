@@ -81,17 +81,17 @@ __device__ __forceinline__ int shift_for(u64 max_abs, int bits) {
 
 // Loads the 8 elements [col, col+8) of a row as float; elements at or beyond D read as 0.
 template <typename T>
-__device__ __forceinline__ void load8(const T* __restrict__ row, int64_t col, int64_t D, bool vec_ok,
+__device__ __forceinline__ void load8(const T* row, int64_t col, int64_t D, bool vec_ok,
                                       float (&f)[8]) {
     if (vec_ok && col + 8 <= D) {
         if constexpr (sizeof(T) == 2) {
-            const uint4 raw = __ldg(reinterpret_cast<const uint4*>(row + col));
+            const uint4 raw = *reinterpret_cast<const uint4*>(row + col);
             const T* h = reinterpret_cast<const T*>(&raw);
 #pragma unroll
             for (int e = 0; e < 8; ++e) f[e] = to_float(h[e]);
         } else {
-            const float4 a = __ldg(reinterpret_cast<const float4*>(row + col));
-            const float4 b = __ldg(reinterpret_cast<const float4*>(row + col) + 1);
+            const float4 a = *reinterpret_cast<const float4*>(row + col);
+            const float4 b = *(reinterpret_cast<const float4*>(row + col) + 1);
             f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w;
             f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
         }
@@ -125,17 +125,17 @@ template <typename T>
 struct RawLane {
     static constexpr int kVecs = sizeof(T) == 2 ? 1 : 2;
     uint4 v[kVecs];
-    __device__ __forceinline__ void load(const T* __restrict__ p) {
+    __device__ __forceinline__ void load(const T* p) {
 #pragma unroll
-        for (int i = 0; i < kVecs; ++i) v[i] = __ldg(reinterpret_cast<const uint4*>(p) + i);
+        for (int i = 0; i < kVecs; ++i) v[i] = reinterpret_cast<const uint4*>(p)[i];
     }
     // the first n (at most 8) elements at p one by one, zeros behind them
-    __device__ __forceinline__ void load_tail(const T* __restrict__ p, int64_t n) {
+    __device__ __forceinline__ void load_tail(const T* p, int64_t n) {
         using Bits = typename std::conditional<sizeof(T) == 2, unsigned short, unsigned int>::type;
         const Bits* src = reinterpret_cast<const Bits*>(p);
         Bits b[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) b[e] = e < n ? __ldg(src + e) : static_cast<Bits>(0);
+        for (int e = 0; e < 8; ++e) b[e] = e < n ? src[e] : static_cast<Bits>(0);
         if constexpr (sizeof(T) == 2) {
             v[0] = make_uint4(b[0] | (static_cast<uint32_t>(b[1]) << 16), b[2] | (static_cast<uint32_t>(b[3]) << 16),
                               b[4] | (static_cast<uint32_t>(b[5]) << 16), b[6] | (static_cast<uint32_t>(b[7]) << 16));
