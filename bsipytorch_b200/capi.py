@@ -36,6 +36,7 @@ SIGNATURES = {
     "bsi_b200_register_key_bounds": (_i32, [_vp, _vp, _i64, _i32]),
     "bsi_b200_unregister_key_bounds": (_i32, [_vp]),
     "bsi_b200_debug_exact_int_tiles": (_i32, [_vp]),
+    "bsi_b200_debug_last_tiles": (_i32, [_vp, _vp]),
     "bsi_b200_recombine_i8": (_i32, [_vp, _i64, _i32, _i64, _vp, _i64, _vp]),
     "bsi_b200_dot_i8": (_i32, [_vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _i64, _i64, _f32, _vp, _i64, _vp, _i32, _vp]),
     "bsi_b200_linear_i8": (_i32, [_vp, _i64, _vp, _i64, _vp, _i64, _vp, _vp, _i64, _i64, _i64, _f32, _vp, _i64, _i32, _vp]),
@@ -113,6 +114,13 @@ def exact_int_tiles() -> int:
     v = C.c_ulonglong(0)
     check(lib().bsi_b200_debug_exact_int_tiles(C.byref(v)), "bsi_b200_debug_exact_int_tiles")
     return v.value
+
+
+def last_tiles():
+    """(columns of a tile, parts along K) of this thread's last dot on the paired tensor-core kernel."""
+    width, parts = C.c_int(0), C.c_int(0)
+    check(lib().bsi_b200_debug_last_tiles(C.byref(width), C.byref(parts)), "bsi_b200_debug_last_tiles")
+    return width.value, parts.value
 
 
 def device_status() -> int:

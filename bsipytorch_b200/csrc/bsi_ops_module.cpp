@@ -1079,6 +1079,8 @@ py::object join_key_sets(const py::list& keys, const py::list& biases) {
     return py::make_tuple(cap, all.defined() ? py::cast(all) : py::object(py::none()), views);
 }
 
+std::atomic<int64_t> g_joint_layers{0};     // layers whose projections ran on a joint image (a test hook)
+
 // One OPT decoder layer (pre-LN attention, ReLU MLP) whose six linears are BSI layers: the same ATen operators in the
 // same order as the module's Python forward and the BSI layers' own kernels, so the same bits. In Python the layer costs
 // 170 us of host time against 75 us of kernels (1024 tokens of OPT-125M). The query, key and value projections read one
@@ -1136,6 +1138,7 @@ py::object opt_layer_forward(const torch::Tensor& x, const py::tuple& norms, con
     }
     at::Tensor q, k, v;
     if (all != nullptr) {
+        ++g_joint_layers;
         LinearTo to{all, &all_bias, at::Tensor(), scaling, H};
         linear_forward(env, flat(norm(x, 0)), dp[0], false, &to, 1);
         q = to.y.narrow(1, 0, H);
@@ -1722,6 +1725,8 @@ PYBIND11_MODULE(bsi_ops, m) {
     m.def("debug_keys_tensors", &debug_keys_tensors);
     m.def("debug_query_tensors", &debug_query_tensors);
     m.def("debug_dot_iacc", &debug_dot_iacc);
+    m.def("debug_joint_layers", []() { return g_joint_layers.exchange(0); },
+          "OPT layers whose projections ran on a joint key image since the last call");
     m.def("ewah_encode_words", &ewah_encode_words, py::arg("words"), py::arg("threshold"));
     m.def("ewah_decode_words", &ewah_decode_words, py::arg("stream"), py::arg("off"), py::arg("len"), py::arg("W"));
     m.def("save_keyset", &save_keyset, py::arg("keyset_cuda_cap"), py::arg("out_dir"),

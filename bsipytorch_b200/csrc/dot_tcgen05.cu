@@ -536,6 +536,9 @@ int pick_bn_pair(int64_t Q, int64_t R, bool any_width) {
     return best;
 }
 
+// Tile width and parts along K of this thread's last paired dot (a test hook: bsi_b200_debug_last_tiles).
+thread_local int t_last_width = 0, t_last_parts = 0;
+
 // How many clusters of 2 * SPLIT CTAs run at once (one CTA per SM whatever the tile width); 0 when the query fails.
 template <int SPLIT>
 int resident_clusters() {
@@ -624,6 +627,8 @@ int dot_i8_pair(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_strid
     // only with bounds (a split adds integers), one plain destination, and no accumulator dump
     const bool may_split = !force_bn && kabs != nullptr && dbg_iacc == nullptr && scatter.n == 0;
     const int parts = may_split ? pick_split(Q, R, chunks, bn, &bn) : 1;
+    t_last_width = bn;
+    t_last_parts = parts;
     if (bn < 64 || bn > 256 || (bn & 31) != 0 || (!any_width && (bn & (bn - 1)) != 0))
         return fail(BSI_ERR_INVALID, "dot_i8: tile width must be a multiple of 32 in [64, 256] (64, 128 or 256 for 16-bit outputs)");
     if (dbg_iacc != nullptr && y_dtype != BSI_DTYPE_F32)
@@ -737,6 +742,14 @@ extern "C" int bsi_b200_device_status(int* status_out) {
     if (int rc = take_peer_status(&pv)) return rc;
     if (v == 0) v = pv;
     *status_out = v;
+    return BSI_OK;
+}
+
+extern "C" int bsi_b200_debug_last_tiles(int* width_out, int* parts_out) {
+    using namespace bsi;
+    if (width_out == nullptr || parts_out == nullptr) return fail(BSI_ERR_INVALID, "debug_last_tiles: null pointer");
+    *width_out = t_last_width;
+    *parts_out = t_last_parts;
     return BSI_OK;
 }
 

@@ -746,8 +746,11 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                         else row_of_lane<float, 8>(qs_row, nrow, chunks, smax, ssum, u2);
                     }
                 }
-                // an infinity anywhere fails the test. By shuffles: as redux.sync the maximum left out some lanes in the split
-                // instantiations (nvcc 12.9), which a row that breaks the bounds on lane 22 showed.
+                // An infinity anywhere fails the test. By shuffles: with redux.sync (nvcc 12.9) an earlier form of this code
+                // had norm = 0 in every warp of one instantiation (256 columns, four parts), and so exact sums beyond 2^24.
+                // Not a divergent warp (a __syncwarp before each changed nothing) nor wrong operands (the other four maxima
+                // were right, and shuffles of the same registers are); writing the operands out made it go away. The split
+                // test has a row beyond the bounds for every width and number of parts.
                 auto most = [](float v) {
 #pragma unroll
                     for (int d = 16; d > 0; d >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, d));

@@ -22,14 +22,18 @@ def test_joint_projections(dtype, B, T, H):
         for m in (attn.q_proj, attn.k_proj, attn.v_proj):
             m.bias.copy_(torch.randn(H, generator=g) * 0.1)         # in place: the joint bias follows
         assert "_joint" in layer.__dict__
+        used = bsipytorch_b200.bsi_ops.debug_joint_layers
+        used()
         got = layer(x)
+        assert used() == 1
         joint = layer.__dict__.pop("_joint")
-        assert torch.equal(got, layer(x))
+        assert torch.equal(got, layer(x)) and used() == 0
         # a projection that changed its bias or its keys no longer runs on the joint image
         layer.__dict__["_joint"] = joint
         attn.k_proj.bias = attn.k_proj.bias + 1.0
         attn.v_proj._bsi_keys_cuda = bsipytorch_b200.bsi_ops.build_bsi_keys_cuda(torch.randn(H, H, generator=g) * 0.05, 2, 0.5)[0]
         changed = layer(x)
+        assert used() == 0
         layer.__dict__.pop("_joint")
         assert torch.equal(changed, layer(x)) and not torch.equal(changed, got)
 

@@ -18,15 +18,25 @@ class _Bounds(C.Structure):
     _fields_ = [("key_bounds", C.c_void_p), ("query_sq", C.c_void_p), ("query_sq_stride", C.c_int64), ("query_abs_max", C.c_int)]
 
 
-# sizes whose widths and parts differ: 256 and 128 columns in 2 and 4 parts, 64 columns (a share of 8 or 16 columns per
-# warp); chunk counts that do not divide, a part without chunks; ragged rows and columns
-@pytest.mark.parametrize("broken", [False, True])
-@pytest.mark.parametrize("Q,R,D", [(512, 2048, 8192), (512, 2040, 4352), (300, 1111, 5000), (40, 500, 8192), (129, 64, 1280), (256, 1500, 2304),
-                                   (33, 65, 16384)])
+# (columns, parts) of every split kernel and of the unsplit ones next to them; chunk counts that do not divide, a part
+# without chunks, ragged rows and columns, shares of 8 and of 16 columns per warp
+PLANS = {(512, 2048, 8192): (128, 2), (300, 1111, 5000): (128, 2), (300, 3000, 16384): (256, 2), (256, 1500, 2304): (64, 2),
+         (40, 500, 8192): (64, 4), (33, 65, 16384): (64, 4), (300, 500, 16384): (128, 4), (300, 1111, 16384): (256, 4),
+         (512, 2040, 4352): (64, 1), (129, 64, 1280): (64, 1), (512, 4000, 1280): (128, 1)}
+
+
+# broken: the row that breaks every bound, which sends its tiles to one pair and the float32 chain
+@pytest.mark.parametrize("broken", [None, 0.5, 1.0])
+@pytest.mark.parametrize("Q,R,D", PLANS)
 def test_split_dot_and_layer(Q, R, D, broken):
     q, k = _inputs.fc1(Q=Q, R=R, D=D, seed=Q + R + D, dtype=torch.float32)
-    if broken:
-        q[Q // 2] *= 3.0e4
+    width, parts = PLANS[Q, R, D]
+    tiles_m, tiles_n = (Q + 255) // 256, (R + width - 1) // width
+    exact = tiles_m * tiles_n * 16 * parts                       # warps that add integers: 16 per tile and part
+    if broken is not None:
+        row = min(int(Q * broken), Q - 1)
+        q[row] *= 3.0e4
+        exact -= tiles_n * (16 * parts - 14)                     # of the row's tiles the other 14 warps of one pair
     chunks, ld = (D + 255) // 256, (D + 255) // 256 * 256
     kb = H.quantize_pack(k.to(DEV), 2, 6, False)
     x = q.to(DEV)
@@ -39,13 +49,15 @@ def test_split_dot_and_layer(Q, R, D, broken):
     capi.check(L.bsi_b200_key_bounds(capi.ptr(kb["q8"]), ld, R, chunks, capi.ptr(bounds), capi.stream_ptr()))
     want = H.dot_i8(q8, scales, kb["q8"], kb["scales"], o.scale_inv(2), capi.ENGINE_SIMT)
     given = _Bounds(bounds.data_ptr(), norms.data_ptr(), chunks, 64)
+    def check_plan():
+        assert capi.last_tiles() == (width, parts) and capi.exact_int_tiles() == exact
     capi.exact_int_tiles()
     out = torch.full((Q, R), float("nan"), device=DEV)
     inv = C.c_float(float(o.scale_inv(2)))
     capi.check(L.bsi_b200_dot_i8_bounded(capi.ptr(q8), ld, capi.ptr(scales), chunks, capi.ptr(kb["q8"]), ld, capi.ptr(kb["scales"]), Q, R,
                                          chunks, inv, capi.ptr(out), R, None, 0, C.byref(given), capi.stream_ptr()))
     assert torch.equal(out.view(torch.int32), want.view(torch.int32))
-    assert capi.exact_int_tiles() > 0 or broken
+    check_plan()
     bias = torch.linspace(-1, 1, R, device=DEV)
     for dtype in (torch.float16, torch.bfloat16):
         y = torch.full((Q, R), float("nan"), dtype=dtype, device=DEV)
@@ -56,4 +68,5 @@ def test_split_dot_and_layer(Q, R, D, broken):
         z = torch.relu(want.to(dtype) + bias.to(dtype))
         z[:, : R // 16 * 8] *= 0.3
         assert torch.equal(y, z)
+        check_plan()
     assert capi.device_status() == 0
