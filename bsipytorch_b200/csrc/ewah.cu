@@ -14,6 +14,7 @@
 //   closes (at the next start, or at W).
 #include <string.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include <mutex>
@@ -430,13 +431,15 @@ __device__ __forceinline__ void load_slice(const u64* __restrict__ base, int W, 
 // which a scan kernel between the passes did before (7 us, most of it latency).
 // How many: slices of more than 128 words (registers for two of them per warp: 3 blocks per SM) take one wave of blocks,
 // so that a warp streams through its slices with loads always in flight, instead of four waves that each began with
-// a wait for memory and for the sums (28672 slices of 256 words, 86 % literals: 43.2 -> 31.2 us); two
-// waves up to 128 words, where more and shorter blocks fit; below, as many blocks as the sums allow.
+// a wait for memory and for the sums (28672 slices of 256 words, 86 % literals: 43.2 -> 31.2 us); six blocks per SM, a
+// wave and a half, up to 128 words, where a block's slices are shorter; below, and for slices that are walked in memory, as
+// many blocks as the sums allow.
 constexpr int kMaxSums = 2048;
 template <int TILES>
 constexpr int kBlocksPerSm = TILES > 4 ? 3 : TILES > 0 ? 4 : 5;
 inline int64_t slices_per_block(int64_t S, int64_t W) {
-    const int64_t blocks = W <= 64 || W > 256 ? kMaxSums : (W <= 128 ? 888 : 444);
+    const int64_t per_sm = W <= 128 ? 6 : kBlocksPerSm<8>;
+    const int64_t blocks = W <= 64 || W > 256 ? kMaxSums : std::min<int64_t>(per_sm * sm_count(), kMaxSums);
     const int64_t least = (S + blocks - 1) / blocks;
     return (least + kWarpsPerBlock - 1) / kWarpsPerBlock * kWarpsPerBlock;
 }

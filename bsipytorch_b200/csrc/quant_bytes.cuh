@@ -31,12 +31,6 @@ __device__ __forceinline__ uint32_t mask_clamp4(uint32_t u0, uint32_t u1, uint32
     return kClamp ? t ^ ((w ^ m) & 0x80808080u) : t ^ (m & 0x80808080u);
 }
 
-// The same with the signs in bit 31 of s0..s3 (e.g. the float bit patterns).
-__device__ __forceinline__ uint32_t sign_clamp4(uint32_t u0, uint32_t u1, uint32_t u2, uint32_t u3, uint32_t s0,
-                                                uint32_t s1, uint32_t s2, uint32_t s3, int bits) {
-    return mask_clamp4<true>(u0, u1, u2, u3, prmt(prmt(s0, s1, 0x00fbu), prmt(s2, s3, 0x00fbu), 0x5410u), bits);
-}
-
 // The reference's two roundings, |v| = floor(|x| * 10^dp + 0.5) and (|v| + [shift > 0] * 2^(shift-1)) >> shift, as two
 // FMAs with round toward zero. An FMA rounds the exact product and sum once, so no operand width matters:
 //   r1 = fma_rz(|x|, mult, 2^22 + 0.5)   floats in [2^22, 2^23) are the multiples of 1/2 and those in [2^23, 2^24) the
