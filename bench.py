@@ -41,8 +41,8 @@ WORKLOADS = {
 L2_BYTES = 126 * 1024 * 1024
 # dram__bytes_read.sum + dram__bytes_write.sum of one dot launch, from the ncu capture summarised
 # under profiles/ (None until a capture of that workload exists).
-NCU_TRAFFIC_BYTES = {"fc1": 18061056, "fc2": 21090000, "pack": 134321152 + 85714944, "pack-lean": 134263552 + 39758592,
-                     "ewah": 58746112 + 39424 + 59124992 + 8368384}
+NCU_TRAFFIC_BYTES = {"fc1": 18066688, "fc2": 21206272, "pack": 134282752 + 81137408, "pack-lean": 134273280 + 37389568,
+                     "ewah": 58760704 + 59137792 + 4631552}
 
 
 def make_inputs(wl, seed=123):
@@ -325,8 +325,8 @@ def run_hbm(args, rank, world, local_rank):
         step(0)
         torch.cuda.synchronize()
         stream_words = int(total.item())
-        # the sizes pass and the emit pass read the words once each, emit writes the stream
-        bytes_step = 2 * S * W * 8 + stream_words * 8 + S * 24
+        # what a call cannot do without; both of its passes read the words
+        bytes_step = S * W * 8 + stream_words * 8 + S * 16      # words once, stream, off / len / flags
         launches, kernel = 2, "ewah_sizes_kernel + ewah_emit_blocks_kernel"
         extra = {"stream_words": stream_words, "input_words": S * W}
     else:
