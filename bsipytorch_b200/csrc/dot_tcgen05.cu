@@ -28,6 +28,8 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "epilogue.cuh"
 #include "quantise.cuh"
@@ -387,6 +389,7 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_kernel(
 }
 
 #include "dot_tcgen05_pair.cuh"
+#include "dot_rows_tcgen05.cuh"
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
@@ -583,7 +586,118 @@ int pick_split(int64_t Q, int64_t R, int64_t chunks, int unsplit_bn, int* bn) {
     return parts;
 }
 
+// ---- dots of few rows (dot_rows_tcgen05.cuh) ------------------------------------------------------------------------
+struct RowsPlan {
+    int nq, parts, per_part, stages, bufs;
+    double us;       // what the launch is expected to take (fused form)
+};
+
+// Query tile, CTAs along K, ring sizes; false where the kernel has no form for the size. The costs are microseconds fitted
+// to layers of 1 .. 32 chunks on an idle GPU: a chunk of 16 rows to quantise 0.62, of 32 rows 1.2, the key stream alone 0.36,
+// and for every part behind the first the hand-over and the folding of its chunks.
+bool plan_rows(int64_t Q, int64_t R, int64_t chunks, bool fused, RowsPlan* out) {
+    const int sms = sm_count();
+    RowsPlan best = {};
+    best.us = 1e30;
+    for (int nq = 16; nq <= 32; nq *= 2) {
+        if (!fused && (nq < Q || (nq == 32 && Q <= 16))) continue;
+        const int64_t tiles = ((R + 127) / 128) * ((Q + nq - 1) / nq);
+        for (int s = 1; s <= 8; s *= 2) {
+            const int64_t per = (chunks + s - 1) / s, parts = (chunks + per - 1) / per;
+            // a split runs in one wave and keeps all of its accumulators; so does the fused form, whose tiles quantise alone
+            if ((s > 1 || fused) && tiles * parts > sms) break;
+            if (s > 1 && (parts == 1 || per > rows::kMaxBufs || per * nq > rows::kTmemCols)) continue;
+            const double rows_of_tile = static_cast<double>(std::min<int64_t>(Q, nq));
+            RowsPlan p = {};
+            if (!fused) p.us = 0.36 * per + (parts - 1) * (0.7 + 0.12 * per);
+            else if (nq == 16) p.us = 3.0 + (0.33 + 0.018 * rows_of_tile) * per + (parts - 1) * (0.6 + 0.15 * per);
+            else p.us = 3.9 + 1.2 * per + (parts - 1) * (0.8 + 0.25 * per);
+            if (p.us >= best.us) continue;
+            p.nq = nq;
+            p.parts = static_cast<int>(parts);
+            p.per_part = static_cast<int>(per);
+            const int64_t left = rows::kSmemBytes - rows::kFixedBytes - (parts > 1 ? rows::kEpiWarps * nq * 128 : 0) - per * nq * 4;
+            p.stages = static_cast<int>(std::min<int64_t>(std::min<int64_t>(rows::kMaxStages, per), left / (rows::kABytes + nq * 2 * BK)));
+            p.bufs = parts > 1 ? p.per_part : p.stages;
+            if (left > 0 && p.stages >= std::min<int64_t>(per, 2)) best = p;
+        }
+    }
+    *out = best;
+    return best.us < 1e30;
+}
+
+template <int NQ, typename OutT, typename XT>
+int launch_rows(const CUtensorMap& mk, const CUtensorMap& mq, const RowsPlan& plan, const rows::Args& a, cudaStream_t stream) {
+    static bool attr_set[64] = {false};
+    int dev = 0;
+    BSI_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64 || !attr_set[dev]) {
+        BSI_CUDA_TRY(cudaFuncSetAttribute(rows::dot_rows_kernel<NQ, OutT, XT>, cudaFuncAttributeMaxDynamicSharedMemorySize, rows::kSmemBytes));
+        if (dev >= 0 && dev < 64) attr_set[dev] = true;
+    }
+    constexpr bool kFuse = !std::is_same<XT, void>::value;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (pdl_enabled()) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (plan.parts > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = static_cast<unsigned>(plan.parts);
+        attr[n].val.clusterDim.y = 1;
+        attr[n++].val.clusterDim.z = 1;
+    }
+    cfg.gridDim = dim3(static_cast<unsigned>((a.R + 127) / 128 * plan.parts), static_cast<unsigned>((a.Q + NQ - 1) / NQ), 1);
+    cfg.blockDim = dim3((2 + rows::kEpiWarps + (kFuse ? rows::kQuantWarps : 0)) * 32, 1, 1);
+    cfg.dynamicSmemBytes = rows::kSmemBytes;
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    BSI_CUDA_TRY(cudaLaunchKernelEx(&cfg, rows::dot_rows_kernel<NQ, OutT, XT>, mk, mq, a));
+    return check_launch("dot_i8 rows launch");
+}
+
+// a8: the packed queries, null in the fused form (whose activations are in `a`).
+int run_rows(const RowsPlan& plan, rows::Args a, const int8_t* a8, int64_t lda, const int8_t* k8, int64_t ldk, int x_dtype, int y_dtype,
+             cudaStream_t stream) {
+    a.parts = plan.parts; a.per_part = plan.per_part; a.stages = plan.stages; a.bufs = plan.bufs;
+    CUtensorMap mk, mq = {};
+    if (int rc = make_map(&mk, k8, a.R, static_cast<int64_t>(a.chunks) * 256, ldk, 128)) return rc;
+    if (a8 != nullptr)
+        if (int rc = make_map(&mq, a8, a.Q, static_cast<int64_t>(a.chunks) * 256, lda, plan.nq)) return rc;
+#define BSI_ROWS(O_, X_) (plan.nq == 16 ? launch_rows<16, O_, X_>(mk, mq, plan, a, stream) : launch_rows<32, O_, X_>(mk, mq, plan, a, stream))
+    if (a8 == nullptr)
+        return x_dtype == BSI_DTYPE_F32 ? BSI_ROWS(float, float) : x_dtype == BSI_DTYPE_F16 ? BSI_ROWS(__half, __half) : BSI_ROWS(__nv_bfloat16, __nv_bfloat16);
+    return y_dtype == BSI_DTYPE_F32 ? BSI_ROWS(float, void) : y_dtype == BSI_DTYPE_F16 ? BSI_ROWS(__half, void) : BSI_ROWS(__nv_bfloat16, void);
+#undef BSI_ROWS
+}
+
 }  // namespace
+
+// Whether a dot of packed queries goes to the rows kernel. 17 to 32 rows, which fill an eighth of a paired tile: always (4096
+// x 16384 float16 layers of 32 rows 20.3 -> 17.5 us, 8192 x 2048 18.2 -> 15.1). Up to 16, where the key-streaming kernel is
+// the other choice: with key tiles for most of the SMs (4096 x 16384, 16 rows: 19.3 -> 16.0 us; 4096 x 11008, 8 rows: 13.5 ->
+// 11.6) and, beyond 8 rows, which that kernel's MMAs are too slow for, from 48 MB of keys on (16384 x 4096: 28.6 -> 24.1);
+// smaller sets it spreads better (8192 x 2048, 16 rows: 11.5 us against 12.5).
+bool rows_fits(int64_t Q, int64_t R, int64_t chunks) {
+    if (Q > 32 || R >= (1 << 24) || chunks >= (1 << 12)) return false;
+    RowsPlan plan;
+    return (Q > 16 || R >= 10240 || (Q > 8 && R * chunks * 256 >= (48 << 20))) && plan_rows(Q, R, chunks, false, &plan);
+}
+
+int dot_rows(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride, const int8_t* k8, int64_t ldk, const float* bw0,
+             const float* bias, int64_t Q, int64_t R, int64_t chunks, float scale_inv, void* out, int64_t ldo, int y_dtype,
+             const Finishing& fin, bool keys_complete, cudaStream_t stream) {
+    RowsPlan plan;
+    if (!plan_rows(Q, R, chunks, false, &plan)) return fail(BSI_ERR_UNSUPPORTED, "dot_i8: no rows form for these sizes");
+    rows::Args a = {};
+    a.qs = qs; a.qs_stride = qs_stride; a.bw0 = bw0; a.bias = bias; a.keys_complete = keys_complete ? 1 : 0;
+    a.Q = static_cast<int>(Q); a.R = static_cast<int>(R); a.chunks = static_cast<int>(chunks);
+    a.scale_inv = scale_inv; a.out = out; a.ldo = ldo; a.fin = fin;
+    return run_rows(plan, a, a8, lda, k8, ldk, 0, y_dtype, stream);
+}
 
 // Paired-CTA engine with the output type and the bias chosen at run time (y_dtype: BSI_DTYPE_*).
 int dot_i8_pair(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride, const int8_t* k8, int64_t ldk,
@@ -743,6 +857,51 @@ extern "C" int bsi_b200_device_status(int* status_out) {
     if (v == 0) v = pv;
     *status_out = v;
     return BSI_OK;
+}
+
+// Where the quantisation in every CTA costs less than a second launch, which the host needs until 12 us have gone by. Up to 16
+// rows the key-streaming kernel's own one-launch form comes first.
+extern "C" int bsi_b200_linear_rows_fits(int64_t Q, int64_t R, int64_t D) {
+    using namespace bsi;
+    const int64_t chunks = (D + 255) / 256;
+    if (Q < 1 || R < 1 || D < 1 || Q > (1 << 16) || R >= (1 << 24) || chunks >= (1 << 12)) return 0;
+    if (Q <= 16 && bsi_b200_linear_decode_fits(Q, R, D)) return 0;
+    RowsPlan plan;
+    return plan_rows(Q, R, chunks, true, &plan) && plan.us <= 10.5 ? 1 : 0;
+}
+
+extern "C" int bsi_b200_linear_rows(const void* x, int x_dtype, int64_t ldx, int64_t D, int decimal_places, int bits, const int8_t* k8,
+                                    int64_t ldk, const float* bw0, const float* bias, int64_t Q, int64_t R, float scale_inv, void* y,
+                                    int64_t ldy, int activation, int64_t scaled_cols, float factor, int engine, bsi_stream_t stream) {
+    using namespace bsi;
+    if ((engine & ~BSI_KEYS_COMPLETE) != BSI_ENGINE_AUTO) return fail(BSI_ERR_INVALID, "linear_rows: engine must be AUTO");
+    if (Q < 0 || R < 0 || D <= 0 || ldx < D) return fail(BSI_ERR_INVALID, "linear_rows: bad sizes");
+    if (Q == 0 || R == 0) return BSI_OK;
+    if (x == nullptr || k8 == nullptr || bw0 == nullptr || y == nullptr) return fail(BSI_ERR_INVALID, "linear_rows: null pointer");
+    const int64_t chunks = (D + 255) / 256;
+    if (ldk < chunks * 256 || (ldk & 15) || (reinterpret_cast<uintptr_t>(k8) & 15))
+        return fail(BSI_ERR_INVALID, "linear_rows: k8 needs 16-byte aligned rows of at least 256*chunks bytes");
+    if (ldy < R) return fail(BSI_ERR_INVALID, "linear_rows: ldy < R");
+    if (bits < 2 || bits > 8) return fail(BSI_ERR_UNSUPPORTED, "linear_rows: bits must be in [2, 8]");
+    if (decimal_places < 0 || decimal_places > 8) return fail(BSI_ERR_UNSUPPORTED, "linear_rows: decimal_places must be in [0, 8]");
+    if (activation != BSI_ACT_NONE && activation != BSI_ACT_RELU) return fail(BSI_ERR_INVALID, "linear_rows: unknown activation");
+    if (scaled_cols < 0 || scaled_cols > R) return fail(BSI_ERR_INVALID, "linear_rows: bad scaled_cols");
+    if (x_dtype != BSI_DTYPE_F32 && x_dtype != BSI_DTYPE_F16 && x_dtype != BSI_DTYPE_BF16)
+        return fail(BSI_ERR_INVALID, "linear_rows: unknown x_dtype");
+    RowsPlan plan;
+    if (!bsi_b200_linear_rows_fits(Q, R, D) || !plan_rows(Q, R, chunks, true, &plan))
+        return fail(BSI_ERR_UNSUPPORTED, "linear_rows: not a size for this form");
+    if (int rc = require_sm100()) return rc;
+    rows::Args a = {};
+    a.x = x; a.ldx = ldx; a.D = D; a.bits = bits; a.bw0 = bw0; a.bias = bias;
+    a.keys_complete = (engine & BSI_KEYS_COMPLETE) != 0 ? 1 : 0;
+    a.Q = static_cast<int>(Q); a.R = static_cast<int>(R); a.chunks = static_cast<int>(chunks);
+    a.scale_inv = scale_inv; a.out = y; a.ldo = ldy;
+    a.fin = Finishing{activation == BSI_ACT_RELU ? 1 : 0, static_cast<int>(scaled_cols), factor};
+    a.dec_mult = 1;
+    for (int i = 0; i < decimal_places; ++i) a.dec_mult *= 10u;
+    a.dec_scale = static_cast<double>(a.dec_mult);
+    return run_rows(plan, a, nullptr, 0, k8, ldk, x_dtype, x_dtype, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int bsi_b200_debug_last_tiles(int* width_out, int* parts_out) {

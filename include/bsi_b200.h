@@ -278,6 +278,14 @@ int bsi_b200_linear_decode_engine(const void* x, int x_dtype, int64_t ldx, int64
                                   float scale_inv, void* y, int64_t ldy, int activation, int64_t scaled_cols, float factor,
                                   int engine, bsi_stream_t stream);
 
+/* The same one launch for layers of more rows, on the tensor cores: 128 key rows per CTA, tiles of up to 128 activations
+ * quantised by the CTAs that need them. For sizes bsi_b200_linear_rows_fits accepts (host function, 1 or 0). */
+int bsi_b200_linear_rows_fits(int64_t Q, int64_t R, int64_t D);
+int bsi_b200_linear_rows(const void* x, int x_dtype, int64_t ldx, int64_t D, int decimal_places, int bits,
+                         const int8_t* k8, int64_t ldk, const float* bw0, const float* bias, int64_t Q, int64_t R,
+                         float scale_inv, void* y, int64_t ldy, int activation, int64_t scaled_cols, float factor,
+                         int engine, bsi_stream_t stream);
+
 /* Linear whose finished output is re-quantised for the next linear inside the epilogue, so that the
  * layer-type [Q, R] matrix is never written: y = activation(cast(out) + cast(bias)) in layer_dtype
  * (BSI_DTYPE_F16 / BF16) is what bsi_b200_linear_i8_act would store; here every 256-column chunk of y

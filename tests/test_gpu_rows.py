@@ -1,0 +1,70 @@
+"""The rows kernel (key rows on the tensor memory's lanes): one-launch layers of more than 16 rows and dots of few rows give
+the bits of the paired tensor-core tiles."""
+import pytest
+import torch
+
+import _capi_helpers as H
+import _inputs
+from bsipytorch_b200 import capi
+from oracle import oracle as o
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+# one row beyond a tile of 16, tiles of 32 rows (more than 148 of 16), 128 and 129 keys, one chunk, operand rings that turn
+# over (more than 6 chunks), two and four parts along K with a shorter last one, ragged depth, keys and rows
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("Q,R,D", [(17, 128, 256), (33, 129, 250), (512, 1100, 1000), (600, 500, 760), (77, 777, 1000), (20, 9000, 2000),
+                                   (16, 2300, 2304), (64, 700, 2800), (13, 3000, 3840), (40, 130, 4096)])
+def test_one_launch_layer_of_many_rows(dtype, Q, R, D, monkeypatch):
+    import bsipytorch_b200
+    ops = bsipytorch_b200.bsi_ops
+    assert capi.lib().bsi_b200_linear_rows_fits(Q, R, D) == 1
+    x, k = _inputs.fc1(Q=Q, R=R, D=D, seed=Q + R + D, dtype=torch.float32)
+    x[1] *= 3.0e3 if dtype == torch.float16 else 3.0e4        # sums beyond 2^24: the order of the chunks shows
+    x[2, D // 3] = float("inf")
+    x[2, 5] = float("nan")
+    x = x.to(dtype).to(DEV)
+    keys = ops.build_bsi_keys_cuda(k.to(DEV), 2)[0]
+    bias = torch.linspace(-1, 1, R, device=DEV)
+    wide = torch.zeros(Q, D + 3, dtype=dtype, device=DEV)
+    wide[:, :D] = x                                           # rows that are not 16-byte aligned
+    for b in (None, bias):
+        monkeypatch.setenv("BSI_B200_ENGINE", "tcgen05")
+        want = ops.bsi_layer_forward(x, keys, b, 2)
+        monkeypatch.delenv("BSI_B200_ENGINE")
+        capi.exact_int_tiles()
+        for _ in range(3):                                    # the later calls read keys ahead of the wait
+            assert torch.equal(ops.bsi_layer_forward(x, keys, b, 2), want)
+            torch.cuda.synchronize()
+        assert torch.equal(ops.bsi_layer_forward(wide[:, :D], keys, b, 2), want)
+        assert capi.exact_int_tiles() == 0                    # no paired tile ran
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = [ops.bsi_layer_forward(x, keys, bias, 2) for _ in range(3)]
+    graph.replay()
+    assert all(torch.equal(y, want) for y in captured)
+    assert capi.device_status() == 0
+
+
+# packed queries: both tile widths, a row that makes every bound fail, parts along K, one scale per row, no room for a split
+@pytest.mark.parametrize("chunk_mode", [True, False])
+@pytest.mark.parametrize("Q,R,D", [(17, 300, 512), (32, 129, 4096), (20, 2100, 8192), (24, 4111, 4352), (1, 10240, 768), (16, 10300, 4096),
+                                   (9, 12288, 4096), (32, 19000, 2560)])
+def test_packed_dot_of_few_rows(Q, R, D, chunk_mode):
+    q, k = _inputs.fc1(Q=Q, R=R, D=D, seed=Q + R + D, dtype=torch.float32)
+    if Q > 1:
+        q[1] *= 3.0e4
+    qa = H.quantize_pack(q.to(DEV), 2, 7, chunk_mode)
+    kb = H.quantize_pack(k.to(DEV), 2, 6, False)
+    got = H.dot_i8(qa["q8"], qa["scales"], kb["q8"], kb["scales"], o.scale_inv(2))
+    want = H.dot_i8(qa["q8"], qa["scales"], kb["q8"], kb["scales"], o.scale_inv(2), 3064)
+    assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+    assert capi.device_status() == 0
+
+
+# where a CTA's share of the quantisation outweighs a second launch, and where the key-streaming kernel has its own form
+def test_one_launch_rule():
+    fits = capi.lib().bsi_b200_linear_rows_fits
+    assert [fits(64, 4096, 4096), fits(64, 2048, 2048), fits(512, 4096, 4096), fits(16, 256, 256), fits(17, 256, 256)] == [0, 1, 0, 0, 1]
