@@ -873,6 +873,7 @@ struct LinearTo {
     at::Tensor y;
     double factor = 1.0;      // of the first `scaled_cols` finished columns (0: of all); 1: none
     int64_t scaled_cols = 0;
+    at::Tensor add;           // [Q, R] of x's type, contiguous: added to the finished output (a residual sum)
 };
 void linear_forward(const Env& env, const at::Tensor& x2d, int decimalPlaces, bool relu, LinearTo* to, int n) {
     TORCH_CHECK(x2d.dim() == 2 && x2d.is_cuda(), "x must be a 2D CUDA tensor");
@@ -916,7 +917,15 @@ void linear_forward(const Env& env, const at::Tensor& x2d, int decimalPlaces, bo
         const int64_t cols = to[i].scaled_cols > 0 ? to[i].scaled_cols : R;
         const int64_t scaled = to[i].factor != 1.0 && cols % 8 == 0 && fused && D > 0 ? cols : 0;
         const float factor = static_cast<float>(to[i].factor);
-        auto rest = [&] { if (to[i].factor != 1.0 && scaled == 0) y.narrow(1, 0, cols).mul_(to[i].factor); };
+        // so does a sum, behind the factor
+        const bool factor_in = to[i].factor == 1.0 || scaled != 0;
+        const bool add_in = factor_in && fused && D > 0 && to[i].add.defined() && to[i].add.scalar_type() == yt && to[i].add.is_contiguous() &&
+                            to[i].add.numel() == Q * R && to[i].add.device() == x2d.device();
+        const void* add = add_in ? to[i].add.data_ptr() : nullptr;
+        auto rest = [&] {
+            if (!factor_in) y.narrow(1, 0, cols).mul_(to[i].factor);
+            if (to[i].add.defined() && !add_in) y.add_(to[i].add);
+        };
         y = at::detail::empty_cuda({Q, R}, yt, x2d.device(), c10::nullopt);
         const float* bptr = nullptr;
         at::Tensor b32;
@@ -944,17 +953,17 @@ void linear_forward(const Env& env, const at::Tensor& x2d, int decimalPlaces, bo
             (Q > 16 || c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None)) {
             check_status(bsi_b200_linear_rows(x.data_ptr(), code, ldx, D, decimalPlaces, bits, keys.b.q8.data_ptr<int8_t>(),
                                               keys.b.q8.size(1), keys.b.scales.data_ptr<float>(), bptr, Q, R, scale_inv,
-                                              y.data_ptr(), R, act, scaled, factor, keys.complete(), current_stream()),
+                                              y.data_ptr(), R, act, scaled, factor, add, R, keys.complete(), current_stream()),
                          "bsi_b200_linear_rows");
             g_last_quantize_ns = g_last_pack_ns = g_last_total_ns = 0;
             rest();
             continue;
         }
         if (one_launch && bsi_b200_linear_decode_fits(Q, R, D)) {
-            check_status(bsi_b200_linear_decode_engine(x.data_ptr(), code, ldx, D, decimalPlaces, bits, keys.b.q8.data_ptr<int8_t>(),
-                                                       keys.b.q8.size(1), keys.b.scales.data_ptr<float>(), bptr, Q, R, scale_inv,
-                                                       y.data_ptr(), R, act, scaled, factor, keys.complete(), current_stream()),
-                         "bsi_b200_linear_decode_engine");
+            check_status(bsi_b200_linear_decode_add(x.data_ptr(), code, ldx, D, decimalPlaces, bits, keys.b.q8.data_ptr<int8_t>(),
+                                                    keys.b.q8.size(1), keys.b.scales.data_ptr<float>(), bptr, Q, R, scale_inv,
+                                                    y.data_ptr(), R, act, scaled, factor, add, R, keys.complete(), current_stream()),
+                         "bsi_b200_linear_decode_add");
             g_last_quantize_ns = g_last_pack_ns = g_last_total_ns = 0;      // no pack of its own to report
             rest();
             continue;
@@ -988,18 +997,18 @@ void linear_forward(const Env& env, const at::Tensor& x2d, int decimalPlaces, bo
         bsi_dot_bounds bounds = dot_bounds(keys, bits, nullptr);
         bounds.query_sq = sq;
         bounds.query_sq_stride = chunks;
-        check_status(bsi_b200_linear_i8_engine(q8, chunks * 256, scales, chunk ? chunks : 0, keys.b.q8.data_ptr<int8_t>(),
-                                               keys.b.q8.size(1), keys.b.scales.data_ptr<float>(), bptr, Q, R, chunks, scale_inv,
-                                               y.data_ptr(), R, code, act, scaled, factor, &bounds,
-                                               engine | (Q <= kFewRows ? keys.complete() : 0), current_stream()),
-                     "bsi_b200_linear_i8_engine");
+        check_status(bsi_b200_linear_i8_add(q8, chunks * 256, scales, chunk ? chunks : 0, keys.b.q8.data_ptr<int8_t>(),
+                                            keys.b.q8.size(1), keys.b.scales.data_ptr<float>(), bptr, Q, R, chunks, scale_inv,
+                                            y.data_ptr(), R, code, act, scaled, factor, add, R, &bounds,
+                                            engine | (Q <= kFewRows ? keys.complete() : 0), current_stream()),
+                     "bsi_b200_linear_i8_add");
         rest();
     }
 }
 
 at::Tensor linear_forward(const Env& env, const at::Tensor& x2d, const PrebuiltBSIKeysCUDA& keys,
-                          const c10::optional<torch::Tensor>& bias, int decimalPlaces, bool relu = false) {
-    LinearTo to{&keys, &bias, at::Tensor(), 1.0};
+                          const c10::optional<torch::Tensor>& bias, int decimalPlaces, bool relu = false, const at::Tensor& add = at::Tensor()) {
+    LinearTo to{&keys, &bias, at::Tensor(), 1.0, 0, add};
     linear_forward(env, x2d, decimalPlaces, relu, &to, 1);
     return to.y;
 }
@@ -1165,11 +1174,10 @@ py::object opt_layer_forward(const torch::Tensor& x, const py::tuple& norms, con
     }
     // query scaled in the model's type, attention with unit scaling: the order HuggingFace's OPT uses
     const at::Tensor a = at::scaled_dot_product_attention(split(q), split(k), split(v), {}, 0.0, true, 1.0);
-    const at::Tensor o = linear_forward(env, flat(a.transpose(1, 2).reshape({B, T, H})), *keys[3], bias[3], dp[3]);
-    // residual sums into the linears' own outputs: the same sums, without an allocation
-    const at::Tensor mid = o.view({B, T, H}).add_(x);
+    // residual sums in the linears' epilogues: the same sums, two launches of a layer's thirteen fewer
+    const at::Tensor mid = linear_forward(env, flat(a.transpose(1, 2).reshape({B, T, H})), *keys[3], bias[3], dp[3], false, flat(x));
     const at::Tensor f = linear_forward(env, flat(norm(mid, 3)), *keys[4], bias[4], dp[4], /*relu=*/true);
-    return py::cast(linear_forward(env, f, *keys[5], bias[5], dp[5]).view({B, T, H}).add_(mid));
+    return py::cast(linear_forward(env, f, *keys[5], bias[5], dp[5], false, mid).view({B, T, H}));
 }
 
 // Quantise + pack activations (query side: chunk scales) into tensors the caller owns: q8 [rows, >= d]

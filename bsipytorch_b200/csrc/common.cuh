@@ -61,11 +61,14 @@ struct RequantDst {
     float* scales[BSI_B200_MAX_PEERS];   // already offset to this linear's first output chunk
 };
 
-// What happens to a finished output value: ReLU, and a factor for the first scaled_cols columns (a multiple of 8).
+// What happens to a finished output value: ReLU, a factor for the first scaled_cols columns (a multiple of 8), and the
+// addition of a matrix of the output's type and shape, rounded once more (a residual sum; null: none).
 struct Finishing {
     int relu;
     int scaled_cols;
     float factor;
+    const void* add;
+    int64_t ld_add;
 };
 
 // Bounds registered for a key image (bsi_b200_register_key_bounds): with them a dot can tell, per tile, that every

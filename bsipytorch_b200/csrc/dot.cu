@@ -198,7 +198,15 @@ extern "C" int bsi_b200_linear_i8_engine(const int8_t* a8, int64_t lda, const fl
                                          const int8_t* k8, int64_t ldk, const float* bw0, const float* bias,
                                          int64_t Q, int64_t R, int64_t chunks, float scale_inv, void* y, int64_t ldy,
                                          int y_dtype, int activation, int64_t scaled_cols, float factor,
-                                         const bsi_dot_bounds* bounds, int engine, bsi_stream_t stream_) {
+                                         const bsi_dot_bounds* bounds, int engine, bsi_stream_t stream) {
+    return bsi_b200_linear_i8_add(a8, lda, qs, qs_stride, k8, ldk, bw0, bias, Q, R, chunks, scale_inv, y, ldy, y_dtype, activation,
+                                  scaled_cols, factor, nullptr, 0, bounds, engine, stream);
+}
+
+extern "C" int bsi_b200_linear_i8_add(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride, const int8_t* k8, int64_t ldk,
+                                      const float* bw0, const float* bias, int64_t Q, int64_t R, int64_t chunks, float scale_inv,
+                                      void* y, int64_t ldy, int y_dtype, int activation, int64_t scaled_cols, float factor,
+                                      const void* add, int64_t ld_add, const bsi_dot_bounds* bounds, int engine, bsi_stream_t stream_) {
     using namespace bsi;
     if (Q < 0 || R < 0 || chunks < 0) return fail(BSI_ERR_INVALID, "linear_i8: negative size");
     if (Q == 0 || R == 0) return BSI_OK;
@@ -221,7 +229,8 @@ extern "C" int bsi_b200_linear_i8_engine(const int8_t* a8, int64_t lda, const fl
     if (int rc = require_sm100()) return rc;
     if (scaled_cols < 0 || scaled_cols > R || (scaled_cols & 7) != 0)
         return fail(BSI_ERR_INVALID, "linear_i8: scaled_cols must be a multiple of 8 in [0, R]");
-    const Finishing fin{activation == BSI_ACT_RELU ? 1 : 0, static_cast<int>(scaled_cols), factor};
+    if (add != nullptr && ld_add < R) return fail(BSI_ERR_INVALID, "linear_i8: ld_add < R");
+    const Finishing fin{activation == BSI_ACT_RELU ? 1 : 0, static_cast<int>(scaled_cols), factor, add, ld_add};
     if (engine == BSI_ENGINE_AUTO && rows_fits(Q, R, chunks))
         return dot_rows(a8, lda, qs, qs_stride, k8, ldk, bw0, bias, Q, R, chunks, scale_inv, y, ldy, y_dtype, fin, keys_complete,
                         static_cast<cudaStream_t>(stream_));
@@ -270,7 +279,7 @@ extern "C" int bsi_b200_linear_i8_scatter(const int8_t* a8, int64_t lda, const f
     }
     if (int rc = require_sm100()) return rc;
     return dot_i8_pair(a8, lda, qs, qs_stride, k8, ldk, bw0, bias, Q, R, chunks, scale_inv, nullptr, ldy, y_dtype,
-                       nullptr, 0, Finishing{activation == BSI_ACT_RELU ? 1 : 0, 0, 1.0f}, &sc, nullptr, resolve_bounds(nullptr, a8, k8, R), static_cast<cudaStream_t>(stream_));
+                       nullptr, 0, Finishing{activation == BSI_ACT_RELU ? 1 : 0, 0, 1.0f, nullptr, 0}, &sc, nullptr, resolve_bounds(nullptr, a8, k8, R), static_cast<cudaStream_t>(stream_));
 }
 
 extern "C" int bsi_b200_linear_i8_requant(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride,
@@ -314,7 +323,7 @@ extern "C" int bsi_b200_linear_i8_requant(const int8_t* a8, int64_t lda, const f
     }
     if (int rc = require_sm100()) return rc;
     return dot_i8_pair(a8, lda, qs, qs_stride, k8, ldk, bw0, bias, Q, R, chunks, scale_inv, q8_dst[0], R, layer_dtype,
-                       nullptr, 0, Finishing{activation == BSI_ACT_RELU ? 1 : 0, 0, 1.0f}, nullptr, &rq, resolve_bounds(nullptr, a8, k8, R), static_cast<cudaStream_t>(stream_));
+                       nullptr, 0, Finishing{activation == BSI_ACT_RELU ? 1 : 0, 0, 1.0f, nullptr, 0}, nullptr, &rq, resolve_bounds(nullptr, a8, k8, R), static_cast<cudaStream_t>(stream_));
 }
 
 extern "C" int bsi_b200_linear_i8(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride,

@@ -240,9 +240,11 @@ __global__ void __launch_bounds__(kThreads, 1) dot_decode_kernel(const DecodeArg
                 const int row = (group * p.rt + tile_i) * 16 + key;
                 const bool last = s + 1 == p.slabs;
                 float w = 0.0f, bv = 0.0f;
+                OutT av = static_cast<OutT>(0.0f);
                 if (last && row < p.R) {
                     w = behind_wait(p.bw0)[row];
                     if (p.bias != nullptr) bv = behind_wait(p.bias)[row];
+                    if (p.fin.add != nullptr) av = behind_wait(static_cast<const OutT*>(p.fin.add))[q * p.fin.ld_add + row];
                 }
                 float* keep = accs + (static_cast<int64_t>(it) * p.rt * p.Q + rq) * 16 + key;
                 float acc = s > 0 ? *keep : 0.0f;
@@ -252,10 +254,11 @@ __global__ void __launch_bounds__(kThreads, 1) dot_decode_kernel(const DecodeArg
                 for (int c = 0; c < len; ++c)
                     acc = __fmaf_rn(static_cast<float>(src[c * (NT * 8 * kPitch)]), sc[c], acc);
                 if (!last) *keep = acc;
-                else if (row < p.R)
-                    static_cast<OutT*>(p.out)[q * p.ldo + row] =
-                        scaled_if<OutT>(relu_if<OutT>(finish<OutT>((acc * w) * p.scale_inv, bv, p.bias != nullptr), p.fin.relu != 0),
-                                        row < p.fin.scaled_cols, p.fin.factor);
+                else if (row < p.R) {
+                    const OutT y = scaled_if<OutT>(relu_if<OutT>(finish<OutT>((acc * w) * p.scale_inv, bv, p.bias != nullptr), p.fin.relu != 0),
+                                                   row < p.fin.scaled_cols, p.fin.factor);
+                    static_cast<OutT*>(p.out)[q * p.ldo + row] = p.fin.add != nullptr ? plus<OutT>(y, av) : y;
+                }
             }
         }
     }
@@ -352,7 +355,15 @@ extern "C" int bsi_b200_linear_decode(const void* x, int x_dtype, int64_t ldx, i
 extern "C" int bsi_b200_linear_decode_engine(const void* x, int x_dtype, int64_t ldx, int64_t D, int decimal_places, int bits,
                                              const int8_t* k8, int64_t ldk, const float* bw0, const float* bias, int64_t Q,
                                              int64_t R, float scale_inv, void* y, int64_t ldy, int activation,
-                                             int64_t scaled_cols, float factor, int engine, bsi_stream_t stream_) {
+                                             int64_t scaled_cols, float factor, int engine, bsi_stream_t stream) {
+    return bsi_b200_linear_decode_add(x, x_dtype, ldx, D, decimal_places, bits, k8, ldk, bw0, bias, Q, R, scale_inv, y, ldy,
+                                      activation, scaled_cols, factor, nullptr, 0, engine, stream);
+}
+
+extern "C" int bsi_b200_linear_decode_add(const void* x, int x_dtype, int64_t ldx, int64_t D, int decimal_places, int bits,
+                                          const int8_t* k8, int64_t ldk, const float* bw0, const float* bias, int64_t Q, int64_t R,
+                                          float scale_inv, void* y, int64_t ldy, int activation, int64_t scaled_cols, float factor,
+                                          const void* add, int64_t ld_add, int engine, bsi_stream_t stream_) {
     using namespace bsi;
     if ((engine & ~BSI_KEYS_COMPLETE) != BSI_ENGINE_AUTO) return fail(BSI_ERR_INVALID, "linear_decode: engine must be AUTO");
     if (Q < 0 || R < 0 || D <= 0 || ldx < D) return fail(BSI_ERR_INVALID, "linear_decode: bad sizes");
@@ -368,6 +379,7 @@ extern "C" int bsi_b200_linear_decode_engine(const void* x, int x_dtype, int64_t
     if (scaled_cols < 0 || scaled_cols > R) return fail(BSI_ERR_INVALID, "linear_decode: bad scaled_cols");
     if (x_dtype != BSI_DTYPE_F32 && x_dtype != BSI_DTYPE_F16 && x_dtype != BSI_DTYPE_BF16)
         return fail(BSI_ERR_INVALID, "linear_decode: unknown x_dtype");
+    if (add != nullptr && ld_add < R) return fail(BSI_ERR_INVALID, "linear_decode: ld_add < R");
     if (!bsi_b200_linear_decode_fits(Q, R, D)) return fail(BSI_ERR_UNSUPPORTED, "linear_decode: too many query chunks for this form");
     if (int rc = require_sm100()) return rc;
     DecodeArgs a = {};
@@ -375,7 +387,7 @@ extern "C" int bsi_b200_linear_decode_engine(const void* x, int x_dtype, int64_t
     a.x = x; a.ldx = ldx; a.D = D; a.bits = bits; a.k8 = k8; a.ldk = ldk; a.bw0 = bw0; a.bias = bias;
     a.Q = static_cast<int>(Q); a.R = static_cast<int>(R); a.chunks = static_cast<int>(chunks);
     a.scale_inv = scale_inv; a.out = y; a.ldo = ldy;
-    a.fin = Finishing{activation == BSI_ACT_RELU ? 1 : 0, static_cast<int>(scaled_cols), factor};
+    a.fin = Finishing{activation == BSI_ACT_RELU ? 1 : 0, static_cast<int>(scaled_cols), factor, add, ld_add};
     a.dec_mult = 1;
     for (int i = 0; i < decimal_places; ++i) a.dec_mult *= 10u;
     a.dec_scale = static_cast<double>(a.dec_mult);

@@ -318,15 +318,27 @@ dot_rows_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
         } else if (ok && row < p.R) {
             OutT* o = static_cast<OutT*>(p.out) + static_cast<int64_t>(q0) * p.ldo + row;
             const bool relu = p.fin.relu != 0, scaled = row < p.fin.scaled_cols;
+            const OutT* a = p.fin.add == nullptr ? nullptr : behind_wait(static_cast<const OutT*>(p.fin.add)) + q0 * p.fin.ld_add + row;
+            OutT add[4], add_next[4];      // of the four queries at hand and of the next four
+            auto fetch_add = [&](int j, OutT (&to)[4]) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (a != nullptr && j + e < nq) to[e] = a[(j + e) * p.fin.ld_add];
+            };
+            fetch_add(0, add);
 #pragma unroll 1
             for (int j = 0; j < nq; j += 4) {
+                fetch_add(j + 4, add_next);
                 const float4 v = *reinterpret_cast<const float4*>(mine + j * 128);
-                const float a[4] = {v.x, v.y, v.z, v.w};
+                const float sum[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    if (j + e < nq)
-                        *o = scaled_if<OutT>(relu_if<OutT>(finish<OutT>((a[e] * w) * p.scale_inv, bv, has_bias), relu), scaled, p.fin.factor);
+                    if (j + e < nq) {
+                        const OutT y = scaled_if<OutT>(relu_if<OutT>(finish<OutT>((sum[e] * w) * p.scale_inv, bv, has_bias), relu), scaled, p.fin.factor);
+                        *o = a != nullptr ? plus<OutT>(y, add[e]) : y;
+                    }
                     o += p.ldo;
+                    add[e] = add_next[e];
                 }
             }
         }

@@ -467,7 +467,7 @@ int launch_tile(const CUtensorMap& ma, const CUtensorMap& mb, const float* qs, i
     return check_launch("dot_i8 tcgen05 launch");
 }
 
-template <int BN, bool DBG, typename OutT, bool REQ = false, int SPLIT = 1>
+template <int BN, bool DBG, typename OutT, bool REQ = false, int SPLIT = 1, bool ADD = false>
 int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo, const CUtensorMap& mt, int vector_store,
                 const float* qs, int64_t qs_stride, const float* bw0, const float* bias, int Q, int R, int chunks,
                 float scale_inv, void* out, int64_t ldo, int32_t* dbg, const ScatterDst& scatter,
@@ -497,10 +497,10 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap&
     int resident = 0;
     if (dev >= 0 && dev < 64) resident = max_clusters[dev];
     if (resident == 0) {
-        BSI_CUDA_TRY(cudaFuncSetAttribute(pair::dot_i8_tcgen05_pair_kernel<BN, DBG, OutT, REQ, SPLIT>,
+        BSI_CUDA_TRY(cudaFuncSetAttribute(pair::dot_i8_tcgen05_pair_kernel<BN, DBG, OutT, REQ, SPLIT, ADD>,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
         cfg.gridDim = dim3(2 * SPLIT * (sm_count() / (2 * SPLIT)), 1, 1);
-        BSI_CUDA_TRY(cudaOccupancyMaxActiveClusters(&resident, pair::dot_i8_tcgen05_pair_kernel<BN, DBG, OutT, REQ, SPLIT>, &cfg));
+        BSI_CUDA_TRY(cudaOccupancyMaxActiveClusters(&resident, pair::dot_i8_tcgen05_pair_kernel<BN, DBG, OutT, REQ, SPLIT, ADD>, &cfg));
         if (resident <= 0) return fail(BSI_ERR_CUDA, "dot_i8: no cluster of 2 CTAs fits on this device");
         if (dev >= 0 && dev < 64) max_clusters[dev] = resident;
     }
@@ -510,7 +510,7 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap&
     }
     const int clusters = SPLIT > 1 || tiles_total < resident ? tiles_total : resident;
     cfg.gridDim = dim3(2 * SPLIT * clusters, 1, 1);
-    BSI_CUDA_TRY(cudaLaunchKernelEx(&cfg, pair::dot_i8_tcgen05_pair_kernel<BN, DBG, OutT, REQ, SPLIT>, ma, mb, mo, mt, vector_store, qs,
+    BSI_CUDA_TRY(cudaLaunchKernelEx(&cfg, pair::dot_i8_tcgen05_pair_kernel<BN, DBG, OutT, REQ, SPLIT, ADD>, ma, mb, mo, mt, vector_store, qs,
                                     qs_stride, bw0, bias, Q, R, chunks, tiles_m, tiles_total, scale_inv, out, ldo, dbg, scatter, requant,
                                     fin, k_abs_sum, q_abs_max, q_sq, q_sq_stride));
     return check_launch("dot_i8 tcgen05 pair launch");
@@ -722,7 +722,7 @@ int dot_i8_pair(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_strid
     }
     if (Q > 0x7fffff00ll || R > 0x7fffff00ll || chunks > 0x400000)
         return fail(BSI_ERR_UNSUPPORTED, "dot_i8: Q, R or chunks too large");
-    const bool any_width = y_dtype == BSI_DTYPE_F32;
+    const bool any_width = y_dtype == BSI_DTYPE_F32 && fin.add == nullptr;      // sums are built for the powers of two
     // bounds of the two images switch on the integer accumulation where it is provably exact
     const float* kabs = bounds.key_bounds;
     const float qabs = static_cast<float>(bounds.query_abs_max);
@@ -755,7 +755,8 @@ int dot_i8_pair(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_strid
     const int esz = y_dtype == BSI_DTYPE_F32 ? 4 : 2;
     const int per16 = 16 / esz;
     const int vector_store =
-        (((reinterpret_cast<uintptr_t>(out) & 15) == 0 && (ldo % per16) == 0 && (R % per16) == 0) ? 1 : 0) |
+        (((reinterpret_cast<uintptr_t>(out) & 15) == 0 && (ldo % per16) == 0 && (R % per16) == 0 &&
+          (fin.add == nullptr || ((reinterpret_cast<uintptr_t>(fin.add) & 15) == 0 && (fin.ld_add % per16) == 0))) ? 1 : 0) |
         (fin.relu ? 2 : 0);   // the kernel's store_flags
     // bulk stores into the one output matrix; several destinations (scatter) keep plain stores
     CUtensorMap mo = {}, mt = {};
@@ -767,8 +768,9 @@ int dot_i8_pair(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_strid
     }
     const int q = static_cast<int>(Q), r = static_cast<int>(R), c = static_cast<int>(chunks);
     if (parts > 1) {
-#define BSI_SPLIT_T(BN_, S_, T_)                                                                                            \
-    launch_pair<BN_, false, T_, false, S_>(ma, mb, mo, mt, store_flags, qs, qs_stride, bw0, bias, q, r, c, scale_inv, out, ldo, \
+#define BSI_SPLIT_T(BN_, S_, T_) (fin.add != nullptr ? BSI_SPLIT_A(BN_, S_, T_, true) : BSI_SPLIT_A(BN_, S_, T_, false))
+#define BSI_SPLIT_A(BN_, S_, T_, A_)                                                                                        \
+    launch_pair<BN_, false, T_, false, S_, A_>(ma, mb, mo, mt, store_flags, qs, qs_stride, bw0, bias, q, r, c, scale_inv, out, ldo, \
                                            nullptr, scatter, requant, fin, kabs, qabs, qsq, qsq_stride, stream)
 #define BSI_SPLIT(BN_, S_)                                                    \
     (y_dtype == BSI_DTYPE_F16    ? BSI_SPLIT_T(BN_, S_, __half)               \
@@ -778,12 +780,18 @@ int dot_i8_pair(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_strid
         return bn == 256 ? BSI_SPLIT(256, 4) : (bn == 128 ? BSI_SPLIT(128, 4) : BSI_SPLIT(64, 4));
 #undef BSI_SPLIT
 #undef BSI_SPLIT_T
+#undef BSI_SPLIT_A
     }
 #define BSI_PAIR_T(BN_, DBG_, T_)                                                                              \
     launch_pair<BN_, DBG_, T_>(ma, mb, mo, mt, store_flags, qs, qs_stride, bw0, bias, q, r, c, scale_inv, out, ldo,  \
                                dbg_iacc, scatter, requant, fin, kabs, qabs, qsq, qsq_stride, stream)
+#define BSI_PAIR_ADD(BN_, T_)                                                                                            \
+    launch_pair<BN_, false, T_, false, 1, true>(ma, mb, mo, mt, store_flags, qs, qs_stride, bw0, bias, q, r, c, scale_inv, out, \
+                                                ldo, dbg_iacc, scatter, requant, fin, kabs, qabs, qsq, qsq_stride, stream)
 #define BSI_PAIR(BN_)                                                                   \
-    (y_dtype == BSI_DTYPE_F16    ? BSI_PAIR_T(BN_, false, __half)                       \
+    (fin.add != nullptr ? (y_dtype == BSI_DTYPE_F16 ? BSI_PAIR_ADD(BN_, __half) : y_dtype == BSI_DTYPE_BF16 ? BSI_PAIR_ADD(BN_, __nv_bfloat16) \
+                                                                                               : BSI_PAIR_ADD(BN_, float)) \
+     : y_dtype == BSI_DTYPE_F16    ? BSI_PAIR_T(BN_, false, __half)                       \
      : y_dtype == BSI_DTYPE_BF16 ? BSI_PAIR_T(BN_, false, __nv_bfloat16)                \
      : dbg_iacc                  ? BSI_PAIR_T(BN_, true, float)                         \
                                  : BSI_PAIR_T(BN_, false, float))
@@ -807,6 +815,7 @@ int dot_i8_pair(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_strid
     }
 #undef BSI_PAIR_F32
 #undef BSI_PAIR
+#undef BSI_PAIR_ADD
 #undef BSI_PAIR_T
 }
 
@@ -872,7 +881,8 @@ extern "C" int bsi_b200_linear_rows_fits(int64_t Q, int64_t R, int64_t D) {
 
 extern "C" int bsi_b200_linear_rows(const void* x, int x_dtype, int64_t ldx, int64_t D, int decimal_places, int bits, const int8_t* k8,
                                     int64_t ldk, const float* bw0, const float* bias, int64_t Q, int64_t R, float scale_inv, void* y,
-                                    int64_t ldy, int activation, int64_t scaled_cols, float factor, int engine, bsi_stream_t stream) {
+                                    int64_t ldy, int activation, int64_t scaled_cols, float factor, const void* add, int64_t ld_add,
+                                    int engine, bsi_stream_t stream) {
     using namespace bsi;
     if ((engine & ~BSI_KEYS_COMPLETE) != BSI_ENGINE_AUTO) return fail(BSI_ERR_INVALID, "linear_rows: engine must be AUTO");
     if (Q < 0 || R < 0 || D <= 0 || ldx < D) return fail(BSI_ERR_INVALID, "linear_rows: bad sizes");
@@ -888,6 +898,7 @@ extern "C" int bsi_b200_linear_rows(const void* x, int x_dtype, int64_t ldx, int
     if (scaled_cols < 0 || scaled_cols > R) return fail(BSI_ERR_INVALID, "linear_rows: bad scaled_cols");
     if (x_dtype != BSI_DTYPE_F32 && x_dtype != BSI_DTYPE_F16 && x_dtype != BSI_DTYPE_BF16)
         return fail(BSI_ERR_INVALID, "linear_rows: unknown x_dtype");
+    if (add != nullptr && ld_add < R) return fail(BSI_ERR_INVALID, "linear_rows: ld_add < R");
     RowsPlan plan;
     if (!bsi_b200_linear_rows_fits(Q, R, D) || !plan_rows(Q, R, chunks, true, &plan))
         return fail(BSI_ERR_UNSUPPORTED, "linear_rows: not a size for this form");
@@ -897,7 +908,7 @@ extern "C" int bsi_b200_linear_rows(const void* x, int x_dtype, int64_t ldx, int
     a.keys_complete = (engine & BSI_KEYS_COMPLETE) != 0 ? 1 : 0;
     a.Q = static_cast<int>(Q); a.R = static_cast<int>(R); a.chunks = static_cast<int>(chunks);
     a.scale_inv = scale_inv; a.out = y; a.ldo = ldy;
-    a.fin = Finishing{activation == BSI_ACT_RELU ? 1 : 0, static_cast<int>(scaled_cols), factor};
+    a.fin = Finishing{activation == BSI_ACT_RELU ? 1 : 0, static_cast<int>(scaled_cols), factor, add, ld_add};
     a.dec_mult = 1;
     for (int i = 0; i < decimal_places; ++i) a.dec_mult *= 10u;
     a.dec_scale = static_cast<double>(a.dec_mult);

@@ -262,6 +262,23 @@ template <typename OutT>
 __device__ __forceinline__ uint4 times(uint4 o, float factor, OutT t) {
     return make_uint4(times2(o.x, factor, t), times2(o.y, factor, t), times2(o.z, factor, t), times2(o.w, factor, t));
 }
+// 16 bytes of finished values plus those of another matrix. A 16-bit add rounds like the float32 add narrowed (see finish2).
+__device__ __forceinline__ uint4 plus16(uint4 a, uint4 b, float) {
+    return make_uint4(__float_as_uint(__uint_as_float(a.x) + __uint_as_float(b.x)), __float_as_uint(__uint_as_float(a.y) + __uint_as_float(b.y)),
+                      __float_as_uint(__uint_as_float(a.z) + __uint_as_float(b.z)), __float_as_uint(__uint_as_float(a.w) + __uint_as_float(b.w)));
+}
+__device__ __forceinline__ uint32_t plus2(uint32_t a, uint32_t b, __half) {
+    const __half2 y = __hadd2(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b));
+    return *reinterpret_cast<const uint32_t*>(&y);
+}
+__device__ __forceinline__ uint32_t plus2(uint32_t a, uint32_t b, __nv_bfloat16) {
+    const __nv_bfloat162 y = __hadd2(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
+    return *reinterpret_cast<const uint32_t*>(&y);
+}
+template <typename OutT>
+__device__ __forceinline__ uint4 plus16(uint4 a, uint4 b, OutT t) {
+    return make_uint4(plus2(a.x, b.x, t), plus2(a.y, b.y, t), plus2(a.z, b.z, t), plus2(a.w, b.w, t));
+}
 __device__ __forceinline__ float cast_bias(float b, float) { return b; }
 __device__ __forceinline__ __half cast_bias(float b, __half) { return __float2half_rn(b); }
 __device__ __forceinline__ __nv_bfloat16 cast_bias(float b, __nv_bfloat16) { return __float2bfloat16_rn(b); }
@@ -362,7 +379,9 @@ __host__ __device__ constexpr int kBlocks() {
 // back in the next tile's main loop while they drain; written with ordinary stores, the output took half of a tile's
 // time at 16 chunks. A warp has one block of its own; places != nullptr (a CTA's last tile, when nothing reads the operand
 // ring any more) gives every block its own place.
-template <typename OutT, int kCols>
+// ADD: a matrix is added to the finished values. An instantiation of its own: skipped by a branch, its few instructions still
+// cost a 512 x 8192 x 2048 dot 0.5 us, since what runs once per tile waits for its instructions to be fetched.
+template <typename OutT, int kCols, bool ADD>
 __device__ __forceinline__ void store_columns(const float (&acc)[kCols], uint8_t* places, uint8_t* own, const float* colw, const OutT* colb,
                                               const CUtensorMap& map_o, const CUtensorMap& map_t, OutT* __restrict__ outp, int64_t ldo,
                                               int row_shift, int row_base, int Q, int col, int R, float scale_inv, bool has_bias, bool relu,
@@ -401,6 +420,23 @@ __device__ __forceinline__ void store_columns(const float (&acc)[kCols], uint8_t
                     if (col + cg + ch * kPerChunk >= fin.scaled_cols) break;
                     uint4* o = reinterpret_cast<uint4*>(dst + ((whole ? (ch ^ (lane & 7)) : (ch ^ ((lane >> 1) & 3))) << 4));
                     *o = times(*o, fin.factor, OutT());
+                }
+            }
+            if (ADD && row_base + lane < Q) {      // likewise, a few loads at a time: the sums need the registers
+                constexpr int kBatch = kCols <= 64 ? 4 : 2;
+                const OutT* a = behind_wait(static_cast<const OutT*>(fin.add)) + static_cast<int64_t>(row_base + lane) * fin.ld_add + col + cg;
+#pragma unroll 1
+                for (int c0 = 0; c0 < nch && cg + c0 * kPerChunk < kCols; c0 += kBatch) {
+                    uint4 add[kBatch];
+#pragma unroll
+                    for (int e = 0; e < kBatch; ++e)
+                        if (col + cg + (c0 + e) * kPerChunk < R) add[e] = *reinterpret_cast<const uint4*>(a + (c0 + e) * kPerChunk);
+#pragma unroll
+                    for (int e = 0; e < kBatch; ++e) {
+                        const int ch = c0 + e;
+                        uint4* o = reinterpret_cast<uint4*>(dst + ((whole ? (ch ^ (lane & 7)) : (ch ^ ((lane >> 1) & 3))) << 4));
+                        if (col + cg + ch * kPerChunk < R) *o = plus16(*o, add[e], OutT());
+                    }
                 }
             }
             if (bulk) {
@@ -449,19 +485,22 @@ __device__ __forceinline__ void store_columns(const float (&acc)[kCols], uint8_t
         const float bv = in ? static_cast<float>(colb[j]) : 0.0f;      // finish() narrows it again: no change
         OutT* o = outp + static_cast<int64_t>(row_base - row_shift + lane / kWide) * ldo + col + j;
         const int rows = in ? Q - row_base - lane / kWide : 0;         // this lane's rows are 32 / kWide apart
+        const OutT* a = !ADD ? nullptr : behind_wait(static_cast<const OutT*>(fin.add)) + static_cast<int64_t>(row_base + lane / kWide) * fin.ld_add + col + j;
 #pragma unroll 8
         for (int i = 0; i < kWide; ++i) {
             const int rr = i * (32 / kWide) + lane / kWide;
             const float v = stage[rr * kWide + (cj ^ (rr & (kWide - 1)))];
-            if (i * (32 / kWide) < rows)
-                *o = scaled_if<OutT>(relu_if<OutT>(finish<OutT>((v * w) * scale_inv, bv, has_bias), relu), col + j < fin.scaled_cols, fin.factor);
+            if (i * (32 / kWide) < rows) {
+                const OutT y = scaled_if<OutT>(relu_if<OutT>(finish<OutT>((v * w) * scale_inv, bv, has_bias), relu), col + j < fin.scaled_cols, fin.factor);
+                *o = ADD ? plus<OutT>(y, a[i * (32 / kWide) * fin.ld_add]) : y;
+            }
             o += (32 / kWide) * ldo;
         }
         __syncwarp();
     }
 }
 
-template <int BN, bool DBG, typename OutT, bool REQ = false, int SPLIT = 1>
+template <int BN, bool DBG, typename OutT, bool REQ = false, int SPLIT = 1, bool ADD = false>
 __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
     const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
     const __grid_constant__ CUtensorMap map_o, const __grid_constant__ CUtensorMap map_t,   // out in boxes of 32 rows x 128 / 64 bytes
@@ -910,7 +949,7 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
 #pragma unroll
                     for (int j = 0; j < kShare; ++j) val[j] = small ? int_to_float_exact(sum[j]) : static_cast<float>(sum[j]);
                     const int cs = col0 + part * kShare;
-                    store_columns<OutT, kShare>(val, nullptr, my_store, colw + cs, colb + cs, map_o, map_t, static_cast<OutT*>(out), ldo, 0,
+                    store_columns<OutT, kShare, ADD>(val, nullptr, my_store, colw + cs, colb + cs, map_o, map_t, static_cast<OutT*>(out), ldo, 0,
                                                 tm * 256 + static_cast<int>(rank) * BM + quad * 32, Q, n0 + cs, R, scale_inv, has_bias, relu,
                                                 fin, store_flags);
                     continue;
@@ -1031,7 +1070,7 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                 row_shift = d * scatter.rows_per_dst;
             }
             const bool last = tile + num_pairs >= tiles_total;
-            store_columns<OutT, kCols>(acc, (store_flags & 4) && last ? smem + ew * kBlocks<OutT, kCols>() * 4096 : nullptr, my_store, colw + col0,
+            store_columns<OutT, kCols, ADD>(acc, (store_flags & 4) && last ? smem + ew * kBlocks<OutT, kCols>() * 4096 : nullptr, my_store, colw + col0,
                                        colb + col0, map_o, map_t, outp, ldo, row_shift, row_base, Q, n0 + col0, R, scale_inv, has_bias, relu,
                                        fin, store_flags);
         }

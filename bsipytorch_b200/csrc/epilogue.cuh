@@ -40,5 +40,11 @@ __device__ __forceinline__ OutT scaled_if(OutT v, bool on, float factor) {
     return on ? static_cast<OutT>(static_cast<float>(v) * factor) : v;
 }
 
+// The finished value plus one of another matrix, rounded to the output type: a separate elementwise addition's result.
+template <typename OutT>
+__device__ __forceinline__ OutT plus(OutT v, OutT add) {
+    return static_cast<OutT>(static_cast<float>(v) + static_cast<float>(add));
+}
+
 }  // namespace
 }  // namespace bsi

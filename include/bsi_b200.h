@@ -279,12 +279,24 @@ int bsi_b200_linear_decode_engine(const void* x, int x_dtype, int64_t ldx, int64
                                   int engine, bsi_stream_t stream);
 
 /* The same one launch for layers of more rows, on the tensor cores: 128 key rows per CTA, tiles of up to 128 activations
- * quantised by the CTAs that need them. For sizes bsi_b200_linear_rows_fits accepts (host function, 1 or 0). */
+ * quantised by the CTAs that need them. For sizes bsi_b200_linear_rows_fits accepts (host function, 1 or 0).
+ * add (rows ld_add apart, may be NULL): see bsi_b200_linear_i8_add. */
 int bsi_b200_linear_rows_fits(int64_t Q, int64_t R, int64_t D);
 int bsi_b200_linear_rows(const void* x, int x_dtype, int64_t ldx, int64_t D, int decimal_places, int bits,
                          const int8_t* k8, int64_t ldk, const float* bw0, const float* bias, int64_t Q, int64_t R,
                          float scale_inv, void* y, int64_t ldy, int activation, int64_t scaled_cols, float factor,
-                         int engine, bsi_stream_t stream);
+                         const void* add, int64_t ld_add, int engine, bsi_stream_t stream);
+
+/* bsi_b200_linear_decode_engine and bsi_b200_linear_i8_engine whose finished output gets a matrix of its type added (rows
+ * ld_add >= R apart, may be NULL), rounded once more: the residual sum of a decoder layer, what y.add_(x) computes. */
+int bsi_b200_linear_decode_add(const void* x, int x_dtype, int64_t ldx, int64_t D, int decimal_places, int bits,
+                               const int8_t* k8, int64_t ldk, const float* bw0, const float* bias, int64_t Q, int64_t R,
+                               float scale_inv, void* y, int64_t ldy, int activation, int64_t scaled_cols, float factor,
+                               const void* add, int64_t ld_add, int engine, bsi_stream_t stream);
+int bsi_b200_linear_i8_add(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride, const int8_t* k8, int64_t ldk,
+                           const float* bw0, const float* bias, int64_t Q, int64_t R, int64_t chunks, float scale_inv,
+                           void* y, int64_t ldy, int y_dtype, int activation, int64_t scaled_cols, float factor,
+                           const void* add, int64_t ld_add, const bsi_dot_bounds* bounds, int engine, bsi_stream_t stream);
 
 /* Linear whose finished output is re-quantised for the next linear inside the epilogue, so that the
  * layer-type [Q, R] matrix is never written: y = activation(cast(out) + cast(bias)) in layer_dtype
