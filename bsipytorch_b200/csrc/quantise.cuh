@@ -158,15 +158,16 @@ struct RawLane {
     // Largest |x| of the lane as a bit pattern of T that orders like the value: NaN and inf above every finite value.
     __device__ __forceinline__ uint32_t abs_max() const {
         if constexpr (sizeof(T) == 2) {
-            const uint32_t m = __vmaxu2(__vmaxu2(v[0].x & 0x7fff7fffu, v[0].y & 0x7fff7fffu),
-                                        __vmaxu2(v[0].z & 0x7fff7fffu, v[0].w & 0x7fff7fffu));
+            // in the type's own arithmetic, whose absolute value is an operand modifier; NaN wins and comes out canonical
+            using P = typename std::conditional<std::is_same<T, __half>::value, __half2, __nv_bfloat162>::type;
+            const P* p = reinterpret_cast<const P*>(&v[0]);
+            const P most = __hmax2_nan(__hmax2_nan(__habs2(p[0]), __habs2(p[1])), __hmax2_nan(__habs2(p[2]), __habs2(p[3])));
+            const uint32_t m = *reinterpret_cast<const uint32_t*>(&most);
             return max(m & 0xffffu, m >> 16);
         } else {
             const uint4& a = v[0];
             const uint4& b = v[kVecs - 1];
-            const uint32_t m = max(max(max(a.x & 0x7fffffffu, a.y & 0x7fffffffu), max(a.z & 0x7fffffffu, a.w & 0x7fffffffu)),
-                                   max(max(b.x & 0x7fffffffu, b.y & 0x7fffffffu), max(b.z & 0x7fffffffu, b.w & 0x7fffffffu)));
-            return m;
+            return most3(most3(most3(a.x, a.y, a.z), a.w, b.x), most3(b.y, b.z, b.w), 0u);
         }
     }
     // The pattern abs_max() returns as a float.
@@ -203,6 +204,12 @@ struct RawLane {
         }
     }
 private:
+    // the largest magnitude of three float32 patterns, NaN above all
+    static __device__ __forceinline__ uint32_t most3(uint32_t a, uint32_t b, uint32_t c) {
+        float d;
+        asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(__uint_as_float(a)), "f"(__uint_as_float(b)), "f"(__uint_as_float(c)));
+        return __float_as_uint(d);
+    }
     static __device__ __forceinline__ uint32_t mag(uint32_t pair, int half, float mult, float inv, float c) {
         if constexpr (std::is_same<T, __half>::value) {
             const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&pair));
