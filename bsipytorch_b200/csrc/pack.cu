@@ -327,6 +327,175 @@ __global__ void __launch_bounds__(256, BSI_PACK_MIN_BLOCKS) quantize_pack_chunk_
     }
 }
 
+// Two units per warp at a time, for 16-bit types: a lane holds 16 consecutive elements, lanes 0 to 15 those of one unit, 16 to 31
+// those of the next. The kernel above is bound by instruction issue (178 a unit with slices, 117 without), and a third of
+// them do not depend on how many elements a lane has: maximum, shift, rounding constants, addresses, the loop. Here they are
+// paid once per two units, the int8 image leaves 16 bytes per lane, and two lanes instead of four trade the slices' bytes
+// (4096 x 16384 float16: 60.7 -> 52.4 us with slices).
+// For more units than warps are resident; below that the kernel above spreads them over twice the warps.
+template <typename T, bool kDense, bool kWords, bool kQ8>
+__global__ void __launch_bounds__(256, BSI_PACK_MIN_BLOCKS) quantize_pack_chunk_pair_kernel(
+    const T* x, FastGeom g, double dec_scale, uint32_t dec_mult, int bits,
+    u64* __restrict__ words, float* __restrict__ scales, int32_t* __restrict__ shifts, int8_t* __restrict__ q8,
+    int vec_ok, float* __restrict__ sq_norms, float* __restrict__ slice_weights) {
+    static_assert(sizeof(T) == 2, "16 elements are two 16-byte vectors");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // as above
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    x = behind_wait(x);
+    __shared__ uint32_t slow_queue[8][kSlowQueue];
+    constexpr int kDepth = 2;
+    const int lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
+    const bool upper = lane >= 16;                    // the second unit's lanes
+    const uint32_t l = lane & 15u;
+    const uint32_t stride = gridDim.x * 16u;
+    const uint32_t first = (blockIdx.x * 8u + warp) * 2u;
+    if (kWords && slice_weights != nullptr) {         // in chunk mode a row's slice weights do not depend on its values
+        const uint32_t n = (g.total / g.chunks) * static_cast<uint32_t>(bits);
+        for (uint32_t i = blockIdx.x * 256u + threadIdx.x; i < n; i += gridDim.x * 256u)
+            slice_weights[i] = slice_weight(static_cast<int>(i % static_cast<uint32_t>(bits)), bits, 1.0f);
+    }
+    if (first >= g.total) return;
+    constexpr bool kRows = !kDense || kWords;
+    const uint32_t stride_rows = kRows ? stride / g.chunks : 0u;
+    const uint32_t stride_chunks = kRows ? stride - stride_rows * g.chunks : 0u;
+    const float mult = static_cast<float>(dec_mult);
+    const bool vec = kDense || vec_ok != 0;
+    const uint32_t lane_col = l * 16u;
+    int nslow = 0;
+
+    struct Pos { uint32_t unit, row, chunk; };        // of the lane's unit
+    struct Raw { RawLane<T> a, b; };
+    auto advance = [&](Pos& p) {
+        p.unit += stride;
+        if constexpr (kRows) {
+            p.row += stride_rows; p.chunk += stride_chunks;
+            if (p.chunk >= g.chunks) { p.chunk -= g.chunks; ++p.row; }
+        }
+    };
+    auto fetch = [&](Raw& r, const Pos& p) {
+        if (p.unit >= g.total) {                      // the last pair of an odd number of units
+            r.a.v[0] = r.b.v[0] = make_uint4(0u, 0u, 0u, 0u);
+        } else if constexpr (kDense) {
+            const T* src = x + (p.unit * 256u + lane_col);
+            r.a.load(src);
+            r.b.load(src + 8);
+        } else {
+            const uint32_t col = p.chunk * 256u + lane_col;
+            const T* src = x + static_cast<int64_t>(p.row) * g.ldx;
+            const int64_t left = static_cast<int64_t>(g.D) - static_cast<int64_t>(col);
+            if (vec && left >= 16) {
+                r.a.load(src + col);
+                r.b.load(src + col + 8);
+            } else {
+                r.a.load_tail(src + (left > 0 ? col : 0u), left);
+                r.b.load_tail(src + (left > 8 ? col + 8u : 0u), left - 8);
+            }
+        }
+    };
+    auto process = [&](const Raw& r, const Pos& p) {
+        const uint32_t m = max(r.a.abs_max(), r.b.abs_max());
+        const uint32_t m0 = __reduce_max_sync(0xffffffffu, upper ? 0u : m), m1 = __reduce_max_sync(0xffffffffu, upper ? m : 0u);
+        const float amax = RawLane<T>::abs_value(upper ? m1 : m0);
+        const int shift = fast_group_shift(amax, mult, bits);
+        const bool there = p.unit < g.total;
+        const uint32_t slow = __ballot_sync(0xffffffffu, there && shift < 0);
+        if (slow != 0u) {                             // NaN, infinity, beyond 2^23: either unit may be one
+            if (slow & 1u) {
+                if (nslow < kSlowQueue && lane == 0) slow_queue[warp][nslow] = p.unit;
+                ++nslow;
+            }
+            if (slow >> 31) {
+                if (nslow < kSlowQueue && lane == 31) slow_queue[warp][nslow] = p.unit;
+                ++nslow;
+            }
+        }
+        const bool store = there && shift >= 0;
+        // one group in a hundred or so has a value at the clamp: the others skip its steps
+        u64 pa, pb;
+        if (__any_sync(0xffffffffu, store && needs_clamp(amax, mult, shift, bits))) {
+            pa = r.a.template quantise<true>(mult, shift, bits);
+            pb = r.b.template quantise<true>(mult, shift, bits);
+        } else {
+            pa = r.a.template quantise<false>(mult, shift, bits);
+            pb = r.b.template quantise<false>(mult, shift, bits);
+        }
+        uint32_t al = static_cast<uint32_t>(pa), ah = static_cast<uint32_t>(pa >> 32), bl = static_cast<uint32_t>(pb), bh = static_cast<uint32_t>(pb >> 32);
+        if (sq_norms != nullptr) {                    // see fast_chunk
+            int n2 = __dp4a(static_cast<int>(al), static_cast<int>(al), __dp4a(static_cast<int>(ah), static_cast<int>(ah), 0));
+            n2 = __dp4a(static_cast<int>(bl), static_cast<int>(bl), __dp4a(static_cast<int>(bh), static_cast<int>(bh), n2));
+            const int n0 = __reduce_add_sync(0xffffffffu, upper ? 0 : n2), n1 = __reduce_add_sync(0xffffffffu, upper ? n2 : 0);
+            if (store && l == 0) sq_norms[p.unit] = static_cast<float>(upper ? n1 : n0) * __uint_as_float(static_cast<uint32_t>(127 + 2 * shift) << 23);
+        }
+        if (store && l == 0) {
+            scales[p.unit] = __uint_as_float(static_cast<uint32_t>(127 + shift) << 23);   // 2^shift
+            if (shifts != nullptr) shifts[p.unit] = shift;
+        }
+        if constexpr (kQ8) {
+            const uint32_t q8_off = kDense ? p.unit * 256u + lane_col : p.row * g.ld8 + p.chunk * 256u + lane_col;
+            if (store) *reinterpret_cast<uint4*>(q8 + q8_off) = make_uint4(al, ah, bl, bh);
+        }
+        if constexpr (kWords) {
+            transpose8x8_halves(al, ah);              // byte s: the lane's first eight bits of slice s (ah: slices 4 to 7)
+            transpose8x8_halves(bl, bh);              // ... and its next eight
+            // even lanes collect slices 0 to 3 of both lanes of their pair, odd lanes slices 4 to 7
+            const bool odd = (lane & 1) != 0;
+            const uint32_t ga = __shfl_xor_sync(0xffffffffu, odd ? al : ah, 1), gb = __shfl_xor_sync(0xffffffffu, odd ? bl : bh, 1);
+            const uint32_t ka = odd ? ah : al, kb = odd ? bh : bl;
+            const uint32_t a0 = odd ? ga : ka, b0 = odd ? gb : kb, a1 = odd ? ka : ga, b1 = odd ? kb : gb;      // even lane's, odd lane's
+            const uint32_t e0 = __byte_perm(a0, b0, 0x5140), e2 = __byte_perm(a0, b0, 0x7362);      // slice s: bytes a, b; then slice s + 1
+            const uint32_t o0 = __byte_perm(a1, b1, 0x5140), o2 = __byte_perm(a1, b1, 0x7362);
+            if (store && p.chunk * 4u + (l >> 2) < g.W) {
+                const int s0 = odd ? 4 : 0;
+                uint8_t* out = reinterpret_cast<uint8_t*>(words) +
+                               (p.row * g.row_bytes + p.chunk * 32u + (l & 14u) * 2u + static_cast<uint32_t>(s0) * g.slice_bytes);
+                if (s0 < bits) *reinterpret_cast<uint32_t*>(out) = __byte_perm(e0, o0, 0x5410);
+                if (s0 + 1 < bits) *reinterpret_cast<uint32_t*>(out + g.slice_bytes) = __byte_perm(e0, o0, 0x7632);
+                if (s0 + 2 < bits) *reinterpret_cast<uint32_t*>(out + 2u * g.slice_bytes) = __byte_perm(e2, o2, 0x5410);
+                if (s0 + 3 < bits) *reinterpret_cast<uint32_t*>(out + 3u * g.slice_bytes) = __byte_perm(e2, o2, 0x7632);
+            }
+        }
+    };
+
+    Pos cur, nxt;
+    cur.unit = first + (upper ? 1u : 0u);
+    cur.row = kRows ? cur.unit / g.chunks : 0u;
+    cur.chunk = kRows ? cur.unit - cur.row * g.chunks : 0u;
+    nxt = cur;
+    Raw buf[kDepth];
+#pragma unroll
+    for (int j = 0; j < kDepth; ++j) {
+        fetch(buf[j], nxt);
+        advance(nxt);
+    }
+    const uint32_t end = g.total + (upper ? 1u : 0u);       // a warp stays together: its first unit decides
+    while (cur.unit < end) {
+#pragma unroll
+        for (int j = 0; j < kDepth; ++j) {
+            if (cur.unit < end) {
+                const Raw r = buf[j];
+                fetch(buf[j], nxt);
+                process(r, cur);
+                advance(cur);
+                advance(nxt);
+            }
+        }
+    }
+    if (nslow == 0) return;
+    __syncwarp();
+    const int64_t ld8 = kDense ? g.D : g.ld8;
+    if (nslow <= kSlowQueue) {
+        for (int i = 0; i < nslow; ++i)
+            generic_unit<T>(x, slow_queue[warp][i], g.D, g.ldx, dec_scale, dec_mult, bits, g.chunks, g.W, words, scales,
+                            shifts, q8, ld8, vec, lane, 0.0f, sq_norms);
+    } else {
+        for (uint32_t unit = first; unit < g.total; unit += stride)
+            for (uint32_t u = unit; u < min(unit + 2u, g.total); ++u)
+                generic_unit<T>(x, u, g.D, g.ldx, dec_scale, dec_mult, bits, g.chunks, g.W, words, scales, shifts, q8,
+                                ld8, vec, lane, 0.0f, sq_norms);
+    }
+}
+
 // Destinations of the multi-destination pack: the same int8 image / chunk scales go to each of them.
 struct MultiDst {
     int n_q8, n_scales;
@@ -899,14 +1068,13 @@ __global__ void __launch_bounds__(256) cast_bias_kernel(const float* __restrict_
 namespace bsi {
 namespace {
 // Blocks of 256 threads of `kernel` that fit the current device at once (cached per kernel).
-template <typename K>
-int64_t resident_blocks(K kernel) {
+template <auto kernel>
+int64_t resident_blocks() {
     static thread_local int cached_dev = -1;
-    static thread_local K cached_fn = nullptr;
     static thread_local int cached = 0;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) { set_error("quantize_pack: cudaGetDevice failed"); return -1; }
-    if (dev != cached_dev || kernel != cached_fn) {
+    if (dev != cached_dev) {
         int per_sm = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 256, 0) != cudaSuccess || per_sm <= 0) {
             set_error("quantize_pack: occupancy query failed");
@@ -914,7 +1082,6 @@ int64_t resident_blocks(K kernel) {
         }
         cached = per_sm * sm_count();
         cached_dev = dev;
-        cached_fn = kernel;
     }
     return cached;
 }
@@ -937,9 +1104,19 @@ struct PackArgs {
 
 template <typename T, bool kDense, bool kWords, bool kQ8>
 int launch_chunk_fast(const T* x, const PackArgs& a) {
-    const int64_t resident = resident_blocks(quantize_pack_chunk_fast_kernel<T, kDense, kWords, kQ8>);
+    // one unit per warp and turn while a turn takes them all, else two (16-bit types)
+    auto kernel = quantize_pack_chunk_fast_kernel<T, kDense, kWords, kQ8>;
+    int64_t resident = resident_blocks<quantize_pack_chunk_fast_kernel<T, kDense, kWords, kQ8>>();
     if (resident <= 0) return BSI_ERR_CUDA;
     int64_t blocks = (a.rows * a.chunks + 7) / 8;
+    if constexpr (sizeof(T) == 2) {
+        if (blocks > resident) {
+            kernel = quantize_pack_chunk_pair_kernel<T, kDense, kWords, kQ8>;
+            resident = resident_blocks<quantize_pack_chunk_pair_kernel<T, kDense, kWords, kQ8>>();
+            if (resident <= 0) return BSI_ERR_CUDA;
+            blocks = (a.rows * a.chunks + 15) / 16;
+        }
+    }
     blocks = blocks < resident ? blocks : resident;
     FastGeom g;
     g.total = static_cast<uint32_t>(a.rows * a.chunks);
@@ -959,7 +1136,7 @@ int launch_chunk_fast(const T* x, const PackArgs& a) {
     cfg.stream = a.stream;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 1 : 0;
-    BSI_CUDA_TRY(cudaLaunchKernelEx(&cfg, quantize_pack_chunk_fast_kernel<T, kDense, kWords, kQ8>, x, g, a.dec_scale, a.dec_mult,
+    BSI_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, x, g, a.dec_scale, a.dec_mult,
                                     a.bits, a.words, a.scales, a.shifts, a.q8, a.vec_ok, a.sq_norms, a.slice_weights));
     return BSI_OK;
 }
@@ -1158,7 +1335,7 @@ extern "C" int bsi_b200_quantize_pack_multi(const void* x, int dtype, int64_t ro
     }
 #define BSI_LAUNCH_MULTI(T)                                                                                 \
     do {                                                                                                    \
-        const int64_t resident = resident_blocks(quantize_pack_multi_kernel<T>);                            \
+        const int64_t resident = resident_blocks<quantize_pack_multi_kernel<T>>();                            \
         if (resident <= 0) return BSI_ERR_CUDA;                                                             \
         int64_t blocks = (rows * chunks + 7) / 8;                                                           \
         blocks = blocks < resident ? blocks : resident;                                                     \
