@@ -237,7 +237,7 @@ struct PrebuiltBSIQueryCUDA {
 
 template <typename T>
 T* from_capsule(const py::capsule& cap, const char* name) {
-    TORCH_CHECK(cap.name() != nullptr && std::string(cap.name()) == name, "Expected a ", name, " capsule");
+    TORCH_CHECK(cap.name() != nullptr && std::strcmp(cap.name(), name) == 0, "Expected a ", name, " capsule");
     return reinterpret_cast<T*>(cap.get_pointer());
 }
 
@@ -1028,7 +1028,8 @@ py::object bsi_layer_forward(const torch::Tensor& x, const py::capsule& keyset_c
     auto* keys = from_capsule<PrebuiltBSIKeysCUDA>(keyset_cuda_cap, "PrebuiltBSIKeysCUDA");
     TORCH_CHECK(x.dim() >= 1, "x must have at least one dimension");
     const at::AutoDispatchBelowADInplaceOrView below;       // nothing here is recorded for gradients
-    at::Tensor x2d = x.detach();
+    // a detached alias costs 0.3 us, and a plain tensor that wants no gradients needs none
+    at::Tensor x2d = x.requires_grad() || x.unsafeGetTensorImpl()->is_python_dispatch() ? x.detach() : x;
     if (x2d.dim() != 2) x2d = x2d.reshape({-1, x2d.size(-1)});
     if (env.fp32 != nullptr && std::strcmp(env.fp32, "0") != 0) x2d = x2d.to(at::kFloat);   // verify_accuracy_bsi.py:126
     at::Tensor y = linear_forward(env, x2d, *keys, bias, decimalPlaces);

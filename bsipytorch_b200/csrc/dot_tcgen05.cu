@@ -605,7 +605,8 @@ bool plan_rows(int64_t Q, int64_t R, int64_t chunks, bool fused, RowsPlan* out) 
         for (int s = 1; s <= 8; s *= 2) {
             const int64_t per = (chunks + s - 1) / s, parts = (chunks + per - 1) / per;
             // a split runs in one wave and keeps all of its accumulators; so does the fused form, whose tiles quantise alone
-            if ((s > 1 || fused) && tiles * parts > sms) break;
+            // (of 148 SMs, clusters of four use 132 at once and clusters of eight 120)
+            if ((s > 1 || fused) && tiles * parts > (s <= 2 ? sms : s == 4 ? sms * 9 / 10 : sms * 5 / 6)) break;
             if (s > 1 && (parts == 1 || per > rows::kMaxBufs || per * nq > rows::kTmemCols)) continue;
             const double rows_of_tile = static_cast<double>(std::min<int64_t>(Q, nq));
             RowsPlan p = {};
@@ -900,7 +901,7 @@ extern "C" int bsi_b200_linear_rows(const void* x, int x_dtype, int64_t ldx, int
         return fail(BSI_ERR_INVALID, "linear_rows: unknown x_dtype");
     if (add != nullptr && ld_add < R) return fail(BSI_ERR_INVALID, "linear_rows: ld_add < R");
     RowsPlan plan;
-    if (!bsi_b200_linear_rows_fits(Q, R, D) || !plan_rows(Q, R, chunks, true, &plan))
+    if (Q > (1 << 16) || R >= (1 << 24) || chunks >= (1 << 12) || !plan_rows(Q, R, chunks, true, &plan))
         return fail(BSI_ERR_UNSUPPORTED, "linear_rows: not a size for this form");
     if (int rc = require_sm100()) return rc;
     rows::Args a = {};
