@@ -875,6 +875,7 @@ extern "C" int bsi_b200_linear_rows_fits(int64_t Q, int64_t R, int64_t D) {
     using namespace bsi;
     const int64_t chunks = (D + 255) / 256;
     if (Q < 1 || R < 1 || D < 1 || Q > (1 << 16) || R >= (1 << 24) || chunks >= (1 << 12)) return 0;
+    if (((R + 127) >> 7) * ((Q + 31) >> 5) > sm_count()) return 0;      // more tiles than a wave has: no need to plan
     if (Q <= 16 && bsi_b200_linear_decode_fits(Q, R, D)) return 0;
     RowsPlan plan;
     return plan_rows(Q, R, chunks, true, &plan) && plan.us <= 10.5 ? 1 : 0;
