@@ -16,6 +16,7 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -251,6 +252,10 @@ void same_device(const at::Tensor& a, const at::Tensor& b, const char* what) {
     TORCH_CHECK(!a.defined() || !b.defined() || !a.is_cuda() || !b.is_cuda() || a.device() == b.device(), what,
                 ": tensors live on different CUDA devices (", a.device(), " and ", b.device(), ")");
 }
+
+// Whether a mode or transform listens to operators (dispatch and fake-tensor modes, functorch levels, tracers): then every
+// operator that a call would issue is issued, for the mode to see, to change or to refuse.
+bool observed() { return !(c10::impl::tls_local_dispatch_key_set().included_ - c10::default_included_set).empty(); }
 
 uint64_t g_last_quantize_ns = 0, g_last_pack_ns = 0, g_last_total_ns = 0;
 
@@ -920,7 +925,7 @@ void linear_forward(const Env& env, const at::Tensor& x2d, int decimalPlaces, bo
         // so does a sum, behind the factor
         const bool factor_in = to[i].factor == 1.0 || scaled != 0;
         const bool add_in = factor_in && fused && D > 0 && to[i].add.defined() && to[i].add.scalar_type() == yt && to[i].add.is_contiguous() &&
-                            to[i].add.numel() == Q * R && to[i].add.device() == x2d.device();
+                            to[i].add.numel() == Q * R && to[i].add.device() == x2d.device() && !observed();
         const void* add = add_in ? to[i].add.data_ptr() : nullptr;
         auto rest = [&] {
             if (!factor_in) y.narrow(1, 0, cols).mul_(to[i].factor);
@@ -1029,7 +1034,7 @@ py::object bsi_layer_forward(const torch::Tensor& x, const py::capsule& keyset_c
     TORCH_CHECK(x.dim() >= 1, "x must have at least one dimension");
     const at::AutoDispatchBelowADInplaceOrView below;       // nothing here is recorded for gradients
     // a detached alias costs 0.3 us, and a plain tensor that wants no gradients needs none
-    at::Tensor x2d = x.requires_grad() || x.unsafeGetTensorImpl()->is_python_dispatch() ? x.detach() : x;
+    at::Tensor x2d = x.requires_grad() || x.unsafeGetTensorImpl()->is_python_dispatch() || observed() ? x.detach() : x;
     if (x2d.dim() != 2) x2d = x2d.reshape({-1, x2d.size(-1)});
     if (env.fp32 != nullptr && std::strcmp(env.fp32, "0") != 0) x2d = x2d.to(at::kFloat);   // verify_accuracy_bsi.py:126
     at::Tensor y = linear_forward(env, x2d, *keys, bias, decimalPlaces);

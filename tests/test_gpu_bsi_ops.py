@@ -8,6 +8,8 @@ import os
 import numpy as np
 import pytest
 import torch
+from torch._subclasses.fake_tensor import FakeTensorMode
+from torch.utils._python_dispatch import TorchDispatchMode
 
 import _capi_helpers as H
 import _inputs
@@ -287,3 +289,29 @@ def test_outlier_clipping_env(bsi_ops, monkeypatch):
     sc = torch.empty(40, 4, dtype=torch.float32, device=DEV)
     with pytest.raises(RuntimeError, match="BSI_FIXED_CLIP_K"):
         bsi_ops.pack_queries_into(q.to(DEV), q8, sc, 2)
+
+
+class _Ops(TorchDispatchMode):
+    def __init__(self):
+        super().__init__()
+        self.seen = []
+
+    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+        self.seen.append(func)
+        return func(*args, **(kwargs or {}))
+
+
+# a mode sees the layer's operators and can refuse a call, also where a plain tensor needs no operator at all
+@pytest.mark.parametrize("shape", [(20, 512), (2, 10, 512)])
+def test_layer_is_seen_by_modes_and_transforms(bsi_ops, shape):
+    layer = BSIQuantizedLinear(torch.nn.Linear(512, 300, device="cuda"), decimalPlaces=2)
+    x = torch.randn(shape, device="cuda")
+    with torch.no_grad():
+        y = layer(x)
+        with _Ops() as ops:
+            assert torch.equal(layer(x), y)
+        assert torch.ops.aten.detach.default in ops.seen
+        with pytest.raises(AssertionError, match="FakeTensor"), FakeTensorMode():
+            layer(x)
+        with pytest.raises(RuntimeError):                     # wrapped by the transform's level: no storage to read
+            torch.func.jvp(lambda t: layer(x) * t, (torch.ones((), device="cuda"),), (torch.ones((), device="cuda"),))

@@ -2,6 +2,7 @@
 import pytest
 import torch
 import torch.autograd.forward_ad as forward_ad
+from torch.utils._python_dispatch import TorchDispatchMode
 
 from bsipytorch_b200 import opt
 
@@ -101,6 +102,26 @@ def test_tensor_subclasses_and_function_modes_see_the_layer():
             assert layer._native(x) is not None
     assert type(tagged) is _Tagged and torch.equal(tagged.as_subclass(torch.Tensor), want) and torch.equal(got, want)
     assert mode.names.count("layer_norm") == 2 and "scaled_dot_product_attention" in mode.names
+
+
+class _Ops(TorchDispatchMode):
+    def __init__(self):
+        super().__init__()
+        self.seen = []
+
+    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+        self.seen.append(func)
+        return func(*args, **(kwargs or {}))
+
+
+def test_dispatch_modes_see_the_residual_sums():
+    layer, x = _layer(torch.float16)
+    with torch.no_grad():
+        want = layer(x)
+        with _Ops() as ops:
+            got = layer(x)
+    assert torch.equal(got, want)
+    assert ops.seen.count(torch.ops.aten.add_.Tensor) == 2
 
 
 def test_residual_sums_pass_forward_tangents_on():
