@@ -246,8 +246,8 @@ __device__ __forceinline__ uint4 finish16(const float* acc, const float* colw, c
 }
 // 16 bytes of finished values times a factor, rounded to the output type again.
 __device__ __forceinline__ uint4 times(uint4 o, float factor, float) {
-    return make_uint4(__float_as_uint(__uint_as_float(o.x) * factor), __float_as_uint(__uint_as_float(o.y) * factor),
-                      __float_as_uint(__uint_as_float(o.z) * factor), __float_as_uint(__uint_as_float(o.w) * factor));
+    return make_uint4(__float_as_uint(__fmul_rn(__uint_as_float(o.x), factor)), __float_as_uint(__fmul_rn(__uint_as_float(o.y), factor)),
+                      __float_as_uint(__fmul_rn(__uint_as_float(o.z), factor)), __float_as_uint(__fmul_rn(__uint_as_float(o.w), factor)));
 }
 __device__ __forceinline__ uint32_t times2(uint32_t v, float factor, __half) {
     const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&v));
@@ -264,8 +264,8 @@ __device__ __forceinline__ uint4 times(uint4 o, float factor, OutT t) {
 }
 // 16 bytes of finished values plus those of another matrix. A 16-bit add rounds like the float32 add narrowed (see finish2).
 __device__ __forceinline__ uint4 plus16(uint4 a, uint4 b, float) {
-    return make_uint4(__float_as_uint(__uint_as_float(a.x) + __uint_as_float(b.x)), __float_as_uint(__uint_as_float(a.y) + __uint_as_float(b.y)),
-                      __float_as_uint(__uint_as_float(a.z) + __uint_as_float(b.z)), __float_as_uint(__uint_as_float(a.w) + __uint_as_float(b.w)));
+    auto sum = [](uint32_t p, uint32_t q) { return __float_as_uint(__fadd_rn(__uint_as_float(p), __uint_as_float(q))); };
+    return make_uint4(sum(a.x, b.x), sum(a.y, b.y), sum(a.z, b.z), sum(a.w, b.w));
 }
 __device__ __forceinline__ uint32_t plus2(uint32_t a, uint32_t b, __half) {
     const __half2 y = __hadd2(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b));

@@ -4,6 +4,9 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+// The steps below follow one another and a product of the caller's (sum x weight x scale). Their float32 additions and products
+// are the intrinsics that no compiler contracts: a bias, a factor or a residual sum is rounded as by an operator of its own,
+// whatever the code around it is specialised to.
 namespace bsi {
 namespace {
 
@@ -14,17 +17,17 @@ template <typename OutT>
 __device__ __forceinline__ OutT finish(float v, float bias, bool has_bias);
 template <>
 __device__ __forceinline__ float finish<float>(float v, float bias, bool has_bias) {
-    return has_bias ? v + bias : v;
+    return has_bias ? __fadd_rn(v, bias) : v;
 }
 template <>
 __device__ __forceinline__ __half finish<__half>(float v, float bias, bool has_bias) {
     const __half h = __float2half_rn(v);
-    return has_bias ? __float2half_rn(__half2float(h) + __half2float(__float2half_rn(bias))) : h;
+    return has_bias ? __float2half_rn(__fadd_rn(__half2float(h), __half2float(__float2half_rn(bias)))) : h;
 }
 template <>
 __device__ __forceinline__ __nv_bfloat16 finish<__nv_bfloat16>(float v, float bias, bool has_bias) {
     const __nv_bfloat16 h = __float2bfloat16_rn(v);
-    return has_bias ? __float2bfloat16_rn(__bfloat162float(h) + __bfloat162float(__float2bfloat16_rn(bias))) : h;
+    return has_bias ? __float2bfloat16_rn(__fadd_rn(__bfloat162float(h), __bfloat162float(__float2bfloat16_rn(bias)))) : h;
 }
 
 // max(v, 0) on the finished output value when the layer's activation is fused (NaN stays NaN).
@@ -37,13 +40,13 @@ __device__ __forceinline__ OutT relu_if(OutT v, bool relu) {
 // layer's output by a scalar computes (OPT's query scaling).
 template <typename OutT>
 __device__ __forceinline__ OutT scaled_if(OutT v, bool on, float factor) {
-    return on ? static_cast<OutT>(static_cast<float>(v) * factor) : v;
+    return on ? static_cast<OutT>(__fmul_rn(static_cast<float>(v), factor)) : v;
 }
 
 // The finished value plus one of another matrix, rounded to the output type: a separate elementwise addition's result.
 template <typename OutT>
 __device__ __forceinline__ OutT plus(OutT v, OutT add) {
-    return static_cast<OutT>(static_cast<float>(v) + static_cast<float>(add));
+    return static_cast<OutT>(__fadd_rn(static_cast<float>(v), static_cast<float>(add)));
 }
 
 }  // namespace
