@@ -894,7 +894,10 @@ __global__ void __launch_bounds__(256, CPW * RawLane<T>::kVecs <= 8 ? 4 : 2) qua
     }
     uint32_t amax_bits = 0;
 #pragma unroll
-    for (int i = 0; i < CPW; ++i) amax_bits = max(amax_bits, raw[i].abs_max());
+    for (int i = 0; i < CPW; ++i) {
+        if constexpr (sizeof(T) == 4) amax_bits = max(amax_bits, raw[i].abs_max_masked());
+        else amax_bits = max(amax_bits, raw[i].abs_max());
+    }
     amax_bits = __reduce_max_sync(0xffffffffu, amax_bits);
     if (lane == 0) wmax[warp] = amax_bits;
     __syncthreads();
