@@ -37,6 +37,7 @@ SIGNATURES = {
     "bsi_b200_unregister_key_bounds": (_i32, [_vp]),
     "bsi_b200_debug_exact_int_tiles": (_i32, [_vp]),
     "bsi_b200_debug_last_tiles": (_i32, [_vp, _vp]),
+    "bsi_b200_debug_last_rows": (_i32, [_vp, _vp, _vp, _vp, _vp]),
     "bsi_b200_recombine_i8": (_i32, [_vp, _i64, _i32, _i64, _vp, _i64, _vp]),
     "bsi_b200_dot_i8": (_i32, [_vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _i64, _i64, _f32, _vp, _i64, _vp, _i32, _vp]),
     "bsi_b200_linear_i8": (_i32, [_vp, _i64, _vp, _i64, _vp, _i64, _vp, _vp, _i64, _i64, _i64, _f32, _vp, _i64, _i32, _vp]),
@@ -125,6 +126,14 @@ def last_tiles():
     width, parts = C.c_int(0), C.c_int(0)
     check(lib().bsi_b200_debug_last_tiles(C.byref(width), C.byref(parts)), "bsi_b200_debug_last_tiles")
     return width.value, parts.value
+
+
+def last_rows():
+    """(launches, query rows of a tile, parts along K, chunks of a part, chunks in the ring): the rows kernels this thread has
+    launched since it last asked, and the last one's plan."""
+    v = [C.c_int(0) for _ in range(5)]
+    check(lib().bsi_b200_debug_last_rows(*map(C.byref, v)), "bsi_b200_debug_last_rows")
+    return tuple(i.value for i in v)
 
 
 def device_status() -> int:

@@ -22,7 +22,7 @@ int dot_decode(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride
                const float* bias, int64_t Q, int64_t R, int64_t chunks, float scale_inv, void* out, int64_t ldo, int y_dtype,
                const Finishing& fin, bool keys_complete, cudaStream_t stream, bool* taken);
 
-bool rows_fits(int64_t Q, int64_t R, int64_t chunks);
+bool rows_fits(int64_t Q, int64_t R, int64_t chunks, const bsi_dot_bounds& bounds, int64_t qs_stride);
 int dot_rows(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride, const int8_t* k8, int64_t ldk, const float* bw0,
              const float* bias, int64_t Q, int64_t R, int64_t chunks, float scale_inv, void* out, int64_t ldo, int y_dtype,
              const Finishing& fin, bool keys_complete, cudaStream_t stream);
@@ -149,7 +149,7 @@ extern "C" int bsi_b200_dot_i8_bounded(const int8_t* a8, int64_t lda, const floa
         engine = BSI_ENGINE_TCGEN05;
     }
     if (engine == BSI_ENGINE_AUTO) {
-        if (dbg_iacc == nullptr && rows_fits(Q, R, chunks))
+        if (dbg_iacc == nullptr && rows_fits(Q, R, chunks, Q > 16 && Q <= 32 ? resolve_bounds(bounds, a8, k8, R) : bsi_dot_bounds{}, qs_stride))
             return dot_rows(a8, lda, qs, qs_stride, k8, ldk, bw0, nullptr, Q, R, chunks, scale_inv, out, ldo, BSI_DTYPE_F32, Finishing{},
                             keys_complete, stream);
         if (dbg_iacc == nullptr && decode_fits(Q, R, chunks)) {
@@ -231,7 +231,7 @@ extern "C" int bsi_b200_linear_i8_add(const int8_t* a8, int64_t lda, const float
         return fail(BSI_ERR_INVALID, "linear_i8: scaled_cols must be a multiple of 8 in [0, R]");
     if (add != nullptr && ld_add < R) return fail(BSI_ERR_INVALID, "linear_i8: ld_add < R");
     const Finishing fin{activation == BSI_ACT_RELU ? 1 : 0, static_cast<int>(scaled_cols), factor, add, ld_add};
-    if (engine == BSI_ENGINE_AUTO && rows_fits(Q, R, chunks))
+    if (engine == BSI_ENGINE_AUTO && rows_fits(Q, R, chunks, Q > 16 && Q <= 32 ? resolve_bounds(bounds, a8, k8, R) : bsi_dot_bounds{}, qs_stride))
         return dot_rows(a8, lda, qs, qs_stride, k8, ldk, bw0, bias, Q, R, chunks, scale_inv, y, ldy, y_dtype, fin, keys_complete,
                         static_cast<cudaStream_t>(stream_));
     if (engine == BSI_ENGINE_AUTO && decode_fits(Q, R, chunks)) {

@@ -561,8 +561,8 @@ int resident_clusters() {
 // Split along K or not, and the tile width to split at: *bn and the number of parts, 1 for no split. The costs are cycles
 // fitted to runs of 2 .. 64 chunks at widths 64, 128 and 256: 820 + 1.3 bn per chunk, and beside the chunks 7000 + 25 bn
 // without a split, 7500 + 55 bn with two parts, 12000 + 47 bn with four (clusters of eight start later). A split takes one
-// wave of clusters (33 of four CTAs and 15 of eight fit) and has to save a fifteenth.
-int pick_split(int64_t Q, int64_t R, int64_t chunks, int unsplit_bn, int* bn) {
+// wave of clusters (33 of four CTAs and 15 of eight fit) and has to save a fifteenth. *cycles: the cost of what is split.
+int pick_split(int64_t Q, int64_t R, int64_t chunks, int unsplit_bn, int* bn, double* cycles) {
     const int64_t mt = (Q + 255) / 256, pairs = sm_count() / 2;
     if (mt * ((R + unsplit_bn - 1) / unsplit_bn) > pairs) return 1;
     auto cost = [&](int w, double fixed, double per_column, int64_t parts) {
@@ -577,7 +577,7 @@ int pick_split(int64_t Q, int64_t R, int64_t chunks, int unsplit_bn, int* bn) {
             if (mt * ((R + w - 1) / w) > room) continue;
             const double c = s == 2 ? cost(w, 7500.0, 55.0, 2) : cost(w, 12000.0, 47.0, 4);
             if (c < best) {
-                best = c;
+                best = *cycles = c;
                 parts = s;
                 *bn = w;
             }
@@ -627,6 +627,10 @@ bool plan_rows(int64_t Q, int64_t R, int64_t chunks, bool fused, RowsPlan* out) 
     return best.us < 1e30;
 }
 
+// Rows kernels this thread has launched since it last asked, and the last one's plan (a test hook: bsi_b200_debug_last_rows).
+thread_local int t_rows_launches = 0;
+thread_local RowsPlan t_last_rows = {};
+
 template <int NQ, typename OutT, typename XT>
 int launch_rows(const CUtensorMap& mk, const CUtensorMap& mq, const RowsPlan& plan, const rows::Args& a, cudaStream_t stream) {
     static bool attr_set[64] = {false};
@@ -668,6 +672,8 @@ int run_rows(const RowsPlan& plan, rows::Args a, const int8_t* a8, int64_t lda, 
     if (int rc = make_map(&mk, k8, a.R, static_cast<int64_t>(a.chunks) * 256, ldk, 128)) return rc;
     if (a8 != nullptr)
         if (int rc = make_map(&mq, a8, a.Q, static_cast<int64_t>(a.chunks) * 256, lda, plan.nq)) return rc;
+    ++t_rows_launches;
+    t_last_rows = plan;
 #define BSI_ROWS(O_, X_) (plan.nq == 16 ? launch_rows<16, O_, X_>(mk, mq, plan, a, stream) : launch_rows<32, O_, X_>(mk, mq, plan, a, stream))
     if (a8 == nullptr)
         return x_dtype == BSI_DTYPE_F32 ? BSI_ROWS(float, float) : x_dtype == BSI_DTYPE_F16 ? BSI_ROWS(__half, __half) : BSI_ROWS(__nv_bfloat16, __nv_bfloat16);
@@ -677,15 +683,34 @@ int run_rows(const RowsPlan& plan, rows::Args a, const int8_t* a8, int64_t lda, 
 
 }  // namespace
 
-// Whether a dot of packed queries goes to the rows kernel. 17 to 32 rows, which fill an eighth of a paired tile: always (4096
-// x 16384 float16 layers of 32 rows 20.3 -> 17.5 us, 8192 x 2048 18.2 -> 15.1). Up to 16, where the key-streaming kernel is
-// the other choice: with key tiles for most of the SMs (4096 x 16384, 16 rows: 19.3 -> 16.0 us; 4096 x 11008, 8 rows: 13.5 ->
-// 11.6) and, beyond 8 rows, which that kernel's MMAs are too slow for, from 48 MB of keys on (16384 x 4096: 28.6 -> 24.1);
-// smaller sets it spreads better (8192 x 2048, 16 rows: 11.5 us against 12.5).
-bool rows_fits(int64_t Q, int64_t R, int64_t chunks) {
+// Whether the paired tiles, split along K, are the shorter way for 17 to 32 rows: with few key tiles and a deep K, where the
+// rows kernel's parts hand their sums on one after another and the split adds all parts at once (16384 x 512, 32 rows: 15.4 us
+// against 19.1; 8192 x 512: 11.1 against 12.5; 6144 x 512: 10.2 against 10.8; the other way 8192 x 1024: 13.5 against 12.5, 4096
+// x 512: 8.5 against 8.6). Only where its bounds are given and quickly read (rows of whole 16-byte vectors): without them the
+// split does not happen or starts late (4608 x 4608: 21.9 us against 9.5). Both costs as above, in microseconds of a replayed
+// graph: beside its chunks and hand-overs the rows kernel takes 2.1 + 0.2 per part + 0.045 per row, a split (1900 cycles to
+// the microsecond) 0.1 less for every tile that a wave of clusters of eight would still have room for.
+static bool split_is_shorter(int64_t Q, int64_t R, int64_t chunks, const RowsPlan& rows_plan, const bsi_dot_bounds& bounds, int64_t qs_stride) {
+    if (rows_plan.parts == 1 || bounds.key_bounds == nullptr || bounds.query_sq == nullptr || qs_stride < chunks ||
+        bounds.query_sq_stride < chunks || ((chunks | qs_stride | bounds.query_sq_stride) & 3) != 0)
+        return false;
+    int bn = pick_bn_pair(Q, R, false);
+    double cycles = 0.0;
+    if (pick_split(Q, R, chunks, bn, &bn, &cycles) == 1) return false;
+    const double split_us = cycles / 1900.0 - 0.1 * static_cast<double>(15 - (R + bn - 1) / bn);
+    return split_us < rows_plan.us + 2.1 + 0.2 * rows_plan.parts + 0.045 * static_cast<double>(Q);
+}
+
+// Whether a dot of packed queries goes to the rows kernel. 17 to 32 rows, which fill an eighth of a paired tile: but for the
+// case above (4096 x 16384 float16 layers of 32 rows 20.3 -> 17.5 us, 8192 x 2048 18.2 -> 15.1). Up to 16, where the
+// key-streaming kernel is the other choice: with key tiles for most of the SMs (4096 x 16384, 16 rows: 19.3 -> 16.0 us; 4096 x
+// 11008, 8 rows: 13.5 -> 11.6) and, beyond 8 rows, which that kernel's MMAs are too slow for, from 48 MB of keys on (16384 x
+// 4096: 28.6 -> 24.1); smaller sets it spreads better (8192 x 2048, 16 rows: 11.5 us against 12.5).
+bool rows_fits(int64_t Q, int64_t R, int64_t chunks, const bsi_dot_bounds& bounds, int64_t qs_stride) {
     if (Q > 32 || R >= (1 << 24) || chunks >= (1 << 12)) return false;
     RowsPlan plan;
-    return (Q > 16 || R >= 10240 || (Q > 8 && R * chunks * 256 >= (48 << 20))) && plan_rows(Q, R, chunks, false, &plan);
+    if (Q > 16) return plan_rows(Q, R, chunks, false, &plan) && !split_is_shorter(Q, R, chunks, plan, bounds, qs_stride);
+    return (R >= 10240 || (Q > 8 && R * chunks * 256 >= (48 << 20))) && plan_rows(Q, R, chunks, false, &plan);
 }
 
 int dot_rows(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride, const int8_t* k8, int64_t ldk, const float* bw0,
@@ -741,7 +766,8 @@ int dot_i8_pair(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_strid
     }
     // only with bounds (a split adds integers), one plain destination, and no accumulator dump
     const bool may_split = !force_bn && kabs != nullptr && dbg_iacc == nullptr && scatter.n == 0;
-    const int parts = may_split ? pick_split(Q, R, chunks, bn, &bn) : 1;
+    double cycles = 0.0;
+    const int parts = may_split ? pick_split(Q, R, chunks, bn, &bn, &cycles) : 1;
     t_last_width = bn;
     t_last_parts = parts;
     if (bn < 64 || bn > 256 || (bn & 31) != 0 || (!any_width && (bn & (bn - 1)) != 0))
@@ -915,6 +941,19 @@ extern "C" int bsi_b200_linear_rows(const void* x, int x_dtype, int64_t ldx, int
     for (int i = 0; i < decimal_places; ++i) a.dec_mult *= 10u;
     a.dec_scale = static_cast<double>(a.dec_mult);
     return run_rows(plan, a, nullptr, 0, k8, ldk, x_dtype, x_dtype, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int bsi_b200_debug_last_rows(int* launches_out, int* queries_out, int* parts_out, int* chunks_out, int* stages_out) {
+    using namespace bsi;
+    if (launches_out == nullptr || queries_out == nullptr || parts_out == nullptr || chunks_out == nullptr || stages_out == nullptr)
+        return fail(BSI_ERR_INVALID, "debug_last_rows: null pointer");
+    *launches_out = t_rows_launches;
+    *queries_out = t_last_rows.nq;
+    *parts_out = t_last_rows.parts;
+    *chunks_out = t_last_rows.per_part;
+    *stages_out = t_last_rows.stages;
+    t_rows_launches = 0;
+    return BSI_OK;
 }
 
 extern "C" int bsi_b200_debug_last_tiles(int* width_out, int* parts_out) {

@@ -235,6 +235,9 @@ int bsi_b200_debug_exact_int_tiles(unsigned long long* count_out);
 /* Test hook: columns of a tile and parts along K (1: no split) of the calling thread's last dot on the paired tensor-core
  * kernel. In a split dot every warp of every part counts above where the tile's bounds hold, those of one part elsewhere. */
 int bsi_b200_debug_last_tiles(int* width_out, int* parts_out);
+/* Test hook: rows kernels (bsi_b200_linear_rows, dots of few rows) that the calling thread has launched since it last called
+ * this, and of the last one: query rows of a tile, parts along K, chunks of a part, chunks in the operand ring. */
+int bsi_b200_debug_last_rows(int* launches_out, int* queries_out, int* parts_out, int* chunks_out, int* stages_out);
 
 /* The same bounds handed to a dot directly, without the registry (host struct of device pointers; key_bounds NULL: none,
  * query_sq NULL: no Cauchy-Schwarz bound). bounds == NULL: bsi_b200_dot_i8 / bsi_b200_linear_i8_act. */

@@ -64,6 +64,28 @@ def test_packed_dot_of_few_rows(Q, R, D, chunk_mode):
     assert capi.device_status() == 0
 
 
+# deep K over few key tiles: the paired tiles split along K add all parts at once, where their bounds are given and read as
+# whole vectors; from 16 key tiles on, at fewer chunks or without bounds the rows kernel
+@pytest.mark.parametrize("Q,R,D,rows", [(32, 512, 8192, 0), (17, 130, 8192, 0), (32, 960, 16384, 0), (24, 2048, 8192, 1), (32, 512, 4096, 1),
+                                        (32, 512, 7936, 1)])
+def test_deep_dots_of_few_keys_take_the_shorter_way(Q, R, D, rows):
+    import bsipytorch_b200
+    ops = bsipytorch_b200.bsi_ops
+    q, k = _inputs.fc1(Q=Q, R=R, D=D, seed=Q + R + D, dtype=torch.float32)
+    keys = ops.build_bsi_keys_cuda(k.to(DEV), 2)[0]
+    queries = ops.build_bsi_queries_cuda_batch_packed(q.to(DEV), 2)
+    capi.last_rows()
+    got = ops.batch_dot_product_multiquery_cuda_batch_caps(queries, keys)[0]
+    assert capi.last_rows()[0] == rows
+    if not rows:
+        assert capi.last_tiles()[1] > 1
+    t, b = ops.debug_query_batch_tensors(queries), ops.debug_keys_tensors(keys)
+    call = lambda: H.dot_i8(t["q8"], t["scales"], b["q8"], b["scales"].reshape(-1), o.scale_inv(2))      # noqa: E731
+    assert torch.equal(call().view(torch.int32), got.view(torch.int32))
+    assert capi.last_rows()[0] == 1                            # no bounds: no split
+    assert capi.device_status() == 0
+
+
 # where a CTA's share of the quantisation outweighs a second launch, and where the key-streaming kernel has its own form
 def test_one_launch_rule():
     fits = capi.lib().bsi_b200_linear_rows_fits
