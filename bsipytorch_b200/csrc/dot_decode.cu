@@ -328,6 +328,15 @@ bool decode_fits(int64_t Q, int64_t R, int64_t chunks) {
     return Q <= kMaxQueries && R <= (1 << 27) && chunks <= 4096;
 }
 
+// The share of the kernel's warps that have a chunk of their own: as many warps as the next power of two share a row tile
+// (5 chunks: 5 of 8, 9 chunks: 9 of 16).
+double decode_share(int64_t Q, int64_t chunks) {
+    const int64_t most = Q <= 8 ? 32 : 16, slabs = (chunks + most - 1) / most, slab = (chunks + slabs - 1) / slabs;
+    int64_t kw = 1;
+    while (kw < kWarps && kw < slab) kw *= 2;
+    return static_cast<double>(slab) / static_cast<double>(kw * ((slab + kw - 1) / kw));
+}
+
 int dot_decode(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride, const int8_t* k8, int64_t ldk, const float* bw0,
                const float* bias, int64_t Q, int64_t R, int64_t chunks, float scale_inv, void* out, int64_t ldo, int y_dtype,
                const Finishing& fin, bool keys_complete, cudaStream_t stream, bool* taken) {

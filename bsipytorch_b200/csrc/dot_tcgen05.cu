@@ -701,16 +701,35 @@ static bool split_is_shorter(int64_t Q, int64_t R, int64_t chunks, const RowsPla
     return split_us < rows_plan.us + 2.1 + 0.2 * rows_plan.parts + 0.045 * static_cast<double>(Q);
 }
 
+double decode_share(int64_t Q, int64_t chunks);
+
+// Up to 16 rows and more key tiles than SMs: the rows kernel starts another wave of CTAs, each with its set-up and nothing beside
+// it on the SM, and a wave that is not full takes its SMs' time all the same, where the key-streaming kernel goes on. It pays
+// where that kernel leaves a quarter of its warps without a chunk (5 chunks: 20480 x 1280, 1 row, 8.2 -> 7.5 us; 10 chunks: 33664 x
+// 2560, 16 rows, 25.9 -> 18.5) or where long waves are nearly full (37888 x 4096, 1 row, 29.4 -> 26.0, 30000 x 4096, 16 rows,
+// 26.7 -> 25.4; 8192 deep from three quarters on, 30000 rows 42.9 -> 40.6, and beyond 8 rows whatever the fill, 26000 rows 46.2
+// -> 41.6). It loses elsewhere: 19072 x 4096, 1 row, 16.4 us against 19.2; 50272 x 768, 8 rows, 10.9 against 13.2; 50272 x
+// 2048, 1 row, 19.4 against 20.4.
+static bool more_waves_pay(int64_t Q, int64_t R, int64_t chunks) {
+    const int64_t tiles = (R + 127) / 128, sms = sm_count(), waves = (tiles + sms - 1) / sms;
+    if (waves == 1) return true;
+    const double fill = static_cast<double>(tiles) / static_cast<double>(waves * sms);
+    if (chunks >= 5 && decode_share(Q, chunks) <= 0.75) return true;
+    const double least = chunks >= 24 ? (Q > 8 ? 0.0 : 0.75) : chunks >= 14 ? (Q > 8 ? 0.75 : 0.85) : 2.0;
+    return fill >= least;
+}
+
 // Whether a dot of packed queries goes to the rows kernel. 17 to 32 rows, which fill an eighth of a paired tile: but for the
 // case above (4096 x 16384 float16 layers of 32 rows 20.3 -> 17.5 us, 8192 x 2048 18.2 -> 15.1). Up to 16, where the
 // key-streaming kernel is the other choice: with key tiles for most of the SMs (4096 x 16384, 16 rows: 19.3 -> 16.0 us; 4096 x
 // 11008, 8 rows: 13.5 -> 11.6) and, beyond 8 rows, which that kernel's MMAs are too slow for, from 48 MB of keys on (16384 x
-// 4096: 28.6 -> 24.1); smaller sets it spreads better (8192 x 2048, 16 rows: 11.5 us against 12.5).
+// 4096: 28.6 -> 24.1); smaller sets it spreads better (8192 x 2048, 16 rows: 11.5 us against 12.5), and most
+// sets of more than one wave too (above).
 bool rows_fits(int64_t Q, int64_t R, int64_t chunks, const bsi_dot_bounds& bounds, int64_t qs_stride) {
     if (Q > 32 || R >= (1 << 24) || chunks >= (1 << 12)) return false;
     RowsPlan plan;
     if (Q > 16) return plan_rows(Q, R, chunks, false, &plan) && !split_is_shorter(Q, R, chunks, plan, bounds, qs_stride);
-    return (R >= 10240 || (Q > 8 && R * chunks * 256 >= (48 << 20))) && plan_rows(Q, R, chunks, false, &plan);
+    return (R >= 10240 || (Q > 8 && R * chunks * 256 >= (48 << 20))) && more_waves_pay(Q, R, chunks) && plan_rows(Q, R, chunks, false, &plan);
 }
 
 int dot_rows(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride, const int8_t* k8, int64_t ldk, const float* bw0,

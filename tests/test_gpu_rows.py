@@ -86,6 +86,22 @@ def test_deep_dots_of_few_keys_take_the_shorter_way(Q, R, D, rows):
     assert capi.device_status() == 0
 
 
+# up to 16 rows and more key tiles than SMs: the key-streaming kernel, but for chunks that leave its warps idle (5 of 8, 10 of 16) and
+# for long waves that are nearly full
+@pytest.mark.parametrize("Q,R,D,rows", [(1, 18944, 512, 1), (1, 18945, 512, 0), (8, 50272, 768, 0), (16, 19072, 4096, 0), (16, 28416, 4096, 1), (8, 28416, 4096, 0), (16, 20000, 1280, 1),
+                                        (3, 37888, 4096, 1), (9, 20001, 2560, 1), (16, 19000, 6912, 1), (4, 19000, 6912, 0)])
+def test_few_rows_and_more_key_tiles_than_sms(Q, R, D, rows):
+    q, k = _inputs.fc1(Q=Q, R=R, D=D, seed=Q + R + D, dtype=torch.float32)
+    qa = H.quantize_pack(q.to(DEV), 2, 7, True)
+    kb = H.quantize_pack(k.to(DEV), 2, 6, False)
+    capi.last_rows()
+    got = H.dot_i8(qa["q8"], qa["scales"], kb["q8"], kb["scales"], o.scale_inv(2))
+    assert capi.last_rows()[0] == rows
+    want = H.dot_i8(qa["q8"], qa["scales"], kb["q8"], kb["scales"], o.scale_inv(2), 3064)
+    assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+    assert capi.device_status() == 0
+
+
 # where a CTA's share of the quantisation outweighs a second launch, and where the key-streaming kernel has its own form
 def test_one_launch_rule():
     fits = capi.lib().bsi_b200_linear_rows_fits
