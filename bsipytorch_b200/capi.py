@@ -49,6 +49,7 @@ SIGNATURES = {
     "bsi_b200_linear_decode": (_i32, [_vp, _i32, _i64, _i64, _i32, _i32, _vp, _i64, _vp, _vp, _i64, _i64, _f32, _vp, _i64, _i32, _i64, _f32, _vp]),
     "bsi_b200_linear_decode_engine": (_i32, [_vp, _i32, _i64, _i64, _i32, _i32, _vp, _i64, _vp, _vp, _i64, _i64, _f32, _vp, _i64, _i32, _i64, _f32, _i32, _vp]),
     "bsi_b200_linear_rows_fits": (_i32, [_i64, _i64, _i64]),
+    "bsi_b200_linear_rows_ways": (_i32, [_i64, _i64, _i64, _i32]),
     "bsi_b200_linear_rows": (_i32, [_vp, _i32, _i64, _i64, _i32, _i32, _vp, _i64, _vp, _vp, _i64, _i64, _f32, _vp, _i64, _i32, _i64, _f32, _vp, _i64, _i32, _vp]),
     "bsi_b200_linear_decode_add": (_i32, [_vp, _i32, _i64, _i64, _i32, _i32, _vp, _i64, _vp, _vp, _i64, _i64, _f32, _vp, _i64, _i32, _i64, _f32, _vp, _i64, _i32, _vp]),
     "bsi_b200_linear_i8_add": (_i32, [_vp, _i64, _vp, _i64, _vp, _i64, _vp, _vp, _i64, _i64, _i64, _f32, _vp, _i64, _i32, _i32, _i64, _f32, _vp, _i64, _vp, _i32, _vp]),

@@ -952,10 +952,10 @@ void linear_forward(const Env& env, const at::Tensor& x2d, int decimalPlaces, bo
             rest();
             continue;
         }
-        // One launch instead of two, 3.5 us of host time less. A replayed graph has no such cost, and up to 16 rows the
-        // key-streaming kernel behind a packer is the shorter one on the GPU (12 x 3072 x 768: 5.2 us against 7.5).
-        if (one_launch && bsi_b200_linear_rows_fits(Q, R, D) &&
-            (Q > 16 || c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None)) {
+        // one launch instead of two where it is the shorter way; whether a graph records is asked only where that decides
+        const int ways = one_launch ? bsi_b200_linear_rows_ways(Q, R, D, code) : 0;
+        if (ways == (BSI_ROWS_ISSUED | BSI_ROWS_REPLAYED) ||
+            (ways == BSI_ROWS_ISSUED && c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None)) {
             check_status(bsi_b200_linear_rows(x.data_ptr(), code, ldx, D, decimalPlaces, bits, keys.b.q8.data_ptr<int8_t>(),
                                               keys.b.q8.size(1), keys.b.scales.data_ptr<float>(), bptr, Q, R, scale_inv,
                                               y.data_ptr(), R, act, scaled, factor, add, R, keys.complete(), current_stream()),

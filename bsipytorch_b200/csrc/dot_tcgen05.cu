@@ -914,16 +914,44 @@ extern "C" int bsi_b200_device_status(int* status_out) {
     return BSI_OK;
 }
 
-// Where the quantisation in every CTA costs less than a second launch, which the host needs until 12 us have gone by. Up to 16
-// rows the key-streaming kernel's own one-launch form comes first.
-extern "C" int bsi_b200_linear_rows_fits(int64_t Q, int64_t R, int64_t D) {
+// Where one launch, with the quantisation in every CTA, is the shorter way. Issued one by one, two launches take the host 10 us and
+// more (a layer's call through its module), the kernel 0.5 us more than the plan says; the lines are where the two met:
+//   tiles of 32 rows   17 to 32 rows always (24 x 1280 -> 16256 float32: 8.8 us against 12.6), else up to four chunks (56 x 1280 ->
+//                      7808, five: 10.7 against 9.4)
+//   17 rows and more   up to 10.2 us (374 x 3055 -> 739, 10.4 by the plan: 15.3 against 12.9)
+//   up to 16 rows      the key-streaming kernel's own one-launch form comes first, and behind a packer that kernel or, from 10240 keys
+//                      on, this one is the other way: up to 9.6 us (16 x 4352 -> 2185, 10.1: 10.7 against 10.1), up to 8.2 where
+//                      the depth is no whole number of vectors (14 x 3291 -> 207, 8.7: 11.3 against 10.1), up to 10.3 from 12 MB of
+//                      keys on, which the GPU needs longer than 10 us for (9 x 5104 -> 8960: 13.0 against 19.1), and not from
+//                      40 MB on where the rows kernel reads packed rows (4 x 4096 -> 11000: 15.1 against 13.3)
+static bool one_launch_plan(int64_t Q, int64_t R, int64_t D, bsi::RowsPlan* plan) {
     using namespace bsi;
     const int64_t chunks = (D + 255) / 256;
-    if (Q < 1 || R < 1 || D < 1 || Q > (1 << 16) || R >= (1 << 24) || chunks >= (1 << 12)) return 0;
-    if (((R + 127) >> 7) * ((Q + 31) >> 5) > sm_count()) return 0;      // more tiles than a wave has: no need to plan
-    if (Q <= 16 && bsi_b200_linear_decode_fits(Q, R, D)) return 0;
-    RowsPlan plan;
-    return plan_rows(Q, R, chunks, true, &plan) && plan.us <= 10.5 ? 1 : 0;
+    if (Q < 1 || R < 1 || D < 1 || Q > (1 << 16) || R >= (1 << 24) || chunks >= (1 << 12)) return false;
+    if (((R + 127) >> 7) * ((Q + 31) >> 5) > sm_count()) return false;      // more tiles than a wave has: no need to plan
+    if (Q <= 16 && bsi_b200_linear_decode_fits(Q, R, D)) return false;
+    if (!plan_rows(Q, R, chunks, true, plan)) return false;
+    const int64_t keys = R * chunks * 256;
+    if (Q <= 16) {
+        if (R >= 10240 && keys >= (40 << 20)) return false;
+        return plan->us <= (keys >= (12 << 20) ? 10.3 : (D & 7) != 0 ? 8.2 : 9.6);
+    }
+    return plan->us <= (plan->nq == 16 ? 10.2 : Q <= 32 ? 10.5 : 8.8);
+}
+
+// A replayed graph has no host cost. Up to 16 rows the key-streaming kernel behind a packer is the shorter way there (12 x 3072 x
+// 768: 5.2 us against 7.5), and more than 32 rows in tiles of 32 lose to packer and paired tiles where those store whole vectors
+// of 16 bits (512 x 1024 -> 1024 7.3 us against 9.2, 472 x 768 -> 640 6.8 against 8.2, 232 x 256 -> 1920 5.9 against 6.6; ragged
+// columns 432 x 768 -> 660 9.0 against 8.3; float32 169 x 256 -> 2688 6.3 against 5.6, 69 x 768 -> 5504 7.2 against 7.3).
+extern "C" int bsi_b200_linear_rows_ways(int64_t Q, int64_t R, int64_t D, int x_dtype) {
+    bsi::RowsPlan plan;
+    if (!one_launch_plan(Q, R, D, &plan)) return 0;
+    const bool replayed = Q > 16 && (plan.nq == 16 || Q <= 32 || (R & 7) != 0 || x_dtype == BSI_DTYPE_F32);
+    return BSI_ROWS_ISSUED | (replayed ? BSI_ROWS_REPLAYED : 0);
+}
+
+extern "C" int bsi_b200_linear_rows_fits(int64_t Q, int64_t R, int64_t D) {
+    return (bsi_b200_linear_rows_ways(Q, R, D, BSI_DTYPE_F32) & BSI_ROWS_ISSUED) != 0 ? 1 : 0;
 }
 
 extern "C" int bsi_b200_linear_rows(const void* x, int x_dtype, int64_t ldx, int64_t D, int decimal_places, int bits, const int8_t* k8,

@@ -281,10 +281,15 @@ int bsi_b200_linear_decode_engine(const void* x, int x_dtype, int64_t ldx, int64
                                   float scale_inv, void* y, int64_t ldy, int activation, int64_t scaled_cols, float factor,
                                   int engine, bsi_stream_t stream);
 
-/* The same one launch for layers of more rows, on the tensor cores: 128 key rows per CTA, tiles of up to 128 activations
- * quantised by the CTAs that need them. For sizes bsi_b200_linear_rows_fits accepts (host function, 1 or 0).
+/* The same one launch for layers of more rows, on the tensor cores: 128 key rows per CTA, tiles of 16 or 32 activations
+ * quantised by the CTAs that need them. bsi_b200_linear_rows_fits (host function, 1 or 0): sizes where that is the shorter way
+ * for launches issued one by one, about 500 x 1024 x 1024 or 128 x 2048 x 2048; bsi_b200_linear_rows_ways tells it from a
+ * replayed graph, whose launches cost the host nothing. The call itself takes every size whose CTAs fit one wave.
  * add (rows ld_add apart, may be NULL): see bsi_b200_linear_i8_add. */
+#define BSI_ROWS_ISSUED 1    /* the shorter way for launches issued one by one */
+#define BSI_ROWS_REPLAYED 2  /* and in a replayed graph */
 int bsi_b200_linear_rows_fits(int64_t Q, int64_t R, int64_t D);
+int bsi_b200_linear_rows_ways(int64_t Q, int64_t R, int64_t D, int x_dtype);
 int bsi_b200_linear_rows(const void* x, int x_dtype, int64_t ldx, int64_t D, int decimal_places, int bits,
                          const int8_t* k8, int64_t ldk, const float* bw0, const float* bias, int64_t Q, int64_t R,
                          float scale_inv, void* y, int64_t ldy, int activation, int64_t scaled_cols, float factor,

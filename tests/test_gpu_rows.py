@@ -102,7 +102,35 @@ def test_few_rows_and_more_key_tiles_than_sms(Q, R, D, rows):
     assert capi.device_status() == 0
 
 
-# where a CTA's share of the quantisation outweighs a second launch, and where the key-streaming kernel has its own form
+# where a CTA's share of the quantisation outweighs a second launch, tiles of 32 rows and five chunks among them, a depth of no
+# whole vectors, and where the key-streaming kernel has its own form or packed rows are read faster
 def test_one_launch_rule():
-    fits = capi.lib().bsi_b200_linear_rows_fits
+    L = capi.lib()
+    fits, replayed = L.bsi_b200_linear_rows_fits, lambda *size: L.bsi_b200_linear_rows_ways(*size) >> 1      # noqa: E731
     assert [fits(64, 4096, 4096), fits(64, 2048, 2048), fits(512, 4096, 4096), fits(16, 256, 256), fits(17, 256, 256)] == [0, 1, 0, 0, 1]
+    assert [fits(374, 739, 3055), fits(56, 7808, 1280), fits(24, 16256, 1280), fits(48, 7552, 1024)] == [0, 0, 1, 1]
+    assert [fits(14, 207, 3291), fits(14, 207, 3328), fits(16, 2185, 4352), fits(9, 8960, 5104), fits(4, 11000, 4096)] == [0, 1, 0, 1, 0]
+    h, f = capi.DTYPE_F16, capi.DTYPE_F32
+    assert [replayed(512, 1024, 1024, h), replayed(512, 1024, 1024, f), replayed(432, 660, 768, h), replayed(64, 2048, 2048, h),
+            replayed(24, 16256, 1280, h), replayed(13, 3000, 3840, h)] == [0, 1, 1, 1, 1, 0]
+
+
+# the route a captured layer takes: more than 32 rows in tiles of 32 go to packer and paired tiles, the bits are the same
+@pytest.mark.parametrize("dtype,Q,R,D,rows", [(torch.float16, 472, 640, 768, 0), (torch.bfloat16, 232, 1920, 256, 0), (torch.float32, 232, 1920, 256, 1),
+                                              (torch.float16, 64, 777, 2816, 1)])
+def test_captured_layers_take_the_shorter_way(dtype, Q, R, D, rows):
+    import bsipytorch_b200
+    ops = bsipytorch_b200.bsi_ops
+    x, k = _inputs.fc1(Q=Q, R=R, D=D, seed=Q + R + D, dtype=dtype)
+    x, bias = x.to(DEV), torch.linspace(-1, 1, R, device=DEV)
+    keys = ops.build_bsi_keys_cuda(k.to(DEV), 2)[0]
+    capi.last_rows()
+    want = ops.bsi_layer_forward(x, keys, bias, 2)
+    assert capi.last_rows()[0] == 1
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = ops.bsi_layer_forward(x, keys, bias, 2)
+    assert capi.last_rows()[0] == rows
+    graph.replay()
+    assert torch.equal(got, want)
+    assert capi.device_status() == 0
