@@ -13,14 +13,18 @@ DEV = "cuda"
 
 
 # one row beyond a tile of 16, tiles of 32 rows (more than 148 of 16), 128 and 129 keys, one chunk, operand rings that turn
-# over (more than 6 chunks), two and four parts along K with a shorter last one, ragged depth, keys and rows
+# over (more than 6 chunks), also of parts along K, whose stages are free once multiplied (8 and 7 chunks in a ring of 6), two and
+# four parts with a shorter last one, ragged depth, keys and rows; plan: query rows of a tile, parts, chunks of a part, ring
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
-@pytest.mark.parametrize("Q,R,D", [(17, 128, 256), (33, 129, 250), (512, 1100, 1000), (600, 500, 760), (77, 777, 1000), (20, 9000, 2000),
-                                   (16, 2300, 2304), (64, 700, 2800), (13, 3000, 3840), (40, 130, 4096)])
-def test_one_launch_layer_of_many_rows(dtype, Q, R, D, monkeypatch):
+@pytest.mark.parametrize("Q,R,D,plan", [(17, 128, 256, (16, 1, 1, 1)), (33, 129, 250, (16, 1, 1, 1)), (512, 1100, 1000, (32, 1, 4, 4)),
+                                        (600, 500, 760, (32, 1, 3, 3)), (77, 777, 1000, (16, 2, 2, 2)), (20, 9000, 2000, (16, 1, 8, 6)),
+                                        (16, 2300, 2304, (16, 3, 3, 3)), (64, 700, 2800, (16, 4, 3, 3)), (13, 3000, 3840, (16, 4, 4, 4)),
+                                        (40, 130, 4096, (16, 4, 4, 4)), (64, 2048, 4096, (16, 2, 8, 6)), (50, 1999, 3835, (16, 2, 8, 6))])
+def test_one_launch_layer_of_many_rows(dtype, Q, R, D, plan, monkeypatch):
     import bsipytorch_b200
     ops = bsipytorch_b200.bsi_ops
     assert capi.lib().bsi_b200_linear_rows_fits(Q, R, D) == 1
+    capi.last_rows()
     x, k = _inputs.fc1(Q=Q, R=R, D=D, seed=Q + R + D, dtype=torch.float32)
     x[1] *= 3.0e3 if dtype == torch.float16 else 3.0e4        # sums beyond 2^24: the order of the chunks shows
     x[2, D // 3] = float("inf")
@@ -34,12 +38,12 @@ def test_one_launch_layer_of_many_rows(dtype, Q, R, D, monkeypatch):
         monkeypatch.setenv("BSI_B200_ENGINE", "tcgen05")
         want = ops.bsi_layer_forward(x, keys, b, 2)
         monkeypatch.delenv("BSI_B200_ENGINE")
-        capi.exact_int_tiles()
+        assert capi.last_rows()[0] == 0
         for _ in range(3):                                    # the later calls read keys ahead of the wait
             assert torch.equal(ops.bsi_layer_forward(x, keys, b, 2), want)
             torch.cuda.synchronize()
         assert torch.equal(ops.bsi_layer_forward(wide[:, :D], keys, b, 2), want)
-        assert capi.exact_int_tiles() == 0                    # no paired tile ran
+        assert capi.last_rows() == (4,) + plan
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph):
         captured = [ops.bsi_layer_forward(x, keys, bias, 2) for _ in range(3)]
@@ -58,7 +62,9 @@ def test_packed_dot_of_few_rows(Q, R, D, chunk_mode):
         q[1] *= 3.0e4
     qa = H.quantize_pack(q.to(DEV), 2, 7, chunk_mode)
     kb = H.quantize_pack(k.to(DEV), 2, 6, False)
+    capi.last_rows()
     got = H.dot_i8(qa["q8"], qa["scales"], kb["q8"], kb["scales"], o.scale_inv(2))
+    assert capi.last_rows()[:2] == (1, 16 if Q <= 16 else 32)
     want = H.dot_i8(qa["q8"], qa["scales"], kb["q8"], kb["scales"], o.scale_inv(2), 3064)
     assert torch.equal(got.view(torch.int32), want.view(torch.int32))
     assert capi.device_status() == 0
