@@ -283,7 +283,7 @@ int bsi_b200_linear_decode_engine(const void* x, int x_dtype, int64_t ldx, int64
 
 /* The same one launch for layers of more rows, on the tensor cores: 128 key rows per CTA, tiles of 16 or 32 activations
  * quantised by the CTAs that need them. bsi_b200_linear_rows_fits (host function, 1 or 0): sizes where that is the shorter way
- * for launches issued one by one, about 500 x 1024 x 1024 or 128 x 2048 x 2048; bsi_b200_linear_rows_ways tells it from a
+ * for launches issued one by one, about 512 x 1024 x 1024 or 144 x 2048 x 2048; bsi_b200_linear_rows_ways tells it from a
  * replayed graph, whose launches cost the host nothing. The call itself takes every size whose CTAs fit one wave.
  * add (rows ld_add apart, may be NULL): see bsi_b200_linear_i8_add. */
 #define BSI_ROWS_ISSUED 1    /* the shorter way for launches issued one by one */
