@@ -609,40 +609,40 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsLow));
         if (is_producer) {
             // ---------------- TMA producers ----------------
-            // One thread needs ~450 cycles per k-block (empty wait, expect_tx, two tensor copies), which
-            // is slower than the MMAs consume narrow tiles; warps 0 and 2 therefore take the k-blocks
-            // in turn. Stage s = it % kStages is always filled by the producer that owns `it`.
+            // Warps 0 and 2 take the k-blocks in turn. The whole warp walks the loop, as the issuers do, with stage, parity and
+            // coordinates carried along, and one elected lane issues.
             constexpr int kProducers = 2;
             const int me = warp >> 1;
+            int s = me, kb = me;                       // stage of this warp's next k-block, the k-block
+            uint32_t ph = 1;
             bool ok = true;
-            auto load = [&](int it, int kb, int tm, int tn) {
-                const int s = it % kStages;
-                const uint32_t ph = static_cast<uint32_t>(it / kStages) & 1u;
-                if (!wait_or_abort(empty_bar(s), ph ^ 1u, actx, 1)) return false;
-                if (leader) mbar_expect_tx(full_bar(s), 2u * C::kStageBytes);
-                const uint32_t a_dst = smem_base + s * C::kStageBytes;
-                tma_load_2d_pair(a_dst, &map_a, (c_lo * 2 + kb) * BK, tm * 256 + static_cast<int>(rank) * BM, leader_full0 + 8u * s);
-                tma_load_2d_pair(a_dst + C::kABytes, &map_b, (c_lo * 2 + kb) * BK, tn * BN + static_cast<int>(rank) * C::kHalfN,
-                                 leader_full0 + 8u * s);
-                return true;
-            };
-            int done = 0;
-            if constexpr (SPLIT > 1) {
-                // the first ring round goes out before the vote: it is the part's own beginning either way
-                done = min(kStages, num_kb);
-                if (lane == 0)
-                    for (int it = me; it < done && ok; it += kProducers) ok = load(it, it, pair_id % tiles_m, pair_id / tiles_m);
+            auto load = [&](int x, int ya, int yb) {
+                ok = __all_sync(0xffffffffu, wait_or_abort(empty_bar(s), ph, actx, 1));
+                if (!ok) return;
+                if (elect_one()) {
+                    const uint32_t a_dst = smem_base + s * C::kStageBytes, bar = leader_full0 + 8u * s;
+                    if (leader) mbar_expect_tx(full_bar(s), 2u * C::kStageBytes);
+                    tma_load_2d_pair(a_dst, &map_a, x, ya, bar);
+                    tma_load_2d_pair(a_dst + C::kABytes, &map_b, x, yb, bar);
+                }
                 __syncwarp();
-                cluster_sync_all();
-                if (*vote) num_kb = part == 0 ? 2 * chunks : done;
+                s += kProducers;
+                if (s >= kStages) { s -= kStages; ph ^= 1u; }
+            };
+            for (int tile = pair_id; tile < tiles_total && ok; tile += num_pairs) {
+                const int ya = tile % tiles_m * 256 + static_cast<int>(rank) * BM;
+                const int yb = tile / tiles_m * BN + static_cast<int>(rank) * C::kHalfN;
+                if constexpr (SPLIT > 1) {
+                    // the first ring round goes out before the vote: it is the part's own beginning either way
+                    const int done = min(kStages, num_kb);
+                    for (; kb < done && ok; kb += kProducers) load((c_lo * 2 + kb) * BK, ya, yb);
+                    cluster_sync_all();
+                    if (*vote) num_kb = part == 0 ? 2 * chunks : done;
+                } else {
+                    kb = me;
+                }
+                for (; kb < num_kb && ok; kb += kProducers) load((c_lo * 2 + kb) * BK, ya, yb);
             }
-            if (lane == 0) {
-                int it = 0;
-                for (int tile = pair_id; tile < tiles_total && ok; tile += num_pairs)
-                    for (int kb = 0; kb < num_kb && ok; ++kb, ++it)
-                        if (it >= done && it % kProducers == me) ok = load(it, kb, tile % tiles_m, tile / tiles_m);
-            }
-            __syncwarp();
         } else {
             if constexpr (SPLIT > 1) cluster_sync_all();
             if (leader) {
