@@ -110,9 +110,14 @@ __device__ __forceinline__ bool elect_one() {
     return pred != 0;
 }
 
+// Without release: with it an arrival waits for every memory access the warp has under way, 1000 to 1200 cycles here. Where
+// something was written for the other CTAs, a fence of its own stands in front (fence_cluster), in the threads that wrote.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void fence_cluster() { asm volatile("fence.acq_rel.cluster;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_arrive();
+    cluster_wait();
 }
 
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
@@ -176,6 +181,7 @@ __device__ __forceinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, con
             if (now - t0 > kWait) {
                 *a.flag = 1;
                 store_flag_cluster(a.peer_flag, 1);
+                fence_cluster();
                 atomicCAS(&g_device_status, 0, 16 + site);
                 return false;
             }
@@ -402,7 +408,7 @@ __device__ __forceinline__ void store_columns(const float (&acc)[kCols], uint8_t
             const int cg = g * kRoundCols;
             uint8_t* block = places != nullptr ? places + g * 4096 : own;
             if (bulk && places == nullptr) {
-                if (lane == 0) tma_store_wait_read();
+                if (elect_one()) tma_store_wait_read();
                 __syncwarp();
             }
             uint8_t* dst = block + lane * (nch * 16);
@@ -442,7 +448,7 @@ __device__ __forceinline__ void store_columns(const float (&acc)[kCols], uint8_t
             if (bulk) {
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
-                if (lane == 0 && row_base < Q && col + cg < R)      // rows and columns beyond the matrix are clipped
+                if (row_base < Q && col + cg < R && elect_one())    // rows and columns beyond the matrix are clipped
                     tma_store_2d(whole ? &map_o : &map_t, smem_u32(block), col + cg, row_base);
             } else {
                 __syncwarp();
@@ -468,7 +474,7 @@ __device__ __forceinline__ void store_columns(const float (&acc)[kCols], uint8_t
     // warp's 4 KB, then kWide adjacent columns of 32 / kWide rows at a time, so that a store covers consecutive addresses.
     constexpr int kWide = kCols < 32 ? (kCols & -kCols) : 32;
     if (store_flags & 4) {
-        if (lane == 0) tma_store_wait_read();
+        if (elect_one()) tma_store_wait_read();
         __syncwarp();
     }
     float* stage = reinterpret_cast<float*>(own);
@@ -576,9 +582,10 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncwarp();
-    // Cluster barrier split around the TMEM allocation: arrive now (thread 0's barrier inits are
-    // released by its own arrive), wait after the allocation, so the two latencies overlap.
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    // Cluster barrier split around the TMEM allocation: arrive now (warp 0's barrier inits are
+    // released by its own arrive, the others have written nothing), wait after the allocation, so the two latencies overlap.
+    if (warp == 0) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    else cluster_arrive();
     const bool is_producer = warp == 0 || warp == 2;
     uint32_t tmem_base = 0;
     if (is_producer) {
@@ -635,8 +642,9 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                 if constexpr (SPLIT > 1) {
                     // the first ring round goes out before the vote: it is the part's own beginning either way
                     const int done = min(kStages, num_kb);
+                    cluster_arrive();
                     for (; kb < done && ok; kb += kProducers) load((c_lo * 2 + kb) * BK, ya, yb);
-                    cluster_sync_all();
+                    cluster_wait();
                     if (*vote) num_kb = part == 0 ? 2 * chunks : done;
                 } else {
                     kb = me;
@@ -644,29 +652,30 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                 for (; kb < num_kb && ok; kb += kProducers) load((c_lo * 2 + kb) * BK, ya, yb);
             }
         } else {
-            if constexpr (SPLIT > 1) cluster_sync_all();
+            // The vote is the epilogue's; the chunks that the accumulators hold go before it, the part's own beginning either way.
+            if constexpr (SPLIT > 1) cluster_arrive();
+            const int mi = warp >> 1;
+            int total = my_chunks;
+            const int early = SPLIT > 1 ? min(kAccBufs, my_chunks) : 0;
+            auto voted = [&] {
+                cluster_wait();
+                if (*vote) total = part == 0 ? chunks : 0;
+            };
             if (leader) {
             // ---------------- MMA issuers (leader CTA) ----------------
             // The whole warp walks the loop (so that addresses and descriptors stay in the uniform
-            // datapath) and one elected lane issues the tensor-core instructions. A chunk costs an issuer about 770
-            // cycles (three barrier waits, eight MMAs, three commits), more than the MMAs of tiles up to 160 columns
-            // take, so warps 1 and 3 issue alternate chunks; they share nothing but the order of the rings.
+            // datapath) and one elected lane issues the tensor-core instructions. A chunk takes an issuer about 500
+            // cycles (three barrier waits, eight MMAs, three commits), the MMAs 500 + 2 per column of the tile (A and half of B
+            // from shared memory at 64 bytes a cycle), so warps 1 and 3 issue alternate chunks; they share nothing but the
+            // order of the rings.
             constexpr uint32_t idesc = umma_idesc_pair(BN);
-            const int mi = warp >> 1;
-            int total = ((tiles_total - pair_id + num_pairs - 1) / num_pairs) * my_chunks;
-            if constexpr (SPLIT > 1) {
-                if (*vote) {
-                    total = part == 0 ? chunks : 0;
-                    // this part's copies are in flight for nothing: they have to land before the CTAs go
-                    if (part != 0 && mi == 0)
-                        for (int st = 0; st < min(kStages, num_kb); ++st)
-                            if (!wait_or_abort(full_bar(st), 0, actx, 2)) break;
-                }
-            }
+            if constexpr (SPLIT == 1) total = ((tiles_total - pair_id + num_pairs - 1) / num_pairs) * my_chunks;
             int s = 2 * mi;
             uint32_t ph = 0;
             bool ok = true;
-            for (int cc = mi; cc < total && ok; cc += 2) {
+            int cc = mi;
+            auto issue = [&](int upto) {
+            for (; cc < upto && ok; cc += 2) {
                 const int b = cc % kAccBufs;
                 const uint32_t tph = static_cast<uint32_t>(cc / kAccBufs) & 1u;
                 if (!wait_or_abort(tempty_bar(b), tph ^ 1u, actx, 3)) { ok = false; break; }
@@ -693,15 +702,31 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                 s += 2;                                    // the other issuer's chunk
                 if (s >= kStages) { s -= kStages; ph ^= 1u; }
             }
+            };
+            if constexpr (SPLIT > 1) {
+                issue(early);
+                voted();
+            }
+            issue(total);
+            if (SPLIT > 1 && total == 0 && mi == 0)        // copies that no MMA waited for have to land before the CTAs go
+                for (int st = 2 * early; st < min(kStages, num_kb); ++st)
+                    if (!wait_or_abort(full_bar(st), 0, actx, 2)) break;
             if (!ok && lane == 0) {
                 umma_commit(drain_bar);
                 const long long t0 = clock64();
                 while (!mbar_try(drain_bar, 0) && clock64() - t0 < kWait / 64) {}
             }
-            __syncwarp();
+            } else if constexpr (SPLIT > 1) {
+                voted();
             }
+            if (SPLIT > 1 && total == 0)                   // likewise the MMAs whose sums nobody reads
+                for (int cc = mi; cc < early; cc += 2)
+                    if (!wait_or_abort(tfull_bar(cc), 0, actx, 4)) break;
+            __syncwarp();
         }
         if constexpr (SPLIT > 1) cluster_sync_all();      // the operand rings are free
+        __syncwarp();
+        cluster_arrive();
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsHigh));
         // ---------------- epilogue ----------------
@@ -806,8 +831,10 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
             int n_chunks = my_chunks;
             bool whole_tile = SPLIT == 1;      // this pair does all chunks and stores all columns
             if constexpr (SPLIT > 1) {
-                if (!exact && lane < 2 * SPLIT)
+                if (!exact && lane < 2 * SPLIT) {
                     store_flag_cluster(map_to_cta(smem_u32(const_cast<int*>(vote)), static_cast<uint32_t>(lane)), 1);
+                    fence_cluster();
+                }
                 __syncwarp();
                 cluster_sync_all();
                 if (*vote) {
@@ -815,6 +842,8 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                     n_chunks = part == 0 ? chunks : 0;
                 }
             }
+            // The last round of accumulators has no user after this one, and its arrivals could reach the leader after its end.
+            const int hand_back = (SPLIT > 1 ? n_chunks : (tiles_total - pair_id + num_pairs - 1) / num_pairs * my_chunks) - kAccBufs;
             // the chunk scale of the next chunk is loaded a whole chunk ahead: a scattered load per lane (32 rows) that
             // would otherwise stand in front of every fold
             float qnext = qs_row[qs_stride ? min(c_lo, chunks - 1) : 0];
@@ -846,7 +875,7 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                         // every column of the buffer is in registers: hand it back before the last piece is folded in
                         tc_fence_before();
                         __syncwarp();
-                        if (lane == 0) mbar_arrive_cluster(leader_tempty0 + 8u * b);
+                        if (lane == 0 && cc < hand_back) mbar_arrive_cluster(leader_tempty0 + 8u * b);
                     }
                     if (exact) {
 #pragma unroll
@@ -882,6 +911,10 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                         }
                     }
                 }
+            }
+            if constexpr (!REQ && SPLIT == 1) {
+                __syncwarp();
+                if (tile + num_pairs >= tiles_total) cluster_arrive();
             }
             // the half's key scales and bias into shared memory: behind the first barrier nobody reads the last tile's
             asm volatile("bar.sync %0, 128;" ::"r"(2 + half) : "memory");
@@ -926,6 +959,8 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                     __syncwarp();
                     ok = wait_or_abort(sum_bar, 0, actx, 6);
                 }
+                __syncwarp();
+                cluster_arrive();
                 if (add_up) {
                     if (!ok) continue;
                     int sum[kShare];
@@ -1005,6 +1040,7 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                             if (*actx.flag || clock64() - t0 > kWait) {
                                 *actx.flag = 1;
                                 store_flag_cluster(actx.peer_flag, 1);
+                                fence_cluster();
                                 atomicCAS(&g_device_status, 0, 16 + 7);
                                 ok = false;
                                 break;
@@ -1074,7 +1110,11 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                                        colb + col0, map_o, map_t, outp, ldo, row_shift, row_base, Q, n0 + col0, R, scale_inv, has_bias, relu,
                                        fin, store_flags);
         }
-        if (lane == 0) tma_store_wait_read();      // shared memory is read until then
+        if constexpr (REQ) {
+            __syncwarp();
+            cluster_arrive();
+        }
+        if (elect_one()) tma_store_wait_read();    // shared memory is read until then
     }
 
     if (threadIdx.x == 0 && *abort_flag) {
@@ -1084,8 +1124,9 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
     }
     tc_fence_before();
     __syncthreads();
-    __syncwarp();
-    cluster_sync_all();  // the peer may still be reading this CTA's smem or arriving on its barriers
+    // The peer may still be reading this CTA's shared memory or arriving on its barriers: every warp has arrived as soon as it
+    // was done with the other CTAs' memory, the epilogue's before their last stores.
+    cluster_wait();
     if (warp == 1) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;"
