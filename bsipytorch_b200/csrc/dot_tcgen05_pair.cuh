@@ -307,50 +307,49 @@ __device__ __forceinline__ float4 zero_of<float4>() { return make_float4(0.0f, 0
 template <>
 __device__ __forceinline__ float zero_of<float>() { return 0.0f; }
 
-// Over 32 rows of per-chunk scales (and sums of squares; norms may be null), `units` vectors V each: the largest scale,
-// the largest sum of a row's scales, the largest sum of a row's squares, spread over the lanes (the caller takes the
-// maximum over them). Neighbouring lanes read neighbouring vectors of a row and add up by shuffles: with a row per lane
-// every load touched 32 lines, 7 thousand cycles for 64 chunks.
+// Of 32 rows of per-chunk scales (and sums of squares; norms may be null), `units` vectors V each: the largest scale, the
+// largest sum of a row's scales, the largest sum of a row's squares, spread over the lanes (the caller takes the maximum over
+// them). Eight lanes read neighbouring vectors of a row, with eight rows per lane in flight, so that a load touches 4 rows'
+// lines instead of 32 and up to 32 chunks of both arrays take one trip to memory (16 loads in turns of 8: 6400 cycles with
+// the reductions, now 3000). The rows' sums are then halved over the lanes, which takes 7 exchanges instead of 24.
 template <typename V>
 __device__ __forceinline__ void row_stats(const float* qs, int64_t qs_stride, const float* norms, int64_t n_stride,
                                           int first_row, int Q, int units, float& smax, float& ssum, float& u2) {
-    constexpr int kMost = sizeof(V) == 16 ? 8 : 32;      // lanes on a row at most
-    constexpr int kRows = 4;                             // rows per lane group in flight
     const int lane = threadIdx.x & 31;
-    int lg = 0;
-    while ((1 << lg) < units && (1 << lg) < kMost) ++lg;
-    const int group = 1 << lg, sub = lane & (group - 1);
-    for (int it = 0; it < group; it += kRows) {
-        float m[kRows], t[kRows], n[kRows];
+    const int sub = lane & 7;
+    float t[8], n[8];
 #pragma unroll
-        for (int h = 0; h < kRows; ++h) m[h] = t[h] = n[h] = 0.0f;
-        for (int u0 = 0; u0 < units; u0 += group) {
-            V a[kRows], b[kRows];
+    for (int h = 0; h < 8; ++h) t[h] = n[h] = 0.0f;
+    for (int u0 = 0; u0 < units; u0 += 8) {
+        V a[8], b[8];
 #pragma unroll
-            for (int h = 0; h < kRows; ++h) {
-                const int r = first_row + (((it + h) << 5) >> lg) + (lane >> lg);
-                const bool in = it + h < group && u0 + sub < units && r < Q;
-                a[h] = in ? reinterpret_cast<const V*>(qs + r * qs_stride)[u0 + sub] : zero_of<V>();
-                b[h] = in && norms != nullptr ? reinterpret_cast<const V*>(norms + r * n_stride)[u0 + sub] : zero_of<V>();
-            }
-#pragma unroll
-            for (int h = 0; h < kRows; ++h) {
-                m[h] = fmaxf(m[h], most4(a[h]));
-                t[h] += sum4(a[h]);
-                n[h] += sum4(b[h]);
-            }
+        for (int h = 0; h < 8; ++h) {
+            const int r = first_row + h * 4 + (lane >> 3);
+            const bool in = u0 + sub < units && r < Q;
+            a[h] = in ? reinterpret_cast<const V*>(qs + r * qs_stride)[u0 + sub] : zero_of<V>();
+            b[h] = in && norms != nullptr ? reinterpret_cast<const V*>(norms + r * n_stride)[u0 + sub] : zero_of<V>();
         }
 #pragma unroll
-        for (int h = 0; h < kRows; ++h) {
-            for (int d = 1; d < group; d <<= 1) {
-                t[h] += __shfl_xor_sync(0xffffffffu, t[h], d);
-                n[h] += __shfl_xor_sync(0xffffffffu, n[h], d);
-            }
-            smax = fmaxf(smax, m[h]);
-            ssum = fmaxf(ssum, t[h]);
-            u2 = fmaxf(u2, n[h]);
+        for (int h = 0; h < 8; ++h) {
+            smax = fmaxf(smax, most4(a[h]));
+            t[h] += sum4(a[h]);
+            n[h] += sum4(b[h]);
         }
     }
+#pragma unroll
+    for (int d = 4; d > 0; d >>= 1) {        // a lane keeps half of its rows, with both lanes' sums
+        const bool upper = (lane & d) != 0;
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            if (h < d) {
+                const float gt = __shfl_xor_sync(0xffffffffu, upper ? t[h] : t[h + d], d), gn = __shfl_xor_sync(0xffffffffu, upper ? n[h] : n[h + d], d);
+                t[h] = (upper ? t[h + d] : t[h]) + gt;
+                n[h] = (upper ? n[h + d] : n[h]) + gn;
+            }
+        }
+    }
+    ssum = t[0];
+    u2 = n[0];
 }
 
 // The same for one row per lane: kAhead vectors of each array in flight.
@@ -761,6 +760,10 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                 if (has_bias) own_b = behind_wait(bias)[n0 + col0 + own];
             }
 
+            // The chunk scale of the next chunk is loaded a whole chunk ahead, the first one in front of the bounds: a scattered load per
+            // lane (32 rows) that would otherwise stand in front of every fold.
+            float qnext = qs_row[qs_stride ? min(c_lo, chunks - 1) : 0];
+
             // Integer accumulation where it provably equals the float32 chain: the chunk terms I_c * 2^shift are
             // integers, so while every prefix sum stays below 2^24 in magnitude no float32 addition rounds and
             // acc += I_c << shift in int32 gives the same bits. With A the largest query magnitude, a prefix is at
@@ -776,19 +779,14 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
             if (k_abs_sum != nullptr && ok) {
                 // of the warp's key rows: the largest sum of |k| over a row and over one chunk, the largest sum of k^2
                 const float* k_sums = behind_wait(k_abs_sum);
-                float ktot = 0.0f, kchk = 0.0f, k2 = 0.0f;
-                if (lane * 4 < kCols) {
-                    float kv[12];
+                constexpr int kPer = (kCols + 31) / 32;       // key rows per lane
+                float kv[3][kPer];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const int col = min(n0 + col0 + lane * 4 + e, R - 1);
-                        kv[e] = k_sums[col];
-                        kv[4 + e] = k_sums[R + col];
-                        kv[8 + e] = k_sums[2 * static_cast<int64_t>(R) + col];
-                    }
-                    ktot = fmaxf(fmaxf(kv[0], kv[1]), fmaxf(kv[2], kv[3]));
-                    kchk = fmaxf(fmaxf(kv[4], kv[5]), fmaxf(kv[6], kv[7]));
-                    k2 = fmaxf(fmaxf(kv[8], kv[9]), fmaxf(kv[10], kv[11]));
+                for (int e = 0; e < kPer; ++e) {
+                    const int col = min(n0 + col0 + min(e * 32 + lane, kCols - 1), R - 1);
+                    kv[0][e] = k_sums[col];
+                    kv[1][e] = k_sums[R + col];
+                    kv[2][e] = k_sums[2 * static_cast<int64_t>(R) + col];
                 }
                 // of the warp's query rows: the largest and the largest summed 2^shift of a row, the largest sum of squares
                 float smax = 0.0f, ssum = 0.0f, u2 = 0.0f;
@@ -810,20 +808,30 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                         else row_of_lane<float, 8>(qs_row, nrow, chunks, smax, ssum, u2);
                     }
                 }
-                // An infinity anywhere fails the test. By shuffles: with redux.sync (nvcc 12.9) an earlier form of this code
+                float ktot = kv[0][0], kchk = kv[1][0], k2 = kv[2][0];
+#pragma unroll
+                for (int e = 1; e < kPer; ++e) {
+                    ktot = fmaxf(ktot, kv[0][e]);
+                    kchk = fmaxf(kchk, kv[1][e]);
+                    k2 = fmaxf(k2, kv[2][e]);
+                }
+                // An infinity anywhere fails the test. By shuffles, all six maxima side by side: with redux.sync (nvcc 12.9) an earlier form of this code
                 // had norm = 0 in every warp of one instantiation (256 columns, four parts), and so exact sums beyond 2^24.
                 // Not a divergent warp (a __syncwarp before each changed nothing) nor wrong operands (the other four maxima
                 // were right, and shuffles of the same registers are); writing the operands out made it go away. The split
                 // test has a row beyond the bounds for every width and number of parts.
-                auto most = [](float v) {
+                float most[6] = {smax, ssum, u2, ktot, kchk, k2};
 #pragma unroll
-                    for (int d = 16; d > 0; d >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, d));
-                    return v;
-                };
-                const float su = most(smax), tu = most(ssum), ku = most(ktot), cu = most(kchk);
+                for (int d = 16; d > 0; d >>= 1) {
+                    float got[6];
+#pragma unroll
+                    for (int e = 0; e < 6; ++e) got[e] = __shfl_xor_sync(0xffffffffu, most[e], d);
+#pragma unroll
+                    for (int e = 0; e < 6; ++e) most[e] = fmaxf(most[e], got[e]);
+                }
                 // the sums above round (relative 2^-24 per addition, at most a few thousand additions): 0.999 covers it
-                const float first = fminf(su * ku, tu * cu) * q_abs_max;
-                const float norm = q_sq != nullptr && qs_stride ? most(u2) * most(k2) : __uint_as_float(0x7f800000u);
+                const float first = fminf(most[0] * most[3], most[1] * most[4]) * q_abs_max;
+                const float norm = q_sq != nullptr && qs_stride ? most[2] * most[5] : __uint_as_float(0x7f800000u);
                 exact = first < 16777216.0f * 0.999f || norm < 281474976710656.0f * 0.999f;      // 2^24, 2^48
                 small = first < 4194304.0f * 0.999f || norm < 17592186044416.0f * 0.999f;        // 2^22, 2^44
             }
@@ -844,9 +852,6 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
             }
             // The last round of accumulators has no user after this one, and its arrivals could reach the leader after its end.
             const int hand_back = (SPLIT > 1 ? n_chunks : (tiles_total - pair_id + num_pairs - 1) / num_pairs * my_chunks) - kAccBufs;
-            // the chunk scale of the next chunk is loaded a whole chunk ahead: a scattered load per lane (32 rows) that
-            // would otherwise stand in front of every fold
-            float qnext = qs_row[qs_stride ? min(c_lo, chunks - 1) : 0];
             for (int c = 0; c < n_chunks && ok; ++c, ++cc) {
                 const int b = cc % kAccBufs;
                 const uint32_t tph = static_cast<uint32_t>(cc / kAccBufs) & 1u;
