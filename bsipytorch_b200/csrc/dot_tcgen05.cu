@@ -193,6 +193,16 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, int32_t (&r)[32]) {
 }
 
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// The same with the registers of the load named, so that nothing touches them before: for loads under way beside other work.
+__device__ __forceinline__ void tmem_ld_wait_for(int32_t (&r)[32]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]),
+                   "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]), "+r"(r[16]), "+r"(r[17]),
+                   "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]),
+                   "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
+                 :
+                 : "memory");
+}
 
 template <int BN, bool DBG>
 __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_kernel(
@@ -467,7 +477,7 @@ int launch_tile(const CUtensorMap& ma, const CUtensorMap& mb, const float* qs, i
     return check_launch("dot_i8 tcgen05 launch");
 }
 
-template <int BN, bool DBG, typename OutT, bool REQ = false, int SPLIT = 1, bool ADD = false>
+template <int BN, bool DBG, typename OutT, bool REQ = false, int SPLIT = 1, bool ADD = false, bool ONE = false>
 int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo, const CUtensorMap& mt, int vector_store,
                 const float* qs, int64_t qs_stride, const float* bw0, const float* bias, int Q, int R, int chunks,
                 float scale_inv, void* out, int64_t ldo, int32_t* dbg, const ScatterDst& scatter,
@@ -497,10 +507,10 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap&
     int resident = 0;
     if (dev >= 0 && dev < 64) resident = max_clusters[dev];
     if (resident == 0) {
-        BSI_CUDA_TRY(cudaFuncSetAttribute(pair::dot_i8_tcgen05_pair_kernel<BN, DBG, OutT, REQ, SPLIT, ADD>,
+        BSI_CUDA_TRY(cudaFuncSetAttribute(pair::dot_i8_tcgen05_pair_kernel<BN, DBG, OutT, REQ, SPLIT, ADD, ONE>,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
         cfg.gridDim = dim3(2 * SPLIT * (sm_count() / (2 * SPLIT)), 1, 1);
-        BSI_CUDA_TRY(cudaOccupancyMaxActiveClusters(&resident, pair::dot_i8_tcgen05_pair_kernel<BN, DBG, OutT, REQ, SPLIT, ADD>, &cfg));
+        BSI_CUDA_TRY(cudaOccupancyMaxActiveClusters(&resident, pair::dot_i8_tcgen05_pair_kernel<BN, DBG, OutT, REQ, SPLIT, ADD, ONE>, &cfg));
         if (resident <= 0) return fail(BSI_ERR_CUDA, "dot_i8: no cluster of 2 CTAs fits on this device");
         if (dev >= 0 && dev < 64) max_clusters[dev] = resident;
     }
@@ -508,9 +518,14 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap&
         *max_clusters_out = resident;
         return BSI_OK;
     }
+    if constexpr (!ONE && !DBG && !REQ && SPLIT == 1) {
+        if (tiles_total <= resident && (vector_store & 4))
+            return launch_pair<BN, DBG, OutT, REQ, SPLIT, ADD, true>(ma, mb, mo, mt, vector_store, qs, qs_stride, bw0, bias, Q, R, chunks, scale_inv, out,
+                                                                     ldo, dbg, scatter, requant, fin, k_abs_sum, q_abs_max, q_sq, q_sq_stride, stream);
+    }
     const int clusters = SPLIT > 1 || tiles_total < resident ? tiles_total : resident;
     cfg.gridDim = dim3(2 * SPLIT * clusters, 1, 1);
-    BSI_CUDA_TRY(cudaLaunchKernelEx(&cfg, pair::dot_i8_tcgen05_pair_kernel<BN, DBG, OutT, REQ, SPLIT, ADD>, ma, mb, mo, mt, vector_store, qs,
+    BSI_CUDA_TRY(cudaLaunchKernelEx(&cfg, pair::dot_i8_tcgen05_pair_kernel<BN, DBG, OutT, REQ, SPLIT, ADD, ONE>, ma, mb, mo, mt, vector_store, qs,
                                     qs_stride, bw0, bias, Q, R, chunks, tiles_m, tiles_total, scale_inv, out, ldo, dbg, scatter, requant,
                                     fin, k_abs_sum, q_abs_max, q_sq, q_sq_stride));
     return check_launch("dot_i8 tcgen05 pair launch");

@@ -250,6 +250,12 @@ __device__ __forceinline__ uint4 finish16(const float* acc, const float* colw, c
                           finish2(scaled2(acc + 6, v.z, v.w, scale2), b.w, has_bias, relu, OutT()));
     }
 }
+// The same without bias and ReLU, float32.
+__device__ __forceinline__ uint4 finish16_plain(const float* acc, const float* colw, uint64_t scale2) {
+    const float4 w = *reinterpret_cast<const float4*>(colw);
+    const float2 a = scaled2(acc, w.x, w.y, scale2), c = scaled2(acc + 2, w.z, w.w, scale2);
+    return make_uint4(__float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(c.x), __float_as_uint(c.y));
+}
 // 16 bytes of finished values times a factor, rounded to the output type again.
 __device__ __forceinline__ uint4 times(uint4 o, float factor, float) {
     return make_uint4(__float_as_uint(__fmul_rn(__uint_as_float(o.x), factor)), __float_as_uint(__fmul_rn(__uint_as_float(o.y), factor)),
@@ -505,7 +511,106 @@ __device__ __forceinline__ void store_columns(const float (&acc)[kCols], uint8_t
     }
 }
 
-template <int BN, bool DBG, typename OutT, bool REQ = false, int SPLIT = 1, bool ADD = false>
+// Folds the last chunk in (accumulators at taddr in tensor memory) and stores the tile, where a pair has one tile (ONE): block
+// by block of 32 columns, the next one's accumulators on their way while one is finished, so that the first bulk store leaves 2000
+// cycles earlier than with everything folded and turned into floats first. What bounds the rest is shared memory (a block is
+// written once and read once) and the stores, 30 bytes a cycle and SM. kind: float32 chain, or int32 sums below 2^22 / 2^24 in
+// magnitude. Every block has its own place in the operand ring, which nothing reads any more. done(): called when the
+// accumulators have been read. Finished from a rolled loop over raw sums in shared memory, with a third of the code, the same
+// dots took 5 to 10 % longer: two more passes over shared memory.
+enum SumKind { kFloatSums = 0, kSmallInts = 1, kInts = 2 };
+template <typename OutT, int kCols, bool ADD, typename Done>
+__device__ __forceinline__ void fold_and_store(const float (&acc)[kCols], uint32_t taddr, float qscale, int kind, uint8_t* places, const float* colw,
+                                               const OutT* colb, const CUtensorMap& map_o, const CUtensorMap& map_t, int row_base, int Q,
+                                               int col, int R, float scale_inv, bool has_bias, bool relu, const Finishing& fin, Done done) {
+    const int lane = threadIdx.x & 31;
+    constexpr int E = static_cast<int>(sizeof(OutT));
+    constexpr int kPerChunk = 16 / E;
+    constexpr int kRoundCols = 128 / E;
+    constexpr int kFull = kCols / kRoundCols;
+    constexpr int kGroups = (kCols + 31) / 32;               // of 32 columns, the last one of 16 where that is left
+    const uint64_t scale2 = pack2(scale_inv, scale_inv);
+    const bool plain = E == 4 && !has_bias && !relu;
+    const int qmul = kind == kFloatSums ? 0 : __float2int_rn(qscale);
+    int32_t v[2][32];
+    if (kCols >= 32) tmem_ld32(taddr, v[0]); else tmem_ld16(taddr, v[0]);
+#pragma unroll
+    for (int g = 0; g < kGroups; ++g) {
+        const int c0 = g * 32, n = kCols - c0 < 32 ? kCols - c0 : 32;
+        int32_t (&now)[32] = v[g & 1];
+        tmem_ld_wait_for(now);
+        if (g + 1 < kGroups) {
+            if (kCols - c0 - 32 >= 32) tmem_ld32(taddr + c0 + 32, v[(g + 1) & 1]); else tmem_ld16(taddr + c0 + 32, v[(g + 1) & 1]);
+        } else {
+            tc_fence_before();
+            done();
+        }
+        float f[32];
+        if (kind == kSmallInts) {
+#pragma unroll
+            for (int e = 0; e < 32; ++e)
+                if (e < n) f[e] = int_to_float_exact(now[e] * qmul + __float_as_int(acc[c0 + e]));
+        } else if (kind == kInts) {
+#pragma unroll
+            for (int e = 0; e < 32; ++e)
+                if (e < n) f[e] = static_cast<float>(now[e] * qmul + __float_as_int(acc[c0 + e]));
+        } else {
+#pragma unroll
+            for (int e = 0; e < 32; ++e)
+                if (e < n) f[e] = __fmaf_rn(int_to_float_exact(now[e]), qscale, acc[c0 + e]);
+        }
+        const int round = c0 / kRoundCols, cg = round * kRoundCols;
+        const bool whole = round < kFull;
+        uint8_t* block = places + round * 4096;
+        uint8_t* dst = block + lane * (whole ? 128 : 64);
+        auto finish_pieces = [&](auto with) {
+#pragma unroll
+            for (int j = 0; j < 32; j += kPerChunk) {
+                if (j < n) {
+                    const int ch = (c0 + j - cg) / kPerChunk;
+                    *reinterpret_cast<uint4*>(dst + ((whole ? (ch ^ (lane & 7)) : (ch ^ ((lane >> 1) & 3))) << 4)) = with(j);
+                }
+            }
+        };
+        if (plain) finish_pieces([&](int j) { return finish16_plain(f + j, colw + c0 + j, scale2); });
+        else finish_pieces([&](int j) { return finish16<OutT>(f + j, colw + c0 + j, colb + c0 + j, scale2, has_bias, relu); });
+        if (c0 + n == cg + kRoundCols || c0 + n == kCols) {
+            const int nch = whole ? 8 : 4;
+            auto piece = [&](int row, int ch) { return reinterpret_cast<uint4*>(block + row * (nch * 16) + ((whole ? (ch ^ (row & 7)) : (ch ^ ((row >> 1) & 3))) << 4)); };
+            if (col + cg < fin.scaled_cols) {      // a second look at the lane's own row, so that other blocks pay one branch
+#pragma unroll 1
+                for (int ch = 0; ch < nch && col + cg + ch * kPerChunk < fin.scaled_cols; ++ch) *piece(lane, ch) = times(*piece(lane, ch), fin.factor, OutT());
+            }
+            if constexpr (ADD) {                   // likewise, neighbouring lanes on neighbouring pieces of a row, four loads at a time
+                const int tch = lane & (nch - 1), trow = lane / nch, step = 32 / nch;
+                const OutT* a = behind_wait(static_cast<const OutT*>(fin.add)) + static_cast<int64_t>(row_base + trow) * fin.ld_add + col + cg + tch * kPerChunk;
+                const bool in = col + cg + tch * kPerChunk < R;
+                __syncwarp();
+#pragma unroll 1
+                for (int i0 = 0; i0 < nch; i0 += 4) {
+                    uint4 add[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (in && row_base + trow + (i0 + e) * step < Q) add[e] = *reinterpret_cast<const uint4*>(a + (i0 + e) * step * fin.ld_add);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (in && row_base + trow + (i0 + e) * step < Q) {
+                            uint4* o = piece(trow + (i0 + e) * step, tch);
+                            *o = plus16(*o, add[e], OutT());
+                        }
+                }
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (row_base < Q && col + cg < R && elect_one())    // rows and columns beyond the matrix are clipped
+                tma_store_2d(whole ? &map_o : &map_t, smem_u32(block), col + cg, row_base);
+        }
+    }
+}
+
+// ONE: no more tiles than pairs, bulk stores. An instantiation of its own, because the store phase beside the other one made
+// kernels with several tiles per pair 2 to 10 % slower.
+template <int BN, bool DBG, typename OutT, bool REQ = false, int SPLIT = 1, bool ADD = false, bool ONE = false>
 __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
     const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
     const __grid_constant__ CUtensorMap map_o, const __grid_constant__ CUtensorMap map_t,   // out in boxes of 32 rows x 128 / 64 bytes
@@ -515,6 +620,7 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
     void* __restrict__ out, int64_t ldo, int32_t* __restrict__ dbg_iacc, const ScatterDst scatter,
     const RequantDst requant, const Finishing fin, const float* __restrict__ k_abs_sum, float q_abs_max,
     const float* __restrict__ q_sq, int64_t q_sq_stride) {
+    static_assert(!ONE || (!DBG && !REQ && SPLIT == 1), "one tile per pair: plain dots and layers");
     using C = Cfg<BN, OutT, REQ, SPLIT>;
     constexpr int kStages = C::kStages;
     constexpr int kCols = BN / 2;              // accumulator columns per epilogue warp: a multiple of 16
@@ -852,7 +958,8 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
             }
             // The last round of accumulators has no user after this one, and its arrivals could reach the leader after its end.
             const int hand_back = (SPLIT > 1 ? n_chunks : (tiles_total - pair_id + num_pairs - 1) / num_pairs * my_chunks) - kAccBufs;
-            for (int c = 0; c < n_chunks && ok; ++c, ++cc) {
+            const int here = ONE ? n_chunks - 1 : n_chunks;      // the store phase has the last one
+            for (int c = 0; c < here && ok; ++c, ++cc) {
                 const int b = cc % kAccBufs;
                 const uint32_t tph = static_cast<uint32_t>(cc / kAccBufs) & 1u;
                 const float qscale = qnext;
@@ -917,7 +1024,7 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                     }
                 }
             }
-            if constexpr (!REQ && SPLIT == 1) {
+            if constexpr (!REQ && SPLIT == 1 && !ONE) {
                 __syncwarp();
                 if (tile + num_pairs >= tiles_total) cluster_arrive();
             }
@@ -996,6 +1103,22 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
                 }
                 if (!whole_tile) continue;
             }
+            const int row_base = tm * 256 + static_cast<int>(rank) * BM + quad * 32;
+            if constexpr (ONE) {
+                const int b = cc % kAccBufs;
+                ok = __all_sync(0xffffffffu, ok && wait_or_abort(tfull_bar(b), static_cast<uint32_t>(cc / kAccBufs) & 1u, actx, 4));
+                if (!ok) {
+                    cluster_arrive();
+                    break;
+                }
+                tc_fence_after();
+                if (exact && lane == 0) atomicAdd(&g_exact_int_tiles, 1ull);
+                fold_and_store<OutT, kCols, ADD>(acc, tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(b * C::kAccStride + col0),
+                                                 qnext, !exact ? kFloatSums : small ? kSmallInts : kInts, smem + ew * kBlocks<OutT, kCols>() * 4096,
+                                                 colw + col0, colb + col0, map_o, map_t, row_base, Q, n0 + col0, R, scale_inv, has_bias, relu, fin,
+                                                 [] { __syncwarp(); cluster_arrive(); });
+                break;
+            }
             if (!ok) continue;
             if (exact) {
                 // the int32 sums (below 2^24 in magnitude) as floats: what the float32 chain would hold. Below 2^22 by an
@@ -1011,7 +1134,6 @@ __global__ void __launch_bounds__(kThreads, 1) dot_i8_tcgen05_pair_kernel(
             }
 
             // ---- tile result: out = (acc * bw0[r]) * scale_inv ----
-            const int row_base = tm * 256 + static_cast<int>(rank) * BM + quad * 32;
             if constexpr (REQ) {
                 static_assert(BN == 256 && !DBG && sizeof(OutT) == 2, "re-quantisation: 256-wide tiles, 16-bit layer type");
                 {
