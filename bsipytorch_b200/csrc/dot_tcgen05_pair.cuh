@@ -417,6 +417,19 @@ __device__ __forceinline__ void store_columns(const float (&acc)[kCols], uint8_t
                 __syncwarp();
             }
             uint8_t* dst = block + lane * (nch * 16);
+            // The matrix to add, on its way while the block is finished, neighbouring lanes on neighbouring pieces of a row: loaded
+            // behind it, a row per lane, it made the store phase of a 256 x 256 tile twice as long.
+            uint4 add[8];
+            if constexpr (ADD) {
+                const OutT* a = behind_wait(static_cast<const OutT*>(fin.add)) + col + cg + (lane & (nch - 1)) * kPerChunk;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int r = row_base + i * (32 / nch) + lane / nch;
+                    add[i] = make_uint4(0u, 0u, 0u, 0u);
+                    if (i < nch && r < Q && col + cg + (lane & (nch - 1)) * kPerChunk < R)
+                        add[i] = *reinterpret_cast<const uint4*>(a + static_cast<int64_t>(r) * fin.ld_add);
+                }
+            }
 #pragma unroll
             for (int ch = 0; ch < 8; ++ch) {
                 if (ch < nch) {
@@ -433,22 +446,15 @@ __device__ __forceinline__ void store_columns(const float (&acc)[kCols], uint8_t
                     *o = times(*o, fin.factor, OutT());
                 }
             }
-            if (ADD && row_base + lane < Q) {      // likewise, a few loads at a time: the sums need the registers
-                constexpr int kBatch = kCols <= 64 ? 4 : 2;
-                const OutT* a = behind_wait(static_cast<const OutT*>(fin.add)) + static_cast<int64_t>(row_base + lane) * fin.ld_add + col + cg;
-#pragma unroll 1
-                for (int c0 = 0; c0 < nch && cg + c0 * kPerChunk < kCols; c0 += kBatch) {
-                    uint4 add[kBatch];
+            if constexpr (ADD) {
+                __syncwarp();
 #pragma unroll
-                    for (int e = 0; e < kBatch; ++e)
-                        if (col + cg + (c0 + e) * kPerChunk < R) add[e] = *reinterpret_cast<const uint4*>(a + (c0 + e) * kPerChunk);
-#pragma unroll
-                    for (int e = 0; e < kBatch; ++e) {
-                        const int ch = c0 + e;
-                        uint4* o = reinterpret_cast<uint4*>(dst + ((whole ? (ch ^ (lane & 7)) : (ch ^ ((lane >> 1) & 3))) << 4));
-                        if (col + cg + ch * kPerChunk < R) *o = plus16(*o, add[e], OutT());
+                for (int i = 0; i < 8; ++i)
+                    if (i < nch) {
+                        uint4* o = reinterpret_cast<uint4*>(block + (i * (32 / nch) + lane / nch) * (nch * 16) +
+                                                            (((lane & (nch - 1)) ^ (whole ? (i * 4 + (lane >> 3)) & 7 : ((i * 8 + (lane >> 2)) >> 1) & 3)) << 4));
+                        *o = plus16(*o, add[i], OutT());     // beyond the matrix: clipped or not stored
                     }
-                }
             }
             if (bulk) {
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -545,6 +551,26 @@ __device__ __forceinline__ void fold_and_store(const float (&acc)[kCols], uint32
             tc_fence_before();
             done();
         }
+        const int round = c0 / kRoundCols, cg = round * kRoundCols;
+        const bool whole = round < kFull;
+        const int nch = whole ? 8 : 4;
+        // as in store_columns; four loads of a wide tile's block, for the sake of registers, wait until the block is finished
+        constexpr int kAhead = kCols <= 64 ? 8 : 4;
+        const int tch = lane & (nch - 1), trow = lane / nch, step = 32 / nch;
+        const bool in = col + cg + tch * kPerChunk < R;
+        auto fetch = [&](int i) {
+            const int r = row_base + trow + i * step;
+            if (!in || r >= Q) return make_uint4(0u, 0u, 0u, 0u);
+            return *reinterpret_cast<const uint4*>(behind_wait(static_cast<const OutT*>(fin.add)) + static_cast<int64_t>(r) * fin.ld_add + col + cg + tch * kPerChunk);
+        };
+        uint4 add[kAhead];
+        if constexpr (ADD) {
+            if (c0 == cg) {
+#pragma unroll
+                for (int i = 0; i < kAhead; ++i)
+                    if (i < nch) add[i] = fetch(i);
+            }
+        }
         float f[32];
         if (kind == kSmallInts) {
 #pragma unroll
@@ -559,8 +585,6 @@ __device__ __forceinline__ void fold_and_store(const float (&acc)[kCols], uint32
             for (int e = 0; e < 32; ++e)
                 if (e < n) f[e] = __fmaf_rn(int_to_float_exact(now[e]), qscale, acc[c0 + e]);
         }
-        const int round = c0 / kRoundCols, cg = round * kRoundCols;
-        const bool whole = round < kFull;
         uint8_t* block = places + round * 4096;
         uint8_t* dst = block + lane * (whole ? 128 : 64);
         auto finish_pieces = [&](auto with) {
@@ -575,30 +599,16 @@ __device__ __forceinline__ void fold_and_store(const float (&acc)[kCols], uint32
         if (plain) finish_pieces([&](int j) { return finish16_plain(f + j, colw + c0 + j, scale2); });
         else finish_pieces([&](int j) { return finish16<OutT>(f + j, colw + c0 + j, colb + c0 + j, scale2, has_bias, relu); });
         if (c0 + n == cg + kRoundCols || c0 + n == kCols) {
-            const int nch = whole ? 8 : 4;
             auto piece = [&](int row, int ch) { return reinterpret_cast<uint4*>(block + row * (nch * 16) + ((whole ? (ch ^ (row & 7)) : (ch ^ ((row >> 1) & 3))) << 4)); };
             if (col + cg < fin.scaled_cols) {      // a second look at the lane's own row, so that other blocks pay one branch
 #pragma unroll 1
                 for (int ch = 0; ch < nch && col + cg + ch * kPerChunk < fin.scaled_cols; ++ch) *piece(lane, ch) = times(*piece(lane, ch), fin.factor, OutT());
             }
-            if constexpr (ADD) {                   // likewise, neighbouring lanes on neighbouring pieces of a row, four loads at a time
-                const int tch = lane & (nch - 1), trow = lane / nch, step = 32 / nch;
-                const OutT* a = behind_wait(static_cast<const OutT*>(fin.add)) + static_cast<int64_t>(row_base + trow) * fin.ld_add + col + cg + tch * kPerChunk;
-                const bool in = col + cg + tch * kPerChunk < R;
+            if constexpr (ADD) {
                 __syncwarp();
-#pragma unroll 1
-                for (int i0 = 0; i0 < nch; i0 += 4) {
-                    uint4 add[4];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        if (in && row_base + trow + (i0 + e) * step < Q) add[e] = *reinterpret_cast<const uint4*>(a + (i0 + e) * step * fin.ld_add);
-#pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        if (in && row_base + trow + (i0 + e) * step < Q) {
-                            uint4* o = piece(trow + (i0 + e) * step, tch);
-                            *o = plus16(*o, add[e], OutT());
-                        }
-                }
+                for (int i = 0; i < 8; ++i)
+                    if (i < nch) *piece(trow + i * step, tch) = plus16(*piece(trow + i * step, tch), i < kAhead ? add[i < kAhead ? i : 0] : fetch(i), OutT());
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
