@@ -1191,7 +1191,16 @@ py::object opt_layer_forward(const torch::Tensor& x, const py::tuple& norms, con
 // scales [rows, d/256] float32, contiguous. This is the first half of bsi_linear_forward, split off so
 // that a tensor-parallel layer can pack its own column block straight into the buffer the ranks
 // exchange. d must be a multiple of 256.
-void pack_queries_into(torch::Tensor x2d, torch::Tensor q8, torch::Tensor scales, int decimalPlaces) {
+// sq_norms [rows, d/256] float32, where given: the chunks' sums of squares, with which a dot proves its integer route exact.
+const float* chunk_norms(const c10::optional<torch::Tensor>& norms, const torch::Tensor& q8, int64_t rows, int64_t chunks) {
+    if (!norms.has_value() || !norms->defined()) return nullptr;
+    TORCH_CHECK(norms->is_cuda() && norms->scalar_type() == at::kFloat && norms->is_contiguous() && norms->numel() == rows * chunks,
+                "sq_norms must be contiguous float32 [rows, d/256]");
+    same_device(q8, *norms, "packed activations and their sums of squares");
+    return norms->data_ptr<float>();
+}
+
+void pack_queries_into(torch::Tensor x2d, torch::Tensor q8, torch::Tensor scales, int decimalPlaces, c10::optional<torch::Tensor> sq_norms) {
     const Env env;
     require_fixed_queries(env, "pack_queries_into");
     TORCH_CHECK(x2d.dim() == 2 && x2d.is_cuda(), "x must be a 2D CUDA tensor");
@@ -1210,11 +1219,12 @@ void pack_queries_into(torch::Tensor x2d, torch::Tensor q8, torch::Tensor scales
     TORCH_CHECK(d % 256 == 0, "d must be a multiple of 256");
     TORCH_CHECK(q8.size(0) == rows && q8.size(1) >= d, "q8 shape mismatch");
     TORCH_CHECK(scales.numel() == rows * (d / 256), "scales shape mismatch");
+    float* norms = const_cast<float*>(chunk_norms(sq_norms, q8, rows, d / 256));
     if (rows == 0 || d == 0) return;
-    check_status(bsi_b200_quantize_pack(x.data_ptr(), dtype_code(x), rows, d, x.stride(0), decimalPlaces,
-                                        env.bits_queries(), 1, nullptr, scales.data_ptr<float>(), nullptr,
-                                        q8.data_ptr<int8_t>(), q8.stride(0), current_stream()),
-                 "bsi_b200_quantize_pack");
+    check_status(bsi_b200_quantize_pack_norms(x.data_ptr(), dtype_code(x), rows, d, x.stride(0), decimalPlaces,
+                                              env.bits_queries(), 1, 0.0f, nullptr, scales.data_ptr<float>(), nullptr,
+                                              q8.data_ptr<int8_t>(), q8.stride(0), norms, current_stream()),
+                 "bsi_b200_quantize_pack_norms");
 }
 
 // Second half of bsi_linear_forward: the dot of already packed activations with a key set, cast to
@@ -1222,7 +1232,7 @@ void pack_queries_into(torch::Tensor x2d, torch::Tensor q8, torch::Tensor scales
 // [Q, d/256] float32 contiguous.
 at::Tensor linear_from_packed(torch::Tensor q8, torch::Tensor scales, py::capsule keyset_cuda_cap,
                               c10::optional<torch::Tensor> bias, int decimalPlaces, py::object out_dtype, bool relu,
-                              int64_t scaled_columns, double factor) {
+                              int64_t scaled_columns, double factor, c10::optional<torch::Tensor> sq_norms, c10::optional<torch::Tensor> add) {
     auto* keys = from_capsule<PrebuiltBSIKeysCUDA>(keyset_cuda_cap, "PrebuiltBSIKeysCUDA");
     TORCH_CHECK(q8.dim() == 2 && q8.is_cuda() && q8.scalar_type() == at::kChar && q8.stride(1) == 1, "q8 must be int8 [Q, d]");
     TORCH_CHECK(scales.is_cuda() && scales.scalar_type() == at::kFloat && scales.is_contiguous(), "scales must be contiguous float32");
@@ -1249,16 +1259,25 @@ at::Tensor linear_from_packed(torch::Tensor q8, torch::Tensor scales, py::capsul
     }
     const int code = yt == at::kHalf ? BSI_DTYPE_F16 : (yt == at::kBFloat16 ? BSI_DTYPE_BF16 : BSI_DTYPE_F32);
     const Env env;
-    const bsi_dot_bounds bounds = dot_bounds(*keys, env.bits_queries(), nullptr);
-    check_status(bsi_b200_linear_i8_engine(q8.data_ptr<int8_t>(), q8.stride(0), scales.data_ptr<float>(), chunks,
-                                           keys->b.q8.data_ptr<int8_t>(), keys->b.q8.size(1),
-                                           keys->b.scales.data_ptr<float>(), bptr, Q, R, chunks,
-                                           static_cast<float>(scale_inv), y.data_ptr(), R, code,
-                                           relu ? BSI_ACT_RELU : BSI_ACT_NONE, scaled_columns, static_cast<float>(factor), &bounds,
-                                           (env.engine_free() ? BSI_ENGINE_AUTO : BSI_ENGINE_TCGEN05) |
-                                               (Q <= kFewRows ? keys->complete() : 0),
-                                           current_stream()),
-                 "bsi_b200_linear_i8_engine");
+    bsi_dot_bounds bounds = dot_bounds(*keys, env.bits_queries(), nullptr);
+    bounds.query_sq = chunk_norms(sq_norms, q8, Q, chunks);
+    bounds.query_sq_stride = chunks;
+    const void* addend = nullptr;
+    if (add.has_value() && add->defined()) {
+        TORCH_CHECK(add->is_cuda() && add->scalar_type() == yt && add->dim() == 2 && add->size(0) == Q && add->size(1) == R && add->is_contiguous(),
+                    "add must be a contiguous [Q, R] matrix of the output's type");
+        same_device(q8, *add, "packed activations and the matrix to add");
+        addend = add->data_ptr();
+    }
+    check_status(bsi_b200_linear_i8_add(q8.data_ptr<int8_t>(), q8.stride(0), scales.data_ptr<float>(), chunks,
+                                        keys->b.q8.data_ptr<int8_t>(), keys->b.q8.size(1),
+                                        keys->b.scales.data_ptr<float>(), bptr, Q, R, chunks,
+                                        static_cast<float>(scale_inv), y.data_ptr(), R, code,
+                                        relu ? BSI_ACT_RELU : BSI_ACT_NONE, scaled_columns, static_cast<float>(factor), addend, R, &bounds,
+                                        (env.engine_free() ? BSI_ENGINE_AUTO : BSI_ENGINE_TCGEN05) |
+                                            (Q <= kFewRows ? keys->complete() : 0),
+                                        current_stream()),
+                 "bsi_b200_linear_i8_add");
     return y;
 }
 
@@ -1363,7 +1382,7 @@ void linear_from_packed_scatter(torch::Tensor q8, torch::Tensor scales, py::caps
 void linear_from_packed_requant(torch::Tensor q8, torch::Tensor scales, py::capsule keyset_cuda_cap,
                                 c10::optional<torch::Tensor> bias, int decimalPlaces, py::object layer_dtype, bool relu,
                                 std::vector<int64_t> q8_ptrs, int64_t ld8, std::vector<int64_t> scale_ptrs,
-                                int64_t scale_ld) {
+                                int64_t scale_ld, c10::optional<torch::Tensor> sq_norms) {
     const Env env;
     require_fixed_queries(env, "linear_from_packed_requant");
     env.check_clip("linear_from_packed_requant");
@@ -1395,6 +1414,15 @@ void linear_from_packed_requant(torch::Tensor q8, torch::Tensor scales, py::caps
     for (int64_t p : q8_ptrs) qd.push_back(reinterpret_cast<int8_t*>(static_cast<intptr_t>(p)));
     for (int64_t p : scale_ptrs) sd.push_back(reinterpret_cast<float*>(static_cast<intptr_t>(p)));
     keys->register_bounds(Env().bits_queries());
+    // the sums of squares are registered for the time of the call, which has no other way to take them
+    struct Registered {
+        const int8_t* a8;
+        ~Registered() { if (a8 != nullptr) bsi_b200_unregister_query_bounds(a8); }
+    } registered{nullptr};
+    if (const float* norms = chunk_norms(sq_norms, q8, Q, chunks)) {
+        check_status(bsi_b200_register_query_bounds(q8.data_ptr<int8_t>(), norms, chunks), "bsi_b200_register_query_bounds");
+        registered.a8 = q8.data_ptr<int8_t>();
+    }
     check_status(bsi_b200_linear_i8_requant(q8.data_ptr<int8_t>(), q8.stride(0), scales.data_ptr<float>(), chunks,
                                             keys->b.q8.data_ptr<int8_t>(), keys->b.q8.size(1),
                                             keys->b.scales.data_ptr<float>(), bptr, Q, R, chunks,
@@ -1726,12 +1754,13 @@ PYBIND11_MODULE(bsi_ops, m) {
           py::arg("joint") = py::none(),
           "One OPT decoder layer over BSI linears; None where the environment asks for another form of the layers");
     m.def("pack_queries_into", &pack_queries_into, py::arg("x2d"), py::arg("q8"), py::arg("scales"),
-          py::arg("decimal_places"), "Pack activations into caller-owned int8 / chunk-scale tensors");
+          py::arg("decimal_places"), py::arg("sq_norms") = py::none(),
+          "Pack activations into caller-owned int8 / chunk-scale tensors; sq_norms: their chunks' sums of squares as well");
     m.def("linear_from_packed", &linear_from_packed, py::arg("q8"), py::arg("scales"), py::arg("keyset_cuda_cap"),
           py::arg("bias"), py::arg("decimal_places"), py::arg("out_dtype"), py::arg("relu") = false,
-          py::arg("scaled_columns") = 0, py::arg("factor") = 1.0,
+          py::arg("scaled_columns") = 0, py::arg("factor") = 1.0, py::arg("sq_norms") = py::none(), py::arg("add") = py::none(),
           "Dot of packed activations with a key set, cast + bias (+ ReLU) fused; the first scaled_columns output columns (a "
-          "multiple of 8) times factor");
+          "multiple of 8) times factor; sq_norms: the activations' sums of squares (pack_queries_into); add: a matrix added at the end");
     m.def("peer_alloc", &peer_alloc, py::arg("nbytes"), "Zero-filled device buffer other local processes can map: (uint8 tensor, handle bytes)");
     m.def("peer_open", &peer_open, py::arg("handle"), "Map a peer's buffer; returns its device address here");
     m.def("peer_close", &peer_close, py::arg("ptr"));
@@ -1739,7 +1768,7 @@ PYBIND11_MODULE(bsi_ops, m) {
           "Bounded flag barrier over the ranks, enqueued on the current stream");
     m.def("linear_from_packed_requant", &linear_from_packed_requant, py::arg("q8"), py::arg("scales"),
           py::arg("keyset_cuda_cap"), py::arg("bias"), py::arg("decimal_places"), py::arg("layer_dtype"), py::arg("relu"),
-          py::arg("q8_ptrs"), py::arg("ld8"), py::arg("scale_ptrs"), py::arg("scale_ld"));
+          py::arg("q8_ptrs"), py::arg("ld8"), py::arg("scale_ptrs"), py::arg("scale_ld"), py::arg("sq_norms") = py::none());
     m.def("add_layernorm_pack", &add_layernorm_pack, py::arg("x"), py::arg("delta"), py::arg("weight"), py::arg("bias"),
           py::arg("eps"), py::arg("q8_ptrs"), py::arg("ld8"), py::arg("scale_ptrs"), py::arg("scale_ld"), py::arg("decimal_places"));
     m.def("pack_queries_multi", &pack_queries_multi, py::arg("x2d"), py::arg("q8_ptrs"), py::arg("ld8"),

@@ -55,25 +55,26 @@ class BsiDeviceOps:
         cap, mem, num_keys, d, w = self.m.build_bsi_keys_cuda(weight.float(), self.dp, self.threshold)
         return cap
 
-    def pack_into(self, x2d, q8, scales):
-        self.m.pack_queries_into(x2d, q8, scales, self.dp)
+    def pack_into(self, x2d, q8, scales, norms=None):
+        self.m.pack_queries_into(x2d, q8, scales, self.dp, norms)
 
-    def linear(self, q8, scales, keys, bias, out_dtype, relu=False):
-        return self.m.linear_from_packed(q8, scales, keys, bias, self.dp, out_dtype, relu)
+    def linear(self, q8, scales, keys, bias, out_dtype, relu=False, norms=None, add=None):
+        """norms: the packed activations' chunk sums of squares; add: a matrix added to the output in the epilogue."""
+        return self.m.linear_from_packed(q8, scales, keys, bias, self.dp, out_dtype, relu, 0, 1.0, norms, add)
 
-    def linear_scaled(self, q8, scales, keys, bias, out_dtype, columns, factor):
+    def linear_scaled(self, q8, scales, keys, bias, out_dtype, columns, factor, norms=None):
         """linear whose first `columns` output columns (a multiple of 8) are multiplied by `factor` in the epilogue."""
-        return self.m.linear_from_packed(q8, scales, keys, bias, self.dp, out_dtype, False, columns, factor)
+        return self.m.linear_from_packed(q8, scales, keys, bias, self.dp, out_dtype, False, columns, factor, norms)
 
     def add_ln_pack(self, x, delta, ln, q8_ptrs, ld8, scale_ptrs, scale_ld):
         """x + delta (delta may be None), LayerNorm `ln` of the sum, packed to the given addresses; returns the sum."""
         return self.m.add_layernorm_pack(x, delta, ln.weight, ln.bias, ln.eps, q8_ptrs, ld8, scale_ptrs, scale_ld, self.dp)
 
-    def linear_requant(self, q8, scales, keys, bias, layer_dtype, relu, q8_ptrs, ld8, scale_ptrs, scale_ld):
+    def linear_requant(self, q8, scales, keys, bias, layer_dtype, relu, q8_ptrs, ld8, scale_ptrs, scale_ld, norms=None):
         """Linear whose output is re-quantised for the next linear inside its epilogue and stored to the given
         addresses (needs a 16-bit layer type and a multiple of 256 output features)."""
         self.m.linear_from_packed_requant(q8, scales, keys, bias, self.dp, layer_dtype, relu, q8_ptrs, ld8,
-                                          scale_ptrs, scale_ld)
+                                          scale_ptrs, scale_ld, norms)
 
 
 def _align(n: int, a: int = 256) -> int:
@@ -245,12 +246,12 @@ class TPDecoderLayer(nn.Module):
         return recv.view(G, Q // G, Rl).permute(1, 0, 2).reshape(Q // G, G * Rl)
 
     # -- forward ---------------------------------------------------------------------------------
-    def _qkv(self, q8, sc):
+    def _qkv(self, q8, sc, norms=None):
         """[Q, 3 * H/G], the query block scaled in the model's type (HuggingFace's OPT scales it before an attention with
         unit scaling): in the epilogue on the extension, where the separate pass over a strided block cost 42 us."""
         Hl, factor = self.h_hi - self.h_lo, self.head_dim ** -0.5
         if isinstance(self.ops, BsiDeviceOps) and Hl % 8 == 0:
-            return self.ops.linear_scaled(q8, sc, self.keys_qkv, self.bias_qkv, self.dtype, Hl, factor)
+            return self.ops.linear_scaled(q8, sc, self.keys_qkv, self.bias_qkv, self.dtype, Hl, factor, norms)
         qkv = self.ops.linear(q8, sc, self.keys_qkv, self.bias_qkv, self.dtype)
         qkv[:, :Hl] *= factor
         return qkv
@@ -304,11 +305,41 @@ class TPDecoderLayer(nn.Module):
         to_owner(px.C2_q8, px.C2_sc, self.keys_fc2, self.bias_fc2)
         return x_loc, px.T
 
+    def forward_whole(self, x, B, T):
+        """The layer on one rank with the CUDA extension: the packers leave the chunks' sums of squares for the dots' integer
+        route, and both residual sums are taken in the epilogue of the linear in front of them (one rounding in the layer's
+        type, as x + delta does)."""
+        Q, ops, dt, dev = B * T, self.ops, self.dtype, x.device
+
+        def pack(h):
+            D = h.shape[1]
+            q8 = torch.empty(Q, D, dtype=torch.int8, device=dev)
+            sc, sq = torch.empty(2, Q, D // 256, dtype=torch.float32, device=dev)
+            ops.pack_into(h, q8, sc, sq)
+            return q8, sc, sq
+
+        q8, sc, sq = pack(self.self_attn_layer_norm(x))
+        attn = self._attention(self._qkv(q8, sc, sq), B, T)
+        q8, sc, sq = pack(attn)
+        x = ops.linear(q8, sc, self.keys_out, self.bias_out, dt, norms=sq, add=x)
+        q8, sc, sq = pack(self.final_layer_norm(x))
+        if self.fuse_requant:
+            Fd = self.cfg.ffn_dim
+            q8f = torch.empty(Q, Fd, dtype=torch.int8, device=dev)
+            scf = torch.empty(Q, Fd // 256, dtype=torch.float32, device=dev)
+            ops.linear_requant(q8, sc, self.keys_fc1, self.bias_fc1, dt, True, [q8f.data_ptr()], Fd, [scf.data_ptr()], Fd // 256, sq)
+            q8, sc, sq = q8f, scf, None
+        else:
+            q8, sc, sq = pack(ops.linear(q8, sc, self.keys_fc1, self.bias_fc1, dt, relu=True, norms=sq))
+        return ops.linear(q8, sc, self.keys_fc2, self.bias_fc2, dt, norms=sq, add=x), None
+
     def forward(self, x_loc, delta, B, T, px=None):
         """(x, delta) -> (x, delta): `delta` is the fc2 output of the previous layer for the own tokens, not yet
-        added to the residual stream `x` (None at the first layer)."""
+        added to the residual stream `x` (None at the first layer, and where the epilogue has added it)."""
         if px is not None:
             return self.forward_peer(x_loc, delta, B, T, px)
+        if self.world == 1 and not self.fuse_ln and isinstance(self.ops, BsiDeviceOps):
+            return self.forward_whole(x_loc if delta is None else x_loc + delta, B, T)
         Q = B * T
         ops, dt = self.ops, self.dtype
         H = self.cfg.hidden_size
@@ -381,7 +412,7 @@ class TPOPTForCausalLM(nn.Module):
         x, delta = self.embed_tokens(ids) + self.embed_positions(pos), None
         for layer in self.layers:
             x, delta = layer(x, delta, b, T, px)
-        return self.final_layer_norm(x + delta)
+        return self.final_layer_norm(x if delta is None else x + delta)
 
     def _micro(self, B, T):
         """Number of micro-batches for a [B, T] input: with peer exchange the batch is split into groups of
