@@ -972,6 +972,138 @@ __global__ void __launch_bounds__(256, CPW * RawLane<T>::kVecs <= 8 ? 4 : 2) qua
     }
 }
 
+// The same for what a key build asks for, every output. The kernel above was bound by instruction issue (266 a chunk of 256
+// elements, 77 % of the slots), so nothing is decided per chunk here that is known before: WPR warps on a row and CPW chunks each
+// are constants (all addresses a base and an immediate), the clamp and the 64-bit path are chosen once per row, and the outputs are
+// there. The largest magnitude comes from signed and unsigned maxima of the patterns, three at a time, without masking each. 174
+// instructions a chunk, 16384 x 4096 float32: 82.8 -> 64.3 us (385 MB, 93 % of the copy rate), 50000 x 768 57.7 -> 40.1.
+// kWhole: rows of whole chunks on 16-byte vectors; else the last chunk's lanes look at what is left.
+template <typename T, int CPW, int WPR, bool kWhole>
+__global__ void __launch_bounds__(256, CPW * RawLane<T>::kVecs <= 8 ? 4 : 2) quantize_pack_row_build_kernel(
+    const T* __restrict__ x, uint32_t rows, int64_t D, uint32_t ldx, int vec_ok, double dec_scale, uint32_t dec_mult, int bits, int chunks, uint32_t W,
+    u64* __restrict__ words, float* __restrict__ scales, int32_t* __restrict__ shifts, int8_t* __restrict__ q8, uint32_t ld8,
+    float* __restrict__ slice_weights, float* __restrict__ bounds) {
+    __shared__ uint32_t wmax[8];
+    __shared__ int wsum[3][8];
+    const int lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
+    const int sub = warp & (WPR - 1);
+    const uint32_t row = blockIdx.x * (8u / WPR) + static_cast<uint32_t>(warp / WPR);
+    const bool row_ok = row < rows;
+    const int mine = row_ok ? (chunks - sub + WPR - 1) / WPR : 0;        // chunks sub, sub + WPR, .. of the row
+    const T* xr = x + static_cast<size_t>(row_ok ? row : 0u) * ldx;
+    const T* src = xr + sub * 256 + lane * 8;
+
+    RawLane<T> raw[CPW];
+#pragma unroll
+    for (int i = 0; i < CPW; ++i) {
+        if (kWhole && i < mine) {
+            raw[i].load(src + i * WPR * 256);
+        } else if (!kWhole && i < mine) {
+            const int64_t left = D - (sub + i * WPR) * 256 - lane * 8;
+            if (vec_ok && left >= 8) raw[i].load(src + i * WPR * 256);
+            else raw[i].load_tail(left > 0 ? src + i * WPR * 256 : xr, left);
+        } else {
+#pragma unroll
+            for (int e = 0; e < RawLane<T>::kVecs; ++e) raw[i].v[e] = make_uint4(0u, 0u, 0u, 0u);
+        }
+    }
+    uint32_t amax_bits = 0;
+    if constexpr (sizeof(T) == 4) {
+        int positive = 0;           // positive patterns order as signed, negative ones above them as unsigned numbers
+        uint32_t negative = 0;
+#pragma unroll
+        for (int i = 0; i < CPW; ++i) {
+#pragma unroll
+            for (int e = 0; e < RawLane<T>::kVecs; ++e) {
+                const uint4& a = raw[i].v[e];
+                positive = __vimax3_s32(__vimax3_s32(positive, static_cast<int>(a.x), static_cast<int>(a.y)), static_cast<int>(a.z), static_cast<int>(a.w));
+                negative = __vimax3_u32(__vimax3_u32(negative, a.x, a.y), a.z, a.w);
+            }
+        }
+        amax_bits = max(static_cast<uint32_t>(positive), (negative >> 31) != 0u ? negative & 0x7fffffffu : 0u);
+    } else {
+#pragma unroll
+        for (int i = 0; i < CPW; ++i) amax_bits = max(amax_bits, raw[i].abs_max());
+    }
+    amax_bits = __reduce_max_sync(0xffffffffu, amax_bits);
+    if constexpr (WPR > 1) {
+        if (lane == 0) wmax[warp] = amax_bits;
+        __syncthreads();
+        const int group = warp & ~(WPR - 1);
+#pragma unroll
+        for (int i = 0; i < WPR; ++i) amax_bits = max(amax_bits, wmax[group + i]);
+    }
+    const float mult = static_cast<float>(dec_mult);
+    int shift = fast_group_shift(RawLane<T>::abs_value(amax_bits), mult, bits);
+    const bool fast = shift >= 0;
+    const bool clamp = fast && needs_clamp(RawLane<T>::abs_value(amax_bits), mult, shift, bits);
+    if (!fast) shift = generic_row_shift<T>(xr, chunks, D, dec_scale, dec_mult, bits, vec_ok, lane);
+
+    int asum = 0, amax_chunk = 0, qsum = 0;
+    const int s0 = first_slice(lane);
+    const bool first_there = s0 < bits, second_there = s0 + 1 < bits;
+    int8_t* q8_out = q8 + static_cast<size_t>(row_ok ? row : 0u) * ld8 + sub * 256 + lane * 8;
+    // half word (lane / 4) % 2 of the lane's word in slice s0, and in the slice after it
+    uint32_t* w_out = reinterpret_cast<uint32_t*>(words + (static_cast<size_t>(row_ok ? row : 0u) * bits + s0) * W + sub * 4 + (lane >> 3)) + ((lane >> 2) & 1);
+    uint32_t* w_out1 = w_out + 2u * W;
+    const int words_left = static_cast<int>(W) - sub * 4 - (lane >> 3);      // the lane's word exists while this is positive
+    auto emit = [&](u64 packed, int i) {
+        *reinterpret_cast<u64*>(q8_out + i * WPR * 256) = packed;
+        uint32_t w0, w1;
+        slice_pieces(packed, lane, w0, w1);
+        if (kWhole || words_left > i * WPR * 4) {
+            if (first_there) w_out[i * WPR * 8] = w0;
+            if (second_there) w_out1[i * WPR * 8] = w1;
+        }
+        int a;
+        chunk_sums(packed, a, qsum);
+        asum += a;
+        amax_chunk = max(amax_chunk, a);
+    };
+    if (fast && !clamp) {
+#pragma unroll
+        for (int i = 0; i < CPW; ++i)
+            if (i < mine) emit(raw[i].template quantise<false>(mult, shift, bits), i);
+    } else if (fast) {
+#pragma unroll
+        for (int i = 0; i < CPW; ++i)
+            if (i < mine) emit(raw[i].template quantise<true>(mult, shift, bits), i);
+    } else {
+#pragma unroll 1
+        for (int i = 0; i < mine; ++i)
+            emit(generic_row_chunk<T>(xr, sub + i * WPR, D, dec_scale, dec_mult, bits, vec_ok, lane, shift), i);
+    }
+    qsum = __reduce_add_sync(0xffffffffu, qsum);
+    const float scale = __uint_as_float(static_cast<uint32_t>(127 + shift) << 23);      // 2^shift, shift <= 62
+    if (row_ok && sub == 0) {
+        if (lane == 0) {
+            scales[row] = scale;
+            if (shifts != nullptr) shifts[row] = shift;
+        }
+        if (lane < bits) slice_weights[static_cast<size_t>(row) * bits + lane] = slice_weight(lane, bits, scale);
+    }
+    if constexpr (WPR > 1) {
+        if (lane == 0) {
+            wsum[0][warp] = asum;
+            wsum[1][warp] = amax_chunk;
+            wsum[2][warp] = qsum;
+        }
+        __syncthreads();
+    }
+    if (row_ok && sub == 0 && lane == 0) {
+#pragma unroll
+        for (int i = 1; i < WPR; ++i) {
+            asum += wsum[0][warp + i];
+            amax_chunk = max(amax_chunk, wsum[1][warp + i]);
+            qsum += wsum[2][warp + i];
+        }
+        bounds[row] = static_cast<float>(asum);
+        bounds[static_cast<size_t>(rows) + row] = static_cast<float>(amax_chunk);
+        bounds[2 * static_cast<size_t>(rows) + row] = static_cast<float>(qsum);
+    }
+}
+
 // Bounds of an int8 image that exists already (loaded key sets, rows too long for the kernel above): one warp per row.
 __global__ void __launch_bounds__(256) key_bounds_kernel(const int8_t* __restrict__ q8, int64_t rows, int64_t chunks,
                                                          int64_t ld8, float* __restrict__ bounds) {
@@ -1151,10 +1283,19 @@ int launch_slice_weights(const float* scales, const PackArgs& a) {
     return BSI_OK;
 }
 
+template <typename T, int CPW, int WPR, bool kWhole>
+int launch_row_build(const T* x, const PackArgs& a, unsigned grid) {
+    quantize_pack_row_build_kernel<T, CPW, WPR, kWhole><<<grid, 256, 0, a.stream>>>(
+        x, static_cast<uint32_t>(a.rows), a.D, static_cast<uint32_t>(a.ldx), a.vec_ok, a.dec_scale, a.dec_mult, a.bits,
+        static_cast<int>(a.chunks), static_cast<uint32_t>(a.W), a.words, a.scales, a.shifts, a.q8, static_cast<uint32_t>(a.ld8),
+        a.slice_weights, a.key_bounds);
+    return BSI_OK;
+}
+
 // Row mode: the register-resident kernel for rows of up to 64 chunks (8 warps x 8 chunks), decimal_places in [0, 8]
 // and no clipping; the two-pass 64-bit kernel otherwise. As few warps on a row (1, 2, 4 or 8) as leave each four chunks at
 // most, more than that only on the longest rows: what a row costs beside its chunks is paid per warp (16384 x 4096
-// float32: 96 us with 8 warps of 2 chunks, 84 us with 4 of 4; 4096 x 768: 9.2 us with 4 warps of 1, 7.2 us with 2 of 2).
+// float32, an earlier form: 96 us with 8 warps of 2 chunks, 84 us with 4 of 4; 4096 x 768: 9.2 us with 4 warps of 1, 7.2 us with 2 of 2).
 template <typename T>
 int launch_row(const T* x, const PackArgs& a) {
     if (a.dec_mult == 0u || a.clip_k > 0.0f || a.chunks > 64) {
@@ -1176,6 +1317,16 @@ int launch_row(const T* x, const PackArgs& a) {
     const int64_t per_block = 8 >> wpr_log2;
     const unsigned grid = static_cast<unsigned>((a.rows + per_block - 1) / per_block);
     const int cpw = static_cast<int>((a.chunks + (1 << wpr_log2) - 1) >> wpr_log2);
+    if (a.words != nullptr && a.q8 != nullptr && a.scales != nullptr && a.slice_weights != nullptr && a.key_bounds != nullptr &&
+        a.rows < (1ll << 31) && a.ldx < (1ll << 31) && a.ld8 < (1ll << 31)) {
+        const bool whole = a.vec_ok && a.D == a.chunks * 256;
+#define BSI_ROW_BUILD(CPW, WPR) (whole ? launch_row_build<T, CPW, WPR, true>(x, a, grid) : launch_row_build<T, CPW, WPR, false>(x, a, grid))
+        if (wpr_log2 == 0) return cpw <= 1 ? BSI_ROW_BUILD(1, 1) : cpw <= 2 ? BSI_ROW_BUILD(2, 1) : BSI_ROW_BUILD(4, 1);
+        if (wpr_log2 == 1) return BSI_ROW_BUILD(4, 2);
+        if (wpr_log2 == 2) return BSI_ROW_BUILD(4, 4);
+        return cpw <= 4 ? BSI_ROW_BUILD(4, 8) : BSI_ROW_BUILD(8, 8);
+#undef BSI_ROW_BUILD
+    }
 #define BSI_ROW_FAST(CPW)                                                                                              \
     quantize_pack_row_fast_kernel<T, CPW><<<grid, 256, 0, a.stream>>>(                                                 \
         x, a.rows, a.D, a.ldx, a.dec_scale, a.dec_mult, a.bits, static_cast<int>(a.chunks), a.W, wpr_log2, a.words,    \
