@@ -496,6 +496,109 @@ __global__ void __launch_bounds__(256, BSI_PACK_MIN_BLOCKS) quantize_pack_chunk_
     }
 }
 
+// The same for what a query batch and a layer ask for (int8 image, scales and sums of squares; kWords: slices and their weights)
+// of rows of whole chunks on 16-byte vectors. The kernel above is bound by instruction issue (167 a unit, 77 % of the slots), so a
+// warp takes G turns of two units each of one row here: all loads go out together, addresses are a base and an immediate, and
+// nothing is asked per unit that the launch knows. 4096 x 16384 float16 with slices 51.1 -> 45.9 us (5.7 TB/s, 88 % of the copy rate),
+// 512 x 8192 5.5 -> 4.6. (float32, one unit per turn: 65.6 -> 63.6 us with slices, 71 -> 74 without; not built.)
+template <typename T, int G, bool kWords>
+__global__ void __launch_bounds__(256, 4) quantize_pack_chunk_turns_kernel(
+    const T* x, uint32_t rows, uint32_t per_row /* warps */, uint32_t chunks, double dec_scale, uint32_t dec_mult, int bits,
+    u64* __restrict__ words, float* __restrict__ scales, int8_t* __restrict__ q8, float* __restrict__ sq_norms,
+    float* __restrict__ slice_weights) {
+    static_assert(sizeof(T) == 2, "16 elements are two 16-byte vectors");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // as above
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    x = behind_wait(x);
+    const int lane = threadIdx.x & 31;
+    const bool upper = lane >= 16;                        // the second unit's lanes
+    const uint32_t l = lane & 15u;
+    const uint32_t item = blockIdx.x * 8u + (threadIdx.x >> 5);
+    const uint32_t row = item / per_row, c0 = (item - row * per_row) * (2u * G);       // first chunk
+    if (kWords) {                                         // in chunk mode a row's slice weights do not depend on its values
+        const uint32_t n = rows * static_cast<uint32_t>(bits);
+        for (uint32_t i = blockIdx.x * 256u + threadIdx.x; i < n; i += gridDim.x * 256u)
+            slice_weights[i] = slice_weight(static_cast<int>(i % static_cast<uint32_t>(bits)), bits, 1.0f);
+    }
+    if (row >= rows) return;
+    const uint32_t D = chunks * 256u, W = chunks * 4u;
+    const int turns = static_cast<int>(min((chunks - c0 + 1u) / 2u, static_cast<uint32_t>(G)));
+    const uint32_t chunk = c0 + (upper ? 1u : 0u);        // the lane's, in turn 0
+    const size_t at = static_cast<size_t>(row) * D + chunk * 256u + l * 16u;
+    const float mult = static_cast<float>(dec_mult);
+    struct Raw { RawLane<T> a, b; };
+    Raw raw[G];
+#pragma unroll
+    for (int i = 0; i < G; ++i) {
+        if (i < turns && chunk + 2u * i < chunks) {
+            raw[i].a.load(x + at + i * 512);
+            raw[i].b.load(x + at + i * 512 + 8);
+        } else {
+            raw[i].a.v[0] = raw[i].b.v[0] = make_uint4(0u, 0u, 0u, 0u);
+        }
+    }
+    int8_t* q8_out = q8 + at;
+    float* scale_out = scales + (row * chunks + chunk);
+    float* sq_out = sq_norms + (row * chunks + chunk);
+    const uint32_t slice_words = 2u * W;                  // 32-bit words per slice
+    const bool odd = (lane & 1) != 0;                     // even lanes collect slices 0 to 3 of both lanes of their pair, odd lanes 4 to 7
+    const int s0 = odd ? 4 : 0;
+    uint32_t* w_out = nullptr;
+    if (kWords) w_out = reinterpret_cast<uint32_t*>(words + (static_cast<size_t>(row) * bits + s0) * W) + chunk * 8u + (l >> 1);
+    uint32_t slow = 0;                                    // bit i: turn i has a unit of the 64-bit path; bit 16 + i: the lane's is one
+#pragma unroll
+    for (int i = 0; i < G; ++i) {
+        if (i >= turns) break;
+        const Raw& r = raw[i];
+        const uint32_t m = max(r.a.abs_max(), r.b.abs_max());
+        const uint32_t m0 = __reduce_max_sync(0xffffffffu, upper ? 0u : m), m1 = __reduce_max_sync(0xffffffffu, upper ? m : 0u);
+        const float amax = RawLane<T>::abs_value(upper ? m1 : m0);
+        const int shift = fast_group_shift(amax, mult, bits);
+        const bool there = chunk + 2u * i < chunks;
+        const bool store = there && shift >= 0;
+        if (__any_sync(0xffffffffu, there && shift < 0)) slow |= (1u << i) | (there && shift < 0 ? 0x10000u << i : 0u);
+        u64 pa, pb;
+        if (__any_sync(0xffffffffu, store && needs_clamp(amax, mult, shift, bits))) {      // one group in a hundred or so
+            pa = r.a.template quantise<true>(mult, shift, bits);
+            pb = r.b.template quantise<true>(mult, shift, bits);
+        } else {
+            pa = r.a.template quantise<false>(mult, shift, bits);
+            pb = r.b.template quantise<false>(mult, shift, bits);
+        }
+        uint32_t al = static_cast<uint32_t>(pa), ah = static_cast<uint32_t>(pa >> 32), bl = static_cast<uint32_t>(pb), bh = static_cast<uint32_t>(pb >> 32);
+        int n2 = __dp4a(static_cast<int>(al), static_cast<int>(al), __dp4a(static_cast<int>(ah), static_cast<int>(ah), 0));      // see fast_chunk
+        n2 = __dp4a(static_cast<int>(bl), static_cast<int>(bl), __dp4a(static_cast<int>(bh), static_cast<int>(bh), n2));
+        const int n0 = __reduce_add_sync(0xffffffffu, upper ? 0 : n2), n1 = __reduce_add_sync(0xffffffffu, upper ? n2 : 0);
+        if (store && l == 0u) {
+            scale_out[i * 2] = __uint_as_float(static_cast<uint32_t>(127 + shift) << 23);      // 2^shift
+            sq_out[i * 2] = static_cast<float>(upper ? n1 : n0) * __uint_as_float(static_cast<uint32_t>(127 + 2 * shift) << 23);
+        }
+        if (store) *reinterpret_cast<uint4*>(q8_out + i * 512) = make_uint4(al, ah, bl, bh);
+        if constexpr (kWords) {
+            transpose8x8_halves(al, ah);                  // as in the kernel above
+            transpose8x8_halves(bl, bh);
+            const uint32_t ga = __shfl_xor_sync(0xffffffffu, odd ? al : ah, 1), gb = __shfl_xor_sync(0xffffffffu, odd ? bl : bh, 1);
+            const uint32_t ka = odd ? ah : al, kb = odd ? bh : bl;
+            const uint32_t a0 = odd ? ga : ka, b0 = odd ? gb : kb, a1 = odd ? ka : ga, b1 = odd ? kb : gb;
+            const uint32_t e0 = __byte_perm(a0, b0, 0x5140), e2 = __byte_perm(a0, b0, 0x7362);
+            const uint32_t o0 = __byte_perm(a1, b1, 0x5140), o2 = __byte_perm(a1, b1, 0x7362);
+            if (store) {
+                uint32_t* w = w_out + i * 16;
+                if (s0 < bits) w[0] = __byte_perm(e0, o0, 0x5410);
+                if (s0 + 1 < bits) w[slice_words] = __byte_perm(e0, o0, 0x7632);
+                if (s0 + 2 < bits) w[2u * slice_words] = __byte_perm(e2, o2, 0x5410);
+                if (s0 + 3 < bits) w[3u * slice_words] = __byte_perm(e2, o2, 0x7632);
+            }
+        }
+    }
+    if ((slow & 0xffffu) == 0u) return;
+#pragma unroll 1
+    for (int u = 0; u < 2 * turns; ++u)
+        if (__shfl_sync(0xffffffffu, slow, (u & 1) * 16) & (0x10000u << (u >> 1)))
+            generic_unit<T>(x, static_cast<int64_t>(row) * chunks + c0 + u, D, D, dec_scale, dec_mult, bits, chunks, W, kWords ? words : nullptr,
+                            scales, nullptr, q8, D, true, lane, 0.0f, sq_norms);
+}
+
 // Destinations of the multi-destination pack: the same int8 image / chunk scales go to each of them.
 struct MultiDst {
     int n_q8, n_scales;
@@ -1237,6 +1340,38 @@ struct PackArgs {
     float* key_bounds;    // row mode only
 };
 
+// Turns per warp: four, two or one, as many as leave a block for every place on the chip and few lanes without a unit (a row's
+// last warp and, for an odd number of chunks, its last turn are not full: 2500 x 2304 with four turns 7.6 us, pair kernel 6.5).
+// Below that the other kernels spread the units better.
+template <typename T, bool kWords>
+int launch_chunk_turns(const T* x, const PackArgs& a, bool* taken) {
+    *taken = false;
+    const int64_t turns = (a.chunks + 1) / 2, places = static_cast<int64_t>(sm_count()) * 4;
+    int g = 4;
+    auto fits = [&] {
+        const int64_t warps = (turns + g - 1) / g;
+        return (a.rows * warps + 7) / 8 >= places && warps * g * 2 * 8 <= a.chunks * 9;
+    };
+    while (g > 1 && !fits()) g /= 2;
+    if (!fits()) return BSI_OK;
+    const int64_t per_row = (turns + g - 1) / g, blocks = (a.rows * per_row + 7) / 8;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = dim3(static_cast<unsigned>(blocks), 1, 1);
+    cfg.blockDim = dim3(256, 1, 1);
+    cfg.stream = a.stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 1 : 0;
+    auto kernel = g == 4 ? quantize_pack_chunk_turns_kernel<T, 4, kWords>
+                         : g == 2 ? quantize_pack_chunk_turns_kernel<T, 2, kWords> : quantize_pack_chunk_turns_kernel<T, 1, kWords>;
+    BSI_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, x, static_cast<uint32_t>(a.rows), static_cast<uint32_t>(per_row), static_cast<uint32_t>(a.chunks),
+                                    a.dec_scale, a.dec_mult, a.bits, a.words, a.scales, a.q8, a.sq_norms, a.slice_weights));
+    *taken = true;
+    return BSI_OK;
+}
+
 template <typename T, bool kDense, bool kWords, bool kQ8>
 int launch_chunk_fast(const T* x, const PackArgs& a) {
     // one unit per warp and turn while a turn takes them all, else two (16-bit types)
@@ -1359,6 +1494,13 @@ int launch_chunk(const T* x, const PackArgs& a) {
     }
     const bool dense = a.vec_ok && a.ldx == a.D && (a.D & 255) == 0 && (a.q8 == nullptr || a.ld8 == a.D);
     const bool w = a.words != nullptr, q = a.q8 != nullptr;
+    if constexpr (sizeof(T) == 2) {
+        if (dense && q && a.sq_norms != nullptr && a.shifts == nullptr && w == (a.slice_weights != nullptr)) {
+            bool taken = false;
+            const int rc = w ? launch_chunk_turns<T, true>(x, a, &taken) : launch_chunk_turns<T, false>(x, a, &taken);
+            if (rc != BSI_OK || taken) return rc;
+        }
+    }
     if (dense) {
         if (w && q) return launch_chunk_fast<T, true, true, true>(x, a);
         if (q) return launch_chunk_fast<T, true, false, true>(x, a);
