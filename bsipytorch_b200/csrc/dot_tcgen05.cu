@@ -477,6 +477,10 @@ int launch_tile(const CUtensorMap& ma, const CUtensorMap& mb, const float* qs, i
     return check_launch("dot_i8 tcgen05 launch");
 }
 
+// How many clusters of 2 * SPLIT CTAs run at once (one CTA per SM whatever the instantiation); 0 when the query fails.
+template <int SPLIT>
+int resident_clusters();
+
 template <int BN, bool DBG, typename OutT, bool REQ = false, int SPLIT = 1, bool ADD = false, bool ONE = false>
 int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo, const CUtensorMap& mt, int vector_store,
                 const float* qs, int64_t qs_stride, const float* bw0, const float* bias, int Q, int R, int chunks,
@@ -484,7 +488,7 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap&
                 const RequantDst& requant, const Finishing& fin, const float* k_abs_sum, float q_abs_max, const float* q_sq, int64_t q_sq_stride,
                 cudaStream_t stream, int* max_clusters_out = nullptr /* only asks how many clusters fit at once */) {
     using C = pair::Cfg<BN, OutT, REQ, SPLIT>;
-    static int max_clusters[64] = {0};   // per instantiation
+    static bool attr_set[64] = {false};   // per instantiation
     int dev = 0;
     BSI_CUDA_TRY(cudaGetDevice(&dev));
     const int tiles_m = (Q + 255) / 256;
@@ -504,26 +508,22 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap&
     cfg.stream = stream;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 2 : 1;
-    int resident = 0;
-    if (dev >= 0 && dev < 64) resident = max_clusters[dev];
-    if (resident == 0) {
+    if (dev < 0 || dev >= 64 || !attr_set[dev]) {
         BSI_CUDA_TRY(cudaFuncSetAttribute(pair::dot_i8_tcgen05_pair_kernel<BN, DBG, OutT, REQ, SPLIT, ADD, ONE>,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
-        cfg.gridDim = dim3(2 * SPLIT * (sm_count() / (2 * SPLIT)), 1, 1);
-        BSI_CUDA_TRY(cudaOccupancyMaxActiveClusters(&resident, pair::dot_i8_tcgen05_pair_kernel<BN, DBG, OutT, REQ, SPLIT, ADD, ONE>, &cfg));
-        if (resident <= 0) return fail(BSI_ERR_CUDA, "dot_i8: no cluster of 2 CTAs fits on this device");
-        if (dev >= 0 && dev < 64) max_clusters[dev] = resident;
+        if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
     if (max_clusters_out != nullptr) {
-        *max_clusters_out = resident;
+        cfg.gridDim = dim3(2 * SPLIT * (sm_count() / (2 * SPLIT)), 1, 1);
+        BSI_CUDA_TRY(cudaOccupancyMaxActiveClusters(max_clusters_out, pair::dot_i8_tcgen05_pair_kernel<BN, DBG, OutT, REQ, SPLIT, ADD, ONE>, &cfg));
         return BSI_OK;
     }
-    if constexpr (!ONE && !DBG && !REQ && SPLIT == 1) {
-        if (tiles_total <= resident && (vector_store & 4))
-            return launch_pair<BN, DBG, OutT, REQ, SPLIT, ADD, true>(ma, mb, mo, mt, vector_store, qs, qs_stride, bw0, bias, Q, R, chunks, scale_inv, out,
-                                                                     ldo, dbg, scatter, requant, fin, k_abs_sum, q_abs_max, q_sq, q_sq_stride, stream);
+    int clusters = tiles_total;
+    if constexpr (SPLIT == 1 && !ONE) {
+        const int resident = resident_clusters<1>();
+        if (resident <= 0) return fail(BSI_ERR_CUDA, "dot_i8: no cluster of 2 CTAs fits on this device");
+        clusters = tiles_total < resident ? tiles_total : resident;
     }
-    const int clusters = SPLIT > 1 || tiles_total < resident ? tiles_total : resident;
     cfg.gridDim = dim3(2 * SPLIT * clusters, 1, 1);
     BSI_CUDA_TRY(cudaLaunchKernelEx(&cfg, pair::dot_i8_tcgen05_pair_kernel<BN, DBG, OutT, REQ, SPLIT, ADD, ONE>, ma, mb, mo, mt, vector_store, qs,
                                     qs_stride, bw0, bias, Q, R, chunks, tiles_m, tiles_total, scale_inv, out, ldo, dbg, scatter, requant,
@@ -557,7 +557,6 @@ int pick_bn_pair(int64_t Q, int64_t R, bool any_width) {
 // Tile width and parts along K of this thread's last paired dot (a test hook: bsi_b200_debug_last_tiles).
 thread_local int t_last_width = 0, t_last_parts = 0;
 
-// How many clusters of 2 * SPLIT CTAs run at once (one CTA per SM whatever the tile width); 0 when the query fails.
 template <int SPLIT>
 int resident_clusters() {
     static int cached[64] = {0};
@@ -845,19 +844,26 @@ int dot_i8_pair(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_strid
 #undef BSI_SPLIT_T
 #undef BSI_SPLIT_A
     }
+    // no more tiles than pairs, bulk stores: an instantiation of its own
+    const bool one = (store_flags & 4) != 0 && dbg_iacc == nullptr && requant.n == 0 && (Q + 255) / 256 * ((R + bn - 1) / bn) <= resident_clusters<1>();
+#define BSI_PAIR_ONE(BN_, T_, ADD_)                                                                                      \
+    launch_pair<BN_, false, T_, false, 1, ADD_, true>(ma, mb, mo, mt, store_flags, qs, qs_stride, bw0, bias, q, r, c, scale_inv, out, \
+                                                      ldo, nullptr, scatter, requant, fin, kabs, qabs, qsq, qsq_stride, stream)
 #define BSI_PAIR_T(BN_, DBG_, T_)                                                                              \
+    (one && !DBG_) ? BSI_PAIR_ONE(BN_, T_, false) :                                                            \
     launch_pair<BN_, DBG_, T_>(ma, mb, mo, mt, store_flags, qs, qs_stride, bw0, bias, q, r, c, scale_inv, out, ldo,  \
                                dbg_iacc, scatter, requant, fin, kabs, qabs, qsq, qsq_stride, stream)
 #define BSI_PAIR_ADD(BN_, T_)                                                                                            \
+    one ? BSI_PAIR_ONE(BN_, T_, true) :                                                                                  \
     launch_pair<BN_, false, T_, false, 1, true>(ma, mb, mo, mt, store_flags, qs, qs_stride, bw0, bias, q, r, c, scale_inv, out, \
                                                 ldo, dbg_iacc, scatter, requant, fin, kabs, qabs, qsq, qsq_stride, stream)
 #define BSI_PAIR(BN_)                                                                   \
-    (fin.add != nullptr ? (y_dtype == BSI_DTYPE_F16 ? BSI_PAIR_ADD(BN_, __half) : y_dtype == BSI_DTYPE_BF16 ? BSI_PAIR_ADD(BN_, __nv_bfloat16) \
-                                                                                               : BSI_PAIR_ADD(BN_, float)) \
-     : y_dtype == BSI_DTYPE_F16    ? BSI_PAIR_T(BN_, false, __half)                       \
-     : y_dtype == BSI_DTYPE_BF16 ? BSI_PAIR_T(BN_, false, __nv_bfloat16)                \
-     : dbg_iacc                  ? BSI_PAIR_T(BN_, true, float)                         \
-                                 : BSI_PAIR_T(BN_, false, float))
+    (fin.add != nullptr ? (y_dtype == BSI_DTYPE_F16 ? (BSI_PAIR_ADD(BN_, __half)) : y_dtype == BSI_DTYPE_BF16 ? (BSI_PAIR_ADD(BN_, __nv_bfloat16)) \
+                                                                                               : (BSI_PAIR_ADD(BN_, float))) \
+     : y_dtype == BSI_DTYPE_F16    ? (BSI_PAIR_T(BN_, false, __half))                     \
+     : y_dtype == BSI_DTYPE_BF16 ? (BSI_PAIR_T(BN_, false, __nv_bfloat16))              \
+     : dbg_iacc                  ? (BSI_PAIR_T(BN_, true, float))                       \
+                                 : (BSI_PAIR_T(BN_, false, float)))
     if (requant.n > 0) {
         if (y_dtype == BSI_DTYPE_F16)
             return launch_pair<256, false, __half, true>(ma, mb, mo, mt, store_flags, qs, qs_stride, bw0, bias, q, r, c, scale_inv,
@@ -866,7 +872,7 @@ int dot_i8_pair(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_strid
                                                             scale_inv, out, ldo, nullptr, scatter, requant, fin, kabs, qabs, qsq,
                                                             qsq_stride, stream);
     }
-#define BSI_PAIR_F32(BN_) (dbg_iacc ? BSI_PAIR_T(BN_, true, float) : BSI_PAIR_T(BN_, false, float))
+#define BSI_PAIR_F32(BN_) (dbg_iacc ? (BSI_PAIR_T(BN_, true, float)) : (BSI_PAIR_T(BN_, false, float)))
     switch (bn) {
         case 256: return BSI_PAIR(256);
         case 224: return BSI_PAIR_F32(224);
@@ -879,6 +885,7 @@ int dot_i8_pair(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_strid
 #undef BSI_PAIR_F32
 #undef BSI_PAIR
 #undef BSI_PAIR_ADD
+#undef BSI_PAIR_ONE
 #undef BSI_PAIR_T
 }
 
