@@ -531,9 +531,11 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap&
     return check_launch("dot_i8 tcgen05 pair launch");
 }
 
-// Pair kernel tile width. Measured on the 512 x 8192 x 2048 shape, a pair spends about 650 + 3.1 * BN cycles per
-// 256-deep chunk of a tile (the epilogue's per-column work plus a fixed hand-off cost), and walks through
-// ceil(tiles / pairs) tiles. The widest tile wins unless a narrower one is clearly cheaper (more than 8 %: at equal
+// Pair kernel tile width. The costs, 650 + 3.1 * BN cycles per 256-deep chunk of a tile and ceil(tiles / pairs) tiles, and those of
+// pick_split were fitted to a form of the kernel whose chunks took 980 cycles at every width; they take 500 + 2 * BN now. Over 228
+// sizes (64 .. 2048 rows, 256 .. 12288 columns, 2 .. 64 chunks) what the two pick is within 1.1 % of the best width and split on
+// the mean, a refitted rule within 0.3 %; the difference is at 8192 and more of depth, where unsplit tiles of 64 to 128 columns
+// are 6 to 25 % shorter than the split taken (512 x 3072 x 16384: 32.4 us, 96 columns 26.0). The widest tile wins unless a narrower one is clearly cheaper (more than 8 %: at equal
 // rounds the wider tile also has the shorter fill and store phases). float32 output may use any multiple of 32,
 // the 16-bit layer epilogues (whole 64-column store rounds) the powers of two.
 int pick_bn_pair(int64_t Q, int64_t R, bool any_width) {
@@ -703,7 +705,8 @@ int run_rows(const RowsPlan& plan, rows::Args a, const int8_t* a8, int64_t lda, 
 // x 512: 8.5 against 8.6). Only where its bounds are given and quickly read (rows of whole 16-byte vectors): without them the
 // split does not happen or starts late (4608 x 4608: 21.9 us against 9.5). Both costs as above, in microseconds of a replayed
 // graph: beside its chunks and hand-overs the rows kernel takes 2.1 + 0.2 per part + 0.045 per row, a split (1900 cycles to
-// the microsecond) 0.1 less for every tile that a wave of clusters of eight would still have room for.
+// the microsecond) 0.1 less for every tile that a wave of clusters of eight would still have room for. Split and rows kernel as they
+// were when this was fitted; both have become shorter (512 keys 15.4 -> 10.5 us, 1024 keys on the rows kernel 17.0 -> 13.2).
 static bool split_is_shorter(int64_t Q, int64_t R, int64_t chunks, const RowsPlan& rows_plan, const bsi_dot_bounds& bounds, int64_t qs_stride) {
     if (rows_plan.parts == 1 || bounds.key_bounds == nullptr || bounds.query_sq == nullptr || qs_stride < chunks ||
         bounds.query_sq_stride < chunks || ((chunks | qs_stride | bounds.query_sq_stride) & 3) != 0)

@@ -27,17 +27,16 @@
 //   tempty[b]  leader's copy used: one arrival per epilogue warp of BOTH CTAs (16)
 // The accumulator ring holds 2 or 4 buffers (BN > 128, else): with narrow tiles the MMA issuers run several chunks
 // ahead of the epilogue, which takes the barrier round trip off the critical path.
-// A chunk of a 256 x 224 tile takes 920 to 1050 cycles with integer sums (clock64 marks in every CTA of a 512 x 8192 x
-// 2048 dot), its 8 MMAs 896; the float32 chain costs three instructions per accumulator value instead of one, at one warp
-// instruction per clock and SM sub-partition, next to TMEM loads that slow down while the tensor pipe is busy. What a tile
-// costs beyond its chunks, the bounds and the store phase, went from 20 to 6 thousand cycles with batched bound loads,
-// key scales and bias in shared memory and bulk stores: 4096 x 16384 x 4096, float16 out: 254 -> 189 us (2.9 POPS).
+// What bounds a chunk (clock64 marks in every CTA): the MMAs read A and half of B from shared memory at 64 bytes a cycle, 500 + 2 BN
+// cycles for the chunk's 8 (600 at 64 columns, 750 at 128, 1000 at 224); with the float32 chain, three instructions per
+// accumulator value instead of one, the epilogue is about as long at 256 columns. Beside the chunks a 512 x 8192 x 2048 dot
+// spends 1700 cycles on set-up, 1500 until the first k-block has come, 1000 for the chunk behind it, and 5000 on the store phase.
 // Split along K (SPLIT = 2 or 4): where the tiles leave most SMs idle, a cluster of SPLIT pairs shares one tile, each
 // with a part of the chunks. The chunk terms are integers, so where the bounds of the integer route hold for every warp
 // of the tile (the cluster votes before the first MMA) the parts add up in any order to the float32 chain's bits: every
 // warp sends its sums through distributed shared memory to the pair that owns the columns, which adds and stores them.
 // If a bound fails anywhere, pair 0 does the whole tile on its own with the chain in order, as an unsplit kernel would.
-// 512 x 2048 x 8192 (32 tiles of 256 x 128, 2 pairs each; operands cold): 18.3 -> 17.3 us; 64 x 512 x 16384: 33.8 -> 15.9.
+// 512 x 2048 x 8192 (32 tiles of 256 x 128, 2 pairs each): 13.9 us; 64 x 512 x 16384: 10.5.
 // All waits are bounded; a timeout raises the abort flag of both CTAs and every role drains out.
 #pragma once
 
