@@ -567,6 +567,10 @@ __device__ __forceinline__ void fold_and_store(const float (&acc)[kCols], uint32
     const int qmul = kind == kFloatSums ? 0 : __float2int_rn(qscale);
     int32_t v[2][32];
     if (kCols >= 32) tmem_ld32(taddr, v[0]); else tmem_ld16(taddr, v[0]);
+    // The matrix to add as in store_columns, from a block's first group to its last (two of 16 bits); four loads of a wide tile's
+    // block, for the sake of registers, wait until the block is finished.
+    constexpr int kAhead = kCols <= 64 ? 8 : 4;
+    uint4 add[kAhead];
 #pragma unroll
     for (int g = 0; g < kGroups; ++g) {
         const int c0 = g * 32, n = kCols - c0 < 32 ? kCols - c0 : 32;
@@ -581,8 +585,6 @@ __device__ __forceinline__ void fold_and_store(const float (&acc)[kCols], uint32
         const int round = c0 / kRoundCols, cg = round * kRoundCols;
         const bool whole = round < kFull;
         const int nch = whole ? 8 : 4;
-        // as in store_columns; four loads of a wide tile's block, for the sake of registers, wait until the block is finished
-        constexpr int kAhead = kCols <= 64 ? 8 : 4;
         const int tch = lane & (nch - 1), trow = lane / nch, step = 32 / nch;
         const bool in = col + cg + tch * kPerChunk < R;
         auto fetch = [&](int i) {
@@ -590,7 +592,6 @@ __device__ __forceinline__ void fold_and_store(const float (&acc)[kCols], uint32
             if (!in || r >= Q) return make_uint4(0u, 0u, 0u, 0u);
             return *reinterpret_cast<const uint4*>(behind_wait(static_cast<const OutT*>(fin.add)) + static_cast<int64_t>(r) * fin.ld_add + col + cg + tch * kPerChunk);
         };
-        uint4 add[kAhead];
         if constexpr (ADD) {
             if (c0 == cg) {
 #pragma unroll
