@@ -57,6 +57,8 @@ SIGNATURES = {
     "bsi_b200_quantize_pack_multi": (_i32, [_vp, _i32, _i64, _i64, _i64, _i32, _i32, _i32, _vp, _i64, _i32, _vp, _i64, _vp]),
     "bsi_b200_linear_i8_requant": (_i32, [_vp, _i64, _vp, _i64, _vp, _i64, _vp, _vp, _i64, _i64, _i64, _f32, _i32, _i32, _i32, _i32,
                                           _i32, _vp, _i64, _vp, _i64, _vp]),
+    "bsi_b200_linear_i8_requant_bounded": (_i32, [_vp, _i64, _vp, _i64, _vp, _i64, _vp, _vp, _i64, _i64, _i64, _f32, _i32, _i32, _i32, _i32,
+                                                  _i32, _vp, _i64, _vp, _i64, _vp, _vp]),
     "bsi_b200_add_layernorm_pack": (_i32, [_vp, _vp, _vp, _vp, _f32, _i32, _i64, _i64, _vp, _i32, _i32, _i32, _vp, _i64, _i32, _vp, _i64, _vp]),
     "bsi_b200_peer_alloc": (_i32, [_i64, _vp, _vp]),
     "bsi_b200_peer_free": (_i32, [_vp]),

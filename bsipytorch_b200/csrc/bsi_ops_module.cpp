@@ -1186,13 +1186,8 @@ py::object opt_layer_forward(const torch::Tensor& x, const py::tuple& norms, con
     return py::cast(linear_forward(env, f, *keys[5], bias[5], dp[5], false, mid).view({B, T, H}));
 }
 
-// Quantise + pack activations (query side: chunk scales) into tensors the caller owns: q8 [rows, >= d]
-// int8 (any row stride that is a multiple of 16 bytes, e.g. a column block of a wider matrix) and
-// scales [rows, d/256] float32, contiguous. This is the first half of bsi_linear_forward, split off so
-// that a tensor-parallel layer can pack its own column block straight into the buffer the ranks
-// exchange. d must be a multiple of 256.
 // sq_norms [rows, d/256] float32, where given: the chunks' sums of squares, with which a dot proves its integer route exact.
-const float* chunk_norms(const c10::optional<torch::Tensor>& norms, const torch::Tensor& q8, int64_t rows, int64_t chunks) {
+float* chunk_norms(const c10::optional<torch::Tensor>& norms, const torch::Tensor& q8, int64_t rows, int64_t chunks) {
     if (!norms.has_value() || !norms->defined()) return nullptr;
     TORCH_CHECK(norms->is_cuda() && norms->scalar_type() == at::kFloat && norms->is_contiguous() && norms->numel() == rows * chunks,
                 "sq_norms must be contiguous float32 [rows, d/256]");
@@ -1200,6 +1195,11 @@ const float* chunk_norms(const c10::optional<torch::Tensor>& norms, const torch:
     return norms->data_ptr<float>();
 }
 
+// Quantise + pack activations (query side: chunk scales) into tensors the caller owns: q8 [rows, >= d]
+// int8 (any row stride that is a multiple of 16 bytes, e.g. a column block of a wider matrix) and
+// scales [rows, d/256] float32, contiguous. This is the first half of bsi_linear_forward, split off so
+// that a tensor-parallel layer can pack its own column block straight into the buffer the ranks
+// exchange. d must be a multiple of 256.
 void pack_queries_into(torch::Tensor x2d, torch::Tensor q8, torch::Tensor scales, int decimalPlaces, c10::optional<torch::Tensor> sq_norms) {
     const Env env;
     require_fixed_queries(env, "pack_queries_into");
@@ -1219,7 +1219,7 @@ void pack_queries_into(torch::Tensor x2d, torch::Tensor q8, torch::Tensor scales
     TORCH_CHECK(d % 256 == 0, "d must be a multiple of 256");
     TORCH_CHECK(q8.size(0) == rows && q8.size(1) >= d, "q8 shape mismatch");
     TORCH_CHECK(scales.numel() == rows * (d / 256), "scales shape mismatch");
-    float* norms = const_cast<float*>(chunk_norms(sq_norms, q8, rows, d / 256));
+    float* norms = chunk_norms(sq_norms, q8, rows, d / 256);
     if (rows == 0 || d == 0) return;
     check_status(bsi_b200_quantize_pack_norms(x.data_ptr(), dtype_code(x), rows, d, x.stride(0), decimalPlaces,
                                               env.bits_queries(), 1, 0.0f, nullptr, scales.data_ptr<float>(), nullptr,
@@ -1413,23 +1413,24 @@ void linear_from_packed_requant(torch::Tensor q8, torch::Tensor scales, py::caps
     std::vector<float*> sd;
     for (int64_t p : q8_ptrs) qd.push_back(reinterpret_cast<int8_t*>(static_cast<intptr_t>(p)));
     for (int64_t p : scale_ptrs) sd.push_back(reinterpret_cast<float*>(static_cast<intptr_t>(p)));
-    keys->register_bounds(Env().bits_queries());
-    // the sums of squares are registered for the time of the call, which has no other way to take them
-    struct Registered {
-        const int8_t* a8;
-        ~Registered() { if (a8 != nullptr) bsi_b200_unregister_query_bounds(a8); }
-    } registered{nullptr};
-    if (const float* norms = chunk_norms(sq_norms, q8, Q, chunks)) {
-        check_status(bsi_b200_register_query_bounds(q8.data_ptr<int8_t>(), norms, chunks), "bsi_b200_register_query_bounds");
-        registered.a8 = q8.data_ptr<int8_t>();
+    // given sums of squares go with the call; else the bounds are the registry's
+    bsi_dot_bounds bounds = {};
+    const float* norms = chunk_norms(sq_norms, q8, Q, chunks);
+    if (norms != nullptr) {
+        bounds = dot_bounds(*keys, env.bits_queries(), nullptr);
+        bounds.query_sq = norms;
+        bounds.query_sq_stride = chunks;
+    } else {
+        keys->register_bounds(env.bits_queries());
     }
-    check_status(bsi_b200_linear_i8_requant(q8.data_ptr<int8_t>(), q8.stride(0), scales.data_ptr<float>(), chunks,
-                                            keys->b.q8.data_ptr<int8_t>(), keys->b.q8.size(1),
-                                            keys->b.scales.data_ptr<float>(), bptr, Q, R, chunks,
-                                            static_cast<float>(scale_inv), yt == at::kHalf ? BSI_DTYPE_F16 : BSI_DTYPE_BF16,
-                                            relu ? BSI_ACT_RELU : BSI_ACT_NONE, decimalPlaces, env.bits_queries(),
-                                            static_cast<int>(qd.size()), qd.data(), ld8, sd.data(), scale_ld, current_stream()),
-                 "bsi_b200_linear_i8_requant");
+    check_status(bsi_b200_linear_i8_requant_bounded(q8.data_ptr<int8_t>(), q8.stride(0), scales.data_ptr<float>(), chunks,
+                                                    keys->b.q8.data_ptr<int8_t>(), keys->b.q8.size(1),
+                                                    keys->b.scales.data_ptr<float>(), bptr, Q, R, chunks,
+                                                    static_cast<float>(scale_inv), yt == at::kHalf ? BSI_DTYPE_F16 : BSI_DTYPE_BF16,
+                                                    relu ? BSI_ACT_RELU : BSI_ACT_NONE, decimalPlaces, env.bits_queries(),
+                                                    static_cast<int>(qd.size()), qd.data(), ld8, sd.data(), scale_ld,
+                                                    norms != nullptr ? &bounds : nullptr, current_stream()),
+                 "bsi_b200_linear_i8_requant_bounded");
 }
 
 // Residual add + LayerNorm + activation pack (16-bit layer types). Returns x + delta (delta optional); the

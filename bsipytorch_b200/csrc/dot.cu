@@ -287,7 +287,17 @@ extern "C" int bsi_b200_linear_i8_requant(const int8_t* a8, int64_t lda, const f
                                           int64_t Q, int64_t R, int64_t chunks, float scale_inv,
                                           int layer_dtype, int activation, int decimal_places, int bits,
                                           int n_dst, int8_t* const* q8_dst, int64_t ld8,
-                                          float* const* scale_dst, int64_t scale_ld, bsi_stream_t stream_) {
+                                          float* const* scale_dst, int64_t scale_ld, bsi_stream_t stream) {
+    return bsi_b200_linear_i8_requant_bounded(a8, lda, qs, qs_stride, k8, ldk, bw0, bias, Q, R, chunks, scale_inv, layer_dtype,
+                                              activation, decimal_places, bits, n_dst, q8_dst, ld8, scale_dst, scale_ld, nullptr, stream);
+}
+
+extern "C" int bsi_b200_linear_i8_requant_bounded(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride,
+                                                  const int8_t* k8, int64_t ldk, const float* bw0, const float* bias,
+                                                  int64_t Q, int64_t R, int64_t chunks, float scale_inv,
+                                                  int layer_dtype, int activation, int decimal_places, int bits,
+                                                  int n_dst, int8_t* const* q8_dst, int64_t ld8, float* const* scale_dst,
+                                                  int64_t scale_ld, const bsi_dot_bounds* bounds, bsi_stream_t stream_) {
     using namespace bsi;
     if (Q < 0 || R < 0 || chunks < 0) return fail(BSI_ERR_INVALID, "linear_i8_requant: negative size");
     if (Q == 0 || R == 0) return BSI_OK;
@@ -323,7 +333,7 @@ extern "C" int bsi_b200_linear_i8_requant(const int8_t* a8, int64_t lda, const f
     }
     if (int rc = require_sm100()) return rc;
     return dot_i8_pair(a8, lda, qs, qs_stride, k8, ldk, bw0, bias, Q, R, chunks, scale_inv, q8_dst[0], R, layer_dtype,
-                       nullptr, 0, Finishing{activation == BSI_ACT_RELU ? 1 : 0, 0, 1.0f, nullptr, 0}, nullptr, &rq, resolve_bounds(nullptr, a8, k8, R), static_cast<cudaStream_t>(stream_));
+                       nullptr, 0, Finishing{activation == BSI_ACT_RELU ? 1 : 0, 0, 1.0f, nullptr, 0}, nullptr, &rq, resolve_bounds(bounds, a8, k8, R), static_cast<cudaStream_t>(stream_));
 }
 
 extern "C" int bsi_b200_linear_i8(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride,

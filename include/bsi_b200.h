@@ -322,6 +322,13 @@ int bsi_b200_linear_i8_requant(const int8_t* a8, int64_t lda, const float* qs, i
                                int layer_dtype, int activation, int decimal_places, int bits,
                                int n_dst, int8_t* const* q8_dst, int64_t ld8,
                                float* const* scale_dst, int64_t scale_ld, bsi_stream_t stream);
+/* The same with its bounds handed over (see bsi_dot_bounds; NULL: those of the registry). */
+int bsi_b200_linear_i8_requant_bounded(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_stride,
+                                       const int8_t* k8, int64_t ldk, const float* bw0, const float* bias,
+                                       int64_t Q, int64_t R, int64_t chunks, float scale_inv,
+                                       int layer_dtype, int activation, int decimal_places, int bits,
+                                       int n_dst, int8_t* const* q8_dst, int64_t ld8, float* const* scale_dst, int64_t scale_ld,
+                                       const bsi_dot_bounds* bounds, bsi_stream_t stream);
 
 /* Chunk-mode quantise + pack of activations (int8 image and chunk scales only) written to several
  * places at once: the int8 image to q8_dst[i] + row * ld8 + col for i < n_q8_dst, the chunk scales to
