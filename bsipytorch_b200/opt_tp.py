@@ -251,7 +251,8 @@ class TPDecoderLayer(nn.Module):
         unit scaling): in the epilogue on the extension, where the separate pass over a strided block cost 42 us."""
         Hl, factor = self.h_hi - self.h_lo, self.head_dim ** -0.5
         if isinstance(self.ops, BsiDeviceOps) and Hl % 8 == 0:
-            return self.ops.linear_scaled(q8, sc, self.keys_qkv, self.bias_qkv, self.dtype, Hl, factor, norms)
+            sums = {} if norms is None else {"norms": norms}
+            return self.ops.linear_scaled(q8, sc, self.keys_qkv, self.bias_qkv, self.dtype, Hl, factor, **sums)
         qkv = self.ops.linear(q8, sc, self.keys_qkv, self.bias_qkv, self.dtype)
         qkv[:, :Hl] *= factor
         return qkv
@@ -338,7 +339,7 @@ class TPDecoderLayer(nn.Module):
         added to the residual stream `x` (None at the first layer, and where the epilogue has added it)."""
         if px is not None:
             return self.forward_peer(x_loc, delta, B, T, px)
-        if self.world == 1 and not self.fuse_ln and isinstance(self.ops, BsiDeviceOps):
+        if self.world == 1 and not self.fuse_ln and type(self.ops) is BsiDeviceOps:
             return self.forward_whole(x_loc if delta is None else x_loc + delta, B, T)
         Q = B * T
         ops, dt = self.ops, self.dtype
