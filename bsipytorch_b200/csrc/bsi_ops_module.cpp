@@ -1263,11 +1263,16 @@ at::Tensor linear_from_packed(torch::Tensor q8, torch::Tensor scales, py::capsul
     bounds.query_sq = chunk_norms(sq_norms, q8, Q, chunks);
     bounds.query_sq_stride = chunks;
     const void* addend = nullptr;
+    bool sum_behind = false;
     if (add.has_value() && add->defined()) {
-        TORCH_CHECK(add->is_cuda() && add->scalar_type() == yt && add->dim() == 2 && add->size(0) == Q && add->size(1) == R && add->is_contiguous(),
-                    "add must be a contiguous [Q, R] matrix of the output's type");
+        TORCH_CHECK(add->is_cuda() && add->is_floating_point() && add->dim() == 2 && add->size(0) == Q && add->size(1) == R,
+                    "add must be a floating-point CUDA matrix [Q, R]");
         same_device(q8, *add, "packed activations and the matrix to add");
-        addend = add->data_ptr();
+        // an operator of its own where the epilogue cannot take the matrix as it is, where a mode listens, and where the sum is
+        // to be recorded: in the epilogue it would be none of these
+        sum_behind = add->scalar_type() != yt || !add->is_contiguous() || observed() || add->unsafeGetTensorImpl()->is_python_dispatch() ||
+                     (at::GradMode::is_enabled() && add->requires_grad()) || add->_fw_grad(0).defined();
+        if (!sum_behind) addend = add->data_ptr();
     }
     check_status(bsi_b200_linear_i8_add(q8.data_ptr<int8_t>(), q8.stride(0), scales.data_ptr<float>(), chunks,
                                         keys->b.q8.data_ptr<int8_t>(), keys->b.q8.size(1),
@@ -1278,7 +1283,7 @@ at::Tensor linear_from_packed(torch::Tensor q8, torch::Tensor scales, py::capsul
                                             (Q <= kFewRows ? keys->complete() : 0),
                                         current_stream()),
                  "bsi_b200_linear_i8_add");
-    return y;
+    return sum_behind ? add->add(y) : y;
 }
 
 // ---- peer memory and the stores-as-collectives of the tensor-parallel layer -----------------------
@@ -1761,7 +1766,8 @@ PYBIND11_MODULE(bsi_ops, m) {
           py::arg("bias"), py::arg("decimal_places"), py::arg("out_dtype"), py::arg("relu") = false,
           py::arg("scaled_columns") = 0, py::arg("factor") = 1.0, py::arg("sq_norms") = py::none(), py::arg("add") = py::none(),
           "Dot of packed activations with a key set, cast + bias (+ ReLU) fused; the first scaled_columns output columns (a "
-          "multiple of 8) times factor; sq_norms: the activations' sums of squares (pack_queries_into); add: a matrix added at the end");
+          "multiple of 8) times factor; sq_norms: the activations' sums of squares (pack_queries_into); add: a matrix added at the "
+          "end, as add + y does, in the epilogue where it is contiguous, of the output's type and nobody listens");
     m.def("peer_alloc", &peer_alloc, py::arg("nbytes"), "Zero-filled device buffer other local processes can map: (uint8 tensor, handle bytes)");
     m.def("peer_open", &peer_open, py::arg("handle"), "Map a peer's buffer; returns its device address here");
     m.def("peer_close", &peer_close, py::arg("ptr"));

@@ -37,6 +37,8 @@ import torch
 import torch.distributed as dist
 import torch.nn.functional as F
 from torch import nn
+from torch.overrides import _get_current_function_mode_stack
+from torch.utils._device import DeviceContext
 
 from .opt import CONFIGS, OPTConfig
 
@@ -306,6 +308,13 @@ class TPDecoderLayer(nn.Module):
         to_owner(px.C2_q8, px.C2_sc, self.keys_fc2, self.bias_fc2)
         return x_loc, px.T
 
+    def whole(self, x):
+        """Whether this is one rank with the extension's own operations and its residual sums may ride in epilogues. A function
+        mode or a tensor subclass sees them as operators of their own; what else may look (dispatch modes, gradients, forward-mode
+        tangents) linear_from_packed asks for itself."""
+        return (self.world == 1 and not self.fuse_ln and type(self.ops) is BsiDeviceOps and type(x) is torch.Tensor
+                and not (torch._C._is_torch_function_mode_enabled() and any(type(m) is not DeviceContext for m in _get_current_function_mode_stack())))
+
     def forward_whole(self, x, B, T):
         """The layer on one rank with the CUDA extension: the packers leave the chunks' sums of squares for the dots' integer
         route, and both residual sums are taken in the epilogue of the linear in front of them (one rounding in the layer's
@@ -339,7 +348,7 @@ class TPDecoderLayer(nn.Module):
         added to the residual stream `x` (None at the first layer, and where the epilogue has added it)."""
         if px is not None:
             return self.forward_peer(x_loc, delta, B, T, px)
-        if self.world == 1 and not self.fuse_ln and type(self.ops) is BsiDeviceOps:
+        if self.whole(x_loc):
             return self.forward_whole(x_loc if delta is None else x_loc + delta, B, T)
         Q = B * T
         ops, dt = self.ops, self.dtype
