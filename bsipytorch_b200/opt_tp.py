@@ -37,6 +37,7 @@ import torch
 import torch.distributed as dist
 import torch.nn.functional as F
 from torch import nn
+from torch.nn.modules import module as nn_module
 from torch.overrides import _get_current_function_mode_stack
 from torch.utils._device import DeviceContext
 
@@ -77,6 +78,10 @@ class BsiDeviceOps:
         addresses (needs a 16-bit layer type and a multiple of 256 output features)."""
         self.m.linear_from_packed_requant(q8, scales, keys, bias, self.dp, layer_dtype, relu, q8_ptrs, ld8,
                                           scale_ptrs, scale_ld, norms)
+
+
+# what sees a layer's arguments and results
+_LAYER_HOOKS = ("_forward_hooks", "_forward_pre_hooks", "_backward_hooks", "_backward_pre_hooks")
 
 
 def _align(n: int, a: int = 256) -> int:
@@ -315,10 +320,17 @@ class TPDecoderLayer(nn.Module):
         return (self.world == 1 and not self.fuse_ln and type(self.ops) is BsiDeviceOps and type(x) is torch.Tensor
                 and not (torch._C._is_torch_function_mode_enabled() and any(type(m) is not DeviceContext for m in _get_current_function_mode_stack())))
 
-    def forward_whole(self, x, B, T):
-        """The layer on one rank with the CUDA extension: the packers leave the chunks' sums of squares for the dots' integer
-        route, and both residual sums are taken in the epilogue of the linear in front of them (one rounding in the layer's
-        type, as x + delta does)."""
+    def takes_sum(self, x):
+        """Whether a caller that only wants the sum may ask for it (forward's `summed`): nobody looks at the pair."""
+        d = self.__dict__
+        return (type(self) is TPDecoderLayer and self.whole(x) and "forward" not in d and not any(d[h] for h in _LAYER_HOOKS)
+                and not (nn_module._global_forward_hooks or nn_module._global_forward_pre_hooks))
+
+    def forward_whole(self, x, B, T, summed):
+        """The layer on one rank with the CUDA extension: the packers leave the chunks' sums of squares for the integer route of
+        the dots behind them (not fc1's re-quantising epilogue, so not for fc2 of the 16-bit types), and residual sums are taken
+        in the epilogue of the linear in front of them (one rounding in the layer's type, as x + delta does): out_proj's, and
+        fc2's where the caller wants only the sum."""
         Q, ops, dt, dev = B * T, self.ops, self.dtype, x.device
 
         def pack(h):
@@ -341,15 +353,16 @@ class TPDecoderLayer(nn.Module):
             q8, sc, sq = q8f, scf, None
         else:
             q8, sc, sq = pack(ops.linear(q8, sc, self.keys_fc1, self.bias_fc1, dt, relu=True, norms=sq))
-        return ops.linear(q8, sc, self.keys_fc2, self.bias_fc2, dt, norms=sq, add=x), None
+        o = ops.linear(q8, sc, self.keys_fc2, self.bias_fc2, dt, norms=sq, add=x if summed else None)
+        return (o, None) if summed else (x, o)
 
-    def forward(self, x_loc, delta, B, T, px=None):
+    def forward(self, x_loc, delta, B, T, px=None, summed=False):
         """(x, delta) -> (x, delta): `delta` is the fc2 output of the previous layer for the own tokens, not yet
-        added to the residual stream `x` (None at the first layer, and where the epilogue has added it)."""
+        added to the residual stream `x` (None at the first layer). summed (where takes_sum): (x + delta, None)."""
         if px is not None:
             return self.forward_peer(x_loc, delta, B, T, px)
         if self.whole(x_loc):
-            return self.forward_whole(x_loc if delta is None else x_loc + delta, B, T)
+            return self.forward_whole(x_loc if delta is None else x_loc + delta, B, T, summed)
         Q = B * T
         ops, dt = self.ops, self.dtype
         H = self.cfg.hidden_size
@@ -421,7 +434,10 @@ class TPOPTForCausalLM(nn.Module):
         pos = torch.arange(self.rank * Qn, (self.rank + 1) * Qn, device=input_ids.device) % T + 2   # OPT's offset
         x, delta = self.embed_tokens(ids) + self.embed_positions(pos), None
         for layer in self.layers:
-            x, delta = layer(x, delta, b, T, px)
+            if px is None and isinstance(layer, TPDecoderLayer) and layer.takes_sum(x):
+                x, delta = layer(x, delta, b, T, summed=True)
+            else:
+                x, delta = layer(x, delta, b, T, px)
         return self.final_layer_norm(x if delta is None else x + delta)
 
     def _micro(self, B, T):
