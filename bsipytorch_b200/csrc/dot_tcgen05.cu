@@ -578,7 +578,14 @@ int resident_clusters() {
 // fitted to runs of 2 .. 64 chunks at widths 64, 128 and 256: 820 + 1.3 bn per chunk, and beside the chunks 7000 + 25 bn
 // without a split, 7500 + 55 bn with two parts, 12000 + 47 bn with four (clusters of eight start later). A split takes one
 // wave of clusters (33 of four CTAs and 15 of eight fit) and has to save a fifteenth. *cycles: the cost of what is split.
-int pick_split(int64_t Q, int64_t R, int64_t chunks, int unsplit_bn, int* bn, double* cycles) {
+// sums: the queries' sums of squares are there, so that the vote passes but for rare rows. Without them it rests on the two
+// cheap bounds, which hold for even activations and mostly fail for layer norms' outputs with outliers, and a tile whose vote fails
+// is done by one pair after all: a wager on the values. Taken where it wins at least about as much as it may lose (40 .. 512 rows,
+// 256 .. 4096 columns, float16, split over unsplit): tiles of the unsplit width, four parts from 24 chunks on, 0.53 .. 0.84 where
+// the vote passes and 1.21 .. 1.29 where it fails (64 x 512 x 16384: 10.4 and 25.6 us, unsplit 18.1 and 21.0), two from 48 on,
+// 0.75 .. 0.86 and 1.18 .. 1.22. Not taken: two parts below (32 chunks 0.84 .. 0.92 and 1.22 .. 1.25), wider tiles than unsplit (0.72 ..
+// 1.23 and 1.60 .. 1.90: 512 x 8192 -> 2048 13.3 and 21.5, unsplit 12.0 and 12.8).
+int pick_split(int64_t Q, int64_t R, int64_t chunks, int unsplit_bn, bool sums, int* bn, double* cycles) {
     const int64_t mt = (Q + 255) / 256, pairs = sm_count() / 2;
     if (mt * ((R + unsplit_bn - 1) / unsplit_bn) > pairs) return 1;
     auto cost = [&](int w, double fixed, double per_column, int64_t parts) {
@@ -591,6 +598,7 @@ int pick_split(int64_t Q, int64_t R, int64_t chunks, int unsplit_bn, int* bn, do
         const int64_t room = s == 2 ? resident_clusters<2>() : resident_clusters<4>();
         for (int w = 256; w >= 64; w /= 2) {
             if (mt * ((R + w - 1) / w) > room) continue;
+            if (!sums && (w != unsplit_bn || chunks < (s == 4 ? 24 : 48))) continue;
             const double c = s == 2 ? cost(w, 7500.0, 55.0, 2) : cost(w, 12000.0, 47.0, 4);
             if (c < best) {
                 best = *cycles = c;
@@ -713,7 +721,7 @@ static bool split_is_shorter(int64_t Q, int64_t R, int64_t chunks, const RowsPla
         return false;
     int bn = pick_bn_pair(Q, R, false);
     double cycles = 0.0;
-    if (pick_split(Q, R, chunks, bn, &bn, &cycles) == 1) return false;
+    if (pick_split(Q, R, chunks, bn, true, &bn, &cycles) == 1) return false;
     const double split_us = cycles / 1900.0 - 0.1 * static_cast<double>(15 - (R + bn - 1) / bn);
     return split_us < rows_plan.us + 2.1 + 0.2 * rows_plan.parts + 0.045 * static_cast<double>(Q);
 }
@@ -800,12 +808,10 @@ int dot_i8_pair(const int8_t* a8, int64_t lda, const float* qs, int64_t qs_strid
         const int64_t t256 = mt * ((R + 255) / 256), t224 = mt * ((R + 223) / 224);
         if (t256 <= pairs && t224 <= pairs && t224 > t256) bn = 224;
     }
-    // Only with bounds (a split adds integers), one plain destination, and no accumulator dump. Without the Cauchy-Schwarz bound
-    // the vote mostly fails, and one pair does the whole tile: 512 x 8192 -> 2048 float16 packed without sums of squares 21.7 us,
-    // unsplit 13.1.
-    const bool may_split = !force_bn && kabs != nullptr && (qsq != nullptr || qs_stride == 0) && dbg_iacc == nullptr && scatter.n == 0;
+    // only with bounds (a split adds integers), one plain destination, and no accumulator dump
+    const bool may_split = !force_bn && kabs != nullptr && dbg_iacc == nullptr && scatter.n == 0;
     double cycles = 0.0;
-    const int parts = may_split ? pick_split(Q, R, chunks, bn, &bn, &cycles) : 1;
+    const int parts = may_split ? pick_split(Q, R, chunks, bn, qsq != nullptr || qs_stride == 0, &bn, &cycles) : 1;
     t_last_width = bn;
     t_last_parts = parts;
     if (bn < 64 || bn > 256 || (bn & 31) != 0 || (!any_width && (bn & (bn - 1)) != 0))
