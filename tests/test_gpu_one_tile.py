@@ -18,12 +18,33 @@ class _Bounds(C.Structure):
     _fields_ = [("key_bounds", C.c_void_p), ("query_sq", C.c_void_p), ("query_sq_stride", C.c_int64), ("query_abs_max", C.c_int)]
 
 
-# one chunk (no main loop), fewer chunks than accumulators, more; tiles of 64, 128 and 256 columns; clipped rows and columns, a last
-# block of half a row; a row beyond every bound (float32 chain next to integer sums), sums between 2^22 and 2^24
+def _sum_kinds(q8, scales, k8, width):
+    """Warps of float32 sums, of integer sums below 2^22 and of other integer sums, by the bounds that a warp takes over its 32
+    rows and its half of a tile's columns."""
+    Q, R, chunks = q8.shape[0], k8.shape[0], scales.shape[1]
+    k = k8.double().abs().view(R, chunks, 256).sum(2)
+    rows = [scales.double().amax(1), scales.double().sum(1), ((q8.double().view(Q, chunks, 256) ** 2).sum(2) * scales.double() ** 2).sum(1)]
+    cols = [k.sum(1), k.amax(1), (k8.double() ** 2).sum(1)]
+    blocks, halves = (Q + 255) // 256 * 8, -(-R // width) * 2
+    rows = [torch.nn.functional.pad(r, (0, blocks * 32 - Q)).view(blocks, 32).amax(1) for r in rows]             # no rows: no sums
+    cols = [torch.cat([c, c[-1:].expand(halves * width // 2 - R)]).view(halves, width // 2).amax(1) for c in cols]
+    first = torch.minimum(torch.outer(rows[0], cols[0]), torch.outer(rows[1], cols[1])) * 64
+    norm = torch.outer(rows[2], cols[2])
+    exact = (first < 2.0 ** 24 * 0.999) | (norm < 2.0 ** 48 * 0.999)
+    small = (first < 2.0 ** 22 * 0.999) | (norm < 2.0 ** 44 * 0.999)
+    return int((~exact).sum()), int(small.sum()), int((exact & ~small).sum())
+
+
+# Tiles of every width that the rule takes (float32, else), in one wave; the parts along K where the bounds are there. One chunk (no
+# main loop), fewer chunks than accumulators, more; clipped rows and columns, a last block of half a row, shares of 48 columns with
+# their load of 16; a row beyond every bound (float32 chain next to integer sums), and where scaled sums between 2^22 and 2^24.
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
-@pytest.mark.parametrize("Q,R,D,scale", [(40, 200, 256, 1.0), (257, 72, 512, 1.0), (33, 1000, 2304, 1.0), (300, 4424, 768, 1.0), (129, 9464, 1000, 1.0),
-                                         (250, 16000, 1280, 1.0), (64, 520, 2048, 6.0)])
-def test_one_tile_per_pair(dtype, Q, R, D, scale):
+@pytest.mark.parametrize("Q,R,D,scale,widths,parts", [
+    (40, 200, 256, 1.0, (64, 64), 1), (257, 72, 512, 1.0, (64, 64), 1), (33, 1000, 2304, 1.0, (64, 64), 2), (33, 1000, 1792, 1.0, (64, 64), 1),
+    (300, 4424, 768, 1.0, (128, 128), 1), (129, 9464, 1000, 1.0, (128, 128), 1), (129, 9464, 1000, 8.0, (128, 128), 1),
+    (250, 16000, 1280, 1.0, (224, 256), 1), (64, 520, 2048, 6.0, (64, 64), 2), (64, 520, 1536, 6.0, (64, 64), 1),
+    (200, 6056, 768, 8.0, (96, 128), 1), (130, 12040, 512, 1.0, (192, 256), 1), (100, 10040, 512, 16.0, (192, 256), 1)])
+def test_one_tile_per_pair(dtype, Q, R, D, scale, widths, parts):
     q, k = _inputs.fc1(Q=Q, R=R, D=D, seed=Q + R + D, dtype=torch.float32)
     q *= scale
     q[Q // 2] *= 3.0e4
@@ -41,6 +62,10 @@ def test_one_tile_per_pair(dtype, Q, R, D, scale):
     add = torch.randn(Q, R, generator=g, device=DEV).to(dtype)
     bias = torch.linspace(-1, 1, R, device=DEV)
     given = _Bounds(bounds.data_ptr(), norms.data_ptr(), chunks, 64)
+    width = widths[0 if dtype == torch.float32 else 1]
+    floats, small, large = _sum_kinds(q8, scales, kb["q8"], width)
+    assert floats > 0 and small > 0 and (large > 0 or scale == 1.0)
+    capi.exact_int_tiles()
     for with_bounds in (True, False):
         for b, relu, cols, a in ((None, 0, 0, None), (bias, 0, 0, None), (bias, 1, R // 16 * 8, None), (bias, 0, R // 16 * 8, add), (None, 1, 0, add)):
             y = torch.full((Q + 1, R), -7.0, dtype=dtype, device=DEV)
@@ -48,6 +73,10 @@ def test_one_tile_per_pair(dtype, Q, R, D, scale):
                                                 None if b is None else capi.ptr(b), Q, R, chunks, C.c_float(float(o.scale_inv(2))), capi.ptr(y), R,
                                                 H._DT[dtype], relu, cols, C.c_float(0.3), None if a is None else capi.ptr(a), R,
                                                 C.byref(given) if with_bounds else None, capi.ENGINE_TCGEN05, capi.stream_ptr()))
+            wide = widths[1] if a is not None else 256 if width == 224 and not with_bounds else width      # sums: powers of two
+            assert capi.last_tiles() == (wide, parts if with_bounds else 1) and (Q + 255) // 256 * -(-R // wide) <= 74      # one wave of pairs
+            ints = capi.exact_int_tiles()
+            assert ints == 0 if not with_bounds else ints == small + large or wide != width or parts > 1
             want = dot.to(dtype)
             if b is not None:
                 want = want + b.to(dtype)
