@@ -411,7 +411,9 @@ dot_rows_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
     }
     tc_fence_before();
     __syncthreads();
-    if (p.parts > 1) pair::cluster_sync_all();      // a copy of this CTA's sums may still be on its way
+    // A copy of this CTA's sums may still be on its way: it has landed when its receiver arrives here, which waited for it on its own
+    // barrier. The cluster barrier itself releases nothing, and nothing else is written across.
+    if (p.parts > 1) pair::cluster_sync_all();
     if (warp == 1) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"

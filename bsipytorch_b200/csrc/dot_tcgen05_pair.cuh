@@ -110,7 +110,8 @@ __device__ __forceinline__ bool elect_one() {
 }
 
 // Without release: with it an arrival waits for every memory access the warp has under way, 1000 to 1200 cycles here. Where
-// something was written for the other CTAs, a fence of its own stands in front (fence_cluster), in the threads that wrote.
+// something was written for the other CTAs, a fence of its own stands in front (fence_cluster), in the threads that wrote. Who
+// shares these with another kernel orders its own writes likewise (dot_rows_kernel: its receivers wait for the copies).
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void fence_cluster() { asm volatile("fence.acq_rel.cluster;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
